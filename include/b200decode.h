@@ -188,6 +188,19 @@ int b200_gemm_w4a16_status(int* code);
  * (reference runtime/quant.py:93-97). Used to prove the kernels read the packed format correctly. */
 int b200_dequant_w4a16(const void* Wp, const void* SZ, void* out, int N, int K, int log2G, void* stream);
 
+/* The quantizer (reference runtime/quant.py:17-60): W [N, K], dtype 0 fp16, 1 bf16, 2 fp32, 16B, group G = 8 .. 256 (a
+ * power of two that divides K), clip != 0 with the range search. Writes the outputs that are not NULL: packed int32
+ * [N, K/8], sz half2 [N, K/G], levels q uint8 [N, K], scale and zero fp16 [N, K/G] (both or neither), dequantized fp16
+ * [N, K]. Same levels and parameters as the torch form on a CUDA device. */
+int b200_quantize_w4(const void* W, int dtype, int N, int K, int G, int clip, void* packed, void* sz, void* q, void* scale,
+                     void* zero, void* deq, void* stream);
+/* The columns of one GPTQ block (reference runtime/quant.py:51-90), nb <= 128 of them, nb a multiple of `group`: W fp32,
+ * row pitch ldw, points at the block's first column; U points at element (b0, b0) of the upper factor of the inverse
+ * Hessian, element strides us0, us1. Writes levels Q (row pitch ldq), fp32 scale / zero (pitch lds) and the columns'
+ * errors E (pitch lde), which the caller applies to the columns behind the block. */
+int b200_gptq_block(const float* W, int ldw, int N, int nb, const float* U, long long us0, long long us1, int group,
+                    int clip, void* Q, int ldq, float* scale, float* zero, int lds, float* E, int lde, void* stream);
+
 /* x[H] = emb[tok[0], :]; tok is int64 [1] on the device (the reference's step does this with
  * torch.index_select, runtime/model.py:218). emb fp16 [V, H], x 16B; H % 8 == 0. A token outside [0, V) reads row 0
  * instead of memory outside the table. */

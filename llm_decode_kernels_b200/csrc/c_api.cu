@@ -32,6 +32,11 @@ cudaError_t swiglu_dispatch(const void* gu, void* out, int rows, int I, cudaStre
 cudaError_t prefill_gemm_dispatch(const void* Wp, const void* SZ, const void* X, void* Y, int T, int N, int K, int log2G,
                                   cudaStream_t st);
 int prefill_gemm_max_tokens();
+cudaError_t quantize_w4_dispatch(const void* W, int dtype, int N, int K, int G, int clip, const QuantOut& out,
+                                 cudaStream_t st);
+cudaError_t gptq_block_dispatch(const float* W, int ldw, int N, int nb, const float* U, long long us0, long long us1,
+                                int group, int clip, uint8_t* Q, int ldq, float* S, float* Z, int lds, float* E, int lde,
+                                cudaStream_t st);
 cudaError_t prefill_gemm_status(int* code);
 cudaError_t rope_append_dispatch(void* qkv, const float* cos_t, const float* sin_t, const int* pos, const int* bt,
                                  int bt_stride, void* kc, void* vc, int B, int n_q, int n_kv, int D, int log2P,
@@ -285,6 +290,23 @@ int b200_dequant_w4a16(const void* Wp, const void* SZ, void* out, int N, int K, 
   REQUIRE(log2G >= 3 && log2G < 31 && K % 8 == 0 && K % (1 << log2G) == 0, B200_ERR_SHAPE);
   REQUIRE(aligned16(out), B200_ERR_ALIGN);
   return finish(b200::dequant_w4a16_dispatch(Wp, SZ, out, N, K, log2G, S(stream)));
+}
+
+int b200_quantize_w4(const void* W, int dtype, int N, int K, int G, int clip, void* packed, void* sz, void* q, void* scale,
+                     void* zero, void* deq, void* stream) {
+  REQUIRE(W && N > 0 && K > 0 && dtype >= 0 && dtype <= 2 && !scale == !zero, B200_ERR_ARG);
+  REQUIRE(G >= 8 && G <= 256 && (G & (G - 1)) == 0 && K % G == 0, B200_ERR_SHAPE);
+  REQUIRE(aligned16(W) && aligned16(packed) && aligned16(sz) && aligned16(q) && aligned16(deq), B200_ERR_ALIGN);
+  const b200::QuantOut out = {(uint32_t*)packed, (half2*)sz, (uint2*)q, (half*)scale, (half*)zero, (uint4*)deq};
+  return finish(b200::quantize_w4_dispatch(W, dtype, N, K, G, clip, out, S(stream)));
+}
+
+int b200_gptq_block(const float* W, int ldw, int N, int nb, const float* U, long long us0, long long us1, int group,
+                    int clip, void* Q, int ldq, float* scale, float* zero, int lds, float* E, int lde, void* stream) {
+  REQUIRE(W && U && Q && scale && zero && E && N > 0 && nb > 0, B200_ERR_ARG);
+  REQUIRE(nb <= 128 && group >= 4 && (group & (group - 1)) == 0 && nb % group == 0, B200_ERR_SHAPE);
+  return finish(b200::gptq_block_dispatch(W, ldw, N, nb, U, us0, us1, group, clip, (uint8_t*)Q, ldq, scale, zero, lds, E,
+                                          lde, S(stream)));
 }
 
 int b200_embed_row(const void* emb, const long long* tok, void* x, int H, int V, void* stream) {

@@ -216,6 +216,15 @@ DEVI void mma16832_u8s8(int (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint
 // slots 0-7 (lane l's 16 bytes at 16 l), 512 B for row slots 8-15, 16 x (scale, zero).
 constexpr int kTileUnitBytes = 1088;
 
+// What the quantizer writes; a null pointer leaves that output out. `words` = N K / 8 in element order of W.
+struct QuantOut {
+  uint32_t* packed;    // [words] nibbles in kernel order
+  half2* sz;           // [groups] (scale, zero)
+  uint2* q;            // [words] eight levels, one byte each
+  half *scale, *zero;  // [groups]; both or neither
+  uint4* deq;          // [words] eight fp16 dequantized weights
+};
+
 // Order key for greedy argmax over fp16 logits: larger value wins, then the lower index. One max-reduction
 // over these keys settles value and tie-break together.
 DEVI unsigned long long argmax_key(half v, int idx) {

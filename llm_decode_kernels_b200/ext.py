@@ -14,7 +14,7 @@ swiglu_batched.
 """
 import ctypes
 import math
-from ctypes import c_float, c_int, c_size_t, c_void_p
+from ctypes import c_float, c_int, c_longlong, c_size_t, c_void_p
 from pathlib import Path
 
 import torch
@@ -71,6 +71,10 @@ SIGNATURES = {
     "b200_rope_append_batched": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int,
                                  c_int, c_int, c_int, c_int, c_void_p],
     "b200_dequant_w4a16": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p],
+    "b200_quantize_w4": [c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
+                         c_void_p, c_void_p],
+    "b200_gptq_block": [c_void_p, c_int, c_int, c_int, c_void_p, c_longlong, c_longlong, c_int, c_int, c_void_p, c_int,
+                        c_void_p, c_void_p, c_int, c_void_p, c_int, c_void_p],
     "b200_add_rmsnorm_batched": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_float, c_void_p],
     "b200_swiglu_batched": [c_void_p, c_void_p, c_int, c_int, c_void_p],
     "b200_gemm_w4a16": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p],
@@ -487,6 +491,28 @@ class Ops:
             raise RuntimeError("dequant_w4a16: inconsistent shapes")
         self._check(self.lib.b200_dequant_w4a16(packed.data_ptr(), sz.data_ptr(), out.data_ptr(), N, K,
                                                 _ilog2_exact(int(group), "group"), _stream()), "dequant_w4a16")
+
+    # ---- quantization (called by quant.py) ------------------------------------------------------------------
+    def quantize_w4(self, w, group, clip, packed=None, sz=None, q=None, scale=None, zero=None, deq=None):
+        """w [N, K] fp16 / bf16 / fp32 -> whichever outputs are given: packed int32 [N, K/8], sz fp16 [N, K/G, 2], levels q
+        uint8 [N, K], scale and zero fp16 [N, K/G], dequantized deq fp16 [N, K]."""
+        w = _cuda(w.contiguous(), "w")
+        N, K = w.shape
+        ptr = [None if t is None else t.data_ptr() for t in (packed, sz, q, scale, zero, deq)]
+        with torch.cuda.device(w.device):
+            self._check(self.lib.b200_quantize_w4(
+                w.data_ptr(), (torch.float16, torch.bfloat16, torch.float32).index(w.dtype), N, K, int(group), int(clip),
+                *ptr, _stream()), "quantize_w4")
+
+    def gptq_block(self, W, b0, b1, U, group, clip, Q, S, Z, Eb):
+        """The column loop of GPTQ over columns [b0, b1) of W fp32 [N, K]: levels into Q uint8 [N, K], group parameters
+        into S, Z fp32 [N, K/group], rounding errors into Eb fp32 [N, b1 - b0]. W itself is not changed."""
+        N, K = W.shape
+        with torch.cuda.device(W.device):
+            self._check(self.lib.b200_gptq_block(
+                W.data_ptr() + 4 * b0, K, N, b1 - b0, U.data_ptr() + 4 * (b0 * U.stride(0) + b0 * U.stride(1)),
+                U.stride(0), U.stride(1), int(group), int(clip), Q.data_ptr() + b0, K, S.data_ptr() + 4 * (b0 // group),
+                Z.data_ptr() + 4 * (b0 // group), K // group, Eb.data_ptr(), b1 - b0, _stream()), "gptq_block")
 
     # ---- the prompt: T tokens at once --------------------------------------------------------------------
     def gemm_w4a16(self, packed, sz, x, y, group):

@@ -16,10 +16,13 @@ Format, for a weight W [N, K] (out x in) and group size G along K:
 The bit layout lets a kernel turn `(word >> 4i) & 0x000F000F | 0x64006400` into the half2
 (1024 + q[8j+2i], 1024 + q[8j+2i+1]) with no integer-to-float conversion.
 
-All functions run on the device of their input (torch ops). Quantization is offline work; the
-decode step itself never calls into this file.
+All functions run on the device of their input: quantize, QuantLinear and the column loop of
+quantize_gptq as one kernel each on a CUDA device (csrc/quantize.cu; same results), everything else as
+torch ops. Quantization is offline work; the decode step itself never calls into this file.
 """
 import torch
+
+from . import ext
 
 CLIP_GRID = (1.0, 0.95, 0.9, 0.85, 0.8, 0.75, 0.7)
 
@@ -57,10 +60,27 @@ def group_params(wf, clip=False):
     return best_scale, best_zero
 
 
+def _kernel_takes(w, group):
+    """Whether the CUDA quantizer covers this input: groups of 8 to 256 weights, a power of two (a group is then at most
+    one warp of 8-weight threads), and a floating type it reads."""
+    return (w.is_cuda and w.numel() > 0 and w.dtype in (torch.float16, torch.bfloat16, torch.float32)
+            and 8 <= group <= 256 and group & (group - 1) == 0)
+
+
 def quantize(w: torch.Tensor, group: int, clip: bool = False):
     """[N, K] -> (q uint8 [N, K], scale fp16 [N, K/G], zero fp16 [N, K/G])."""
     N, K = w.shape
     assert K % group == 0, (K, group)
+    if _kernel_takes(w, group):
+        q = torch.empty(N, K, dtype=torch.uint8, device=w.device)
+        s, z = (torch.empty(N, K // group, dtype=torch.float16, device=w.device) for _ in range(2))
+        ext.load().quantize_w4(w, group, clip, q=q, scale=s, zero=z)
+        return q, s, z
+    return _quantize_torch(w, group, clip)
+
+
+def _quantize_torch(w, group, clip=False):
+    N, K = w.shape
     wf = w.to(torch.float32).reshape(N, K // group, group)
     scale, zero = group_params(wf, clip)
     q = _levels(wf, scale, zero)
@@ -88,6 +108,29 @@ def quantize_gptq(w: torch.Tensor, H: torch.Tensor, group: int, clip: bool = Fal
     W[:, dead] = 0
     diag += damp * diag.mean()
     U = torch.linalg.cholesky(torch.cholesky_inverse(torch.linalg.cholesky(H)), upper=True)
+    Q, S, Z = _gptq_columns(W, U, group, clip, block)
+    return Q, S.to(torch.float16), Z.to(torch.float16)
+
+
+def _gptq_columns(W, U, group, clip, block):
+    """Fixes the columns of W fp32 [N, K] left to right (W is used up): levels, scales and zero points."""
+    if not (W.is_cuda and block <= 128 and group >= 4 and group & (group - 1) == 0):
+        return _gptq_columns_torch(W, U, group, clip, block)
+    N, K = W.shape
+    Q = torch.empty(N, K, dtype=torch.uint8, device=W.device)
+    S, Z = (torch.empty(N, K // group, device=W.device) for _ in range(2))
+    E = torch.empty(N, block, device=W.device)
+    ops = ext.load()
+    for b0 in range(0, K, block):
+        b1 = min(b0 + block, K)
+        ops.gptq_block(W, b0, b1, U, group, clip, Q, S, Z, E)
+        if b1 < K:
+            W[:, b1:].addmm_(E[:, :b1 - b0], U[b0:b1, b1:], alpha=-1)
+    return Q, S, Z
+
+
+def _gptq_columns_torch(W, U, group, clip, block):
+    N, K = W.shape
     Q = torch.zeros(N, K, dtype=torch.uint8, device=W.device)
     S = torch.zeros(N, K // group, device=W.device)
     Z = torch.zeros(N, K // group, device=W.device)
@@ -110,7 +153,7 @@ def quantize_gptq(w: torch.Tensor, H: torch.Tensor, group: int, clip: bool = Fal
             Wb[:, i:] -= e[:, None] * Ub[i, i:][None, :]
             Eb[:, i] = e
         W[:, b1:] -= Eb @ U[b0:b1, b1:]
-    return Q, S.to(torch.float16), Z.to(torch.float16)
+    return Q, S, Z
 
 
 def dequantize(q, scale, zero, group: int):
@@ -153,6 +196,14 @@ class QuantLinear:
         per-group range clipping)."""
         self.N, self.K = w.shape
         self.group = group
+        if qsz is None and _kernel_takes(w, group):
+            assert self.K % group == 0, (self.K, group)
+            dev = w.device
+            self.packed = torch.empty(self.N, self.K // 8, dtype=torch.int32, device=dev)
+            self.sz = torch.empty(self.N, self.K // group, 2, dtype=torch.float16, device=dev)
+            self.w_ref = torch.empty(self.N, self.K, dtype=torch.float16, device=dev) if keep_ref else None
+            ext.load().quantize_w4(w, group, clip, packed=self.packed, sz=self.sz, deq=self.w_ref)
+            return
         if qsz is not None:
             q, s, z = (t.to(w.device) for t in qsz)
         else:

@@ -1,0 +1,50 @@
+"""The CUDA quantizer kernels against the torch form of the same functions on the same device."""
+import pytest
+import torch
+
+from llm_decode_kernels_b200 import quant as PQ
+
+pytestmark = pytest.mark.gpu
+
+
+def weights(N, K, dtype, seed):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    w = torch.randn(N, K, generator=g, device="cuda") * 0.02
+    w[0, :K // 2] = 0                       # a group without a range
+    w[N // 2] = w[N // 2].abs() + 0.5       # no zero crossing: levels far beyond 15 before clamping
+    w[N - 1] *= 1e-6                        # scales at their lower bound
+    w[torch.rand(N, K, generator=g, device="cuda") < 2e-3] *= 8
+    return w.to(dtype)
+
+
+@pytest.mark.parametrize("N,K,G", [(1, 8, 8), (3, 96, 32), (257, 384, 64), (1000, 1280, 128), (64, 512, 256), (17, 640, 640)])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("clip", [False, True])
+def test_quantize_kernel_equals_torch_form(N, K, G, dtype, clip):
+    w = weights(N, K, dtype, N + K)
+    q0, s0, z0 = PQ._quantize_torch(w, G, clip)
+    q, s, z = PQ.quantize(w, G, clip)
+    same = ((s == s0) & (z == z0)).repeat_interleave(G, 1)
+    # clipping: two factors of equal error up to the order of the sum may change places
+    assert same.float().mean() >= (1 - 2e-3 if clip else 1)
+    assert torch.equal(q[same], q0[same])
+    ql = PQ.QuantLinear(w, G, clip=clip)
+    assert torch.equal(ql.packed, PQ.pack(q)) and torch.equal(ql.sz, PQ.pack_scale_zero(s, z))
+    assert torch.equal(ql.w_ref, PQ.dequantize(q, s, z, G))
+
+
+@pytest.mark.parametrize("N,K,G,block", [(5, 64, 64, 64), (300, 384, 128, 128), (64, 320, 32, 96), (129, 512, 64, 128)])
+@pytest.mark.parametrize("clip", [False, True])
+def test_gptq_kernel_equals_torch_loop(monkeypatch, N, K, G, block, clip):
+    g = torch.Generator(device="cuda").manual_seed(N)
+    w = weights(N, K, torch.float16, 3)
+    x = torch.randn(4 * K, K, generator=g, device="cuda")
+    H = 2 * x.t() @ (x + 0.5 * x.roll(1, 1)) / x.shape[0]
+    H = (H + H.t()) / 2
+    H[7] = 0
+    H[:, 7] = 0                             # an input that is never active
+    got = PQ.quantize_gptq(w, H, G, clip=clip, block=block)
+    monkeypatch.setattr(PQ, "_gptq_columns", PQ._gptq_columns_torch)
+    ref = PQ.quantize_gptq(w, H, G, clip=clip, block=block)
+    assert (got[0] != ref[0]).float().mean() < 2e-3
+    assert all((a != b).float().mean() < 2e-3 for a, b in zip(got[1:], ref[1:]))
