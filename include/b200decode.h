@@ -180,6 +180,10 @@ int b200_swiglu_batched(const void* gu, void* out, int rows, int I, void* stream
  * if one runs out the CTA frees its tensor memory and returns, and b200_gemm_w4a16_status reports 1 (sticky). */
 int b200_gemm_w4a16(const void* Wp, const void* SZ, const void* X, void* Y, int T, int N, int K, int log2G,
                     void* stream);
+/* The same product from the tile-layout copy (b200_gemv_w4a16_tile_repack) for any T; swiglu != 0: Wt is the paired layout
+ * of [gate; up], N counts outputs and Y = silu(gate) * up. K % 128 == 0, Y 8B. split: 0 = the library's choice, or the number
+ * of CTA pairs (1, 2, 4) that share an output tile by splitting K. Timed-out waits: b200_gemm_w4a16_status. */
+int b200_gemm_w4a16_tiled(const void* Wt, const void* X, void* Y, int T, int N, int K, int swiglu, int split, void* stream);
 int b200_gemm_w4a16_max_tokens(void);
 /* Synchronous read of the status word: 0, or 1 once a bounded wait ran out. */
 int b200_gemm_w4a16_status(int* code);

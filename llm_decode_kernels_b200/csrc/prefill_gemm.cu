@@ -24,7 +24,7 @@
 // their own waits, the CTA waits (bounded) for its copies in flight, still takes part in the cluster barriers, frees
 // its tensor memory and returns; b200_gemm_w4a16_status then reports 1.
 #include "common.cuh"
-#include <cuda.h>
+#include "prefill.h"
 
 namespace b200 {
 
@@ -386,6 +386,16 @@ EncodeTiledFn encode_tiled() {
 
 }  // namespace
 
+bool encode_activation_map(CUtensorMap* map, const void* X, int T, int K, int box_rows) {
+  const EncodeTiledFn encode = encode_tiled();
+  if (!encode) return false;
+  const cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)T}, strides[1] = {(cuuint64_t)K * 2};
+  const cuuint32_t box[2] = {(cuuint32_t)kPfChunk, (cuuint32_t)box_rows}, estr[2] = {1, 1};
+  return encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(X), dims, strides, box, estr,
+                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 // How many ways K is split for a matrix of N rows: the largest power of two, up to the portable cluster size, for
 // which every cluster of the grid is resident at once (the occupancy query knows how many clusters of that size the
 // GPU's processor groups hold) and every split keeps at least two chunks.
@@ -436,15 +446,8 @@ cudaError_t prefill_gemm_dispatch(const void* Wp, const void* SZ, const void* X,
   const int Tpad = (T + 15) / 16 * 16;
   int cols = 32;
   while (cols < Tpad) cols *= 2;
-  const EncodeTiledFn encode = encode_tiled();
-  if (!encode) return cudaErrorNotSupported;
   CUtensorMap xmap;
-  const cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)T}, strides[1] = {(cuuint64_t)K * 2};
-  const cuuint32_t box[2] = {(cuuint32_t)kPfChunk, (cuuint32_t)Tpad}, estr[2] = {1, 1};
-  if (encode(&xmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(X), dims, strides, box, estr,
-             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-    return cudaErrorInvalidValue;
+  if (!encode_activation_map(&xmap, X, T, K, Tpad)) return cudaErrorInvalidValue;
   const size_t stage = (size_t)kPfRows * 128 + (size_t)Tpad * 128;
   int ns = (int)((kPfSmemLimit - 1024) / stage);
   ns = ns > kPfMaxStages ? kPfMaxStages : ns;   // >= kPfMinStages: four stages of the largest tile fit

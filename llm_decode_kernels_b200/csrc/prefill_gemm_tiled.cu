@@ -1,0 +1,517 @@
+// Prompt GEMM from the tile layout:  Y[T, N] = X[T, K] . dequant(W)[N, K]^T for any number of tokens, optionally with SwiGLU
+// (paired [gate; up] layout), fp32 accumulation, fp16 out. The fp16 weights are the format's (dequant_w4a16_kernel), bit for bit.
+//
+// What bounds a W4A16 GEMM here is not the tensor core but what has to reach it: with a 128-row tile per CTA every 64 columns of
+// K bring 32 KB of activations (256 tokens) from the L2 for 512 cycles of MMA, more than the L2 delivers to 148 SMs, and the
+// dequantized weights (16 KB) pass through shared memory twice. So:
+//   * two CTAs on neighbouring SMs work as a pair (cta_group::2): 256 rows of W x up to 256 tokens, each CTA brings 128 rows of
+//     W and half of the tokens - half the activation traffic per MMA cycle;
+//   * the dequantized weights never touch shared memory: a dequantizing thread owns a row, its tcgen05.st puts the row's fp16 pairs
+//     into tensor memory, and the MMA reads its A operand there;
+//   * a CTA pair is persistent: it walks over output tiles, the dequantizing and copying warps run four to six 128-column units
+//     ahead across tile borders, and the epilogue warps empty the accumulator into shared memory (rounded to fp16) before they
+//     store, so the next tile's MMAs wait only for that;
+//   * where there are fewer tiles than pairs, S = 2 or 4 pairs (one cluster) share a tile by splitting K; their fp32 partial tiles
+//     meet through distributed shared memory in a fixed order.
+// Warps: 0-11 dequantize (three groups of four, every third unit: a unit is ~2000 cycles of latency for a warp and 1024 of MMA at
+// 256 tokens), 12-15 epilogue, 16 MMA issue (even CTA of a pair), 17 TMA.
+// Tensor memory: accumulator (128 lanes = rows, one column per token; 128 or 256 columns), then six or four A stages of 64 columns.
+// Loops that run once per launch at small sizes are kept short rather than unrolled: every launch fetches its code anew.
+// Every wait is bounded; a wait that runs out raises the CTA's fail flag, all roles leave, the CTA waits (bounded) for its copies,
+// joins the cluster barriers, frees its tensor memory, and b200_gemm_w4a16_status is non-zero.
+#include "common.cuh"
+#include "prefill.h"
+
+namespace b200 {
+
+namespace {
+
+__device__ int g_tiled_status = 0;   // 0, or the code of the first wait inside prefill_gemm_tiled_kernel that ran out
+
+constexpr int kDqGroups = 3, kDqWarps = 4 * kDqGroups, kEpWarps = 4, kThreads = (kDqWarps + kEpWarps + 2) * 32;
+constexpr int kMmaWarp = kDqWarps + kEpWarps, kTmaWarp = kMmaWarp + 1;
+constexpr int kMaxStages = 6;          // 128-column units in flight: A in tensor memory, B in shared memory
+constexpr int kACols = 64;             // tensor-memory columns of an A stage
+constexpr int kMaxTokens = 256;        // tokens per tile = N of the MMA (a multiple of 32)
+constexpr int kMaxSplit = 4;           // pairs per tile: clusters of at most 8 CTAs
+constexpr int kSpin = 1 << 20;         // polls before a wait gives up ...
+constexpr unsigned long long kWaitNs = 100000000ull;   // ... or this long
+
+enum : int { WAIT_DQ = 1, WAIT_MMA_ACC = 2, WAIT_MMA_B = 3, WAIT_MMA_A = 4, WAIT_TMA = 5, WAIT_EP = 6 };
+
+DEVI uint32_t sa(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+DEVI void bar_init(uint64_t* b, int count) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(sa(b)), "r"(count));
+}
+DEVI uint32_t in_cta(uint32_t local, uint32_t rank) {   // the same shared-memory offset in CTA `rank` of the cluster
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(local), "r"(rank));
+  return r;
+}
+// Arrivals and waits carry no cluster-scope fence: what they order is tensor memory (the tcgen05 fences beside them) and bulk
+// copies (their own transaction counts); an acquire at cluster scope would empty the L1 on every poll.
+DEVI void bar_arrive_cluster(uint32_t addr) {
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(addr) : "memory");
+}
+DEVI void bar_expect(uint64_t* b, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(sa(b)), "r"(bytes) : "memory");
+}
+DEVI bool bar_try(uint64_t* b, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(sa(b)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+DEVI unsigned long long now_ns() {
+  unsigned long long t;
+  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+  return t;
+}
+// false if the phase did not complete within the bound or another role of the CTA has given up
+template <int SLEEP_NS>
+DEVI bool bar_wait(uint64_t* b, uint32_t parity, volatile int* fail, int code) {
+  if (bar_try(b, parity)) return true;
+  const unsigned long long t0 = now_ns();
+#pragma unroll 1
+  for (int i = 0; i < kSpin; ++i) {
+    if (SLEEP_NS > 0) __nanosleep(SLEEP_NS);
+    if (bar_try(b, parity)) return true;
+    if ((i & 31) == 31) {
+      if (*fail) return false;
+      if (now_ns() - t0 > kWaitNs) break;
+    }
+  }
+  *fail = 1;
+  atomicCAS(&g_tiled_status, 0, code);
+  return false;
+}
+DEVI void cluster_barrier() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+DEVI float4 ld_cluster4(uint32_t addr) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
+  return v;
+}
+// K-major tile, 128-byte swizzle: see umma_desc_sw128 in prefill_gemm.cu
+DEVI uint64_t desc_sw128(uint32_t addr) {
+  return (uint64_t)((addr & 0x3FFFFu) >> 4) | (1ull << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61);
+}
+
+DEVI void tmem_ld16(uint32_t addr, uint32_t (&v)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n\t"
+      "tcgen05.wait::ld.sync.aligned;"
+      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
+        "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+      : "r"(addr)
+      : "memory");
+}
+DEVI void tmem_st16(uint32_t addr, const uint32_t (&v)[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(addr),
+      "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]), "r"(v[10]),
+      "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
+      : "memory");
+}
+
+struct Shared {
+  uint64_t a_full[kMaxStages], b_full[kMaxStages], empty[kMaxStages], acc_full, acc_empty;
+  uint32_t tmem;
+  int fail;
+};
+
+// Position in the sequence of 128-column units a CTA works through: the units [u0, u1) of its first tile, of its second, ...
+struct Walk {
+  int tile, u;
+  DEVI void step(int n, int u0, int u1, int stride) {
+    u += n;
+    while (u >= u1) u -= u1 - u0, tile += stride;
+  }
+};
+
+// Stage and how often it has been used before, of a sequence that takes the stages in turn.
+struct Ring {
+  int s, use;
+  DEVI void step(int n, int stages) {
+    s += n;
+    if (s >= stages) s -= stages, ++use;
+  }
+};
+
+// one row's 128 weights of a unit and their (scale, zero)
+struct RowUnit { uint4 w[4]; half2 sz; };
+
+DEVI void ld32(const uint8_t* p, uint4& a, uint4& b) {   // one whole 32-byte sector per lane
+  asm volatile("ld.global.nc.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=r"(a.x), "=r"(a.y), "=r"(a.z), "=r"(a.w), "=r"(b.x), "=r"(b.y), "=r"(b.z), "=r"(b.w)
+               : "l"(p));
+}
+
+// (q - z) * s per pair of weights, as dequant_w4a16_kernel. HI: nibbles at bits 4-7 / 20-23 are taken where they stand, as
+// 1024 + 16 q, and multiplied by s / 16 - the same product whenever s / 16 is exact in fp16 and 1024 + 16 z is sixteen times
+// what 1024 + z rounds z to (sixteenths_exact: not for a subnormal scale); it saves two shifts per word.
+DEVI bool sixteenths_exact(half2 sz) {
+  const half k1024 = __float2half_rn(1024.f), k16 = __float2half_rn(16.f), s = __low2half(sz), z = __high2half(sz);
+  return __heq(__hmul(__hmul(s, __float2half_rn(0.0625f)), k16), s) &&
+         __heq(__hsub(__hfma(z, k16, k1024), k1024), __hmul(__hsub(__hadd(z, k1024), k1024), k16));
+}
+template <bool HI>
+DEVI void dequant_store(const RowUnit& d, uint32_t dst) {
+  const half2 k1024 = __float2half2_rn(1024.f), z2 = __half2half2(__high2half(d.sz)), s2 = __half2half2(__low2half(d.sz));
+  const half2 zl = __hadd2(z2, k1024), zh = __hfma2(z2, __float2half2_rn(16.f), k1024);
+  const half2 s16 = __hmul2(s2, __float2half2_rn(0.0625f));
+#pragma unroll
+  for (int h = 0; h < 4; ++h) {   // 32 columns of K = 16 columns of tensor memory
+    const uint32_t w4[4] = {d.w[h].x, d.w[h].y, d.w[h].z, d.w[h].w};
+    uint32_t o[16];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const uint32_t w = w4[j], wh = w >> 8;
+      o[4 * j] = as_u32(__hmul2(__hsub2(nib_lo(w), zl), s2));
+      o[4 * j + 1] = HI ? as_u32(__hmul2(__hsub2(nib_hi(w), zh), s16)) : as_u32(__hmul2(__hsub2(nib_lo(w >> 4), zl), s2));
+      o[4 * j + 2] = as_u32(__hmul2(__hsub2(nib_lo(wh), zl), s2));
+      o[4 * j + 3] = HI ? as_u32(__hmul2(__hsub2(nib_hi(wh), zh), s16)) : as_u32(__hmul2(__hsub2(nib_lo(w >> 12), zl), s2));
+    }
+    tmem_st16(dst + 16 * h, o);
+  }
+}
+
+// half(silu(gate)) * up for two outputs, the rounding points of swiglu_kernel
+DEVI uint32_t gated2(uint32_t gate, uint32_t up) {
+  const float2 g = __half22float2(as_h2(gate));
+  const half2 s = __floats2half2_rn(__fdividef(g.x, 1.f + __expf(-g.x)), __fdividef(g.y, 1.f + __expf(-g.y)));
+  return as_u32(__hmul2(s, as_h2(up)));
+}
+
+}  // namespace
+
+template <bool SWIGLU>
+__global__ void __launch_bounds__(kThreads, 1)
+prefill_gemm_tiled_kernel(const __grid_constant__ CUtensorMap xmap, const uint8_t* __restrict__ Wt, half* __restrict__ Y, int T,
+                          int N, int row_tiles, int nunit, int nt, int S, int feat_tiles, int tiles, int ns) {
+  extern __shared__ uint8_t raw[];
+  __shared__ Shared sh;
+  uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(raw) + 1023) & ~(uintptr_t)1023);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  uint32_t rank;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+  const int csize = 2 * S, first = blockIdx.x / csize, stride = gridDim.x / csize;
+  const int split = rank >> 1, side = rank & 1;            // which share of K; which half of the pair
+  const uint32_t lead = rank & ~1u;
+  const int u0 = nunit * split / S, u1 = nunit * (split + 1) / S;
+  const int half_bytes = nt * 64, stage_bytes = 2 * half_bytes;   // 64 columns of K x nt / 2 tokens; a unit
+  volatile int* fail = &sh.fail;
+  pdl_launch_dependents();
+
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(sa(&sh.tmem)) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+  }
+  if (tid == 0) {
+    for (int s = 0; s < ns; ++s) {
+      bar_init(&sh.a_full[s], 2 * 4);   // one group of dequantizing warps in each CTA of the pair
+      bar_init(&sh.b_full[s], 1);
+      bar_init(&sh.empty[s], 1);
+    }
+    bar_init(&sh.acc_full, 1);
+    bar_init(&sh.acc_empty, 2 * kEpWarps);
+    sh.fail = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  cluster_barrier();   // the peers' barriers exist before anything arrives on them
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = sh.tmem, tmem_a = tmem + (uint32_t)(512 - kACols * ns);
+
+  if (warp < kDqWarps) {
+    // ---- A: thread = row; group `grp` takes every third unit of the sequence, with the next two in registers
+    const int grp = warp >> 2, r = (warp & 3) * 32 + lane;
+    const uint32_t lanes = (uint32_t)((warp & 3) * 32) << 16;
+    Walk at = {first, u0};
+    at.step(grp, u0, u1, stride);
+    Walk ahead = at;
+    auto load = [&](RowUnit& d) {
+      const int rt = 16 * (ahead.tile % feat_tiles) + 8 * side + (r >> 4);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) d.w[i] = make_uint4(0u, 0u, 0u, 0u);
+      d.sz = __float2half2_rn(0.f);
+      if (ahead.tile < tiles && rt < row_tiles) {   // rows past the matrix: zero words, zero scale
+        const uint8_t* p = Wt + ((size_t)rt * nunit + ahead.u) * kTileUnitBytes;
+        const uint8_t* q = p + 64 * (r & 15);
+        ld32(q, d.w[0], d.w[1]);
+        ld32(q + 32, d.w[2], d.w[3]);
+        d.sz = __ldg(reinterpret_cast<const half2*>(p + 1024) + (r & 15));
+      }
+      ahead.step(kDqGroups, u0, u1, stride);
+    };
+    RowUnit cur, next, after;
+    load(cur);
+    load(next);
+    Ring ring = {grp, 0};
+#pragma unroll 1
+    for (; at.tile < tiles; at.step(kDqGroups, u0, u1, stride)) {
+      load(after);
+      if (ring.use > 0 && !__all_sync(0xffffffffu, bar_wait<64>(&sh.empty[ring.s], (ring.use - 1) & 1, fail, WAIT_DQ))) break;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const uint32_t dst = tmem_a + lanes + (uint32_t)(kACols * ring.s);
+      if (__all_sync(0xffffffffu, sixteenths_exact(cur.sz))) dequant_store<true>(cur, dst);
+      else dequant_store<false>(cur, dst);
+      asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) bar_arrive_cluster(in_cta(sa(&sh.a_full[ring.s]), lead));
+      ring.step(kDqGroups, ns);
+      cur = next;
+      next = after;
+    }
+  } else if (warp == kMmaWarp) {
+    if (side == 0 && lane == 0) {
+      // D fp32, A and B fp16, both K-major, N / 8 in bits 17-22, M / 16 in bits 24-28 (M = 256 over the pair)
+      const uint32_t idesc = (1u << 4) | ((uint32_t)(nt >> 3) << 17) | ((256u >> 4) << 24);
+      const uint16_t both = (uint16_t)(3u << lead);
+      auto commit = [&](uint64_t* bar) {
+        asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(sa(bar)),
+                     "h"(both)
+                     : "memory");
+      };
+      bool ok = true;
+      int done = 0;
+      Ring ring = {0, 0};
+      for (int tile = first; tile < tiles && ok; tile += stride, ++done) {
+        if (done > 0) ok = bar_wait<0>(&sh.acc_empty, (done - 1) & 1, fail, WAIT_MMA_ACC);
+        for (int u = u0; u < u1 && ok; ++u) {
+          ok = bar_wait<0>(&sh.b_full[ring.s], ring.use & 1, fail, WAIT_MMA_B) &&
+               bar_wait<0>(&sh.a_full[ring.s], ring.use & 1, fail, WAIT_MMA_A);
+          if (!ok) break;
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          const uint32_t a = tmem_a + (uint32_t)(kACols * ring.s), bs = sa(base + ring.s * stage_bytes);
+          const uint64_t b0 = desc_sw128(bs), b1 = desc_sw128(bs + half_bytes);
+#pragma unroll
+          for (int k = 0; k < 8; ++k)
+            asm volatile(
+                "{\n\t.reg .pred p;\n\t"
+                "setp.ne.b32 p, %4, 0;\n\t"
+                "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(tmem),
+                "r"(a + 8 * k), "l"((k < 4 ? b0 + 2 * k : b1 + 2 * (k - 4))), "r"(idesc), "r"((u > u0 || k > 0) ? 1u : 0u)
+                : "memory");
+          commit(&sh.empty[ring.s]);
+          ring.step(1, ns);
+        }
+        if (ok) commit(&sh.acc_full);
+      }
+    }
+  } else if (warp == kTmaWarp) {
+    if (lane == 0) {
+      pdl_wait();   // X is the predecessor's output
+      Ring ring = {0, 0};
+      for (Walk at = {first, u0}; at.tile < tiles; at.step(1, u0, u1, stride), ring.step(1, ns)) {
+        uint64_t* full = &sh.b_full[ring.s];
+        if (ring.use > 0 && !bar_wait<0>(&sh.empty[ring.s], (ring.use - 1) & 1, fail, WAIT_TMA)) break;
+        // both CTAs' halves count on the even CTA's barrier
+        if (side == 0) bar_expect(full, 2 * stage_bytes);
+        const uint32_t bar = in_cta(sa(full), lead), dst = sa(base + ring.s * stage_bytes);
+        const int y = (at.tile / feat_tiles) * nt + side * (nt >> 1);
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+          asm volatile(
+              "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
+                  dst + h * half_bytes),
+              "l"(&xmap), "r"(at.u * 128 + 64 * h), "r"(y), "r"(bar)
+              : "memory");
+      }
+      // giving up: let the copies in flight land before the shared memory goes away (the even CTA holds the barriers)
+      if (*fail && side == 0)
+        for (int s = 0; s < ns; ++s) {
+          const int uses = ring.use + (s < ring.s ? 1 : 0);   // how often stage s has been filled
+          for (int i = 0; uses > 0 && i < (1 << 16) && !bar_try(&sh.b_full[s], (uses - 1) & 1); ++i) __nanosleep(64);
+        }
+    }
+  } else {
+    // ---- epilogue: a warp reaches the 32 lanes (rows) of its quarter
+    const int q = warp & 3, et = tid - 32 * kDqWarps;
+    const uint32_t taddr = tmem + ((uint32_t)(32 * q) << 16);
+    half* rows = reinterpret_cast<half*>(base + ns * stage_bytes);   // [token][128 rows]
+    auto epilogue_sync = [] { asm volatile("bar.sync 1, %0;" ::"n"(32 * kEpWarps) : "memory"); };
+    const bool vec = (N & 7) == 0 && (reinterpret_cast<uintptr_t>(Y) & 15) == 0;
+    int done = 0;
+#pragma unroll 1
+    for (int tile = first; tile < tiles; tile += stride, ++done) {
+      const bool ok = __all_sync(0xffffffffu, bar_wait<128>(&sh.acc_full, done & 1, fail, WAIT_EP));
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      if (S > 1) {   // one tile per cluster: park the partial tile P[token][128 rows] as fp32 over the idle stages
+        float* P = reinterpret_cast<float*>(base);
+#pragma unroll 1
+        for (int c = 0; ok && c < nt; c += 16) {
+          uint32_t v[16];
+          tmem_ld16(taddr + c, v);
+#pragma unroll
+          for (int j = 0; j < 16; ++j) P[(c + j) * 128 + 32 * q + lane] = __uint_as_float(v[j]);
+        }
+        break;
+      }
+#pragma unroll 1
+      for (int c = 0; ok && c < nt; c += 16) {
+        uint32_t v[16];
+        tmem_ld16(taddr + c, v);
+#pragma unroll
+        for (int j = 0; j < 16; ++j) rows[(c + j) * 128 + 32 * q + lane] = __float2half_rn(__uint_as_float(v[j]));
+      }
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      epilogue_sync();   // the tile is complete; a warp that gave up has raised the flag before
+      if (*fail) break;
+      if (lane == 0) bar_arrive_cluster(in_cta(sa(&sh.acc_empty), lead));
+      if (done == 0) pdl_wait();   // Y may still be read by the kernel before this one
+      const int t0 = (tile / feat_tiles) * nt, row0 = (tile % feat_tiles) * 256 + side * 128, tn = min(nt, T - t0);
+      constexpr int kPieces = SWIGLU ? 8 : 16;   // pieces of 8 outputs per token
+#pragma unroll 2
+      for (int i = et; i < tn * kPieces; i += 32 * kEpWarps) {
+        const int t = i / kPieces, pc = i % kPieces, f = (SWIGLU ? row0 >> 1 : row0) + 8 * pc;
+        const uint4* src = reinterpret_cast<const uint4*>(rows + t * 128 + (SWIGLU ? 16 : 8) * pc);
+        uint4 o = src[0];
+        if (SWIGLU) {   // rows 16 k + 0..7 are gates, 16 k + 8..15 their up rows
+          const uint4 u = src[1];
+          o = make_uint4(gated2(o.x, u.x), gated2(o.y, u.y), gated2(o.z, u.z), gated2(o.w, u.w));
+        }
+        half* y = Y + (size_t)(t0 + t) * N + f;
+        if (vec && f + 7 < N) {
+          *reinterpret_cast<uint4*>(y) = o;
+        } else {
+          const uint32_t w[4] = {o.x, o.y, o.z, o.w};
+#pragma unroll
+          for (int e = 0; e < 8; ++e)
+            if (f + e < N) y[e] = __ushort_as_half((unsigned short)(w[e >> 1] >> (16 * (e & 1))));
+        }
+      }
+      epilogue_sync();   // `rows` is free for the next tile
+    }
+  }
+  __syncwarp();
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  cluster_barrier();   // partial tiles are parked; every MMA that reads a peer's shared memory has completed
+  if (S > 1 && first < tiles && !*fail) {
+    pdl_wait();
+    // CTA (split, side) finishes tokens split, split + S, ... of its side's rows: sum in split order, four rows a lane
+    const int t_base = (first / feat_tiles) * nt, row0 = (first % feat_tiles) * 256 + side * 128;
+    for (int t = warp * S + split; t < nt && t_base + t < T; t += (kThreads / 32) * S) {
+      const uint32_t local = sa(base) + (uint32_t)((t * 128 + 4 * lane) * sizeof(float));
+      float4 v[kMaxSplit];
+#pragma unroll
+      for (int s = 0; s < kMaxSplit; ++s)
+        if (s < S) v[s] = ld_cluster4(in_cta(local, 2 * s + side));
+      float4 a = v[0];
+#pragma unroll
+      for (int s = 1; s < kMaxSplit; ++s)
+        if (s < S) a.x += v[s].x, a.y += v[s].y, a.z += v[s].z, a.w += v[s].w;
+      half2 h01 = __floats2half2_rn(a.x, a.y), h23 = __floats2half2_rn(a.z, a.w);
+      half* y = Y + (size_t)(t_base + t) * N;
+      if (SWIGLU) {   // rows 16 k + 0..7 gates, 16 k + 8..15 their up rows: two lanes further on
+        const uint32_t u01 = __shfl_xor_sync(0xffffffffu, as_u32(h01), 2), u23 = __shfl_xor_sync(0xffffffffu, as_u32(h23), 2);
+        if ((lane & 2) == 0) {
+          const int f = (row0 >> 1) + 8 * (lane >> 2) + 4 * (lane & 1);
+          const half2 o01 = as_h2(gated2(as_u32(h01), u01)), o23 = as_h2(gated2(as_u32(h23), u23));
+          const half o[4] = {__low2half(o01), __high2half(o01), __low2half(o23), __high2half(o23)};
+#pragma unroll
+          for (int e = 0; e < 4; ++e)
+            if (f + e < N) y[f + e] = o[e];
+        }
+      } else {
+        const int f = row0 + 4 * lane;
+        if (f + 3 < N && (N & 3) == 0) {
+          *reinterpret_cast<uint2*>(y + f) = make_uint2(as_u32(h01), as_u32(h23));
+        } else {
+          const half o[4] = {__low2half(h01), __high2half(h01), __low2half(h23), __high2half(h23)};
+#pragma unroll
+          for (int e = 0; e < 4; ++e)
+            if (f + e < N) y[f + e] = o[e];
+        }
+      }
+    }
+  }
+  if (S > 1) cluster_barrier();   // nobody's shared memory goes away while a peer still reads it
+  if (warp == 0) {
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
+  }
+}
+
+static int resident_clusters(int S, size_t smem) {   // clusters of 2 S CTAs the GPU holds at once; asked once per device
+  static int known[kMaxDevices][kMaxSplit + 1] = {};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return 0;
+  if (known[dev][S] == 0) {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2 * S, attr[0].val.clusterDim.y = 1, attr[0].val.clusterDim.z = 1;
+    cfg.gridDim = dim3(2 * S), cfg.blockDim = dim3(kThreads), cfg.dynamicSmemBytes = smem, cfg.attrs = attr, cfg.numAttrs = 1;
+    int num = 0;
+    if (cudaOccupancyMaxActiveClusters(&num, prefill_gemm_tiled_kernel<false>, &cfg) != cudaSuccess) {
+      (void)cudaGetLastError();
+      num = 0;
+    }
+    known[dev][S] = num > 0 ? num : -1;
+  }
+  return known[dev][S] > 0 ? known[dev][S] : 0;
+}
+
+cudaError_t prefill_gemm_tiled_status(int* code) {
+  return cudaMemcpyFromSymbol(code, g_tiled_status, sizeof(int), 0, cudaMemcpyDeviceToHost);
+}
+
+// Y[T, N]; N = rows of W (swiglu: of outputs, W has 2 N rows in paired layout). force_split: 0, or the S to use.
+cudaError_t prefill_gemm_tiled_dispatch(const void* Wt, const void* X, void* Y, int T, int N, int K, int swiglu, int force_split,
+                                        cudaStream_t st) {
+  const int nunit = K / 128, row_tiles = swiglu ? (N + 7) / 8 : (N + 15) / 16;
+  const int feat_tiles = (row_tiles + 15) / 16, ntt = (T + kMaxTokens - 1) / kMaxTokens;
+  const int nt = ((T + ntt - 1) / ntt + 31) / 32 * 32;   // equal token tiles, so that the last one is not nearly empty
+  const int tiles = feat_tiles * ((T + nt - 1) / nt);
+  const int ns = nt <= 128 ? 6 : 4;   // what tensor memory has left beside the accumulator
+  auto bytes = [](int tokens, int stages) { return 1024 + (size_t)tokens * (128 * stages + 256); };   // stages + fp16 tile
+  const size_t smem = bytes(nt, ns), smem_max = bytes(kMaxTokens, 4);
+  static size_t allowed[2][kMaxDevices] = {};
+  cudaError_t e = allow_dynamic_smem(prefill_gemm_tiled_kernel<false>, smem_max, allowed[0]);
+  if (e == cudaSuccess) e = allow_dynamic_smem(prefill_gemm_tiled_kernel<true>, smem_max, allowed[1]);
+  if (e != cudaSuccess) return e;
+  // Split K where that shortens the longest CTA. Measured, in microseconds: a unit 0.53 at any token count (MMA issue and
+  // dequantization below 256 tokens, the MMA itself at 256); a launch 3.4 and 0.019 per token behind it when a pair works alone,
+  // 4.4 / 5.6 and 0.022 when 2 / 4 pairs exchange partial tiles.
+  int S = 1;
+  double best = 0;
+  for (int c = 1; c <= kMaxSplit; c *= 2) {
+    const int room = resident_clusters(c, smem_max);
+    if (room == 0 || (c > 1 && nunit / c < 2)) continue;
+    const int waves = (tiles + room - 1) / room, units = (nunit + c - 1) / c;
+    const double cost = c == 1 ? 3.4 + 0.019 * (nt - 32) + waves * (units * 0.53 + 0.3)
+                               : waves * (3.2 + 0.6 * c + 0.022 * (nt - 32) + units * 0.53);
+    if (best == 0 || cost < best) best = cost, S = c;
+  }
+  if (force_split) S = force_split;
+  const int room = resident_clusters(S, smem_max);
+  if (room == 0) return cudaErrorNotSupported;
+  CUtensorMap xmap;
+  if (!encode_activation_map(&xmap, X, T, K, nt / 2)) return cudaErrorInvalidValue;
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 2 * S, attr[0].val.clusterDim.y = 1, attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.gridDim = dim3(2 * S * (S > 1 || tiles < room ? tiles : room));
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = attr;
+  cfg.numAttrs = 2;
+  return cudaLaunchKernelEx(&cfg, swiglu ? prefill_gemm_tiled_kernel<true> : prefill_gemm_tiled_kernel<false>, xmap,
+                            (const uint8_t*)Wt, (half*)Y, T, N, row_tiles, nunit, nt, S, feat_tiles, tiles, ns);
+}
+
+}  // namespace b200

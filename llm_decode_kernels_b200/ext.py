@@ -78,6 +78,7 @@ SIGNATURES = {
     "b200_add_rmsnorm_batched": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_float, c_void_p],
     "b200_swiglu_batched": [c_void_p, c_void_p, c_int, c_int, c_void_p],
     "b200_gemm_w4a16": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p],
+    "b200_gemm_w4a16_tiled": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p],
     "b200_gemm_w4a16_max_tokens": [],
     "b200_gemm_w4a16_status": [c_void_p],
     "b200_embed_row": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p],
@@ -527,6 +528,15 @@ class Ops:
             raise RuntimeError("gemm_w4a16: sz must be [N, K/group, 2]")
         self._check(self.lib.b200_gemm_w4a16(packed.data_ptr(), sz.data_ptr(), x.data_ptr(), y.data_ptr(), x.shape[0],
                                              N, K, _ilog2_exact(int(group), "group"), _stream()), "gemm_w4a16")
+
+    def gemm_w4a16_tiled(self, tiled, x, y, N, K, swiglu=False, split=0):
+        """y[T, N] = x[T, K] @ W^T from the tile-layout copy of W, any T. swiglu: the copy is a paired [gate; up] and
+        y[T, N] = silu(gate) * up. split: 0, or how many CTA pairs share a tile (1, 2, 4)."""
+        _cuda(tiled, "tiled", torch.uint8), _cuda(x, "x", torch.float16), _cuda(y, "y", torch.float16)
+        if x.dim() != 2 or x.shape[1] != K or tuple(y.shape) != (x.shape[0], N):
+            raise RuntimeError("gemm_w4a16_tiled: x must be [T, K] and y [T, N]")
+        self._check(self.lib.b200_gemm_w4a16_tiled(tiled.data_ptr(), x.data_ptr(), y.data_ptr(), x.shape[0], int(N), int(K),
+                                                   int(swiglu), int(split), _stream()), "gemm_w4a16_tiled")
 
     def gemm_max_tokens(self):
         return int(self.lib.b200_gemm_w4a16_max_tokens())

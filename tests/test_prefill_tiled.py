@@ -1,0 +1,64 @@
+"""The prompt path on the tile-layout weights: GEMM by CTA pairs, prompt attention, batched RoPE + append."""
+import numpy as np
+import pytest
+import torch
+
+from llm_decode_kernels_b200 import ext, quant as PQ
+from oracle import quant_oracle as Q
+
+pytestmark = pytest.mark.gpu
+dev = "cuda"
+
+
+@pytest.fixture(scope="module")
+def K():
+    return ext.load()
+
+
+def matrix(K, N, Kd, gate_up=False, G=128):
+    torch.manual_seed(N + Kd)
+    ql = PQ.QuantLinear((torch.randn(N, Kd, device=dev) * 0.02).half(), G, keep_ref=True)
+    return ql, K.gemv_tile_repack(ql.packed, ql.sz, G, gate_up=gate_up)
+
+
+def test_one_hot_rows_are_the_dequantized_weights(K):
+    N, Kd, G = 200, 256, 128
+    torch.manual_seed(3)
+    w = (torch.randn(N, Kd) * 0.05).half()
+    w[3] *= 1e-4                                 # a subnormal scale
+    q, s, z = PQ.quantize(w, G, False)
+    packed, sz = PQ.pack(q).to(dev), PQ.pack_scale_zero(s, z).to(dev)
+    tiled = K.gemv_tile_repack(packed, sz, G)
+    want = Q.dequantize(q.numpy(), s.numpy(), z.numpy(), G)
+    y = torch.full((Kd, N), float("nan"), dtype=torch.half, device=dev)
+    K.gemm_w4a16_tiled(tiled, torch.eye(Kd, dtype=torch.half, device=dev), y, N, Kd)
+    assert np.array_equal(y.cpu().numpy().view(np.uint16), want.T.copy().view(np.uint16))
+
+
+# ragged rows and tokens, one unit of K, a tile more than whole ones, more tiles than CTA pairs; every split
+@pytest.mark.parametrize("N,Kd,T", [(256, 128, 1), (1003, 1024, 17), (320, 384, 77), (2560, 2048, 256), (2048, 5632, 300),
+                                    (512, 256, 129), (5000, 512, 1025)])
+@pytest.mark.parametrize("split", [0, 1, 2, 4])
+def test_gemm_tiled(K, N, Kd, T, split):
+    if split > Kd // 128:
+        pytest.skip("more splits than units of K")
+    ql, tiled = matrix(K, N, Kd)
+    x = torch.randn(T, Kd, device=dev).half()
+    y = torch.full((T, N), float("nan"), dtype=torch.half, device=dev)
+    K.gemm_w4a16_tiled(tiled, x, y, N, Kd, split=split)
+    ref = x.float() @ ql.w_ref.float().t()
+    assert ((y.float() - ref).abs().max() / ref.abs().max()).item() <= 2e-3
+    assert K.gemm_status() == 0
+
+
+@pytest.mark.parametrize("I,Kd,T", [(5632, 2048, 256), (1003, 1024, 77), (128, 256, 500)])
+@pytest.mark.parametrize("split", [1, 2])
+def test_gemm_tiled_swiglu(K, I, Kd, T, split):
+    ql, tiled = matrix(K, 2 * I, Kd, gate_up=True)
+    x = torch.randn(T, Kd, device=dev).half()
+    y = torch.full((T, I), float("nan"), dtype=torch.half, device=dev)
+    K.gemm_w4a16_tiled(tiled, x, y, I, Kd, swiglu=True, split=split)
+    gu = (x.float() @ ql.w_ref.float().t()).half()
+    ref = (torch.nn.functional.silu(gu[:, :I].float()).half() * gu[:, I:]).float()
+    assert ((y.float() - ref).abs().max() / ref.abs().max()).item() <= 4e-3
+    assert K.gemm_status() == 0
