@@ -233,6 +233,29 @@ typedef struct b200_step_layer {
   void* vc;
 } b200_step_layer;
 
+/* One chunk of a prompt in one call: T tokens `ids` at positions start .. start + T - 1 go through embedding, all layers (their
+ * K and V rows are appended to the paged caches; attention is causal over positions 0 .. their own) and the final norm, which
+ * is left in `normed`. The reference steps through the prompt (runtime/model.py:267-276). Matrices in tile layout, gate|up
+ * paired; H, n_q D and I multiples of 128; D = 64 or 128; n_q / n_kv a power of two. Everything is device memory except
+ * `layers`, a host array. Float pointers 16B. */
+typedef struct {
+  const b200_step_layer* layers;
+  int L, H, I, n_q, n_kv, D, V, log2P;
+  float eps;
+  const void* emb;        /* fp16 [V, H] */
+  const void* norm_f;     /* fp16 [H] */
+  const float* cos_t;     /* fp32 [positions, D/2] */
+  const float* sin_t;
+  const int* bt;          /* block table of the sequence */
+  const long long* ids;   /* [T] */
+  const int* pos;         /* [T]: start, start + 1, ... */
+  int T, start;
+  void *x, *normed, *qkv, *attn, *o, *act;   /* fp16 work buffers: [T,H] [T,H] [T,(n_q+2n_kv)D] [T,n_q D] [T,H] [T,I] */
+  float* scratch;         /* partials of split attention, or NULL: short prompts behind a long context then run unsplit */
+  size_t scratch_floats;
+} b200_prefill_desc;
+int b200_prefill_chunk(const b200_prefill_desc* d, void* stream);
+
 /* Host-side description of a step; every pointer inside points to device memory. */
 typedef struct b200_step_desc {
   const b200_step_layer* layers;

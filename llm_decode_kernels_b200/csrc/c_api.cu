@@ -5,6 +5,7 @@
 #include "../../include/b200decode.h"
 #include "common.cuh"
 #include "decode_step.h"
+#include "prefill.h"
 #include <string.h>
 
 namespace b200 {
@@ -275,6 +276,28 @@ int b200_gemm_w4a16_status(int* code) {
   if (e == cudaSuccess) e = b200::prefill_gemm_tiled_status(&tiled);
   *code |= tiled;
   return finish(e);
+}
+
+int b200_prefill_chunk(const b200_prefill_desc* d, void* stream) {
+  REQUIRE(d && d->layers && d->emb && d->norm_f && d->cos_t && d->sin_t && d->bt && d->ids && d->pos && d->x && d->normed &&
+              d->qkv && d->attn && d->o && d->act,
+          B200_ERR_ARG);
+  REQUIRE(d->L > 0 && d->H > 0 && d->I > 0 && d->n_q > 0 && d->n_kv > 0 && d->V > 0 && d->T > 0 && d->start >= 0, B200_ERR_ARG);
+  REQUIRE(d->n_q % d->n_kv == 0 && d->log2P >= 0 && d->log2P < 16, B200_ERR_SHAPE);
+  REQUIRE(b200::prefill_attention_takes(d->D, d->n_q, d->n_kv), B200_ERR_SHAPE);
+  REQUIRE(d->H % 128 == 0 && (d->n_q * d->D) % 128 == 0 && d->I % 128 == 0, B200_ERR_SHAPE);
+  REQUIRE(d->H <= 32768 && d->T <= (1 << 20), B200_ERR_LIMIT);
+  for (const void* q : {d->emb, d->norm_f, (const void*)d->cos_t, (const void*)d->sin_t, (const void*)d->x, (const void*)d->normed,
+                        (const void*)d->qkv, (const void*)d->attn, (const void*)d->o, (const void*)d->act, (const void*)d->scratch})
+    REQUIRE(aligned16(q), B200_ERR_ALIGN);
+  b200::PrefillParams p = {};
+  p.layers = reinterpret_cast<const b200::StepLayer*>(d->layers);
+  p.L = d->L; p.H = d->H; p.I = d->I; p.n_q = d->n_q; p.n_kv = d->n_kv; p.D = d->D; p.V = d->V; p.log2P = d->log2P;
+  p.eps = d->eps; p.emb = d->emb; p.norm_f = d->norm_f; p.cos_t = d->cos_t; p.sin_t = d->sin_t; p.bt = d->bt;
+  p.ids = d->ids; p.pos = d->pos; p.T = d->T; p.start = d->start;
+  p.x = d->x; p.normed = d->normed; p.qkv = d->qkv; p.attn = d->attn; p.o = d->o; p.act = d->act;
+  p.scratch = d->scratch; p.scratch_floats = d->scratch ? d->scratch_floats : 0;
+  return finish(b200::prefill_chunk_dispatch(p, S(stream)));
 }
 
 int b200_gemm_w4a16_tiled(const void* Wt, const void* X, void* Y, int T, int N, int K, int swiglu, int split, void* stream) {

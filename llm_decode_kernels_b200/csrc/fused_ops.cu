@@ -140,9 +140,59 @@ __global__ void rope_append_kernel(half* __restrict__ qkv, const float* __restri
   }
 }
 
+// The same for the rows of a prompt: one block per token, 8 pairs per thread in 16-byte pieces. A block per (token, head) of 32
+// threads each, as above, is 164,000 blocks for 4096 tokens and 110 us; this form takes 12.
+__global__ void __launch_bounds__(256)
+rope_append_rows_kernel(half* __restrict__ qkv, const float* __restrict__ cos_t, const float* __restrict__ sin_t,
+                        const int* __restrict__ pos_ptr, const int* __restrict__ bt, int bt_stride, half* __restrict__ kc,
+                        half* __restrict__ vc, int n_q, int n_kv, int D, int log2P) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int b = blockIdx.x, d2 = D >> 1, per_head = D >> 4, heads = n_q + 2 * n_kv;
+  const int pos = pos_ptr[b], page = bt[(size_t)b * bt_stride + (pos >> log2P)], slot = pos & ((1 << log2P) - 1);
+  for (int c = threadIdx.x; c < heads * per_head; c += blockDim.x) {
+    const int head = c / per_head, i = (c - head * per_head) * 8;
+    half* v = qkv + ((size_t)b * heads + head) * D + i;
+    uint4 lo = *reinterpret_cast<const uint4*>(v), hi = *reinterpret_cast<const uint4*>(v + d2);
+    half* dst = v;
+    if (head < n_q + n_kv) {
+      float a[8], bb[8], cs[8], sn[8];
+      unpack8(lo, a);
+      unpack8(hi, bb);
+      const float *cp = cos_t + (size_t)pos * d2 + i, *sp = sin_t + (size_t)pos * d2 + i;
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        *reinterpret_cast<float4*>(cs + 4 * k) = __ldg(reinterpret_cast<const float4*>(cp) + k);
+        *reinterpret_cast<float4*>(sn + 4 * k) = __ldg(reinterpret_cast<const float4*>(sp) + k);
+      }
+      uint32_t r[4], w[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        r[k] = as_u32(__floats2half2_rn(a[2 * k] * cs[2 * k] - bb[2 * k] * sn[2 * k],
+                                        a[2 * k + 1] * cs[2 * k + 1] - bb[2 * k + 1] * sn[2 * k + 1]));
+        w[k] = as_u32(__floats2half2_rn(bb[2 * k] * cs[2 * k] + a[2 * k] * sn[2 * k],
+                                        bb[2 * k + 1] * cs[2 * k + 1] + a[2 * k + 1] * sn[2 * k + 1]));
+      }
+      lo = make_uint4(r[0], r[1], r[2], r[3]);
+      hi = make_uint4(w[0], w[1], w[2], w[3]);
+      if (head >= n_q) dst = kc + ((((size_t)page * n_kv + (head - n_q)) << log2P) + slot) * D + i;
+    } else {
+      dst = vc + ((((size_t)page * n_kv + (head - n_q - n_kv)) << log2P) + slot) * D + i;
+    }
+    *reinterpret_cast<uint4*>(dst) = lo;
+    *reinterpret_cast<uint4*>(dst + d2) = hi;
+  }
+}
+
 cudaError_t rope_append_dispatch(void* qkv, const float* cos_t, const float* sin_t, const int* pos, const int* bt,
                                  int bt_stride, void* kc, void* vc, int B, int n_q, int n_kv, int D, int log2P,
                                  cudaStream_t st) {
+  auto aligned = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };
+  if (B >= 4 && D % 16 == 0 && aligned(qkv) && aligned(cos_t) && aligned(sin_t) && aligned(kc) && aligned(vc)) {
+    B200_LAUNCH(rope_append_rows_kernel, dim3(B), dim3(256), 0, st, (half*)qkv, cos_t, sin_t, pos, bt, bt_stride, (half*)kc,
+                (half*)vc, n_q, n_kv, D, log2P);
+    return cudaPeekAtLastError();
+  }
   B200_LAUNCH(rope_append_kernel, dim3(n_q + 2 * n_kv, B), dim3(D / 2), 0, st, (half*)qkv, cos_t, sin_t, pos, bt,
               bt_stride, (half*)kc, (half*)vc, n_q, n_kv, D, log2P);
   return cudaPeekAtLastError();

@@ -876,6 +876,13 @@ __global__ void paged_attn_combine_kernel(const float* __restrict__ o_part, cons
   out[hq * D + d] = __float2half(acc / L);
 }
 
+cudaError_t attention_combine_dispatch(const float* o_part, const float* m_part, const float* l_part, const int* pos, int PS,
+                                       int max_splits, int n_q, int B, int D, void* out, cudaStream_t st) {
+  B200_LAUNCH(paged_attn_combine_kernel, dim3(n_q, B), dim3(D), 0, st, o_part, m_part, l_part, pos, PS, max_splits, D,
+              (half*)out);
+  return cudaPeekAtLastError();
+}
+
 enum : int { ATTN_REGISTER = 1, ATTN_STAGED = 2, ATTN_MMA = 3 };
 
 template <typename Kern>
@@ -979,11 +986,7 @@ cudaError_t paged_attention_dispatch(int version, const void* q, const void* kc,
                       o_part, m_part, l_part, (half*)out, max_splits, B};
   cudaError_t e = D == 64 ? launch_partial<64>(hpg, kind, a, st) : launch_partial<128>(hpg, kind, a, st);
   if (e != cudaSuccess) return e;
-  if (max_splits > 1) {
-    B200_LAUNCH(paged_attn_combine_kernel, dim3(n_q, B), dim3(D), 0, st, o_part, m_part, l_part, pos, PS, max_splits,
-                D, (half*)out);
-    e = cudaPeekAtLastError();
-  }
+  if (max_splits > 1) e = attention_combine_dispatch(o_part, m_part, l_part, pos, PS, max_splits, n_q, B, D, out, st);
   return e;
 }
 
@@ -1019,11 +1022,8 @@ cudaError_t rope_paged_attention_dispatch(void* qkv, const float* cos_t, const f
   B200_ROPE_CASE(128, 1) B200_ROPE_CASE(128, 2) B200_ROPE_CASE(128, 4) B200_ROPE_CASE(128, 8)
 #undef B200_ROPE_CASE
   if (e != cudaSuccess) return e;
-  if (max_splits > 1 && arrive == nullptr) {   // with an arrival array the last block of each head has combined
-    B200_LAUNCH(paged_attn_combine_kernel, dim3(n_q, 1), dim3(D), 0, st, o_part, m_part, l_part, pos, PS, max_splits, D,
-                (half*)out);
-    e = cudaPeekAtLastError();
-  }
+  if (max_splits > 1 && arrive == nullptr)   // with an arrival array the last block of each head has combined
+    e = attention_combine_dispatch(o_part, m_part, l_part, pos, PS, max_splits, n_q, 1, D, out, st);
   return e;
 }
 

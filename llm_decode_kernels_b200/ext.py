@@ -79,6 +79,7 @@ SIGNATURES = {
     "b200_swiglu_batched": [c_void_p, c_void_p, c_int, c_int, c_void_p],
     "b200_gemm_w4a16": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p],
     "b200_gemm_w4a16_tiled": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p],
+    "b200_prefill_chunk": [c_void_p, c_void_p],
     "b200_gemm_w4a16_max_tokens": [],
     "b200_gemm_w4a16_status": [c_void_p],
     "b200_embed_row": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p],
@@ -99,6 +100,16 @@ class StepDesc(ctypes.Structure):
                 ("norm_f", c_void_p), ("w_head", c_void_p), ("sz_head", c_void_p), ("cos_t", c_void_p),
                 ("sin_t", c_void_p), ("bt", c_void_p), ("tok", c_void_p), ("pos", c_void_p), ("history", c_void_p),
                 ("logits", c_void_p), ("xchg", c_void_p), ("ctrl", c_void_p), ("ctx_cap", c_int), ("grid", c_int), ("trace", c_void_p)]
+
+
+class PrefillDesc(ctypes.Structure):
+    """b200_prefill_desc of include/b200decode.h."""
+    _fields_ = [("layers", c_void_p), ("L", c_int), ("H", c_int), ("I", c_int), ("n_q", c_int), ("n_kv", c_int),
+                ("D", c_int), ("V", c_int), ("log2P", c_int), ("eps", c_float), ("emb", c_void_p), ("norm_f", c_void_p),
+                ("cos_t", c_void_p), ("sin_t", c_void_p), ("bt", c_void_p), ("ids", c_void_p), ("pos", c_void_p),
+                ("T", c_int), ("start", c_int), ("x", c_void_p), ("normed", c_void_p), ("qkv", c_void_p),
+                ("attn", c_void_p), ("o", c_void_p), ("act", c_void_p), ("scratch", c_void_p),
+                ("scratch_floats", c_size_t)]
 
 
 def load_library(build_if_missing=True, path=None):
@@ -537,6 +548,10 @@ class Ops:
             raise RuntimeError("gemm_w4a16_tiled: x must be [T, K] and y [T, N]")
         self._check(self.lib.b200_gemm_w4a16_tiled(tiled.data_ptr(), x.data_ptr(), y.data_ptr(), x.shape[0], int(N), int(K),
                                                    int(swiglu), int(split), _stream()), "gemm_w4a16_tiled")
+
+    def prefill_chunk(self, desc: "PrefillDesc"):
+        """One chunk of a prompt through embedding, layers and final norm (b200_prefill_chunk) on the current stream."""
+        self._check(self.lib.b200_prefill_chunk(ctypes.byref(desc), _stream()), "prefill_chunk")
 
     def gemm_max_tokens(self):
         return int(self.lib.b200_gemm_w4a16_max_tokens())

@@ -16,6 +16,7 @@ teacher-forced.
 This runtime has one backend: the CUDA kernels of libb200decode.so, all weights W4A16. `backend="ref"`,
 `weights="fp16"` and CPU devices are refused; the CPU restatement used for checking lives outside the package.
 """
+import ctypes
 import json
 import math
 from dataclasses import dataclass, field
@@ -333,6 +334,17 @@ class Model:
         self.graph = None               # a captured graph holds the old geometry
         self._setup_persistent_step()
 
+    def _layer_table(self):
+        """Host array of b200_step_layer: the tile-layout matrices, norm weights and caches of every layer."""
+        arr = (ext.StepLayer * self.L)()
+        for i, lw in enumerate(self.layers):
+            for k, name in enumerate(("qkv", "o", "gu", "down")):
+                arr[i].w[k] = lw[name].tiled.data_ptr()
+                arr[i].sz[k] = 0
+            arr[i].ln1, arr[i].ln2 = lw["ln1"].data_ptr(), lw["ln2"].data_ptr()
+            arr[i].kc, arr[i].vc = self.kv[i, 0].data_ptr(), self.kv[i, 1].data_ptr()
+        return arr
+
     def _setup_persistent_step(self):
         """Describe the step for b200_decode_step: device array of per-layer pointers, exchange and control memory.
         The kernel streams the tile-layout copies of the matrices (gate|up in its paired form), the same copies the
@@ -359,13 +371,7 @@ class Model:
         dev = self.cfg.device
         if getattr(self, "_step_static", None) is None:
             grid = torch.cuda.get_device_properties(dev).multi_processor_count
-            arr = (ext.StepLayer * self.L)()
-            for i, lw in enumerate(self.layers):
-                for k, name in enumerate(("qkv", "o", "gu", "down")):
-                    arr[i].w[k] = lw[name].tiled.data_ptr()
-                    arr[i].sz[k] = 0
-                arr[i].ln1, arr[i].ln2 = lw["ln1"].data_ptr(), lw["ln2"].data_ptr()
-                arr[i].kc, arr[i].vc = self.kv[i, 0].data_ptr(), self.kv[i, 1].data_ptr()
+            arr = self._layer_table()
             host = torch.frombuffer(bytearray(bytes(arr)), dtype=torch.uint8)
             nbytes = self.K.decode_step_xchg_bytes(self.L, self.H, self.I, self.n_q, self.n_kv, self.D, grid)
             self._step_static = {"layers": host.to(dev), "xchg": torch.zeros(nbytes, dtype=torch.uint8, device=dev),
@@ -636,6 +642,58 @@ class Model:
                 logits[i].copy_(self.logits)
         return logits
 
+    def _tiled_prefill(self):
+        """Description of the prompt path on the tile-layout matrices (b200_prefill_chunk), or None where the model's shape or
+        configuration rules it out (the prompt then goes through the row-major GEMM in chunks of gemm_max_tokens())."""
+        if not hasattr(self, "_prefill_desc"):
+            every = [lw[n] for lw in self.layers for n in ("qkv", "o", "gu", "down")] + [self.lm_head]
+            group = self.n_q // self.n_kv
+            ok = (all(lin.tiled is not None for lin in every) and all(lw["gu"].paired for lw in self.layers)
+                  and all(k % 128 == 0 for k in (self.H, self.n_q * self.D, self.I)) and self.H <= 32768
+                  and group & (group - 1) == 0 and group <= 128)
+            self._prefill_desc = None
+            if ok:
+                d = ext.PrefillDesc()
+                self._prefill_layers = self._layer_table()
+                d.layers = ctypes.addressof(self._prefill_layers)
+                d.L, d.H, d.I, d.n_q, d.n_kv, d.D, d.V = self.L, self.H, self.I, self.n_q, self.n_kv, self.D, self.V
+                d.log2P, d.eps = self.cfg.page.bit_length() - 1, self.eps
+                d.emb, d.norm_f = self.emb.data_ptr(), self.norm_f.data_ptr()
+                d.cos_t, d.sin_t = self.cos.data_ptr(), self.sin.data_ptr()
+                self._prefill_desc = d
+                self._positions = torch.arange(self.cfg.max_ctx + 1, dtype=torch.int32, device=self.tok.device)
+                self._prefill_work = None
+        return self._prefill_desc
+
+    def _prefill_tiled(self, ids, collect_logits):
+        """prefill() on the tile-layout matrices: chunks of as many tokens as a 256 MB work buffer holds (4096 at most), each one
+        call into the library. Returns (logits of every position or None, final-norm row of the last token)."""
+        d, K, dev, n = self._prefill_desc, self.K, self.tok.device, ids.numel()
+        widths = (self.H, self.H, self.H, (self.n_q + 2 * self.n_kv) * self.D, self.n_q * self.D, self.I)
+        per_token = 2 * sum(widths)
+        chunk = max(256, min(4096, (256 << 20) // per_token // 256 * 256))
+        scratch = 2 * 128 * 2 * 148 * (self.D + 2)     # floats: two waves of attention blocks, 128 query rows each
+        need = min(n, chunk) * per_token + 4 * scratch
+        if self._prefill_work is None or self._prefill_work.numel() < need:
+            self._prefill_work = torch.empty(need, dtype=torch.uint8, device=dev)
+        base = self._prefill_work.data_ptr()
+        d.scratch, d.scratch_floats, d.bt = base, scratch, self.bt.data_ptr()
+        all_logits = torch.empty(n, self.V_full, dtype=torch.half, device=dev) if collect_logits else None
+        for c0 in range(0, n, chunk):
+            T = min(chunk, n - c0)
+            at = base + 4 * scratch
+            for name, w in zip(("x", "normed", "o", "qkv", "attn", "act"), widths):
+                setattr(d, name, at)
+                at += 2 * T * w
+            d.T, d.start = T, self.host_pos + c0
+            d.ids, d.pos = ids.data_ptr() + 8 * c0, self._positions.data_ptr() + 4 * d.start
+            K.prefill_chunk(d)
+            off = d.normed - base
+            normed = self._prefill_work[off:off + 2 * T * self.H].view(torch.half).view(T, self.H)
+            if collect_logits:
+                K.gemm_w4a16_tiled(self.lm_head.tiled, normed, all_logits[c0:c0 + T], self.lm_head.N, self.lm_head.K)
+        return all_logits, normed[T - 1]
+
     def _prefill_state(self, T):
         """Static buffers of a prompt chunk of T tokens (kept per T and attention geometry, so that a recorded graph
         stays valid)."""
@@ -683,15 +741,15 @@ class Model:
         K.add_rmsnorm_batched(x, delta, self.norm_f, normed, self.eps)
 
     def prefill(self, tokens, collect_logits=False, use_graph=True):
-        """Process a prompt T tokens at a time instead of one step per token: every weight matrix is read once per
-        chunk of up to gemm_max_tokens() tokens (b200_gemm_w4a16, tcgen05 tensor cores), the small operators run in
-        their batched forms, and attention runs as a batch of T queries over the same block table, query t seeing
-        the cache up to its own position. The reference has no such path (it steps through the prompt,
+        """Process a prompt T tokens at a time instead of one step per token, on the tcgen05 tensor cores: every weight matrix
+        is read once per chunk (of up to 4096 tokens from the tile-layout copies, one library call per chunk; of up to
+        gemm_max_tokens() from the row-major tensors where those cannot be used), the small operators run in their
+        batched forms, and query t of the chunk attends over the cache up to its own position. The reference has no such path (it steps through the prompt,
         runtime/model.py:267-276). Leaves the runtime exactly where teacher_force(tokens) would: K/V rows of the
         prompt in the cache, self.logits / self.tok from the last prompt token, the position behind the prompt.
         The history entries of the prompt positions before the last are not written. Returns the logits of every
-        prompt position, fp16 [len, V], when collect_logits is set. With use_graph a long prompt replays one CUDA graph
-        per whole chunk from its second chunk on. One GPU, row-major packed weights kept (keep_packed=True)."""
+        prompt position, fp16 [len, V], when collect_logits is set. With use_graph the row-major path replays one CUDA
+        graph per whole chunk from its second chunk on. One GPU, row-major packed weights kept (keep_packed=True)."""
         if self.tp != 1:
             raise ValueError("prefill() is single-GPU; tensor-parallel ranks step through the prompt")
         if self.off:
@@ -713,6 +771,10 @@ class Model:
         dev, K, G = self.tok.device, self.K, self.cfg.group
         if ids.device.type != "cuda":
             ids = ids.pin_memory().to(dev, non_blocking=True)
+        if self._tiled_prefill() is not None:
+            all_logits, last = self._prefill_tiled(ids, collect_logits)
+            self._finish_prefill(n, all_logits, last)
+            return all_logits
         h16 = dict(dtype=torch.half, device=dev)
         # tokens per chunk: the GEMM's limit, and split scratch of at most 256 MB
         chunk = max(1, min(K.gemm_max_tokens(), (256 << 20) // (self.n_q * self.max_splits * self.D * 4)))
@@ -735,15 +797,18 @@ class Model:
                     st["graph"] = graph
             if collect_logits:
                 K.gemm_w4a16(self.lm_head.packed, self.lm_head.sz, st["normed"], all_logits[c0:c0 + T], G)
-        normed = st["normed"]
-        if collect_logits:
+        self._finish_prefill(n, all_logits, st["normed"][T - 1])
+        return all_logits
+
+    def _finish_prefill(self, n, all_logits, last):
+        """Logits of the last prompt token, the token after the prompt, and the position behind it."""
+        if all_logits is not None:
             self.logits.copy_(all_logits[n - 1])
         else:   # only the last position's logits are needed to go on: one GEMV
-            self.linear(self.lm_head, normed[T - 1], self.logits)
+            self.linear(self.lm_head, last, self.logits)
         self.host_pos += n
         self.pos.fill_(self.host_pos - 1)
-        K.argmax(self.logits, self.tok, self.pos, self.history)   # token after the prompt; pos -> host_pos
-        return all_logits
+        self.K.argmax(self.logits, self.tok, self.pos, self.history)   # token after the prompt; pos -> host_pos
 
     def generate(self, prompt, n_new, use_graph=True, prefill=False):
         """Greedy decoding of n_new tokens after `prompt`, each token read back to the host as soon as its step has

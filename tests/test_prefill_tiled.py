@@ -62,3 +62,31 @@ def test_gemm_tiled_swiglu(K, I, Kd, T, split):
     ref = (torch.nn.functional.silu(gu[:, :I].float()).half() * gu[:, I:]).float()
     assert ((y.float() - ref).abs().max() / ref.abs().max()).item() <= 4e-3
     assert K.gemm_status() == 0
+
+
+# heads per group 1 .. 8, both head sizes, pages of 8 .. 64 tokens; prompts of one row block and several, with and without
+# a context before them, and a few tokens behind a long one (the context is then split between blocks)
+@pytest.mark.parametrize("D,n_q,n_kv,page,start,T", [(64, 8, 8, 16, 0, 130), (64, 8, 4, 8, 37, 65), (64, 8, 2, 64, 0, 33),
+                                                     (64, 8, 1, 16, 1500, 5), (64, 16, 2, 16, 700, 200), (128, 8, 1, 16, 0, 70),
+                                                     (128, 4, 4, 16, 1100, 3), (64, 8, 1, 16, 0, 1)])
+def test_prefill_equals_stepping(D, n_q, n_kv, page, start, T):
+    from llm_decode_kernels_b200.model import DecodeConfig, Model
+    from test_model import KERNEL_TOL, hf_cfg, random_state
+    c = hf_cfg(512, 2, n_q, n_kv, 1024, 1000, D=D)
+    m = Model(random_state(c, 3, D), c, DecodeConfig(group=128, max_ctx=start + T + 16, page=page, seed=1))
+    m.prepare(start + T + 8, use_graph=False)
+    m.kv.normal_(generator=torch.Generator(device=dev).manual_seed(2))
+    before = m.kv.clone()
+    ids = torch.randint(0, 1000, (T,), generator=torch.Generator().manual_seed(4))
+    m.reset(start)
+    want = m.teacher_force(ids, use_graph=False, collect_logits=True).float()
+    kv, tok = m.kv.clone().float(), int(m.tok)
+    m.kv.copy_(before)
+    m.reset(start)
+    got = m.prefill(ids, collect_logits=True).float()
+    assert (got - want).abs().max() <= KERNEL_TOL * want.abs().max()
+    assert torch.equal((m.kv != before).any(-1), (kv != before).any(-1))      # the same cache rows
+    assert (m.kv.float() - kv).abs().max() <= KERNEL_TOL * kv.abs().max()
+    assert m.host_pos == start + T and int(m.pos) == start + T and m.K.gemm_status() == 0
+    top = want[-1].sort(descending=True)[0]
+    assert int(m.tok) == tok or top[0] - top[1] <= 2 * KERNEL_TOL * want.abs().max()
