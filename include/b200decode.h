@@ -278,10 +278,15 @@ typedef struct b200_step_desc {
   int grid;            /* CTAs = SMs of the device */
   long long* trace;    /* NULL. (A library built with -DB200_STEP_TRACE, which the normal build never is, fills an
                         * int64 [grid, 8 + 25 (L + 1)] array here with per-CTA globaltimer values inside every phase.) */
+  void* att_xchg;      /* NULL, or b200_decode_step_att_bytes() bytes, zeroed once by the caller: lets attention use every CTA on
+                        * long contexts (without it: at most four slices per query head) */
 } b200_step_desc;
 
 /* Bytes of exchange memory a step of these dimensions needs. */
 size_t b200_decode_step_xchg_bytes(int L, int H, int I, int n_q, int n_kv, int D, int grid);
+
+/* Bytes of the optional wide attention exchange (0: the dimensions leave no CTAs to spare). */
+size_t b200_decode_step_att_bytes(int L, int n_q, int n_kv, int D, int grid);
 
 /* Launch one step. B200_ERR_SHAPE if the dimensions do not fit the kernel (H, n_q D and I multiples of 128, group size
  * a multiple of 128, pages of at most 64 tokens, the shared-memory plan; use the per-operator entry points then),

@@ -365,6 +365,13 @@ size_t b200_decode_step_xchg_bytes(int L, int H, int I, int n_q, int n_kv, int D
   return (per_layer * L + (size_t)grid * 4) * sizeof(uint32_t);
 }
 
+size_t b200_decode_step_att_bytes(int L, int n_q, int n_kv, int D, int grid) {
+  if (L <= 0 || grid <= 0 || n_q <= 0 || n_kv <= 0 || n_q % n_kv) return 0;
+  const int wide = b200::step_att_max(grid, n_q, n_kv);
+  if (wide <= b200::step_att_slices(grid, n_q)) return 0;
+  return b200::step_att_words_per_layer(n_q, D, wide) * L * sizeof(uint32_t);
+}
+
 int b200_decode_step(const b200_step_desc* d, void* stream) {
   static_assert(sizeof(b200_step_layer) == sizeof(b200::StepLayer), "layer structs must match");
   REQUIRE(d && d->layers && d->emb && d->norm_f && d->w_head && d->cos_t && d->sin_t && d->bt &&
@@ -383,25 +390,30 @@ int b200_decode_step(const b200_step_desc* d, void* stream) {
     kmax = K > kmax ? K : kmax;
   }
   REQUIRE(aligned16(d->emb) && aligned16(d->norm_f) && aligned16(d->w_head) && aligned16(d->xchg) &&
-              aligned16(d->ctrl) && aligned16(d->layers),
+              aligned16(d->ctrl) && aligned16(d->layers) && aligned16(d->att_xchg),
           B200_ERR_ALIGN);
   REQUIRE(d->ctx_cap <= (1 << 20), B200_ERR_LIMIT);
 
   b200::StepParams p = {};
   p.layers = reinterpret_cast<const b200::StepLayer*>(d->layers);
   p.L = d->L; p.H = d->H; p.I = d->I; p.n_q = d->n_q; p.n_kv = d->n_kv; p.D = d->D; p.V = d->V;
+  p.n_qkv = n_qkv; p.n_att = n_att;
   p.log2G = d->log2G; p.log2P = d->log2P; p.eps = d->eps;
   p.emb = (const half*)d->emb; p.norm_f = (const half*)d->norm_f; p.w_head = d->w_head; p.sz_head = d->sz_head;
   p.cos_t = d->cos_t; p.sin_t = d->sin_t; p.bt = d->bt; p.tok = d->tok; p.pos = d->pos; p.history = d->history;
   p.logits = (half*)d->logits; p.xchg = (uint32_t*)d->xchg; p.ctrl = (b200::StepCtrl*)d->ctrl;
   p.trace = d->trace;
   p.att_slices = b200::step_att_slices(d->grid, d->n_q);
+  p.att_groups = b200::step_att_groups(d->n_q, d->n_kv);
+  p.att_max = d->att_xchg ? b200::step_att_max(d->grid, d->n_q, d->n_kv) : 0;
+  p.att_xchg = (uint32_t*)d->att_xchg;
+  p.layer_words = (int)b200::step_words_per_layer(d->H, d->I, d->n_q, d->n_kv, d->D, p.att_slices);
+  p.att_layer_words = (int)b200::step_att_words_per_layer(d->n_q, d->D, p.att_max);
   // shared-memory plan
   const int ncw = b200::decode_step_consumer_warps();
   const int resid_bytes = align_up(2 * d->H, 128);
   const int xin_bytes = align_up(2 * kmax, 128);             // two byte digits per activation, as B fragments
   const int xsum_bytes = align_up((kmax / 128) * 8, 128);
-  const int att_bytes = align_up((4 * d->D + ncw * d->D + 2 * ncw + d->D + 64) * 4, 128);
   int part_bytes;
   {
     // partial sums: one float per consumer warp and row slot of the CTA's tiles (16 slots per tile); the layer
@@ -422,8 +434,7 @@ int b200_decode_step(const b200_step_desc* d, void* stream) {
   // attention copies whole KV pages into a stage, K rows in one half and V rows in the other
   const int P = 1 << d->log2P;
   REQUIRE(P <= b200::decode_step_max_kv_tokens() && 4 * d->D * P <= p.stage_w, B200_ERR_SHAPE);
-  const size_t fixed = b200::decode_step_plan_smem(p, resid_bytes, xin_bytes, xsum_bytes, att_bytes, part_bytes,
-                                                   table_bytes);
+  const size_t fixed = b200::decode_step_plan_smem(p, resid_bytes, xin_bytes, xsum_bytes, part_bytes, table_bytes);
   const size_t budget = 227 * 1024;
   REQUIRE(fixed + 2 * (size_t)p.stage_bytes <= budget, B200_ERR_SHAPE);
   int ns = (int)((budget - fixed) / p.stage_bytes);

@@ -51,18 +51,21 @@
 //
 // Phases per layer (the reference's operator order, with the same rounding points as its fused kernels):
 //   A  resid += down[l-1] (layer 0: resid = embedding row);  x = RMSNorm(resid) * ln1;  qkv = Wqkv x
-//   B  attention: query head h is shared by J CTAs (as many as the grid has to spare, at most 4), CTA h + j n_q
-//      taking every J-th 128-token stage of the context: RoPE on q and k, (slice 0) append k, v to the paged cache,
-//      then per-warp online softmax over the slice's cached tokens (from the ring), merged once across warps; the
-//      slice's normalised output and log-sum-exp go to the exchange
-//   C  o = Wo attn, attn merged from the J slices of each head while it is staged
+//   B  attention: RoPE on q and k, append k, v to the paged cache, online softmax over the cached tokens (from the ring).
+//      Short contexts: one CTA per query head. Longer ones: a CTA takes one kv head and one slice of the context for ALL
+//      query heads of the group (up to 8), so every cached row is copied and read once, both contractions as warp-level
+//      MMAs; the slices' normalised outputs and log-sum-exps go to an exchange of their own, and one CTA per head merges
+//      them. (TinyLlama shape at 8192 cached tokens: 695 us a token with up to four CTAs per query head, 440 this way.)
+//   C  o = Wo attn
 //   D  resid += o;  x = RMSNorm(resid) * ln2;  act = SwiGLU(Wgate x, Wup x)
 //   E  down = Wdown act
 // then resid += down;  x = RMSNorm(resid) * norm_f;  logits = Whead x;  per-CTA argmax candidates; CTA 0 merges
 // them (lowest index wins ties), writes tok, history[pos], pos + 1 and the new epoch.
-// Barriers over the consumer threads per phase: one for sum(resid^2) where a norm precedes the GEMV, one between the
-// warps' partial sums and the threads that add them up; the partial-sum buffer alternates between phases so that no
-// third one is needed.
+// The norm's factor rsqrt(mean(resid^2) + eps) multiplies the outputs of the GEMV behind it (x is staged as resid * ln).
+// One barrier over the consumer threads per phase, between the warps' partial sums (and sums of squares) and the threads that
+// add them up; the partial-sum buffer alternates between phases so that no second one is needed.
+// The code of the loop is kept small - one copy of what serves several phases, loops not unrolled where nothing is gained:
+// at 101 KB the fetches of 90 to 180 lines per layer and SM from the L2 were 12 us of a token, at 85 KB there are none.
 //
 // Every wait (mbarrier or tag poll) is bounded. A wait that runs out records a code in StepCtrl::error, raises an
 // abort flag that all later waits honour at once, and the CTA leaves after its copies in flight have landed; the
@@ -86,9 +89,11 @@ constexpr int kSpinLimit = 1 << 18;         // polls / try_waits before a wait g
 constexpr int kHeaderBytes = 2048;
 constexpr int kMaxKvTokens = 128;           // cached tokens per ring stage in attention (3 rounds of 11 warps x 4 tokens)
 constexpr int kKvRounds = (kMaxKvTokens + 4 * kNCW - 1) / (4 * kNCW);
-constexpr int kSliceMinContext = 1152;      // cached tokens from which attention is cut into context slices
-constexpr int kPollBatch = 4;               // exchange granules a lane keeps in flight while it polls (plain staging)
-constexpr int kNormBatch = 2;               // the same where a norm follows: units of the residual stream per pass
+// Units of a row a warp polls and stages together: two, so that nothing spills, where a row is a few units per warp; more for long
+// rows, which are bound by these trips to the L2 (28672 weights: 20 units per warp; 8 layers of the 70B shape 884 -> 858 us).
+// Six or eight at a time spill and lose again.
+constexpr int kBatch = 2, kBatchNorm = 2, kWideBatch = 4, kWideBatchNorm = 3;
+constexpr int kWideUnits = 4;               // units per warp above which a row counts as long
 
 enum : int { ERR_POLL = 1, ERR_FULL = 2, ERR_EMPTY = 3, ERR_TOKEN = 4 };
 
@@ -145,33 +150,49 @@ DEVI void st_tagged(uint32_t* p, uint32_t v) {
   asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
+DEVI void st_tagged2(uint32_t* p, uint32_t a, uint32_t b) {
+  asm volatile("st.relaxed.gpu.global.v2.u32 [%0], {%1, %2};" ::"l"(p), "r"(a), "r"(b) : "memory");
+}
+
 // ---- shared state of one CTA -----------------------------------------------------------------------------------
-// Shared memory: [0, 128) full barriers, [128, 256) empty barriers, 256 abort flag, 272 sum scratch, 512 slices;
+// Shared memory: [0, 128) full barriers, [128, 256) empty barriers, 256 abort flag, 272 sum scratch, 512 slices, 640 plan of
+// the attention, 704 argmax keys, 1024 RoPE factors;
 // from kHeaderBytes on: residual stream, then the areas whose offsets the host put into StepParams (off_*).
 // Pointers into it are formed where they are used (one add of a kernel parameter) instead of being carried in
 // registers through the whole step.
+// How a step's attention is cut: A slices of `per` cached tokens per kv head. two: their partials are merged by one CTA per
+// head, which publishes the attention output (otherwise the CTAs that stage it merge).
+// units: attention units of a layer, dealt to the CTAs in turn.
+struct AttPlan { int A, per, two, refresh, pos, units; };
+
+// The shared memory is named where it is used and not carried as a pointer: a pointer that passes through a function or an asm
+// statement loses its address space, and every access through it becomes a generic one.
+extern __shared__ __align__(128) uint8_t step_smem[];
 struct Cta {
-  uint8_t* smem;
   const StepParams* p;   // the kernel's parameter block (constant bank)
   uint32_t tagw;         // (tag << 16)
 #ifdef B200_STEP_TRACE
   long long* tr;         // this CTA's row of the trace array (thread 0 stamps), or null
 #endif
-  DEVI uint64_t* full(int i) const { return reinterpret_cast<uint64_t*>(smem) + i; }
-  DEVI uint64_t* empty(int i) const { return reinterpret_cast<uint64_t*>(smem) + kMaxStages + i; }
-  DEVI volatile int* abort() const { return reinterpret_cast<volatile int*>(smem + 2 * kMaxStages * 8); }
+  DEVI uint64_t* full(int i) const { return reinterpret_cast<uint64_t*>(step_smem) + i; }
+  DEVI uint64_t* empty(int i) const { return reinterpret_cast<uint64_t*>(step_smem) + kMaxStages + i; }
+  DEVI volatile int* abort() const { return reinterpret_cast<volatile int*>(step_smem + 2 * kMaxStages * 8); }
   // kNCW floats: the warps' shares of sum(resid^2)
-  DEVI float* red() const { return reinterpret_cast<float*>(smem + 2 * kMaxStages * 8 + 16); }
+  DEVI float* red() const { return reinterpret_cast<float*>(step_smem + 2 * kMaxStages * 8 + 16); }
   // [H] residual stream, private copy of the CTA; unit u belongs to warp u % kNCW
-  DEVI half* resid() const { return reinterpret_cast<half*>(smem + kHeaderBytes); }
+  DEVI half* resid() const { return reinterpret_cast<half*>(step_smem + kHeaderBytes); }
   // activations of the running GEMV as byte-digit B fragments, 256 bytes per unit; unit u is written and read by one warp only
-  DEVI half* xin() const { return reinterpret_cast<half*>(smem + p->off_xin); }
-  DEVI float* xsum() const { return reinterpret_cast<float*>(smem + p->off_xsum); }   // [Kmax / 128][2] sum, 2^-s
-  DEVI float* att() const { return reinterpret_cast<float*>(smem + p->off_att); }     // attention scratch
+  DEVI half* xin() const { return reinterpret_cast<half*>(step_smem + p->off_xin); }
+  DEVI float* xsum() const { return reinterpret_cast<float*>(step_smem + p->off_xsum); }   // [Kmax / 128][2] sum, 2^-s
+  DEVI uint8_t* att() const { return step_smem + p->off_att; }                             // attention scratch (att_layout)
+  DEVI const AttPlan& plan() const { return *reinterpret_cast<const AttPlan*>(step_smem + 640); }
+  DEVI unsigned long long* keys() const { return reinterpret_cast<unsigned long long*>(step_smem + 704); }   // [2 kNCW]
+  DEVI float* rope() const { return reinterpret_cast<float*>(step_smem + 1024); }          // [D/2] cos, [D/2] sin, page of pos
   // partial dot products, [warp][row slot], two buffers used by alternate phases
-  DEVI float* part() const { return reinterpret_cast<float*>(smem + p->off_part); }
-  DEVI uint8_t* stage(int slot) const { return smem + p->off_ring + (size_t)slot * p->stage_bytes; }
+  DEVI float* part() const { return reinterpret_cast<float*>(step_smem + p->off_part); }
+  DEVI uint8_t* stage(int slot) const { return step_smem + p->off_ring + (size_t)slot * p->stage_bytes; }
   DEVI StepCtrl* ctrl() const { return p->ctrl; }
+  DEVI const StepLayer& layer(int l) const { return reinterpret_cast<const StepLayer*>(step_smem + p->off_table)[l]; }
 };
 
 // Phase stamps of the instrumented build (-DB200_STEP_TRACE): thread 0 of the CTA stores the nanosecond timer at slot
@@ -224,8 +245,9 @@ DEVI bool wait_bar(const Cta& c, uint64_t* bar, uint32_t parity, int code, unsig
 
 // ---- tagged exchange words -----------------------------------------------------------------------------------------
 // A word of step s carries tag (s mod 65535) + 1, so a word left over from step s - 65535 would pass for a fresh one.
-// That cannot happen: every exchange word (every output row of every phase of every layer, and the argmax
-// candidates) is rewritten in every step, so a word is never more than one step old when it is polled.
+// That cannot happen: the output rows of every phase of every layer and the argmax candidates are rewritten in every
+// step, and the partials of attention slices, of which a short context uses only a few, at least in every 1024th step
+// (refresh_partials).
 DEVI bool tags_ok(const Cta& c, uint4 v) {
   return ((((v.x ^ c.tagw) | (v.y ^ c.tagw) | (v.z ^ c.tagw) | (v.w ^ c.tagw)) >> 16) == 0);
 }
@@ -235,26 +257,26 @@ DEVI uint2 payload(uint4 v) { return make_uint2((v.x & 0xFFFFu) | (v.y << 16), (
 // step's tag; all loads of a round are in flight together. out[k] = the 4 fp16 payloads of granule k as 2 x half2.
 template <int NB>
 DEVI void poll_many(const Cta& c, const uint32_t* base, int stride, int nb, uint2 (&out)[NB]) {
-  constexpr int kPollBatch = NB;
-  uint4 v[kPollBatch];
+  uint4 v[NB];
 #pragma unroll
-  for (int k = 0; k < kPollBatch; ++k)
-    if (k < nb) v[k] = ld_poll4(base + (size_t)k * stride);
+  for (int k = 0; k < NB; ++k)
+    if (k < nb) v[k] = ld_poll4(base + k * stride);
   int spins = 0;
+#pragma unroll 1
   for (;;) {
     bool ok = true;
 #pragma unroll
-    for (int k = 0; k < kPollBatch; ++k)
+    for (int k = 0; k < NB; ++k)
       if (k < nb && !tags_ok(c, v[k])) ok = false;
     if (ok || *c.abort()) break;
     if (++spins > kSpinLimit) { raise(c, ERR_POLL); break; }
     if ((spins & 255) == 0 && ((volatile StepCtrl*)c.ctrl())->abort) { *c.abort() = 1; break; }
 #pragma unroll
-    for (int k = 0; k < kPollBatch; ++k)
-      if (k < nb && !tags_ok(c, v[k])) v[k] = ld_poll4(base + (size_t)k * stride);
+    for (int k = 0; k < NB; ++k)
+      if (k < nb && !tags_ok(c, v[k])) v[k] = ld_poll4(base + k * stride);
   }
 #pragma unroll
-  for (int k = 0; k < kPollBatch; ++k)
+  for (int k = 0; k < NB; ++k)
     if (k < nb) out[k] = payload(v[k]);
 }
 DEVI uint2 poll4(const Cta& c, const uint32_t* p) {
@@ -272,6 +294,7 @@ DEVI void poll_list(const Cta& c, const uint32_t* base, const uint32_t (&off)[NB
   for (int k = 0; k < NB; ++k)
     if ((mask >> k) & 1u) v[k] = ld_poll4(base + off[k]);
   int spins = 0;
+#pragma unroll 1
   for (;;) {
     bool ok = true;
 #pragma unroll
@@ -299,23 +322,22 @@ DEVI void poll_list(const Cta& c, const uint32_t* base, const uint32_t (&off)[NB
 // byte order) or high nibbles (m odd: e2 e6 e3 e7). Granule l = 4 elements of word (l % 8) / 2: elements e0..e3 on
 // even lanes, e4..e7 on odd ones, so a lane pair swaps its packed bytes once and each lane permutes one register.
 // xsum[2 u] = 2^-s sum X (for the zero-point term), xsum[2 u + 1] = 2^-s (both NaN if the unit is not finite).
-DEVI void put_unit(const Cta& c, int u, uint2 v, int lane) {
-  // max|x| of the unit from the bit patterns (the order of non-negative fp16 numbers is the order of their bits)
-  const uint32_t m2 = __vmaxu2(v.x & 0x7FFF7FFFu, v.y & 0x7FFF7FFFu);
-  const uint32_t mx = __reduce_max_sync(0xffffffffu, max(m2 & 0xFFFFu, m2 >> 16));
-  const bool finite = mx < 0x7C00u;                       // no infinity, no NaN
-  const int sh = 28 - max((int)(mx >> 10), 1);            // exponent field e: max|x| in [2^(e-15), 2^(e-14)) -> 2^sh max|x| in [2^13, 2^14)
-  const float sc = __int_as_float((sh + 127) << 23);      // 2^sh, sh in [-2, 27]
-  // round(x * 2^sh) + 128 in the low bits of a float: adding 1.5 * 2^23 + 128 rounds to an integer (nearest even)
+DEVI void put_unit(const Cta& c, int u, float4 v, int lane) {
+  // max|x| of the unit from the bit patterns (the order of non-negative floats is the order of their bits; NaN is above all)
+  const uint32_t mx = __reduce_max_sync(0xffffffffu, max(max(__float_as_uint(v.x) & 0x7FFFFFFFu, __float_as_uint(v.y) & 0x7FFFFFFFu),
+                                                         max(__float_as_uint(v.z) & 0x7FFFFFFFu, __float_as_uint(v.w) & 0x7FFFFFFFu)));
+  const bool finite = mx < 0x7F800000u;                   // no infinity, no NaN
+  const int e = max((int)(mx >> 23), 14);                 // exponent field: max|x| in [2^(e-127), 2^(e-126))
+  const float sc = __int_as_float((267 - e) << 23);       // 2^s, s = 140 - e: 2^s max|x| in [2^13, 2^14)
+  // round(x * 2^s) + 128 in the low bits of a float: adding 1.5 * 2^23 + 128 rounds to an integer (nearest even)
   // and leaves it, in two's complement, in the mantissa. Byte 0 of that, with its top bit flipped, is the lo digit
   // (X & 255 read as a signed byte), byte 1 is the hi digit ((X + 128) >> 8).
   constexpr float kMagic = 12582912.f + 128.f;
-  const float2 a = __half22float2(as_h2(v.x)), b = __half22float2(as_h2(v.y));
-  const uint32_t w0 = __float_as_uint(fmaf(a.x, sc, kMagic)), w1 = __float_as_uint(fmaf(a.y, sc, kMagic));
-  const uint32_t w2 = __float_as_uint(fmaf(b.x, sc, kMagic)), w3 = __float_as_uint(fmaf(b.y, sc, kMagic));
+  const uint32_t w0 = __float_as_uint(fmaf(v.x, sc, kMagic)), w1 = __float_as_uint(fmaf(v.y, sc, kMagic));
+  const uint32_t w2 = __float_as_uint(fmaf(v.z, sc, kMagic)), w3 = __float_as_uint(fmaf(v.w, sc, kMagic));
   const uint32_t kM = __float_as_uint(kMagic);            // w - kM = X
   const int xsum_i = __reduce_add_sync(0xffffffffu, (int)(w0 - kM) + (int)(w1 - kM) + (int)(w2 - kM) + (int)(w3 - kM));
-  const float resc = finite ? __int_as_float((127 - sh) << 23) : __int_as_float(0x7fc00000);   // 2^-sh, or NaN
+  const float resc = finite ? __int_as_float((e - 13) << 23) : __int_as_float(0x7fc00000);   // 2^-s, or NaN
   if (lane == 0) {
     c.xsum()[2 * u] = (float)xsum_i * resc;               // the sum of what the MMAs multiply, rescaled
     c.xsum()[2 * u + 1] = resc;
@@ -332,96 +354,45 @@ DEVI void put_unit(const Cta& c, int u, uint2 v, int lane) {
 }
 
 // x <- E[0..K) (tagged).
+template <int PB>
 DEVI void stage_plain(const Cta& c, const uint32_t* E, int K, int warp, int lane) {
   const int nunit = K >> 7;
-  for (int u0 = warp; u0 < nunit; u0 += kNCW * kPollBatch) {
-    const int nb = min(kPollBatch, (nunit - u0 + kNCW - 1) / kNCW);
-    uint2 v[kPollBatch];
+#pragma unroll 1
+  for (int u0 = warp; u0 < nunit; u0 += kNCW * PB) {
+    const int nb = min(PB, (nunit - u0 + kNCW - 1) / kNCW);
+    uint2 v[PB];
     poll_many(c, E + 128 * u0 + 4 * lane, 128 * kNCW, nb, v);
 #pragma unroll
-    for (int k = 0; k < kPollBatch; ++k)
-      if (k < nb) put_unit(c, u0 + kNCW * k, v[k], lane);
+    for (int k = 0; k < PB; ++k)
+      if (k < nb) {
+        const float2 a = __half22float2(as_h2(v[k].x)), b = __half22float2(as_h2(v[k].y));
+        put_unit(c, u0 + kNCW * k, make_float4(a.x, a.y, b.x, b.y), lane);
+      }
   }
   __syncwarp();
 }
 
-// x <- the attention output, merged from the J context slices of every head while it is staged: slice j of head h
-// left its normalised output o_j (Eatt + j n_att) and its log-sum-exp l_j as two fp16 words, value and remainder
-// (Else + h * step_lse_words(J) + 2 j); x = sum_j e^(l_j - max l) o_j / sum_j e^(l_j - max l). A slice that saw no
-// token has l_j = -inf and o_j = 0. Lane l of the warp that owns unit u holds 4 values of one head.
-// A function of its own, called (with the CTA's state by value, in registers) only in steps with a sliced context:
-// inlined into the one loop body that serves every phase of the step it made the GEMV phases of EVERY step a fifth
-// slower (measured; what the compiler does with that loop depends on everything in it - moving put_unit out of line,
-// which shrinks the body by 12 KB, costs 6 %, and so does doing two tiles at once in gemv()).
-__device__ __noinline__ void stage_attn(const Cta c, const uint32_t* Eatt, const uint32_t* Else, int J, int n_att, int D, int warp,
-                     int lane) {
-  constexpr int NL = (kStepMaxAttSlices + 1) / 2;   // granules of log-sum-exp words per head
-  const int nunit = n_att >> 7, lsew = step_lse_words(J), ng = lsew >> 2;
-  const uint32_t lbase = (uint32_t)(Else - Eatt);
-  for (int u = warp; u < nunit; u += kNCW) {
-    const int i = 128 * u + 4 * lane, h = i / D;
-    // While the slices are still at work the warp polls the log-sum-exp words only: one or two addresses per head,
-    // the same for all lanes of a head, instead of J granules per lane - 148 CTAs polling every partial would keep
-    // the L2 busy with nothing else. When those are there the outputs are too, or nearly (the second poll checks
-    // their tags all the same). One unit at a time: more granules in flight would not fit into the registers, and
-    // this kernel must not spill.
-    uint32_t loff[NL], ooff[kStepMaxAttSlices];   // word offsets from Eatt (Else lies behind it)
-#pragma unroll
-    for (int g = 0; g < NL; ++g) loff[g] = lbase + (uint32_t)(h * lsew + 4 * g);
-#pragma unroll
-    for (int k = 0; k < kStepMaxAttSlices; ++k) ooff[k] = (uint32_t)(k * n_att + i);
-    uint2 lv[NL], v[kStepMaxAttSlices];
-    poll_list(c, Eatt, loff, (1u << ng) - 1u, lv);
-    poll_list(c, Eatt, ooff, (1u << J) - 1u, v);
-    float lse[kStepMaxAttSlices], M = -CUDART_INF_F;
-#pragma unroll
-    for (int k = 0; k < kStepMaxAttSlices; ++k) {
-      lse[k] = -CUDART_INF_F;
-      if (k < J) {
-        const uint2 pr = lv[k >> 1];
-        const float2 f = __half22float2(as_h2((k & 1) ? pr.y : pr.x));   // (value, remainder)
-        lse[k] = f.x + f.y;
-        M = fmaxf(M, lse[k]);
-      }
-    }
-    float W = 0.f, o0 = 0.f, o1 = 0.f, o2 = 0.f, o3 = 0.f;
-#pragma unroll
-    for (int k = 0; k < kStepMaxAttSlices; ++k) {
-      if (k < J) {
-        const float w = __expf(lse[k] - M);   // the slice with the step's own token is never empty: M is finite
-        const float2 x01 = __half22float2(as_h2(v[k].x)), x23 = __half22float2(as_h2(v[k].y));
-        W += w;
-        o0 = fmaf(w, x01.x, o0), o1 = fmaf(w, x01.y, o1), o2 = fmaf(w, x23.x, o2), o3 = fmaf(w, x23.y, o3);
-      }
-    }
-    const float rW = 1.f / W;
-    uint2 o;
-    o.x = as_u32(__floats2half2_rn(o0 * rW, o1 * rW));
-    o.y = as_u32(__floats2half2_rn(o2 * rW, o3 * rW));
-    put_unit(c, u, o, lane);
-  }
-  __syncwarp();
-}
-
-// resid <- resid + delta (delta tagged; or resid <- emb row when E == nullptr), then
-// x <- w * half(float(resid) * rsqrt(mean(resid^2) + eps)).  One barrier over the consumer threads (the sum).
-DEVI void stage_norm(const Cta& c, const uint32_t* E, const half* emb_row, const half* w, int H, float eps, int warp,
-                     int lane) {
+// resid <- resid + delta (delta tagged; or resid <- emb row when E == nullptr), x <- w * resid, and the warp's share of sum(resid^2).
+// The factor rsqrt(mean(resid^2) + eps) of the norm is common to the whole row: it is applied to the outputs (reduce_emit), behind
+// the barrier that is there anyway, and no warp waits for the others here. Waiting cost 0.4 us per norm, 19 us per token.
+template <int NB>
+DEVI void stage_norm(const Cta& c, const uint32_t* E, const half* emb_row, const half* w, int H, int warp, int lane) {
   const int nunit = H >> 7;
   uint2* rs = reinterpret_cast<uint2*>(c.resid());
   const uint2* wg = reinterpret_cast<const uint2*>(w);
-  // the norm weights of the first batch are requested before the poll: their latency hides behind the wait
-  uint2 wv0[kNormBatch];
-#pragma unroll
-  for (int k = 0; k < kNormBatch; ++k)
-    if (warp + kNCW * k < nunit) wv0[k] = __ldg(wg + 32 * (warp + kNCW * k) + lane);
   float ss = 0.f;
-  for (int u0 = warp; u0 < nunit; u0 += kNCW * kNormBatch) {
-    const int nb = min(kNormBatch, (nunit - u0 + kNCW - 1) / kNCW);
-    uint2 d[kNormBatch];
-    if (E) poll_many(c, E + 128 * u0 + 4 * lane, 128 * kNCW, nb, d);
+#pragma unroll 1
+  for (int u0 = warp; u0 < nunit; u0 += kNCW * NB) {
+    const int nb = min(NB, (nunit - u0 + kNCW - 1) / kNCW);
+    uint2 d[NB], wv[NB];
 #pragma unroll
-    for (int k = 0; k < kNormBatch; ++k) {
+    for (int k = 0; k < NB; ++k)   // the norm weights travel while the residual is polled
+      if (k < nb) wv[k] = __ldg(wg + 32 * (u0 + kNCW * k) + lane);
+    if (E) poll_many(c, E + 128 * u0 + 4 * lane, 128 * kNCW, nb, d);
+    float4 x[NB];
+    float sq = 0.f;
+#pragma unroll
+    for (int k = 0; k < NB; ++k) {
       if (k < nb) {
         const int idx = 32 * (u0 + kNCW * k) + lane;
         uint2 r;
@@ -434,37 +405,31 @@ DEVI void stage_norm(const Cta& c, const uint32_t* E, const half* emb_row, const
         }
         rs[idx] = r;
         const float2 a = __half22float2(as_h2(r.x)), b = __half22float2(as_h2(r.y));
-        ss = fmaf(a.x, a.x, fmaf(a.y, a.y, fmaf(b.x, b.x, fmaf(b.y, b.y, ss))));
+        sq = fmaf(a.x, a.x, fmaf(a.y, a.y, fmaf(b.x, b.x, fmaf(b.y, b.y, sq))));
+        const float2 wa = __half22float2(as_h2(wv[k].x)), wb = __half22float2(as_h2(wv[k].y));
+        x[k] = make_float4(a.x * wa.x, a.y * wa.y, b.x * wb.x, b.y * wb.y);
       }
     }
+    ss += warp_sum(sq);   // its shuffles fill the gaps in put_unit's chain
+    put_unit(c, u0, x[0], lane);
+#pragma unroll
+    for (int k = 1; k < NB; ++k)
+      if (k < nb) put_unit(c, u0 + kNCW * k, x[k], lane);
   }
-  ss = warp_sum(ss);
   if (lane == 0) c.red()[warp] = ss;
-  consumer_sync();
-  float tot = 0.f;
-#pragma unroll
-  for (int k = 0; k < kNCW; ++k) tot += c.red()[k];
-  const float rinv = rsqrtf(tot / (float)H + eps);
-  int j = 0;
-  for (int u = warp; u < nunit; u += kNCW, ++j) {
-    const int idx = 32 * u + lane;
-    const uint2 r = rs[idx];   // this lane's own write
-    uint2 wv;
-    if (j < kNormBatch) {
-      wv = wv0[0];
-#pragma unroll
-      for (int k = 1; k < kNormBatch; ++k)
-        if (j == k) wv = wv0[k];
-    } else {
-      wv = __ldg(wg + idx);
-    }
-    const float2 a = __half22float2(as_h2(r.x)), b = __half22float2(as_h2(r.y));
-    uint2 o;
-    o.x = as_u32(__hmul2(as_h2(wv.x), __floats2half2_rn(a.x * rinv, a.y * rinv)));
-    o.y = as_u32(__hmul2(as_h2(wv.y), __floats2half2_rn(b.x * rinv, b.y * rinv)));
-    put_unit(c, u, o, lane);
-  }
   __syncwarp();
+}
+// the factor of the norm, behind a barrier after stage_norm
+DEVI float norm_factor(const Cta& c, int H, float eps) {
+  float v[kNCW];
+#pragma unroll
+  for (int k = 0; k < kNCW; ++k) v[k] = c.red()[k];
+#pragma unroll
+  for (int k = 0; k + 1 < kNCW; k += 2) v[k] += v[k + 1];
+  float tot = v[0];
+#pragma unroll
+  for (int k = 2; k < kNCW; k += 2) tot += v[k];
+  return rsqrtf(tot / (float)H + eps);
 }
 
 // ---- GEMV phase -----------------------------------------------------------------------------------------------------
@@ -482,11 +447,17 @@ struct Slice { int t0, nt; };   // this CTA's tiles [t0, t0 + nt) of a matrix
 struct RingPos {
   int slot;
   uint32_t parity;
-  int count;   // stages passed (the producer's abort path needs it)
+};
+struct ProducerPos : RingPos {
+  int count;   // stages passed (the abort path needs it)
 };
 DEVI void advance(RingPos& r, int ns) {
-  ++r.count;
   if (++r.slot == ns) { r.slot = 0; r.parity ^= 1u; }
+}
+
+DEVI void advance(ProducerPos& r, int ns) {
+  ++r.count;
+  advance(static_cast<RingPos&>(r), ns);
 }
 
 // Whole tiles are dealt to the CTAs as evenly as they go: a GEMV phase of the step is a handful of tile-units per
@@ -503,9 +474,10 @@ DEVI Slice slice_of(int rows, int paired, int cta, int ncta) {
 
 // Producer: issue every stage of one matrix slice, one copy each (a bulk copy costs ~0.2 us to issue whatever its
 // size, so several small copies per stage would make the producer the bottleneck).
-DEVI void produce(const Cta& c, const Mat& m, const Slice& s, RingPos& rp, int lane) {
-  const int nunit = m.K >> 7, NU = s.nt * nunit;
-  const uint8_t* src = m.base + (size_t)s.t0 * nunit * kTileUnitBytes;
+DEVI void produce(const Cta& c, const uint8_t* base, int nunit, const Slice& s, ProducerPos& rp, int lane) {
+  const int NU = s.nt * nunit;
+  const uint8_t* src = base + (size_t)s.t0 * nunit * kTileUnitBytes;
+#pragma unroll 1
   for (int i0 = 0; i0 < NU; i0 += c.p->ups, advance(rp, c.p->ns)) {
     const int slot = rp.slot;
     if (!wait_bar(c, c.empty(slot), rp.parity, ERR_EMPTY, 200)) return;
@@ -519,24 +491,24 @@ DEVI void produce(const Cta& c, const Mat& m, const Slice& s, RingPos& rp, int l
 
 // Cached tokens per attention ring stage: K rows in the first half of the stage, V rows in the second.
 DEVI int kv_tokens_per_stage(const StepParams& p) {
-  int t = min(kMaxKvTokens, p.stage_w / (4 * p.D));
+  int t = min(kMaxKvTokens / (p.D / 64), p.stage_w / (4 * p.D));   // head_dim 128: 64, a team of two warps takes a block
   return t & ~((1 << p.log2P) - 1);
 }
 
-// Producer: the cached K/V rows [0, pos) of one kv head, page by page, for context slice j of J: the stages j, j + J,
-// ... of the context. Whole pages are copied; rows at or beyond pos in the last page are ignored by the consumer.
-DEVI void produce_kv(const Cta& c, const StepParams& p, const StepLayer& ly, int kvh, int j, int J, int pos, RingPos& rp,
-                     int lane) {
-  const int tps = kv_tokens_per_stage(p), pps = tps >> p.log2P;
+// Producer: the cached K/V rows [t0, t1) of one kv head, page by page (t0 is a multiple of the page size). Whole pages are
+// copied; rows at or beyond t1 in the last page are ignored by the consumer.
+DEVI void produce_kv(const Cta& c, const StepParams& p, const StepLayer& ly, int kvh, int t0, int t1, ProducerPos& rp, int lane) {
+  const int tps = kv_tokens_per_stage(p);
   const uint32_t page_bytes = (uint32_t)(p.D * 2) << p.log2P;
-  const int nst = (pos + tps - 1) / tps;
-  for (int st = j; st < nst; st += J, advance(rp, c.p->ns)) {
+#pragma unroll 1
+  for (int t = t0; t < t1; t += tps, advance(rp, c.p->ns)) {
     const int slot = rp.slot;
     if (!wait_bar(c, c.empty(slot), rp.parity, ERR_EMPTY, 200)) return;
-    const int pg0 = st * pps, npg = min(pps, ((pos + (1 << p.log2P) - 1) >> p.log2P) - pg0);
+    const int pg0 = t >> p.log2P, npg = (min(tps, t1 - t) + (1 << p.log2P) - 1) >> p.log2P;
     uint8_t* dst = c.stage(slot);
     if (lane == 0) mbar_expect_tx(c.full(slot), 2 * npg * page_bytes);
     __syncwarp();
+#pragma unroll 1
     for (int pg = lane; pg < npg; pg += 32) {
       const size_t off = ((size_t)p.bt[pg0 + pg] * p.n_kv + kvh) * page_bytes;
       bulk_g2s(dst + pg * page_bytes, reinterpret_cast<const uint8_t*>(ly.kc) + off, page_bytes, c.full(slot));
@@ -580,7 +552,8 @@ DEVI void tile_unit(const Cta& c, const uint8_t* tu, int u, int lane, float& ya,
 // Consumer side of one matrix slice, one warp's share. The slice is the sequence of tile-unit blocks
 // (tile 0 unit 0, tile 0 unit 1, ..., tile 1 unit 0, ...), `ups` of them per ring stage; warp w takes the blocks of
 // units w, w + kNCW, ... of every tile, two at a time where the ring stage holds both (two independent instruction
-// streams for the scheduler to interleave). The activations are re-read from shared memory for every block: keeping
+// streams for the scheduler to interleave). Rows of 2048 weights are 16 units for 11 warps: sharing the last five between two warps
+// each (half of a block's MMAs) evens the warps out on paper, and measured 20 us a token slower than leaving them. The activations are re-read from shared memory for every block: keeping
 // them in registers across tiles was measured and loses - it pushes the kernel over its registers, and a spilled
 // register costs an L2 round trip here. Doing two tiles of a stage together (four independent blocks) was measured
 // too and loses 3 %. When the warp has passed its last unit of a tile, lanes t == 0 leave the
@@ -596,6 +569,7 @@ DEVI void gemv(const Cta& c, const Mat& m, const Slice& s, float* part, int pstr
 #ifdef B200_STEP_TRACE
   long long waited = 0;
 #endif
+#pragma unroll 1
   for (int i0 = 0; i0 < NU; i0 += c.p->ups, advance(rp, c.p->ns)) {
     const int slot = rp.slot;
 #ifdef B200_STEP_TRACE
@@ -608,6 +582,7 @@ DEVI void gemv(const Cta& c, const Mat& m, const Slice& s, float* part, int pstr
     const int end = min(NU, i0 + c.p->ups);
     const uint8_t* sb = c.stage(slot) - (size_t)i0 * kTileUnitBytes;   // block idx of the sequence is at sb + idx * 1088
     if (ok && active) {
+#pragma unroll 1
       while (idx < end) {
         const bool two = u + kNCW < nunit && idx + kNCW < end;   // the next unit of the same tile is in this stage too
         float ya2 = 0.f, yb2 = 0.f;
@@ -639,107 +614,175 @@ DEVI void gemv(const Cta& c, const Mat& m, const Slice& s, float* part, int pstr
 #endif
 }
 
-enum : int { OUT_TAGGED = 0, OUT_SWIGLU = 1, OUT_LOGITS = 2 };
-
-// Sum of one row slot over the nwa warps that hold a share of it, always in the same order. With all warps (rows of
-// 1024 weights and more) the loads are issued together and added as a tree: the loop form would make every load
-// wait for the add before it.
+// Sum of one row slot over the nwa warps that hold a share of it, always in the same order: pairs, then the pair sums. The
+// loads are issued together; a loop would make every one wait for the add before it.
 DEVI float sum_partials(const float* p, int pstride, int nwa) {
-  if (nwa == kNCW) {
-    float v[kNCW];
+  float v[kNCW];
 #pragma unroll
-    for (int k = 0; k < kNCW; ++k) v[k] = p[k * pstride];
+  for (int k = 0; k < kNCW; ++k) v[k] = k < nwa ? p[k * pstride] : 0.f;
 #pragma unroll
-    for (int k = 0; k + 1 < kNCW; k += 2) v[k] += v[k + 1];     // pairs, then the pair sums in order
-    float y = v[0];
+  for (int k = 0; k + 1 < kNCW; k += 2) v[k] += v[k + 1];
+  float y = v[0];
 #pragma unroll
-    for (int k = 2; k < kNCW; k += 2) y += v[k];
-    return y;
-  }
-  float y = 0.f;
-  for (int k = 0; k < nwa; ++k) y += p[k * pstride];
+  for (int k = 2; k < kNCW; k += 2) y += v[k];
   return y;
 }
 
 // After the barrier that follows gemv(): thread i adds the warps' partial sums of row slot i in a fixed order
-// (deterministic) and emits the output.
-//   OUT_TAGGED: E[row] <- tagged y.  OUT_SWIGLU: E[i] <- tagged half(silu(gate_i)) * up_i.
-//   OUT_LOGITS: logits[row] <- y, and `best` tracks this thread's maximum.
-DEVI void reduce_emit(const Cta& c, const Mat& m, const Slice& s, const float* part, int pstride, const int OUT,
-                      uint32_t* E, half* logits, unsigned long long& best, int tid) {
+// (deterministic), multiplies by f (the norm's factor, or 1) and emits the output: E[row] <- tagged y; gate|up: E[i] <- tagged half(silu(gate_i)) * up_i.
+DEVI void reduce_emit(const Cta& c, const Mat& m, const Slice& s, const float* part, int pstride, uint32_t* E, float f, int tid) {
   const int nwa = min(kNCW, m.K >> 7);
-  if (OUT == OUT_SWIGLU) {
+  if (m.paired) {
+#pragma unroll 1
     for (int i = tid; i < 8 * s.nt; i += kNT) {
       const int slot = 16 * (i >> 3) + (i & 7), o = 8 * s.t0 + i;
       if (o >= m.N) continue;
       const float ga = sum_partials(part + slot, pstride, nwa), up = sum_partials(part + slot + 8, pstride, nwa);
-      const half h0 = __float2half(ga), h1 = __float2half(up);
+      const half h0 = __float2half(ga * f), h1 = __float2half(up * f);
       const float gf = __half2float(h0);
       const half sl = __float2half(__fdividef(gf, 1.f + __expf(-gf)));
       st_tagged(E + o, c.tagw | (uint32_t)__half_as_ushort(__hmul(sl, h1)));
     }
     return;
   }
+#pragma unroll 1
   for (int i = tid; i < 16 * s.nt; i += kNT) {
     const int row = 16 * s.t0 + i;
-    if (row >= m.N) continue;
-    const half h = __float2half(sum_partials(part + i, pstride, nwa));
-    if (OUT == OUT_TAGGED) {
-      st_tagged(E + row, c.tagw | (uint32_t)__half_as_ushort(h));
-    } else {
-      logits[row] = h;
-      if (!__hisnan(h)) { const unsigned long long key = argmax_key(h, row); best = key > best ? key : best; }
+    if (row < m.N) st_tagged(E + row, c.tagw | (uint32_t)__half_as_ushort(__float2half(sum_partials(part + i, pstride, nwa) * f)));
+  }
+}
+
+// The same for the LM head: logits[row] <- y; returns the largest key of this thread's rows (argmax_key; 0 = none comparable).
+DEVI unsigned long long emit_logits(const Cta& c, const Slice& s, int tid) {
+  const StepParams& p = *c.p;
+  unsigned long long best = 0ull;
+  const int nwa = min(kNCW, p.H >> 7);
+  const float f = norm_factor(c, p.H, p.eps);
+#pragma unroll 1
+  for (int i = tid; i < 16 * s.nt; i += kNT) {
+    const int row = 16 * s.t0 + i;
+    if (row >= p.V) continue;
+    const half h = __float2half(sum_partials(c.part() + i, p.part_stride_head, nwa) * f);
+    p.logits[row] = h;
+    if (!__hisnan(h)) { const unsigned long long key = argmax_key(h, row); best = key > best ? key : best; }
+  }
+  return best;
+}
+
+// ---- attention -------------------------------------------------------------------------------------------------------
+// The cut of a context of `pos` cached tokens: short ones by attention_head, longer ones in slices by attention_group, merged by a CTA
+// per head in one more exchange (~1.3 us), with every CTA taking part. Build-time knobs for measurements: tokens per slice and
+// where the sliced form begins.
+#ifndef B200_STEP_SLICE_TOKENS
+#define B200_STEP_SLICE_TOKENS 128
+#endif
+#ifndef B200_STEP_TWO_MIN
+#define B200_STEP_TWO_MIN 512
+#endif
+DEVI AttPlan att_plan(const StepParams& p, int pos, uint32_t epoch) {
+  AttPlan r;
+  r.two = p.att_max > 1 && pos * p.D >= 64 * B200_STEP_TWO_MIN;   // by the bytes a CTA would copy for one head
+  const int want = (pos + B200_STEP_SLICE_TOKENS - 1) / B200_STEP_SLICE_TOKENS;
+  const int A = r.two ? min(p.att_max, want) : 1;   // one slice: attention_head
+  const int align = max(16, 1 << p.log2P);
+  r.per = max(align, ((pos + A - 1) / A + align - 1) / align * align);
+  r.A = max(1, (pos + r.per - 1) / r.per);   // no slice is empty
+  r.refresh = (epoch & 1023u) == 0;
+  r.pos = pos;
+  r.units = r.two ? p.att_groups * r.A : p.n_q;
+  return r;
+}
+
+// Attention unit u of a layer: heads [h0, h0 + nh) of one kv head, context slice j.
+struct AttUnit { int kvh, h0, nh, j; };
+DEVI AttUnit att_unit(const StepParams& p, int u) {
+  const int hpg = p.n_q / p.n_kv, nsub = (hpg + 7) >> 3, grp = u % p.att_groups, sub = grp % nsub;
+  AttUnit r;
+  r.kvh = grp / nsub;
+  r.h0 = r.kvh * hpg + 8 * sub;
+  r.nh = min(8, hpg - 8 * sub);
+  r.j = u / p.att_groups;
+  return r;
+}
+
+// Where slice j's partials go: the layer's block of the exchange (few slices) or of the wide exchange (two-level form).
+struct AttOut { uint32_t* o; uint32_t* lse; int lsew; };
+DEVI AttOut att_out(const StepParams& p, int layer, bool two) {
+  const int n_att = p.n_q * p.D;
+  AttOut r;
+  r.o = two ? p.att_xchg + (size_t)layer * p.att_layer_words
+            : p.xchg + (size_t)layer * p.layer_words + (p.n_q + 2 * p.n_kv) * p.D;
+  r.lse = r.o + (size_t)(two ? p.att_max : p.att_slices) * n_att;
+  r.lsew = step_lse_words(two ? p.att_max : p.att_slices);
+  return r;
+}
+
+// fp32 value as an fp16 value and the fp16 remainder, tagged
+DEVI void st_lse(const Cta& c, uint32_t* p, float v) {
+  const half hi = __float2half(v), lo = __float2half(v - __half2float(hi));
+  st_tagged2(p, c.tagw | (uint32_t)__half_as_ushort(hi), c.tagw | (uint32_t)__half_as_ushort(lo));
+}
+
+// Every 1024th step: the partial slots this step leaves alone get the current tag (see "tagged exchange words"). CTA h + k ncta
+// does head h.
+__device__ __noinline__ void refresh_partials(const Cta c, int layer) {
+  const StepParams& p = *c.p;
+  const AttPlan pl = c.plan();
+  const int tid = threadIdx.x, n_att = p.n_q * p.D;
+  for (int h = blockIdx.x; h < p.n_q; h += gridDim.x) {
+    for (int two = 0; two < 2; ++two) {
+      const int slots = two ? p.att_max : p.att_slices;
+      if (two && slots <= p.att_slices) break;
+      const AttOut out = att_out(p, layer, two);
+      const int used = two == pl.two ? pl.A : (two ? 0 : 1), used_l = two == pl.two ? pl.A + (pl.A & 1) : 0;
+      for (int i = used * p.D + tid; i < slots * p.D; i += kNT) st_tagged(out.o + (size_t)(i / p.D) * n_att + h * p.D + i % p.D, c.tagw);
+      for (int i = 2 * used_l + tid; i < out.lsew; i += kNT) st_tagged(out.lse + (size_t)h * out.lsew + i, c.tagw);
     }
   }
 }
 
-// ---- attention for one query head, one context slice ------------------------------------------------------------------
-// All consumer threads of the CTA. q, k, v of this step come from the tagged qkv exchange, the cached tokens of slice
-// j (ring stages j, j + J, ... of the context) from ring stages filled by produce_kv; slice 0 also takes the token
-// of this step and writes it to the cache. Lane (t = lane >> 3, c = lane & 7) of warp w owns token slot 4 w + t of a
-// stage and dims [c D/8, (c+1) D/8) of it; each warp keeps a private online-softmax state, merged once at the end.
-// Output: the slice's normalised partial at Eattn + j n_att and its log-sum-exp at Else (see stage_attn).
+// Rows 0-7 of D (16x8, fp32) += A (16x16, fp16, row) * B (16x8, fp16, col); rows 8-15 of A are zero and of D dropped. Lane (g, t):
+// c = D[g][2t, 2t+1], a0 = A[g][2t, 2t+1], a2 = A[g][2t+8, 2t+9].
+DEVI void mma16816_top(float (&c)[2], uint32_t a0, uint32_t a2, uint32_t b0, uint32_t b1) {
+  asm volatile("{\n\t.reg .f32 x, y;\n\t"
+               "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,x,y}, {%2,%6,%3,%6}, {%4,%5}, {%0,%1,%7,%7};\n\t}"
+               : "+f"(c[0]), "+f"(c[1])
+               : "r"(a0), "r"(a2), "r"(b0), "r"(b1), "r"(0u), "f"(0.f));
+}
+DEVI uint4 lds16(uint32_t addr) {
+  uint4 v;
+  asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr));
+  return v;
+}
+
+// ---- short contexts: one CTA per query head -------------------------------------------------------------------------
+// All consumer threads of the CTA. q, k, v of this step come from the tagged qkv exchange, the cached tokens from ring stages
+// filled by produce_kv. Lane (t = lane >> 3, c = lane & 7) of warp w owns token slot 4 w + t of a stage and dims
+// [c D/8, (c+1) D/8) of it, on the fp32 pipes; each warp keeps a private online-softmax state, merged once at the end. Against
+// attention_group: eight times the copies, but a head per CTA is less work on the way from q to the output, and up to a few
+// hundred tokens that way is what counts (TinyLlama shape, context 128: 359 us a token, 376 with the groups).
 template <int D>
-DEVI void attention_head(const Cta& c, const StepParams& p, const StepLayer& ly, uint32_t* E, int u, int pos,
-                         RingPos& rp, int tid, int trace_at) {
-  // E: the layer's exchange block; u: attention unit = head u % n_q, slice u / n_q. Whatever the publishing code at
-  // the end needs is recomputed there from u and the parameter block: the fold loop in between is where this kernel's
-  // register pressure peaks, and every value carried across it costs a register there.
+DEVI void attention_head(const Cta& c, const StepParams& p, const StepLayer& ly, uint32_t* E, int h, RingPos& rp, int tid,
+                         int trace_at) {
   constexpr int D2 = D / 2, G4 = D / 4, DPL = D / 8;
-  const int warp = tid >> 5, lane = tid & 31, ts = lane >> 3, ch = lane & 7;
-  const int J = p.att_slices, h = u % p.n_q, j = u / p.n_q;
-  const int Js = pos >= kSliceMinContext ? J : 1;            // stride of a slice's stages: 1 = slice 0 takes them all
+  const int warp = tid >> 5, lane = tid & 31, ts = lane >> 3, ch = lane & 7, pos = c.plan().pos;
   const int hpg = p.n_q / p.n_kv, kvh = h / hpg;
   const int tps = kv_tokens_per_stage(p);
-  const int nst = (pos + tps - 1) / tps;                       // stages of the whole context
-  const uint32_t* Eqkv = E;
-  if (j > 0 && (j >= nst || Js == 1)) {
-    // no cached token falls into this slice: an empty partial, without touching q, k, v or the ring
-    uint32_t* Eo = E + (size_t)(p.n_q + 2 * p.n_kv) * D + (size_t)j * p.n_q * D + (size_t)h * D;
-    uint32_t* El = E + (size_t)(p.n_q + 2 * p.n_kv) * D + (size_t)J * p.n_q * D + (size_t)h * step_lse_words(J) + 2 * j;
-    const uint32_t ninf = c.tagw | 0xFC00u;                    // fp16 -inf
-    if (tid < D) st_tagged(Eo + tid, c.tagw);
-    if (tid == 0) {
-      st_tagged(El, ninf);
-      st_tagged(El + 1, c.tagw);
-      if ((J & 1) && j == J - 1) { st_tagged(El + 2, ninf); st_tagged(El + 3, c.tagw); }
-    }
-    return;
-  }
-  float* qf = c.att();                                         // [D] rotated q * 1/sqrt(D)
-  half* knew = reinterpret_cast<half*>(c.att() + D);           // [D] rotated k of this step
+  const int nst = (pos + tps - 1) / tps;
+  float* qf = reinterpret_cast<float*>(c.att());              // [D] rotated q * 1/sqrt(D)
+  half* knew = reinterpret_cast<half*>(qf + D);           // [D] rotated k of this step
   half* vnew = knew + D;                                     // [D]
   half* raw = vnew + D;                                      // [3 D] un-rotated q, k, v
-  float* wo = c.att() + 4 * D;                                 // [kNCW][D] per-warp outputs
+  float* wo = qf + 4 * D;                                 // [kNCW][D] per-warp outputs
   float* wm = wo + kNCW * D;                                 // [kNCW] per-warp max
   float* wl = wm + kNCW;                                     // [kNCW] per-warp sum
-  const float* rope = wl + kNCW;                             // [D/2] cos, [D/2] sin, then the page of this step's token
+  const float* rope = c.rope();
   const int pmask = (1 << p.log2P) - 1;
 
   if (tid < 3 * G4) {
     const int which = tid / G4, g = tid % G4;
     const int head = which == 0 ? h : (which == 1 ? p.n_q + kvh : p.n_q + p.n_kv + kvh);
-    reinterpret_cast<uint2*>(raw)[tid] = poll4(c, Eqkv + (size_t)head * D + 4 * g);
+    reinterpret_cast<uint2*>(raw)[tid] = poll4(c, E + (size_t)head * D + 4 * g);
   }
   consumer_sync();
   if (tid < 2 * D) {
@@ -759,13 +802,13 @@ DEVI void attention_head(const Cta& c, const StepParams& p, const StepLayer& ly,
       } else {
         knew[i] = ra;
         knew[i + D2] = rb;
-        if (h % hpg == 0 && j == 0) { ly.kc[row_new + i] = ra; ly.kc[row_new + i + D2] = rb; }
+        if (h % hpg == 0) { ly.kc[row_new + i] = ra; ly.kc[row_new + i + D2] = rb; }
       }
     } else {
       const int i = tid - D;
       const half v = raw[2 * D + i];
       vnew[i] = v;
-      if (h % hpg == 0 && j == 0) ly.vc[row_new + i] = v;
+      if (h % hpg == 0) ly.vc[row_new + i] = v;
     }
   }
   consumer_sync();
@@ -788,7 +831,7 @@ DEVI void attention_head(const Cta& c, const StepParams& p, const StepLayer& ly,
     float s[kKvRounds];
 #pragma unroll
     for (int r = 0; r < kKvRounds; ++r) {
-      const half* kp = reinterpret_cast<const half*>(c.smem + koff[r]);
+      const half* kp = reinterpret_cast<const half*>(step_smem + koff[r]);
       float kf[DPL], a0 = 0.f, a1 = 0.f;
 #pragma unroll
       for (int d8 = 0; d8 < DPL; d8 += 8) unpack8(*reinterpret_cast<const uint4*>(kp + d8), kf + d8);
@@ -814,7 +857,7 @@ DEVI void attention_head(const Cta& c, const StepParams& p, const StepLayer& ly,
     for (int d = 0; d < DPL; ++d) acc[d] *= alpha;
 #pragma unroll
     for (int r = 0; r < kKvRounds; ++r) {
-      const half* vp = reinterpret_cast<const half*>(c.smem + voff[r]);
+      const half* vp = reinterpret_cast<const half*>(step_smem + voff[r]);
       const float pr = __expf(s[r] - mn);      // a masked slot: e^(-inf) = 0
       l += pr;
       float vf[DPL];
@@ -825,19 +868,18 @@ DEVI void attention_head(const Cta& c, const StepParams& p, const StepLayer& ly,
     }
   };
 
-  // The cached tokens come stage by stage from the ring. The token of this step (rotated k, v in the attention
-  // scratch) belongs to slice 0 and rides along as token number nt of that slice's last stage: a stage holds at most
-  // kMaxKvTokens tokens and the warps' slots cover 4 kNCW kKvRounds > kMaxKvTokens, so there is always a slot for it
-  // and it costs no chain of its own.
+  // The cached tokens come stage by stage from the ring. The token of this step (rotated k, v in the attention scratch)
+  // rides along as token number nt of the last stage: a stage holds at most kMaxKvTokens tokens and the warps' slots cover
+  // 4 kNCW kKvRounds > kMaxKvTokens, so there is always a slot for it and it costs no chain of its own.
   static_assert(4 * kNCW * kKvRounds > kMaxKvTokens, "a stage needs a spare slot for the token of this step");
-  const bool takes_new = j == 0;
-  const uint32_t knew_off = (uint32_t)(reinterpret_cast<const uint8_t*>(knew) - c.smem) + ch * DPL * 2;
-  const uint32_t vnew_off = (uint32_t)(reinterpret_cast<const uint8_t*>(vnew) - c.smem) + ch * DPL * 2;
+  const uint32_t knew_off = (uint32_t)(reinterpret_cast<const uint8_t*>(knew) - step_smem) + ch * DPL * 2;
+  const uint32_t vnew_off = (uint32_t)(reinterpret_cast<const uint8_t*>(vnew) - step_smem) + ch * DPL * 2;
 #ifdef B200_STEP_TRACE
   long long waited = 0;
 #endif
-  for (int st = j; st < nst || (nst == 0 && st == 0); st += Js) {  // nst == 0 (empty cache, slice 0): one pass
-    const bool have = st < nst, last = st + Js >= nst;              // without a ring stage
+#pragma unroll 1
+  for (int st = 0; st < nst || (nst == 0 && st == 0); ++st) {   // an empty cache: one pass without a ring stage
+    const bool have = st < nst, last = st + 1 >= nst;
     const int slot = rp.slot;
 #ifdef B200_STEP_TRACE
     const long long w0 = now_ns();
@@ -855,7 +897,7 @@ DEVI void attention_head(const Cta& c, const StepParams& p, const StepLayer& ly,
 #pragma unroll
       for (int r = 0; r < kKvRounds; ++r) {
         const int jt = 4 * warp + ts + 4 * kNCW * r;   // token slot of the stage
-        valid[r] = jt < nt || (takes_new && last && jt == nt);
+        valid[r] = jt < nt || (last && jt == nt);
         koff[r] = jt < nt ? kbase + (uint32_t)jt * (D * 2) : knew_off;
         voff[r] = jt < nt ? vbase + (uint32_t)jt * (D * 2) : vnew_off;
       }
@@ -898,36 +940,296 @@ DEVI void attention_head(const Cta& c, const StepParams& p, const StepLayer& ly,
       o = fmaf(a, wo[w * D + tid], o);
       L = fmaf(a, wl[w], L);
     }
-    const int Jp = p.att_slices, hp = u % p.n_q, jp = u / p.n_q;
-    uint32_t* Eo = E + (size_t)(p.n_q + 2 * p.n_kv) * D + (size_t)jp * p.n_q * D + (size_t)hp * D;
-    uint32_t* El = E + (size_t)(p.n_q + 2 * p.n_kv) * D + (size_t)Jp * p.n_q * D + (size_t)hp * step_lse_words(Jp) + 2 * jp;
-    const uint32_t ninf = c.tagw | 0xFC00u;
-    st_tagged(Eo + tid, c.tagw | (uint32_t)__half_as_ushort(__float2half(o / L)));
-    if (tid == 0) {   // log-sum-exp of the slice as an fp16 value and the fp16 remainder
-      const float lse = M + __logf(L);
-      const half hi = __float2half(lse), lo = __float2half(lse - __half2float(hi));
-      st_tagged(El, c.tagw | (uint32_t)__half_as_ushort(hi));
-      st_tagged(El + 1, c.tagw | (uint32_t)__half_as_ushort(lo));
-      if ((Jp & 1) && jp == Jp - 1) { st_tagged(El + 2, ninf); st_tagged(El + 3, c.tagw); }
+    st_tagged(E + p.n_qkv + (size_t)h * D + tid, c.tagw | (uint32_t)__half_as_ushort(__float2half(o / L)));
+  }
+  stamp(c, trace_at + 2);
+}
+
+// Scratch of attention_group behind Cta::att().
+template <int D>
+struct AttScratch {
+  half q[8][D + 8];              // rotated queries (padded rows)
+  half k[D], v[D];               // rotated k and v of this step
+  float m[kNCW][8], l[kNCW][8];  // per warp and head: running maximum (base-2 units) and sum
+  float o[kNCW][8][65];          // per warp and head: un-normalised output, 64 dims
+};
+
+// All consumer threads of the CTA. q, k, v of this step come from the tagged qkv exchange, the slice's cached tokens from ring
+// stages filled by produce_kv; the last slice also takes the token of this step and writes it to the cache. A block of 16
+// tokens is one warp's work (block b of the slice: warp b mod kNCW), laid out as in paged_attn_mma_kernel: the heads are rows
+// 0-7 of the MMAs; K and V fragments are read from the row-major pages by permuting the contraction index. The probabilities
+// enter the second contraction twice, as fp16 value and as fp16 remainder, so they count with the precision of fp32.
+template <int D>
+DEVI RingPos attention_group(const Cta& c, int layer, int u, RingPos rp, int trace_at) {
+  constexpr int HALVES = D / 64, TEAMS = kNCW / HALVES, CH = D / 32, NB = 8, D2 = D / 2, D4 = D / 4, PG = D / 8;
+  const int tid = threadIdx.x;
+  const StepParams& p = *c.p;
+  const AttPlan& pl = c.plan();   // in shared memory, re-read where it is needed
+  const AttUnit un = att_unit(p, u);
+  const int warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+  AttScratch<D>& sc = *reinterpret_cast<AttScratch<D>*>(c.att());
+  const int t_begin = un.j * pl.per, t_end = min(pl.pos, t_begin + pl.per);
+  const bool takes_new = un.j == pl.A - 1;
+
+  // q of the group's heads (and k, v): a thread takes dims i .. i + 3 and their rotation partners i + D/2 ..
+  if (tid < (un.nh + (takes_new ? 2 : 0)) * PG) {
+    const int which = tid / PG, i = 4 * (tid % PG);
+    const int row = which < un.nh ? un.h0 + which : (which == un.nh ? p.n_q : p.n_q + p.n_kv) + un.kvh;
+    uint2 r[2];
+    poll_many<2>(c, p.xchg + (size_t)layer * p.layer_words + (size_t)row * D + i, D2, 2, r);
+    if (which <= un.nh) {
+      const float4 cs = *reinterpret_cast<const float4*>(c.rope() + i), sn = *reinterpret_cast<const float4*>(c.rope() + D2 + i);
+      const float2 a0 = __half22float2(as_h2(r[0].x)), a1 = __half22float2(as_h2(r[0].y));
+      const float2 b0 = __half22float2(as_h2(r[1].x)), b1 = __half22float2(as_h2(r[1].y));
+      r[0].x = as_u32(__floats2half2_rn(a0.x * cs.x - b0.x * sn.x, a0.y * cs.y - b0.y * sn.y));
+      r[0].y = as_u32(__floats2half2_rn(a1.x * cs.z - b1.x * sn.z, a1.y * cs.w - b1.y * sn.w));
+      r[1].x = as_u32(__floats2half2_rn(b0.x * cs.x + a0.x * sn.x, b0.y * cs.y + a0.y * sn.y));
+      r[1].y = as_u32(__floats2half2_rn(b1.x * cs.z + a1.x * sn.z, b1.y * cs.w + a1.y * sn.w));
+    }
+    half* dst = which < un.nh ? sc.q[which] : (which == un.nh ? sc.k : sc.v);
+    *reinterpret_cast<uint2*>(dst + i) = r[0];
+    *reinterpret_cast<uint2*>(dst + D2 + i) = r[1];
+    if (which >= un.nh && un.h0 == un.kvh * (p.n_q / p.n_kv)) {   // one unit of the kv head appends the row
+      const int page = reinterpret_cast<const int*>(c.rope())[D], slot = pl.pos & ((1 << p.log2P) - 1);
+      half* row_new = (which == un.nh ? c.layer(layer).kc : c.layer(layer).vc) + ((((size_t)page * p.n_kv + un.kvh) << p.log2P) + slot) * D;
+      *reinterpret_cast<uint2*>(row_new + i) = r[0];
+      *reinterpret_cast<uint2*>(row_new + D2 + i) = r[1];
+    }
+  }
+  consumer_sync();
+  stamp(c, trace_at);
+
+  const float sl2 = 1.44269504088896340736f * rsqrtf((float)D);   // scores in base-2 units
+  // head_dim 128: two warps share a block's scores and take 64 output dims each (32 accumulators more would spill)
+  const int team = warp / HALVES, dim0 = 64 * (warp % HALVES);
+  float m = -CUDART_INF_F, l = 0.f, acc[NB][2];
+#pragma unroll
+  for (int n = 0; n < NB; ++n) acc[n][0] = acc[n][1] = 0.f;
+
+  const uint32_t qaddr = smem_u32(&sc.q[g][t * D4]), kaddr = smem_u32(sc.k), vaddr = smem_u32(sc.v);
+  const int tps = kv_tokens_per_stage(p), bps = tps >> 4;   // tokens and blocks per stage
+  int bid = 0, nblk = 0;                                     // first block of the stage mod kNCW; blocks of the slice
+#ifdef B200_STEP_TRACE
+  long long waited = 0;
+#endif
+#pragma unroll 1
+  for (int t0 = t_begin; t0 < t_end || nblk == 0; t0 += tps) {   // an empty cache: one pass without a ring stage
+    const bool have = t0 < t_end, last = t0 + tps >= t_end;
+    const int slot = rp.slot;
+#ifdef B200_STEP_TRACE
+    const long long w0 = now_ns();
+#endif
+    const bool ok = have ? wait_bar(c, c.full(slot), rp.parity, ERR_FULL) : true;
+#ifdef B200_STEP_TRACE
+    waited += now_ns() - w0;
+#endif
+    const int nt = have ? min(tps, t_end - t0) : 0, ntot = nt + (takes_new && last ? 1 : 0);   // the new token rides behind the last one
+    const uint32_t kst = smem_u32(c.stage(slot)), vst = kst + (uint32_t)(tps * D * 2);
+    int b = team - bid;
+    if (b < 0) b += TEAMS;
+    if (ok && 16 * b < ntot && team < TEAMS) {   // a stage holds at most TEAMS blocks (and one token): one per team
+      const int tok0 = 16 * b;
+      float s[2][2];
+#pragma unroll
+      for (int nb = 0; nb < 2; ++nb) s[nb][0] = s[nb][1] = 0.f;
+      {
+        // a row past the stage's tokens: this step's own (finite; masked unless it is its turn)
+        const int j0 = tok0 + g, j1 = j0 + 8;
+        const uint32_t k0 = (j0 < nt ? kst + j0 * (2 * D) : kaddr) + t * (2 * D4), k1 = (j1 < nt ? kst + j1 * (2 * D) : kaddr) + t * (2 * D4);
+#pragma unroll
+        for (int ch = 0; ch < CH; ++ch) {   // k-steps 2 ch and 2 ch + 1: dims t D/4 + 8 ch + {0 .. 3 | 4 .. 7}; row g = head g, zero beyond the group
+          uint4 q4 = lds16(qaddr + 16 * ch);
+          if (g >= un.nh) q4 = make_uint4(0u, 0u, 0u, 0u);
+          const uint4 ka = lds16(k0 + 16 * ch), kb = lds16(k1 + 16 * ch);
+          mma16816_top(s[0], q4.x, q4.y, ka.x, ka.y);
+          mma16816_top(s[1], q4.x, q4.y, kb.x, kb.y);
+          mma16816_top(s[0], q4.z, q4.w, ka.z, ka.w);
+          mma16816_top(s[1], q4.z, q4.w, kb.z, kb.w);
+        }
+      }
+      float pr[4];   // head g, tokens tok0 + 8 nb + 2 t + {0, 1}
+#pragma unroll
+      for (int nb = 0; nb < 2; ++nb)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) pr[2 * nb + e] = tok0 + 8 * nb + 2 * t + e < ntot ? s[nb][e] * sl2 : -CUDART_INF_F;
+      float mx = fmaxf(fmaxf(pr[0], pr[1]), fmaxf(pr[2], pr[3]));
+      mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+      mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+      const float mn = fmaxf(m, mx), alpha = exp2f(m - mn);   // finite: token tok0 counts
+      m = mn;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) pr[e] = exp2f(pr[e] - mn);
+      l = fmaf(l, alpha, (pr[0] + pr[1]) + (pr[2] + pr[3]));
+#pragma unroll
+      for (int n = 0; n < NB; ++n) acc[n][0] *= alpha, acc[n][1] *= alpha;
+      const half2 h01 = __floats2half2_rn(pr[0], pr[1]), h23 = __floats2half2_rn(pr[2], pr[3]);
+      const float2 f01 = __half22float2(h01), f23 = __half22float2(h23);
+      const uint32_t hi0 = as_u32(h01), hi2 = as_u32(h23);
+      const uint32_t lo0 = as_u32(__floats2half2_rn(pr[0] - f01.x, pr[1] - f01.y)), lo2 = as_u32(__floats2half2_rn(pr[2] - f23.x, pr[3] - f23.y));
+      uint32_t vr[4];   // V rows of tokens 2t, 2t + 1, 2t + 8, 2t + 9
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int jt = tok0 + 2 * t + (e & 1) + 8 * (e >> 1);
+        vr[e] = (jt < nt ? vst + jt * (2 * D) : vaddr) + 16 * g + 2 * dim0;
+      }
+      {
+        const uint4 v0 = lds16(vr[0]), v1 = lds16(vr[1]), v2 = lds16(vr[2]), v3 = lds16(vr[3]);
+        const uint32_t w0[4] = {v0.x, v0.y, v0.z, v0.w}, w1[4] = {v1.x, v1.y, v1.z, v1.w};
+        const uint32_t w2[4] = {v2.x, v2.y, v2.z, v2.w}, w3[4] = {v3.x, v3.y, v3.z, v3.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            const uint32_t sel = e ? 0x7632u : 0x5410u, b0 = __byte_perm(w0[i], w1[i], sel), b1 = __byte_perm(w2[i], w3[i], sel);
+            mma16816_top(acc[2 * i + e], hi0, hi2, b0, b1);
+            mma16816_top(acc[2 * i + e], lo0, lo2, b0, b1);
+          }
+      }
+    }
+    nblk += (ntot + 15) >> 4;
+    bid += bps;
+    while (bid >= TEAMS) bid -= TEAMS;
+    if (have) {
+      __syncwarp();
+      if (lane == 0) mbar_arrive(c.empty(slot));
+      advance(rp, c.p->ns);
+    }
+  }
+  stamp(c, trace_at + 1);
+#ifdef B200_STEP_TRACE
+  stamp_value(c, trace_at + 4, waited);   // a duration: what warp 0 waited for the K/V stages
+#endif
+
+  // merge the teams: acc[n][e] = O[head g][dim0 + 8 (2 t + e) + n]
+  const int nw = min(TEAMS, nblk);
+  l += __shfl_xor_sync(0xffffffffu, l, 1);
+  l += __shfl_xor_sync(0xffffffffu, l, 2);
+  if (team < nw) {
+    if (t == 0) sc.m[warp][g] = m, sc.l[warp][g] = l;
+#pragma unroll
+    for (int n = 0; n < NB; ++n)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) sc.o[warp][g][8 * (2 * t + e) + n] = acc[n][e];
+  }
+  consumer_sync();
+  const AttOut out = att_out(p, layer, pl.two);
+#pragma unroll 1
+  for (int i = tid; i < un.nh * D2; i += kNT) {
+    const int h = i / D2, d = 2 * (i % D2), w0 = d / 64;   // warps w0, w0 + HALVES, ... hold these dims
+    float f[TEAMS], M = -CUDART_INF_F, L = 0.f, o0 = 0.f, o1 = 0.f;   // unrolled: the teams' loads are in flight together
+#pragma unroll
+    for (int k = 0; k < TEAMS; ++k) {
+      f[k] = k < nw ? sc.m[k * HALVES][h] : -CUDART_INF_F;
+      M = fmaxf(M, f[k]);
+    }
+#pragma unroll
+    for (int k = 0; k < TEAMS; ++k) {
+      if (k < nw) {
+        const float w = exp2f(f[k] - M);
+        o0 = fmaf(w, sc.o[k * HALVES + w0][h][d % 64], o0);
+        o1 = fmaf(w, sc.o[k * HALVES + w0][h][d % 64 + 1], o1);
+        L = fmaf(w, sc.l[k * HALVES][h], L);
+      }
+    }
+    const float r = 1.f / L;
+    st_tagged2(out.o + (size_t)un.j * (p.n_q * D) + (size_t)(un.h0 + h) * D + d, c.tagw | (uint32_t)__half_as_ushort(__float2half(o0 * r)),
+               c.tagw | (uint32_t)__half_as_ushort(__float2half(o1 * r)));
+    if (d == 0) {
+      uint32_t* lp = out.lse + (size_t)(un.h0 + h) * out.lsew + 2 * un.j;
+      st_lse(c, lp, M + __log2f(L));
+      if ((pl.A & 1) && un.j == pl.A - 1) st_tagged2(lp + 2, c.tagw | 0xFC00u, c.tagw);   // the other half of the last granule: -inf
     }
   }
   stamp(c, trace_at + 2);
+  return rp;   // the caller's barrier comes before the scratch is used again
+}
+
+// Two-level form: the attention output of head h from its A slices, by all consumer threads of one CTA. Thread (dims 4 k .. 4 k + 3,
+// row s) folds slices s, s + rows, ...; the rows meet in shared memory.
+template <int D>
+DEVI void merge_head(const Cta& c, int layer, int h) {
+  constexpr int G = D / 4, ROWS = kNT / G;
+  const int tid = threadIdx.x;
+  const StepParams& p = *c.p;
+  const int A = c.plan().A, k = tid % G, row = tid / G, n_att = p.n_q * D;
+  const AttOut in = att_out(p, layer, true);
+  float* acc_s = reinterpret_cast<float*>(c.att());   // [ROWS][D]
+  float* m_s = acc_s + ROWS * D;                      // [ROWS] maximum, [ROWS] weight
+  float M = -CUDART_INF_F, W = 0.f, o[4] = {0.f, 0.f, 0.f, 0.f};
+  if (row < ROWS) {
+#pragma unroll 1
+    for (int j = row; j < A; j += 2 * ROWS) {
+      const int j2 = j + ROWS;
+      const uint32_t mask = j2 < A ? 15u : 5u;
+      uint32_t off[4];
+      off[0] = (uint32_t)(j * n_att + h * D + 4 * k);
+      off[1] = (uint32_t)(j2 * n_att + h * D + 4 * k);
+      off[2] = (uint32_t)(in.lse - in.o) + (uint32_t)(h * in.lsew + 4 * (j >> 1));
+      off[3] = (uint32_t)(in.lse - in.o) + (uint32_t)(h * in.lsew + 4 * (j2 >> 1));
+      uint2 v[4];
+      poll_list<4>(c, in.o, off, mask, v);
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        if (e && j2 >= A) break;
+        const float2 f = __half22float2(as_h2(((e ? j2 : j) & 1) ? v[2 + e].y : v[2 + e].x));
+        const float2 x01 = __half22float2(as_h2(v[e].x)), x23 = __half22float2(as_h2(v[e].y));
+        const float lse = f.x + f.y, Mn = fmaxf(M, lse), a = exp2f(M - Mn), w = exp2f(lse - Mn);
+        W = fmaf(W, a, w);
+        o[0] = fmaf(o[0], a, w * x01.x), o[1] = fmaf(o[1], a, w * x01.y);
+        o[2] = fmaf(o[2], a, w * x23.x), o[3] = fmaf(o[3], a, w * x23.y);
+        M = Mn;
+      }
+    }
+    *reinterpret_cast<float4*>(acc_s + row * D + 4 * k) = make_float4(o[0], o[1], o[2], o[3]);
+    if (k == 0) m_s[row] = M, m_s[ROWS + row] = W;
+  }
   consumer_sync();
+  if (tid < D) {
+    float Mx = -CUDART_INF_F, Wt = 0.f, y = 0.f;
+    const int rows = min(ROWS, A);
+    for (int r = 0; r < rows; ++r) Mx = fmaxf(Mx, m_s[r]);
+#pragma unroll 4
+    for (int r = 0; r < rows; ++r) {
+      const float f = exp2f(m_s[r] - Mx);
+      Wt = fmaf(f, m_s[ROWS + r], Wt);
+      y = fmaf(f, acc_s[r * D + tid], y);
+    }
+    st_tagged(att_out(p, layer, false).o + (size_t)h * D + tid, c.tagw | (uint32_t)__half_as_ushort(__float2half(y / Wt)));
+  }
+}
+
+// The sliced form, all of a layer's work of this CTA. Not inlined: it would take registers from the loop that serves every phase of
+// the step. False: the step is aborting.
+struct AttDone { RingPos rp; bool ok; };
+template <int D>
+__device__ __noinline__ AttDone attention_sliced(const Cta c, int layer, RingPos rp, int trace_at) {
+  const StepParams& p = *c.p;
+#pragma unroll 1
+  for (int u = blockIdx.x; u < c.plan().units; u += gridDim.x) {
+    rp = attention_group<D>(c, layer, u, rp, trace_at);
+    if (consumer_sync_or(*c.abort())) return AttDone{rp, false};
+  }
+  // the merging CTAs counted from the far end: they are the first to have no second unit
+#pragma unroll 1
+  for (int h = gridDim.x - 1 - blockIdx.x; h < p.n_q; h += gridDim.x) {
+    merge_head<D>(c, layer, h);
+    if (consumer_sync_or(*c.abort())) return AttDone{rp, false};
+  }
+  return AttDone{rp, true};
 }
 
 }  // namespace
 
 // ---- the kernel ------------------------------------------------------------------------------------------------------
-template <int D>
+template <int D, bool WIDE>
 __global__ void __launch_bounds__(kThreads, 1) decode_step_kernel(const __grid_constant__ StepParams p) {
-  extern __shared__ __align__(128) uint8_t smem[];
+  uint8_t* smem = step_smem;
   Cta c;
-  c.smem = smem;
   c.p = &p;
   // the per-layer pointer table, copied once from global memory: every phase starts from these pointers, and a
   // global load in front of each would put an L2 round trip on the critical path ~10 times per layer
   StepLayer* lys = reinterpret_cast<StepLayer*>(smem + p.off_table);
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int cta = blockIdx.x, ncta = gridDim.x;
 
   if (tid == 0) {
@@ -935,12 +1237,11 @@ __global__ void __launch_bounds__(kThreads, 1) decode_step_kernel(const __grid_c
     *c.abort() = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  const int n_qkv = (p.n_q + 2 * p.n_kv) * p.D, n_att = p.n_q * p.D;
   // This CTA's tiles of the five matrix shapes of a step (qkv, o, gate|up, down, head): computed once (they involve
   // integer divisions) and kept in shared memory for producer and consumers.
   Slice* sl = reinterpret_cast<Slice*>(smem + 512);
   if (tid < 5) {
-    const int rows = tid == 0 ? n_qkv : (tid == 2 ? p.I : (tid == 4 ? p.V : p.H));
+    const int rows = tid == 0 ? p.n_qkv : (tid == 2 ? p.I : (tid == 4 ? p.V : p.H));
     sl[tid] = slice_of(rows, tid == 2, cta, ncta);
   }
   {
@@ -948,40 +1249,30 @@ __global__ void __launch_bounds__(kThreads, 1) decode_step_kernel(const __grid_c
     uint4* dst = reinterpret_cast<uint4*>(lys);
     for (int i = tid; i < p.L * (int)(sizeof(StepLayer) / 16); i += kThreads) dst[i] = __ldg(src + i);
   }
-  __syncthreads();
   const uint32_t epoch = ((volatile StepCtrl*)p.ctrl)->epoch + 1u;
   c.tagw = ((epoch % 65535u) + 1u) << 16;
   const int pos = p.pos[0];
-  const int hpg = p.n_q / p.n_kv;
-  // Context slices per query head in attention (the exchange layout always has room for J). Slicing pays from about
-  // 1200 cached tokens on: below that the K/V copies of 96 more CTAs delay the weight stream (an SM's copy engine takes
-  // ~1 us for the 16 page copies of a stage) and the merge costs the o projection's staging a second trip through
-  // the L2, which together outweigh a fold that is shorter by one or two stages. In a step below the threshold slice
-  // 0 takes the whole context and the others publish empty partials (every exchange word is rewritten in every
-  // step - the tag invariant - but nobody waits for these). Every CTA reads the same pos, so all agree.
-  const int J = p.att_slices;
-  const bool sliced = pos >= kSliceMinContext && J > 1;
-  const int per_layer = (int)step_words_per_layer(p.H, p.I, p.n_q, p.n_kv, p.D, J);   // exchange words per layer
-
+  if (tid == 64) *reinterpret_cast<AttPlan*>(smem + 640) = att_plan(p, pos, epoch);
+  __syncthreads();
   if (warp == kNCW) {
     // ================= producer =================
-    RingPos rp = {0, 1u, 0};   // parity 1: the first pass over a fresh `empty` barrier does not wait
-    for (int l = 0; l < p.L && !*c.abort(); ++l) {
-      const StepLayer& ly = lys[l];
-      const Mat mats[4] = {{(const uint8_t*)ly.w[0], n_qkv, p.H, 0},
-                           {(const uint8_t*)ly.w[1], p.H, n_att, 0},
-                           {(const uint8_t*)ly.w[2], p.I, p.H, 1},
-                           {(const uint8_t*)ly.w[3], p.H, p.I, 0}};
-      produce(c, mats[0], sl[0], rp, lane);
-      for (int u = cta; u < p.n_q * J && !*c.abort(); u += ncta)   // attention unit u: head u % n_q, slice u / n_q
-        if (sliced || u < p.n_q) produce_kv(c, p, ly, (u % p.n_q) / hpg, u / p.n_q, sliced ? J : 1, pos, rp, lane);
-#pragma unroll
-      for (int k = 1; k < 4; ++k)
-        if (!*c.abort()) produce(c, mats[k], sl[k], rp, lane);
-    }
-    if (!*c.abort()) {
-      const Mat head = {(const uint8_t*)p.w_head, p.V, p.H, 0};
-      produce(c, head, sl[4], rp, lane);
+    ProducerPos rp;            // parity 1: the first pass over a fresh `empty` barrier does not wait
+    rp.slot = 0, rp.parity = 1u, rp.count = 0;
+    // one copy of the code for all matrices: it shares the instruction cache with the consumers
+#pragma unroll 1
+    for (int step = 0; step <= 4 * p.L && !*c.abort(); ++step) {
+      const int l = step >> 2, k = step & 3;
+      const bool head = l == p.L;
+      const StepLayer& ly = lys[head ? 0 : l];
+      produce(c, head ? (const uint8_t*)p.w_head : (const uint8_t*)ly.w[k], (k == 1 ? p.n_att : (k == 3 ? p.I : p.H)) >> 7,
+              sl[head ? 4 : k], rp, lane);
+      if (k == 0 && !head)
+        for (int u = cta; u < c.plan().units && !*c.abort(); u += ncta) {
+          const bool two = c.plan().two;
+          const AttUnit un = att_unit(p, u);
+          const int t0 = two ? un.j * c.plan().per : 0;
+          produce_kv(c, p, ly, two ? un.kvh : u / (p.n_q / p.n_kv), t0, min(c.plan().pos, t0 + c.plan().per), rp, lane);
+        }
     }
     // Leave only when every copy issued has landed. On the normal path the consumers have waited on every full
     // barrier already; on abort, wait (bounded) for the full barriers of the stages still in the ring.
@@ -1005,12 +1296,11 @@ __global__ void __launch_bounds__(kThreads, 1) decode_step_kernel(const __grid_c
   c.tr = p.trace ? p.trace + (size_t)cta * (kTraceHead + kTracePerLayer * (p.L + 1)) : nullptr;
 #endif
   stamp(c, 0);
-  RingPos rp = {0, 0u, 0};
-  unsigned long long best = 0ull;
+  RingPos rp = {0, 0u};
   // RoPE factors and the page of this step's token depend only on pos: the attention CTAs fetch them now, off the
-  // critical path, into the attention scratch (first read two barriers into the first attention phase)
-  if (cta < p.n_q * J) {
-    float* rope = c.att() + 4 * p.D + kNCW * p.D + 2 * kNCW;
+  // critical path (first read behind the barriers of the first GEMV)
+  if (cta < c.plan().units) {
+    float* rope = c.rope();
     if (tid < (p.D >> 1)) {
       rope[tid] = p.cos_t[(size_t)pos * (p.D >> 1) + tid];
       rope[(p.D >> 1) + tid] = p.sin_t[(size_t)pos * (p.D >> 1) + tid];
@@ -1022,31 +1312,33 @@ __global__ void __launch_bounds__(kThreads, 1) decode_step_kernel(const __grid_c
   const Mat head = {(const uint8_t*)p.w_head, p.V, p.H, 0};
 #pragma unroll 1
   for (int step = 0; step <= 4 * p.L; ++step) {
+    // Forget what is derived from these between phases: lane constants of the GEMV code would otherwise be kept in
+    // registers through attention, and the kernel would spill.
+    asm volatile("" : "+r"(tid), "+r"(warp), "+r"(lane));
     const int l = step >> 2, ph = step & 3;
     const bool is_head = l == p.L;
     const StepLayer& ly = lys[is_head ? 0 : l];
-    uint32_t* E = p.xchg + (size_t)l * per_layer;
-    uint32_t *Eqkv = E, *Eatt = E + n_qkv, *Else = Eatt + (size_t)J * n_att;
-    uint32_t *Eo = Else + p.n_q * step_lse_words(J), *Eact = Eo + p.H, *Edown = Eact + p.I;
+    uint32_t* E = p.xchg + (size_t)l * p.layer_words;
+    uint32_t *Eqkv = E, *Eatt = E + p.n_qkv, *Else = Eatt + (size_t)p.att_slices * p.n_att;
+    uint32_t *Eo = Else + p.n_q * step_lse_words(p.att_slices), *Eact = Eo + p.H, *Edown = Eact + p.I;
     Mat m;
     const uint32_t* Ein;
     const half* nw = nullptr;   // norm weight: non-null selects "residual add + RMSNorm" staging
     uint32_t* Eout;
-    int out = OUT_TAGGED, n_in = p.H;
+    int n_in = p.H;
     if (ph == 0) {
       Ein = l == 0 ? nullptr : E - p.H;   // down of the previous layer: the last H words of its block
       nw = is_head ? p.norm_f : ly.ln1;
-      m = is_head ? head : Mat{(const uint8_t*)ly.w[0], n_qkv, p.H, 0};
+      m = is_head ? head : Mat{(const uint8_t*)ly.w[0], p.n_qkv, p.H, 0};
       Eout = Eqkv;
-      out = is_head ? OUT_LOGITS : OUT_TAGGED;
     } else if (ph == 1) {
-      Ein = Eatt; n_in = n_att;
-      m = Mat{(const uint8_t*)ly.w[1], p.H, n_att, 0};
+      Ein = Eatt; n_in = p.n_att;
+      m = Mat{(const uint8_t*)ly.w[1], p.H, p.n_att, 0};
       Eout = Eo;
     } else if (ph == 2) {
       Ein = Eo; nw = ly.ln2;
       m = Mat{(const uint8_t*)ly.w[2], p.I, p.H, 1};
-      Eout = Eact; out = OUT_SWIGLU;
+      Eout = Eact;
     } else {
       Ein = Eact; n_in = p.I;
       m = Mat{(const uint8_t*)ly.w[3], p.H, p.I, 0};
@@ -1069,11 +1361,10 @@ __global__ void __launch_bounds__(kThreads, 1) decode_step_kernel(const __grid_c
         }
         emb_row = p.emb + (size_t)tok_in * p.H;
       }
-      stage_norm(c, Ein, emb_row, nw, n_in, p.eps, warp, lane);
+      stage_norm<WIDE ? kWideBatchNorm : kBatchNorm>(c, Ein, emb_row, nw, n_in, warp, lane);
     }
     else if (s.nt > 0) {
-      if (ph == 1 && sliced) stage_attn(c, Eatt, Else, J, n_att, p.D, warp, lane);
-      else stage_plain(c, Ein, n_in, warp, lane);   // one slice: its normalised output is the attention output
+      stage_plain<WIDE ? kWideBatch : kBatch>(c, Ein, n_in, warp, lane);
     }
     const int tr_at = kTraceHead + kTracePerLayer * l + kTracePerPhase * ph;
     stamp(c, tr_at);
@@ -1081,19 +1372,29 @@ __global__ void __launch_bounds__(kThreads, 1) decode_step_kernel(const __grid_c
     stamp(c, tr_at + 2);
     if (consumer_sync_or(*c.abort())) return;
     stamp(c, tr_at + 3);
-    reduce_emit(c, m, s, part, pstride, out, Eout, p.logits, best, tid);
-    stamp(c, tr_at + 4);
     if (is_head) break;
+    reduce_emit(c, m, s, part, pstride, Eout, nw ? norm_factor(c, p.H, p.eps) : 1.f, tid);
+    stamp(c, tr_at + 4);
     if (ph == 0) {
-      for (int u = cta; u < p.n_q * J; u += ncta) {
-        attention_head<D>(c, p, ly, E, u, pos, rp, tid, kTraceHead + kTracePerLayer * l + 4 * kTracePerPhase);
-        if (consumer_sync_or(*c.abort())) return;
+      if (c.plan().refresh) refresh_partials(c, l);
+      const int tr_att = kTraceHead + kTracePerLayer * l + 4 * kTracePerPhase;
+      if (c.plan().two) {
+        const AttDone d = attention_sliced<D>(c, l, rp, tr_att);
+        if (!d.ok) return;
+        rp = d.rp;
+      } else {
+        for (int u = cta; u < p.n_q; u += ncta) {
+          attention_head<D>(c, p, ly, E, u, rp, tid, tr_att);
+          if (consumer_sync_or(*c.abort())) return;
+        }
       }
       stamp(c, kTraceHead + kTracePerLayer * l + 4 * kTracePerPhase + 3);
     }
   }
   // this CTA's candidate: max over its threads' keys
-  unsigned long long* keys = reinterpret_cast<unsigned long long*>(c.att());
+  unsigned long long best = emit_logits(c, sl[4], tid);
+  stamp(c, kTraceHead + kTracePerLayer * p.L + 4);
+  unsigned long long* keys = c.keys();
   {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -1104,7 +1405,7 @@ __global__ void __launch_bounds__(kThreads, 1) decode_step_kernel(const __grid_c
   if (lane == 0) keys[warp] = best;
   if (consumer_sync_or(*c.abort())) return;
   stamp(c, 1);
-  uint32_t* Earg = p.xchg + (size_t)p.L * per_layer;   // [ncta][4] words: idx low 16, idx high 16, value key, valid
+  uint32_t* Earg = p.xchg + (size_t)p.L * p.layer_words;   // [ncta][4] words: idx low 16, idx high 16, value key, valid
   if (tid == 0) {
     unsigned long long b = 0ull;
     for (int k = 0; k < kNCW; ++k) b = keys[k] > b ? keys[k] : b;
@@ -1145,15 +1446,19 @@ __global__ void __launch_bounds__(kThreads, 1) decode_step_kernel(const __grid_c
   }
 }
 
-// Lays the fixed areas out behind the header (sizes in, offsets out); returns where the ring starts.
-size_t decode_step_plan_smem(StepParams& p, int resid_bytes, int xin_bytes, int xsum_bytes, int att_bytes,
-                             int part_bytes, int table_bytes) {
+// Lays the fixed areas out behind the header (sizes in, offsets out); returns where the ring starts. The attention scratch shares
+// the activations' area where that is large enough: a GEMV's x is dead when attention runs and the other way round.
+size_t decode_step_plan_smem(StepParams& p, int resid_bytes, int xin_bytes, int xsum_bytes, int part_bytes, int table_bytes) {
+  const int att_bytes = p.D == 64 ? (int)sizeof(AttScratch<64>) : (int)sizeof(AttScratch<128>);
+  static_assert(sizeof(AttScratch<64>) >= (kNT / 16 * 64 + 2 * (kNT / 16)) * 4 && sizeof(AttScratch<128>) >= (kNT / 32 * 128 + 2 * (kNT / 32)) * 4,
+                "merge_head works in the same scratch");
+  const bool shared = xin_bytes >= att_bytes;
   p.off_xin = kHeaderBytes + resid_bytes;
   p.off_xsum = p.off_xin + xin_bytes;
-  p.off_att = p.off_xsum + xsum_bytes;
-  p.off_part = p.off_att + att_bytes;
+  p.off_part = p.off_xsum + xsum_bytes;
   p.off_table = p.off_part + part_bytes;
-  p.off_ring = p.off_table + table_bytes;
+  p.off_att = shared ? p.off_xin : p.off_table + table_bytes;
+  p.off_ring = p.off_table + table_bytes + (shared ? 0 : (att_bytes + 127) / 128 * 128);
   return (size_t)p.off_ring;
 }
 int decode_step_threads() { return kThreads; }
@@ -1162,18 +1467,13 @@ int decode_step_consumer_warps() { return kNCW; }
 int decode_step_max_kv_tokens() { return kMaxKvTokens; }
 
 cudaError_t decode_step_launch(const StepParams& p, int grid, size_t smem, cudaStream_t st) {
-  // the shared-memory limit of a kernel is a per-device attribute
-  static bool configured[64] = {};
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
+  const int kmax = p.H > p.I ? (p.H > p.n_att ? p.H : p.n_att) : (p.I > p.n_att ? p.I : p.n_att);
+  const bool wide = kmax > 128 * kNCW * kWideUnits;
+  auto kern = p.D == 64 ? (wide ? decode_step_kernel<64, true> : decode_step_kernel<64, false>)
+                        : (wide ? decode_step_kernel<128, true> : decode_step_kernel<128, false>);
+  static size_t allowed[4][kMaxDevices] = {};
+  const cudaError_t e = allow_dynamic_smem(kern, smem, allowed[2 * (p.D == 128) + wide]);
   if (e != cudaSuccess) return e;
-  if (dev < 0 || dev >= 64 || !configured[dev]) {
-    e = cudaFuncSetAttribute(decode_step_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(decode_step_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-    if (e != cudaSuccess) return e;
-    if (dev >= 0 && dev < 64) configured[dev] = true;
-  }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(kThreads);
@@ -1184,8 +1484,7 @@ cudaError_t decode_step_launch(const StepParams& p, int grid, size_t smem, cudaS
   attr[0].val.cooperative = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return p.D == 64 ? cudaLaunchKernelEx(&cfg, decode_step_kernel<64>, p)
-                   : cudaLaunchKernelEx(&cfg, decode_step_kernel<128>, p);
+  return cudaLaunchKernelEx(&cfg, kern, p);
 }
 
 }  // namespace b200

@@ -28,6 +28,7 @@ struct StepCtrl {
 struct StepParams {
   const StepLayer* layers;
   int L, H, I, n_q, n_kv, D, V, log2G, log2P;
+  int n_qkv, n_att;   // (n_q + 2 n_kv) D, n_q D
   float eps;
   const half* emb;
   const half* norm_f;
@@ -50,13 +51,17 @@ struct StepParams {
   int stage_bytes, ns;   // stage pitch and number of stages of the ring
   int part_stride;       // row slots per warp in a partial-sum buffer of the layer phases (two buffers)
   int part_stride_head;  // the same for the LM head (one buffer over the same area)
-  int att_slices;        // J: context slices per query head in attention (step_att_slices)
+  int att_slices;        // J: partial attention outputs per query head a layer's exchange block has room for (step_att_slices)
+  int att_groups;        // attention units per slice: kv heads x groups of up to 8 query heads
+  int att_max;           // slices the wide attention exchange has room for (0: there is none)
+  int layer_words, att_layer_words;   // exchange words of a layer: step_words_per_layer, step_att_words_per_layer
+  uint32_t* att_xchg;    // wide attention exchange, step_att_words_per_layer words per layer
 };
 
-// Attention of the step: query head h is worked on by J CTAs, slice j taking the ring stages j, j + J, ... of the
-// cached context; J = as many as the grid has CTAs for, at most kStepMaxAttSlices. Each slice publishes a normalised
-// partial output and its log-sum-exp (two fp16 words: value and remainder); the CTAs that stage the attention output
-// for the o projection merge the J partials while they stage.
+// Attention of the step: a unit of work is one kv head (at most 8 of its query heads) and one slice of the context. Each slice
+// publishes, per query head, a normalised partial output and its log-sum-exp (two fp16 words: value and remainder). A layer's
+// exchange block has room for J = at most kStepMaxAttSlices of them, which the CTAs that stage the attention output merge; the
+// wide attention exchange has room for as many as the grid has CTAs per group, merged by one CTA per head.
 #ifndef B200_STEP_MAX_SLICES
 #define B200_STEP_MAX_SLICES 4   // build-time knob for measurements: 1 = one CTA per query head
 #endif
@@ -67,13 +72,21 @@ inline int step_att_slices(int grid, int n_q) {
 }
 // exchange words per query head for the log-sum-exps: pairs (value, remainder) per slice, padded to whole granules
 __host__ __device__ inline int step_lse_words(int J) { return (2 * J + 3) & ~3; }
+inline int step_att_groups(int n_q, int n_kv) { return n_kv * ((n_q / n_kv + 7) / 8); }
+inline int step_att_max(int grid, int n_q, int n_kv) {
+  const int j = grid / step_att_groups(n_q, n_kv);
+  return j > 64 ? 64 : j;
+}
+// words of one layer in the wide attention exchange
+__host__ __device__ inline size_t step_att_words_per_layer(int n_q, int D, int slices) {
+  return (size_t)slices * n_q * D + (size_t)n_q * step_lse_words(slices);
+}
 // exchange words of one layer: qkv, J partial attention outputs, log-sum-exps, o, act, down
 __host__ __device__ inline size_t step_words_per_layer(int H, int I, int n_q, int n_kv, int D, int J) {
   return (size_t)(n_q + 2 * n_kv) * D + (size_t)J * n_q * D + (size_t)n_q * step_lse_words(J) + H + I + H;
 }
 
-size_t decode_step_plan_smem(StepParams& p, int resid_bytes, int xin_bytes, int xsum_bytes, int att_bytes,
-                             int part_bytes, int table_bytes);
+size_t decode_step_plan_smem(StepParams& p, int resid_bytes, int xin_bytes, int xsum_bytes, int part_bytes, int table_bytes);
 int decode_step_threads();
 int decode_step_max_stages();
 int decode_step_consumer_warps();

@@ -86,8 +86,8 @@ class DecodeConfig:
                                  # prepared context cap is within PERSISTENT_MAX_CTX
 
 
-PERSISTENT_MAX_CTX = 10240   # beyond this the one-launch-per-operator step, whose attention uses every SM, is faster
-                             # (measured us per token at 2048 / 8192: persistent 468 / 697, multi-kernel 652 / 755)
+PERSISTENT_MAX_CTX = 1 << 20  # what the kernel takes; the one-launch-per-operator step is slower at every context (measured us
+                             # per token at 2048 / 16384 / 65000: persistent 403 / 467 / 665, multi-kernel 650 / 995 / 2278)
 
 
 class Linear:
@@ -374,7 +374,9 @@ class Model:
             arr = self._layer_table()
             host = torch.frombuffer(bytearray(bytes(arr)), dtype=torch.uint8)
             nbytes = self.K.decode_step_xchg_bytes(self.L, self.H, self.I, self.n_q, self.n_kv, self.D, grid)
+            wide = self.K.decode_step_att_bytes(self.L, self.n_q, self.n_kv, self.D, grid)
             self._step_static = {"layers": host.to(dev), "xchg": torch.zeros(nbytes, dtype=torch.uint8, device=dev),
+                                 "att_xchg": torch.zeros(wide, dtype=torch.uint8, device=dev),
                                  "ctrl": torch.zeros(4, dtype=torch.int32, device=dev), "grid": grid}
         st = self._step_static
         d = ext.StepDesc()
@@ -386,6 +388,7 @@ class Model:
         d.cos_t, d.sin_t, d.bt = self.cos.data_ptr(), self.sin.data_ptr(), self.bt.data_ptr()
         d.tok, d.pos, d.history = self.tok.data_ptr(), self.pos.data_ptr(), self.history.data_ptr()
         d.logits, d.xchg, d.ctrl = self.logits.data_ptr(), st["xchg"].data_ptr(), st["ctrl"].data_ptr()
+        d.att_xchg = st["att_xchg"].data_ptr() or None
         d.ctx_cap, d.grid = min(self.ctx_cap, self.cfg.max_ctx + 1), st["grid"]
         self._step_desc = d
 

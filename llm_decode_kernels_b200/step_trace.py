@@ -12,7 +12,7 @@ the CTAs and the slowest CTA:
     mma           this warp's tile-units are multiplied (the interval up to the stamp, without those waits)
     barrier       all warps of the CTA have left their partial sums
     emit          the partial sums are added and the outputs stored
-and the attention phase on the CTAs that own a head (the others go straight on and wait in the next staging).
+and the attention phase on the CTAs that have a unit of it (the others go straight on and wait in the next staging).
 The normal build carries none of this; numbers printed here are for finding the slow phase, not benchmark values.
 """
 import argparse
@@ -57,7 +57,6 @@ def main():
     g = torch.Generator().manual_seed(0)
     m.teacher_force(torch.randint(0, c.vocab_size, (a.ctx,), generator=g), use_graph=False)
     torch.cuda.synchronize()
-    n_att = m.n_q                                   # CTAs 0 .. n_q-1 run attention
     acc, totals = [], []
     for _ in range(a.reps):
         trace.zero_()
@@ -99,7 +98,7 @@ def main():
             res["phases_us"][f"{name}.{what}"] = {"median_cta": round(float(np.median(col)), 3),
                                                   "slowest_cta": round(float(col.max()), 3)}
     for j, what in enumerate(ATT_STAMPS):
-        col = d[:n_att, 4 * PER_PHASE + j]
+        col = d[d[:, 4 * PER_PHASE] > 0, 4 * PER_PHASE + j]     # the CTAs with an attention unit
         res["phases_us"][f"attention.{what}"] = {"median_cta": round(float(np.median(col)), 3),
                                                  "slowest_cta": round(float(col.max()), 3)}
     res["layer_us_median_cta"] = round(float(np.median(d[:, :4 * PER_PHASE].sum(axis=1))), 3)

@@ -422,3 +422,33 @@ def test_rope_tables_match_oracle():
     for D in (64, 128):
         a, b = rope_tables(100, D), R.rope_tables(100, D)
         assert torch.equal(a[0], b[0]) and torch.equal(a[1], b[1])
+
+
+# The step's attention: one CTA per head below 512 cached tokens (256 at head_dim 128), slices of 16-token blocks merged by a CTA per
+# head above. Groups of 1 .. 16 query heads per kv head, a first step on an empty cache, both sides of the change, ends of
+# blocks, ring stages and slices, more slices than the ring has stages, pages of 64.
+@pytest.mark.parametrize("D,n_q,n_kv,page", [(64, 16, 1, 16), (64, 8, 8, 16), (64, 8, 2, 64), (128, 8, 1, 16), (128, 4, 4, 32)])
+def test_persistent_attention_forms_match_the_multi_kernel_step(D, n_q, n_kv, page):
+    c = hf_cfg(512, 2, n_q, n_kv, 1024, 1000, D=D)
+    sd = random_state(c, 31, D)
+    cap = 4700
+    models = [Model(sd, c, DecodeConfig(max_ctx=cap, seed=4, page=page, step_kernel=k)) for k in ("persistent", "multi")]
+    kv = torch.randn(models[0].kv.shape, generator=torch.Generator(device="cuda").manual_seed(1), device="cuda").half()
+    pair = models[:2 if n_q // n_kv in (1, 2, 4, 8) else 1]   # the per-operator attention has no other groups: prefill's has 16
+    for m in pair:
+        m.prepare(cap - 16, use_graph=False)
+        m.kv.copy_(kv)
+    for ctx in (0, 15, 127, 128, 255, 256, 511, 512, 513, 640, 1023, 2049, 4600):
+        outs = []
+        for m in pair:
+            m.reset(ctx)
+            outs.append(m.teacher_force([17, 23], use_graph=False, collect_logits=True).float())
+            assert m.step_error() == 0
+        if len(pair) == 2:
+            scale = outs[1].abs().max()
+            assert (outs[0] - outs[1]).abs().max() <= KERNEL_TOL * scale, ctx
+        else:
+            m = pair[0]
+            m.reset(ctx)
+            want = m.prefill([17, 23], collect_logits=True).float()
+            assert (outs[0] - want).abs().max() <= KERNEL_TOL * want.abs().max(), ctx
