@@ -635,8 +635,7 @@ class Model:
         if n and (int(ids.min()) < 0 or int(ids.max()) >= self.V_full):
             raise ValueError(f"token ids must lie in [0, {self.V_full})")
         dev = self.tok.device
-        if ids.device.type != "cuda":
-            ids = (ids.pin_memory() if n else ids).to(dev, non_blocking=True)
+        ids = _ids_to(ids, dev)
         logits = torch.empty(n, self.V_full, dtype=torch.half, device=dev) if collect_logits else None
         for i in range(n):
             self.tok.copy_(ids[i:i + 1])
@@ -772,8 +771,7 @@ class Model:
         if self.host_pos + n > limit:
             raise RuntimeError(f"context {self.host_pos + n} exceeds the prepared attention cap {limit}; call prepare()")
         dev, K, G = self.tok.device, self.K, self.cfg.group
-        if ids.device.type != "cuda":
-            ids = ids.pin_memory().to(dev, non_blocking=True)
+        ids = _ids_to(ids, dev)
         if self._tiled_prefill() is not None:
             all_logits, last = self._prefill_tiled(ids, collect_logits)
             self._finish_prefill(n, all_logits, last)
@@ -858,6 +856,12 @@ class Model:
     def bytes_per_token(self, ctx):
         wb = self.weight_bytes()
         return wb["body"] + wb["lm_head"] + wb["embedding_row"] + self.kv_bytes_per_token(ctx)
+
+
+def _ids_to(ids, dev):
+    """Token ids on the device. Not through fresh pinned memory: a first pinned allocation takes tens of milliseconds, and the
+    few KB of a prompt leave pageable memory before an asynchronous copy returns anyway."""
+    return ids if ids.device.type == "cuda" else ids.to(dev, non_blocking=True)
 
 
 def rope_tables(max_pos: int, head_dim: int = 64, theta: float = 10000.0, device="cpu"):
