@@ -1,4 +1,5 @@
-"""Build libb200decode.so in-tree with nvcc for sm_100a (no torch headers, no JIT cache).
+"""Build libb200decode.so in-tree with nvcc for sm_100a (no torch headers, no JIT cache), and _host.so, the Python face's native
+call path, with the C++ compiler against torch's headers.
 
     python -m llm_decode_kernels_b200.build [--force] [--verbose]
 
@@ -17,6 +18,7 @@ PKG = Path(__file__).resolve().parent
 CSRC = PKG / "csrc"
 INCLUDE = PKG.parent / "include"
 LIB = PKG / "libb200decode.so"
+HOST = PKG / "_host.so"          # the operators' call path (csrc/host_ops.cpp), a CPython extension module
 
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-lineinfo", "-std=c++17",
               "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr"]
@@ -76,6 +78,27 @@ def build(force=False, verbose=False, defines=(), lib=LIB):
     return lib
 
 
+def build_host(force=False, verbose=False):
+    """Compile _host.so if it is stale. Returns its path."""
+    src = CSRC / "host_ops.cpp"
+    if not force and HOST.exists() and HOST.stat().st_mtime >= src.stat().st_mtime:
+        return HOST
+    import sysconfig
+    import torch
+    root = Path(torch.__file__).resolve().parent
+    cuda = Path(nvcc()).resolve().parents[1]
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}", "-I", sysconfig.get_paths()["include"],
+           "-I", str(root / "include"), "-I", str(root / "include/torch/csrc/api/include"), "-I", str(cuda / "include"),
+           str(src), "-o", str(HOST), "-L", str(root / "lib"), "-ltorch_python", "-ltorch_cpu", "-lc10", "-lc10_cuda"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if verbose or r.returncode:
+        sys.stderr.write(f"--- {src.name}\n{r.stdout}{r.stderr}")
+    if r.returncode:
+        raise RuntimeError(f"{cmd[0]} failed on {src.name}")
+    return HOST
+
+
 if __name__ == "__main__":
-    p = build(force="--force" in sys.argv, verbose="--verbose" in sys.argv)
-    print(p)
+    for step in (build, build_host):
+        print(step(force="--force" in sys.argv, verbose="--verbose" in sys.argv))

@@ -22,6 +22,7 @@ import torch
 _LIB = None
 _OPS = None
 LIB_PATH = Path(__file__).resolve().parent / "libb200decode.so"
+HOST_PATH = LIB_PATH.with_name("_host.so")
 
 # name -> argtypes, exactly the declarations of include/b200decode.h (checked by tests/test_abi.py)
 SIGNATURES = {
@@ -172,11 +173,25 @@ def _stream():
     return torch.cuda.current_stream().cuda_stream
 
 
+def _load_host(lib):
+    """The native call path (csrc/host_ops.cpp), built first if it is absent, bound to `lib`."""
+    if not HOST_PATH.exists():
+        from . import build as _build
+        _build.build_host()
+    from . import _host
+    _host.bind({n: ctypes.cast(getattr(lib, n), c_void_p).value for n in _host.names()[0]})
+    return _host
+
+
 class Ops:
-    """The operator set. Every method launches on torch's current CUDA stream and returns None."""
+    """The operator set. Every method launches on torch's current CUDA stream and returns None. The operators a decode step is
+    made of are called through native code that makes the same checks; what it does not accept comes to the methods here."""
 
     def __init__(self, lib):
         self.lib = lib
+        host = _load_host(lib)
+        for name in host.names()[1]:
+            setattr(self, name, host.operator(name, getattr(self, name)))
 
     def _check(self, code, what):
         if code != 0:

@@ -93,3 +93,22 @@ def test_python_face_refuses_cpu_tensors():
         K.swiglu(torch.zeros(256, dtype=torch.float16), x)
     with pytest.raises(RuntimeError, match="CUDA tensor"):
         K.add_rmsnorm(x, None, x, x, 1e-5)
+
+
+def test_native_call_path_mirrors_the_methods():
+    """Every operator of the native call path takes the arguments of the method it stands in for, and hands what it does not
+    accept to that method."""
+    import inspect
+    ops = ext.Ops(ext.load_library())
+    from llm_decode_kernels_b200 import _host
+    for name, (args, required) in _host.names()[1].items():
+        params = list(inspect.signature(getattr(ext.Ops, name)).parameters.values())[1:]
+        assert [p.name for p in params] == list(args), name
+        assert sum(p.default is p.empty for p in params) == required, name
+        assert getattr(ops, name).__doc__ == getattr(ext.Ops, name).__doc__
+    with pytest.raises(RuntimeError, match="gu must be a contiguous CUDA tensor"):
+        ops.swiglu(None, out=None)
+    with pytest.raises(TypeError):
+        ops.swiglu(1, 2, 3)
+    with pytest.raises(TypeError):
+        ops.swiglu(gu=1, nonsense=2)
