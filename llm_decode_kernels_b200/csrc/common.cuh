@@ -212,6 +212,15 @@ DEVI void mma16832_u8s8(int (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint
                : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
+// Rows 0-7 of D (16x8, fp32) += A (16x16, fp16, row) * B (16x8, fp16, col); rows 8-15 of A are zero and of D dropped. Lane (g, t):
+// c = D[g][2t, 2t+1], a0 = A[g][2t, 2t+1], a2 = A[g][2t+8, 2t+9].
+DEVI void mma16816_top(float (&c)[2], uint32_t a0, uint32_t a2, uint32_t b0, uint32_t b1) {
+  asm volatile("{\n\t.reg .f32 x, y;\n\t"
+               "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,x,y}, {%2,%6,%3,%6}, {%4,%5}, {%0,%1,%7,%7};\n\t}"
+               : "+f"(c[0]), "+f"(c[1])
+               : "r"(a0), "r"(a2), "r"(b0), "r"(b1), "r"(0u), "f"(0.f));
+}
+
 // Bytes of one (16-row tile, 128-column unit) block of the tile layout (gemv_tile_repack_kernel): 512 B for row
 // slots 0-7 (lane l's 16 bytes at 16 l), 512 B for row slots 8-15, 16 x (scale, zero).
 constexpr int kTileUnitBytes = 1088;

@@ -741,14 +741,6 @@ __device__ __noinline__ void refresh_partials(const Cta c, int layer) {
   }
 }
 
-// Rows 0-7 of D (16x8, fp32) += A (16x16, fp16, row) * B (16x8, fp16, col); rows 8-15 of A are zero and of D dropped. Lane (g, t):
-// c = D[g][2t, 2t+1], a0 = A[g][2t, 2t+1], a2 = A[g][2t+8, 2t+9].
-DEVI void mma16816_top(float (&c)[2], uint32_t a0, uint32_t a2, uint32_t b0, uint32_t b1) {
-  asm volatile("{\n\t.reg .f32 x, y;\n\t"
-               "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,x,y}, {%2,%6,%3,%6}, {%4,%5}, {%0,%1,%7,%7};\n\t}"
-               : "+f"(c[0]), "+f"(c[1])
-               : "r"(a0), "r"(a2), "r"(b0), "r"(b1), "r"(0u), "f"(0.f));
-}
 DEVI uint4 lds16(uint32_t addr) {
   uint4 v;
   asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr));

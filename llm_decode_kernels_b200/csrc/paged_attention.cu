@@ -7,6 +7,8 @@
 // of tokens [i P, (i+1) P) of sequence b; context length of sequence b = pos[b] + 1, read on the device so one
 // captured graph serves every step. Split s of a sequence owns tokens [s PS, min(ctx, (s+1) PS)).
 //
+// Versions 0 and 3 take paged_attn_cluster_kernel (one launch, see there) where cluster_ctas() says so. Otherwise:
+//
 // Three partial kernels (the `version` of the entry points) share the grid (n_kv, max_splits, B); a block handles ALL
 // heads of one kv group, so every K/V byte is fetched from HBM once. Version 3, paged_attn_mma_kernel, is the default
 // and is described where it is defined; it builds on version 2:
@@ -847,6 +849,254 @@ paged_attn_mma_kernel(const half* __restrict__ q, const half* __restrict__ kc, c
   }
 }
 
+// ---- clusters: the whole call in one launch ------------------------------------------------------------------------------------
+// The C CTAs of a cluster (C <= 8) share one kv head of one sequence, all query heads of the group; CTA r, warp w takes the
+// 16-token blocks r + C w, + 8 C, ... Every warp has a ring of its own, filled by its own cp.async (16 bytes a lane, a row by 8 or 16
+// lanes): no barrier in the loop, and no limit from the bulk-copy engine, which handles the page of one kv head (2 KB) in the time
+// of 8 KB. Arithmetic as in paged_attn_mma_kernel. The warps meet in shared memory, the CTAs through distributed shared memory: no
+// partials in global memory and no combine launch. (The fragments straight from the cache into registers, two blocks ahead, take 167
+// registers; at 128 the spills make every load wait for itself.)
+// Eight sequences of 128 .. 8192 tokens (34 MB): 21.2 us with the ring kernel and its combine, 12.3 here; one sequence of 512: 6.5 ->
+// 3.9 us. Two stages at head_dim 64 (two CTAs an SM; three stages are 5 % slower), three at 128 (one CTA).
+constexpr int kClWarps = 8, kClThreads = kClWarps * 32;
+template <int D> constexpr int cluster_stages() { return D == 64 ? 2 : 3; }
+template <int D> constexpr size_t cluster_smem() { return (size_t)kClWarps * cluster_stages<D>() * 2 * 16 * D * sizeof(half); }
+
+// 8 c .. 8 c + 7 of the dims [t D/4, (t + 1) D/4) of a head, rotated (rotate-half RoPE: fp32, fp16 result)
+template <int D>
+DEVI uint4 rotated8(const half* head, const float* cs, const float* sn, int t, int c) {
+  const int i0 = (t & 1) * (D / 4) + 8 * c;   // index among the D/2 pairs
+  float a[8], bb[8], co[8], si[8];
+  unpack8(*reinterpret_cast<const uint4*>(head + i0), a);
+  unpack8(*reinterpret_cast<const uint4*>(head + D / 2 + i0), bb);
+#pragma unroll
+  for (int v = 0; v < 2; ++v) {
+    *reinterpret_cast<float4*>(co + 4 * v) = *reinterpret_cast<const float4*>(cs + i0 + 4 * v);
+    *reinterpret_cast<float4*>(si + 4 * v) = *reinterpret_cast<const float4*>(sn + i0 + 4 * v);
+  }
+  uint32_t r[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    half h[2];
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const int i = 2 * k + e;
+      h[e] = __float2half(t < 2 ? a[i] * co[i] - bb[i] * si[i] : bb[i] * co[i] + a[i] * si[i]);
+    }
+    r[k] = as_u32(__halves2half2(h[0], h[1]));
+  }
+  return make_uint4(r[0], r[1], r[2], r[3]);
+}
+
+// ROPE: q is the step's raw qkv vector ([B, (n_q + 2 n_kv) D]), see paged_attn_mma_kernel: the CTA whose block holds the step's own
+// token rotates k, writes the row to the caches and keeps it in shared memory, from where the warp puts it in its fragments.
+template <int D, int HPG, bool ROPE>
+__global__ void __launch_bounds__(kClThreads, D == 64 ? 2 : 1)
+paged_attn_cluster_kernel(const half* __restrict__ q, const half* __restrict__ kc, const half* __restrict__ vc,
+                          const int* __restrict__ bt, int bt_stride, const int* __restrict__ pos_ptr, int n_kv, int log2P, int cap,
+                          float sl2, half* __restrict__ out, const RopeArgs ra) {
+  constexpr int CH = D / 32, VC = D / 64, NB = D / 8, NS = cluster_stages<D>();
+  pdl_launch_dependents();
+  __shared__ float wm[kClWarps][HPG], wl[kClWarps][HPG];
+  __shared__ __align__(16) float po[HPG * D], pm[HPG], pl[HPG];
+  __shared__ __align__(16) half new_s[ROPE ? 2 * D : 8];   // k and v of the step's own token
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+  const int kvh = blockIdx.x, rank = blockIdx.y, C = gridDim.y, b = blockIdx.z, n_q = n_kv * HPG;
+  pdl_wait();
+  const int pos = pos_ptr[b], ctx = min(pos + 1, cap), nblk = (ctx + 15) >> 4, stride = kClWarps * C, first = rank + C * warp;
+  const int* btb = bt + (size_t)b * bt_stride;
+  const int pmask = (1 << log2P) - 1;
+
+  // the warp's ring: stage = K rows then V rows of 16 tokens, piece p of row r at p ^ (r & 1) (K reads are then free of conflicts)
+  constexpr int PP = D / 8, HALF = 16 * D * 2, STAGE = 2 * HALF;   // pieces per row; bytes
+  extern __shared__ __align__(128) uint8_t ring_raw[];
+  const uint32_t ring = sm_u32(ring_raw) + warp * (NS * STAGE);
+  int page_lo = 0, page_hi = 0;   // pages of tokens 0 .. 7 / 8 .. 15 of the warp's next 32 blocks: lane i holds its i-th
+  auto load = [&](int i, int slot) {
+    const int blk = first + i * stride;
+    if ((i & 31) == 0) {
+      const int mine = blk + lane * stride, j = 16 * mine;
+      if (mine < nblk) {
+        page_lo = __ldg(btb + (j >> log2P));
+        page_hi = log2P >= 4 || j + 8 >= ctx ? page_lo : __ldg(btb + ((j + 8) >> log2P));
+      }
+    }
+    if (blk < nblk) {
+      const int tok0 = 16 * blk, lo = __shfl_sync(0xffffffffu, page_lo, i & 31), hi = __shfl_sync(0xffffffffu, page_hi, i & 31);
+      const uint32_t dst = ring + slot * STAGE;
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const size_t base = ((((size_t)(h ? hi : lo) * n_kv + kvh) << log2P) + ((tok0 + 8 * h) & pmask)) * D;
+#pragma unroll
+        for (int k = 0; k < 8 * PP / 32; ++k) {
+          const int idx = lane + 32 * k, r = 8 * h + idx / PP, p = idx % PP;
+          const size_t off = base + (idx / PP) * D + p * 8;
+          const uint32_t to = dst + r * (2 * D) + ((p ^ (r & 1)) << 4);
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to), "l"(kc + off) : "memory");
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to + HALF), "l"(vc + off) : "memory");
+        }
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+#pragma unroll
+  for (int i = 0; i < NS - 1; ++i) load(i, i);
+  // Q fragments: row g = head g of the group (zero beyond it), k-step kk holds dims t D/4 + 4 kk + {0,1 | 2,3}
+  uint4 qf[CH];
+  const half* qkv = q + (size_t)b * (ROPE ? n_q + 2 * n_kv : n_q) * D;
+  const half* qh = qkv + (size_t)(kvh * HPG + (g < HPG ? g : 0)) * D;
+  const float *cs = ROPE ? ra.cos_t + (size_t)pos * (D / 2) : nullptr, *sn = ROPE ? ra.sin_t + (size_t)pos * (D / 2) : nullptr;
+#pragma unroll
+  for (int c = 0; c < CH; ++c) {
+    qf[c] = ROPE ? rotated8<D>(qh, cs, sn, t, c) : reinterpret_cast<const uint4*>(qh + t * (D / 4))[c];
+    if (g >= HPG) qf[c] = make_uint4(0u, 0u, 0u, 0u);
+  }
+  int i_new = -1;   // which of this warp's blocks holds the new token
+  if (ROPE && pos < ctx && ((pos >> 4) - rank) % C == 0) {   // in this CTA
+    const int nb = (pos >> 4) - rank;
+    if (nb >= C * warp && (nb / C - warp) % kClWarps == 0) i_new = (nb / C - warp) / kClWarps;
+    if (tid < 4 * CH) {
+      const half *kraw = qkv + (size_t)(n_q + kvh) * D, *vraw = kraw + (size_t)n_kv * D;
+      const int tt = tid / CH, c = tid % CH, d0 = tt * (D / 4) + 8 * c;
+      const uint4 k = rotated8<D>(kraw, cs, sn, tt, c), v = *reinterpret_cast<const uint4*>(vraw + d0);
+      *reinterpret_cast<uint4*>(new_s + d0) = k;
+      *reinterpret_cast<uint4*>(new_s + D + d0) = v;
+      const size_t row = ((((size_t)__ldg(btb + (pos >> log2P)) * n_kv + kvh) << log2P) + (pos & pmask)) * D + d0;
+      *reinterpret_cast<uint4*>(ra.kc_w + row) = k;
+      *reinterpret_cast<uint4*>(ra.vc_w + row) = v;
+    }
+  }
+  if (ROPE) __syncthreads();
+
+  float m = -CUDART_INF_F, l = 0.f, acc[NB][2];
+#pragma unroll
+  for (int n = 0; n < NB; ++n) acc[n][0] = acc[n][1] = 0.f;
+  int slot = 0;
+#pragma unroll 1
+  for (int i = 0; first + i * stride < nblk; ++i) {
+    __syncwarp();   // every lane is done with the stage that is filled next
+    load(i + NS - 1, slot == 0 ? NS - 1 : slot - 1);
+    asm volatile("cp.async.wait_group %0;" ::"n"(NS - 1) : "memory");
+    __syncwarp();
+    const uint8_t* ks = ring_raw + (ring - sm_u32(ring_raw)) + slot * STAGE;
+    const uint8_t* vs = ks + HALF;
+    if (++slot == NS) slot = 0;
+    const int left = ctx - 16 * (first + i * stride);   // tokens of the block that count, >= 1
+    if (ROPE && i == i_new) {
+      const int j = pos & 15;
+      if (lane < 2 * PP) {
+        const int isv = lane >= PP, p = lane - isv * PP;
+        *reinterpret_cast<uint4*>(const_cast<uint8_t*>(isv ? vs : ks) + j * (2 * D) + ((p ^ (j & 1)) << 4)) =
+            *reinterpret_cast<const uint4*>(new_s + isv * D + 8 * p);
+      }
+      __syncwarp();
+    }
+    float s[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
+#pragma unroll
+    for (int c = 0; c < CH; ++c)
+#pragma unroll
+      for (int nb = 0; nb < 2; ++nb) {
+        const uint4 k = *reinterpret_cast<const uint4*>(ks + (8 * nb + g) * (2 * D) + (((t * CH + c) ^ (g & 1)) << 4));
+        mma16816_top(s[nb], qf[c].x, qf[c].y, k.x, k.y);
+        mma16816_top(s[nb], qf[c].z, qf[c].w, k.z, k.w);
+      }
+    float p[4];   // head g, tokens 8 nb + 2 t + {0, 1}; rows past the context hold anything: masked
+#pragma unroll
+    for (int nb = 0; nb < 2; ++nb)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) p[2 * nb + e] = 8 * nb + 2 * t + e < left ? s[nb][e] * sl2 : -CUDART_INF_F;
+    float mx = fmaxf(fmaxf(p[0], p[1]), fmaxf(p[2], p[3]));
+    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+    const float mn = fmaxf(m, mx), alpha = exp2f(m - mn);
+    m = mn;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) p[e] = exp2f(p[e] - mn);
+    l = l * alpha + (p[0] + p[1]) + (p[2] + p[3]);
+#pragma unroll
+    for (int n = 0; n < NB; ++n) acc[n][0] *= alpha, acc[n][1] *= alpha;
+    const uint32_t pa0 = as_u32(__floats2half2_rn(p[0], p[1])), pa2 = as_u32(__floats2half2_rn(p[2], p[3]));
+#pragma unroll
+    for (int c = 0; c < VC; ++c) {
+      uint32_t w0[4], w1[4], w2[4], w3[4];
+      auto row = [&](int r, uint32_t (&w)[4]) {   // 0 * NaN is NaN: rows past the context count as zeros
+        uint4 v = *reinterpret_cast<const uint4*>(vs + r * (2 * D) + (((8 * c + g) ^ (r & 1)) << 4));
+        if (r >= left) v = make_uint4(0u, 0u, 0u, 0u);
+        w[0] = v.x, w[1] = v.y, w[2] = v.z, w[3] = v.w;
+      };
+      row(2 * t, w0), row(2 * t + 1, w1), row(2 * t + 8, w2), row(2 * t + 9, w3);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        mma16816_top(acc[8 * c + 2 * k], pa0, pa2, __byte_perm(w0[k], w1[k], 0x5410), __byte_perm(w2[k], w3[k], 0x5410));
+        mma16816_top(acc[8 * c + 2 * k + 1], pa0, pa2, __byte_perm(w0[k], w1[k], 0x7632), __byte_perm(w2[k], w3[k], 0x7632));
+      }
+    }
+  }
+
+  // the warps of the CTA: acc[n][e] = O[head g][dim 64 (n / 8) + 8 (2 t + e) + n % 8]
+  l += __shfl_xor_sync(0xffffffffu, l, 1);
+  l += __shfl_xor_sync(0xffffffffu, l, 2);
+  static_assert(NS * STAGE >= 8 * (D + 1) * 4, "a warp's output fits over its ring");
+  float* wo = reinterpret_cast<float*>(ring_raw);   // [warp] at the warp's ring, which is idle now: [HPG][D + 1]
+  constexpr int WO = NS * STAGE / 4;
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  __syncwarp();
+  if (g < HPG) {
+    if (t == 0) wm[warp][g] = m, wl[warp][g] = l;
+#pragma unroll
+    for (int n = 0; n < NB; ++n)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) wo[warp * WO + g * (D + 1) + 64 * (n / 8) + 8 * (2 * t + e) + n % 8] = acc[n][e];
+  }
+  __syncthreads();
+  half* o_row = out + ((size_t)b * n_q + kvh * HPG) * D;
+  for (int i = tid; i < HPG * D; i += kClThreads) {
+    const int h = i / D, d = i % D;
+    float M = -CUDART_INF_F, o = 0.f, L = 0.f;
+#pragma unroll
+    for (int w = 0; w < kClWarps; ++w) M = fmaxf(M, wm[w][h]);
+    if (M > -CUDART_INF_F) {   // a CTA without a block: nothing
+#pragma unroll
+      for (int w = 0; w < kClWarps; ++w) {
+        const float a = exp2f(wm[w][h] - M);
+        o = fmaf(a, wo[w * WO + h * (D + 1) + d], o);
+        L = fmaf(a, wl[w][h], L);
+      }
+    }
+    if (C == 1) o_row[i] = __float2half(o / L);
+    else po[i] = o;
+    if (d == 0) pm[h] = M, pl[h] = L;
+  }
+  if (C == 1) return;
+  // the CTAs of the cluster: CTA r finishes every C-th output
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+  auto peer = [](const float* p, int r) {
+    uint32_t a;
+    float v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(sm_u32(p)), "r"(r));
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+    return v;
+  };
+  for (int i = rank + C * tid; i < HPG * D; i += C * kClThreads) {
+    const int h = i / D;
+    float mv[8], lv[8], ov[8], M = -CUDART_INF_F, o = 0.f, L = 0.f;
+#pragma unroll
+    for (int r = 0; r < 8; ++r) mv[r] = r < C ? peer(pm + h, r) : -CUDART_INF_F;
+#pragma unroll
+    for (int r = 0; r < 8; ++r) lv[r] = r < C ? peer(pl + h, r) : 0.f, ov[r] = r < C ? peer(po + i, r) : 0.f;
+#pragma unroll
+    for (int r = 0; r < 8; ++r) M = fmaxf(M, mv[r]);   // finite: CTA 0 has a block
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+      const float a = exp2f(mv[r] - M);
+      o = fmaf(a, ov[r], o);
+      L = fmaf(a, lv[r], L);
+    }
+    o_row[i] = __float2half(o / L);
+  }
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
 // Grid (n_q, B), D threads: thread d merges dim d of one head over the live splits.
 __global__ void paged_attn_combine_kernel(const float* __restrict__ o_part, const float* __restrict__ m_part,
                                           const float* __restrict__ l_part, const int* __restrict__ pos_ptr, int PS,
@@ -883,16 +1133,6 @@ cudaError_t attention_combine_dispatch(const float* o_part, const float* m_part,
   return cudaPeekAtLastError();
 }
 
-enum : int { ATTN_REGISTER = 1, ATTN_STAGED = 2, ATTN_MMA = 3 };
-
-template <typename Kern>
-static cudaError_t allow_ring(Kern kern, size_t bytes, bool* done) {
-  if (*done) return cudaSuccess;   // the ring needs more than the default 48 KB of dynamic shared memory
-  const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-  if (e == cudaSuccess) *done = true;
-  return e;
-}
-
 struct AttnArgs {
   const half *q, *kc, *vc;
   const int* bt;
@@ -904,6 +1144,55 @@ struct AttnArgs {
   half* out;
   int max_splits, B;
 };
+
+template <int D>
+static cudaError_t launch_cluster(const AttnArgs& a, int hpg, int C, const RopeArgs* rope, cudaStream_t st) {
+  auto kern = hpg == 1   ? (rope ? paged_attn_cluster_kernel<D, 1, true> : paged_attn_cluster_kernel<D, 1, false>)
+              : hpg == 2 ? (rope ? paged_attn_cluster_kernel<D, 2, true> : paged_attn_cluster_kernel<D, 2, false>)
+              : hpg == 4 ? (rope ? paged_attn_cluster_kernel<D, 4, true> : paged_attn_cluster_kernel<D, 4, false>)
+                         : (rope ? paged_attn_cluster_kernel<D, 8, true> : paged_attn_cluster_kernel<D, 8, false>);
+  static size_t allowed[8][b200::kMaxDevices] = {};
+  const cudaError_t e = allow_dynamic_smem(kern, cluster_smem<D>(), allowed[2 * (hpg == 1 ? 0 : hpg == 2 ? 1 : hpg == 4 ? 2 : 3) + (rope != nullptr)]);
+  if (e != cudaSuccess) return e;
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 1, attr[0].val.clusterDim.y = C, attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.gridDim = dim3(a.n_kv, C, a.B);
+  cfg.blockDim = dim3(kClThreads);
+  cfg.dynamicSmemBytes = cluster_smem<D>();
+  cfg.stream = st;
+  cfg.attrs = attr;
+  cfg.numAttrs = 2;
+  const long long cap = (long long)a.PS * a.max_splits;
+  return cudaLaunchKernelEx(&cfg, kern, a.q, a.kc, a.vc, a.bt, a.bt_stride, a.pos, a.n_kv, a.log2P,
+                            (int)(cap < (1 << 30) ? cap : 1 << 30), a.scale * 1.44269504088896340736f, a.out,
+                            rope ? *rope : RopeArgs{nullptr, nullptr, nullptr, nullptr});
+}
+
+// CTAs per cluster for a call, or 0 where clusters do not serve it: as many as are resident at once (two an SM at head_dim 64, one at
+// 128; a second wave of them pays the whole latency of a call again: 8 x 1000 tokens of 8 heads at 128, 25 us with 512 CTAs), eight
+// at most. Not for pages below 8 tokens, nor where few CTAs would walk a long context (less than half of the chip and more than 16
+// blocks a warp at the cap): the splits of the ring kernel then put more of the chip to work.
+static int cluster_ctas(int B, int n_kv, int D, int log2P, int PS, int max_splits) {
+  const long long pairs = (long long)B * n_kv, slots = kNumSMs * (D == 64 ? 2 : 1);
+  int C = 1;
+  while (C < 8 && pairs * C * 2 <= slots) C *= 2;
+  return log2P >= 3 && (pairs * C >= kNumSMs / 2 || (long long)PS * max_splits <= 16ll * 16 * kClWarps * C) ? C : 0;
+}
+
+enum : int { ATTN_REGISTER = 1, ATTN_STAGED = 2, ATTN_MMA = 3 };
+
+template <typename Kern>
+static cudaError_t allow_ring(Kern kern, size_t bytes, bool* done) {
+  if (*done) return cudaSuccess;   // the ring needs more than the default 48 KB of dynamic shared memory
+  const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  if (e == cudaSuccess) *done = true;
+  return e;
+}
+
 
 template <int D, int HPG, int KH>
 static cudaError_t launch_mma(const AttnArgs& a, int dev, cudaStream_t st) {
@@ -984,6 +1273,9 @@ cudaError_t paged_attention_dispatch(int version, const void* q, const void* kc,
   if (kind == ATTN_MMA && (reinterpret_cast<uintptr_t>(q) & 7u)) kind = ATTN_STAGED;   // Q fragments: 8-byte loads
   const AttnArgs a = {(const half*)q, (const half*)kc, (const half*)vc, bt, bt_stride, pos, n_kv, log2P, PS, scale,
                       o_part, m_part, l_part, (half*)out, max_splits, B};
+  const int C = version == 0 || version == 3 ? cluster_ctas(B, n_kv, D, log2P, PS, max_splits) : 0;
+  const bool aligned = ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(kc) | reinterpret_cast<uintptr_t>(vc)) & 15u) == 0;
+  if (C && aligned) return D == 64 ? launch_cluster<64>(a, hpg, C, nullptr, st) : launch_cluster<128>(a, hpg, C, nullptr, st);
   cudaError_t e = D == 64 ? launch_partial<64>(hpg, kind, a, st) : launch_partial<128>(hpg, kind, a, st);
   if (e != cudaSuccess) return e;
   if (max_splits > 1) e = attention_combine_dispatch(o_part, m_part, l_part, pos, PS, max_splits, n_q, B, D, out, st);
@@ -1003,7 +1295,7 @@ cudaError_t rope_paged_attention_dispatch(void* qkv, const float* cos_t, const f
                                           int* arrive, cudaStream_t st) {
   const int hpg = n_q / n_kv;
   const bool ring_ok = log2P >= 3 && log2P <= 6 && PS % (1 << log2P) == 0;
-  if (!ring_ok) {
+  if (!ring_ok && !cluster_ctas(1, n_kv, D, log2P, PS, max_splits)) {
     const cudaError_t e = rope_append_dispatch(qkv, cos_t, sin_t, pos, bt, 1 << 30, kc, vc, 1, n_q, n_kv, D, log2P, st);
     if (e != cudaSuccess) return e;
     return paged_attention_dispatch(0, qkv, kc, vc, bt, 1 << 30, pos, 1, n_q, n_kv, D, log2P, PS, max_splits, o_part,
@@ -1015,6 +1307,8 @@ cudaError_t rope_paged_attention_dispatch(void* qkv, const float* cos_t, const f
   const AttnArgs a = {(const half*)qkv, (const half*)kc, (const half*)vc, bt, 1 << 30, pos, n_kv, log2P, PS,
                       1.0f / sqrtf((float)D), o_part, m_part, l_part, (half*)out, max_splits, 1};
   const RopeArgs r = {cos_t, sin_t, (half*)kc, (half*)vc};
+  if (const int C = cluster_ctas(1, n_kv, D, log2P, PS, max_splits))
+    return D == 64 ? launch_cluster<64>(a, hpg, C, &r, st) : launch_cluster<128>(a, hpg, C, &r, st);
   cudaError_t e = cudaErrorInvalidValue;
 #define B200_ROPE_CASE(DD, H) \
   if (D == DD && hpg == H) e = launch_mma_rope<DD, H>(a, r, arrive, dev, st);

@@ -376,6 +376,43 @@ def test_attention_batched(K, D, n_q, n_kv, B):
 
 
 # ---- 6. fused operators ---------------------------------------------------------------------------------
+# Cluster kernel: 8, 4, 2 and 1 CTAs per sequence and kv head, sequences of unequal length (CTAs and warps without a block, ends
+# inside a block), pages of 8 (two per block) to 128, a cap below the position, page slots past the context poisoned.
+@pytest.mark.parametrize("B,n_q,n_kv,D,page,ctxs", [(1, 8, 1, 64, 8, [129]), (3, 8, 8, 128, 16, [1, 16, 700]), (2, 16, 4, 64, 128, [2047, 33]),
+                                                    (16, 16, 8, 64, 32, [5, 300]), (40, 16, 8, 128, 16, [17, 64, 255])])
+def test_attention_in_clusters(K, B, n_q, n_kv, D, page, ctxs):
+    torch.manual_seed(B)
+    ctxs = [ctxs[i % len(ctxs)] for i in range(B)]
+    pages = [-(-c // page) for c in ctxs]
+    kc = torch.full((sum(pages), n_kv, page, D), float("nan"), dtype=torch.half, device=dev)
+    vc = kc.clone()
+    bt = torch.zeros(B, max(pages), dtype=torch.int32, device=dev)
+    perm, at, ref = torch.randperm(sum(pages)), 0, []
+    q = torch.randn(B, n_q, D, device=dev).half()
+    for b, (c, n) in enumerate(zip(ctxs, pages)):
+        bt[b, :n] = perm[at:at + n].int().to(dev)
+        at += n
+        for j in range(0, c, page):
+            m = min(page, c - j)
+            kc[bt[b, j // page], :, :m] = torch.randn(n_kv, m, D, device=dev).half()
+            vc[bt[b, j // page], :, :m] = torch.randn(n_kv, m, D, device=dev).half()
+        ref.append(R.paged_attention_ref(q[b].cpu(), kc.cpu(), vc.cpu(), bt[b].cpu(), c, page))
+    pos = torch.tensor([c - 1 for c in ctxs], dtype=torch.int32, device=dev)
+    PS = 48
+    S = -(-max(ctxs) // PS)
+    scratch = [torch.empty(B, n_q, S, *w, device=dev) for w in ((D,), (), ())]
+    out = torch.full((B, n_q, D), float("nan"), dtype=torch.half, device=dev)
+    K.paged_attention_batched(q, kc, vc, bt, pos, PS, *scratch, out)
+    for b in range(B):
+        assert rel_err(out[b], ref[b]) <= ATTN_TOL, b
+    if max(ctxs) > PS:      # the cap of the split geometry: tokens beyond it do not count
+        one = [t[:, :, :1].contiguous() for t in scratch]
+        K.paged_attention_batched(q, kc, vc, bt, pos, PS, *one, out)
+        b = ctxs.index(max(ctxs))
+        want = R.paged_attention_ref(q[b].cpu(), kc.cpu(), vc.cpu(), bt[b].cpu(), PS, page)
+        assert rel_err(out[b], want) <= ATTN_TOL
+
+
 @pytest.mark.parametrize("H", [2048, 8192, 128, 4104])
 def test_add_rmsnorm(K, H):
     torch.manual_seed(H)
