@@ -6,9 +6,9 @@
 
 namespace b200 {
 
-// Tensor map of activations X fp16 [T, K]: boxes of 64 columns x box_rows tokens, 128-byte swizzle, zeros past T. False if the
-// driver refuses (alignment).
-bool encode_activation_map(CUtensorMap* map, const void* X, int T, int K, int box_rows);
+// Tensor map of activations X fp16 [T, K], 128-byte swizzle, zeros past T: coordinates (column in a 64-column chunk, token, chunk),
+// boxes of 64 columns x box_rows tokens x chunks. False if the driver refuses (alignment).
+bool encode_activation_map(CUtensorMap* map, const void* X, int T, int K, int box_rows, int chunks);
 
 // One chunk of a prompt: T tokens at positions start .. start + T - 1 of the sequence whose block table is bt.
 struct PrefillParams {

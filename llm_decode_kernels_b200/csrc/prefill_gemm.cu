@@ -108,12 +108,13 @@ DEVI void umma_commit(uint64_t* bar) {
                : "memory");
 }
 
-// one 2-D tile of the activations into this CTA's shared memory; completion counts bytes on the stage's mbarrier
-DEVI void tma_load_2d(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
+// one tile of the activations (a 64-column chunk of tokens from y on) into this CTA's shared memory; completion counts bytes on
+// the stage's mbarrier
+DEVI void tma_load(void* dst, const CUtensorMap* map, int chunk, int y, uint64_t* bar) {
   asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(
           smem_addr(dst)),
-      "l"(map), "r"(x), "r"(y), "r"(smem_addr(bar))
+      "l"(map), "r"(0), "r"(y), "r"(chunk), "r"(smem_addr(bar))
       : "memory");
 }
 
@@ -291,7 +292,7 @@ prefill_gemm_kernel(const __grid_constant__ CUtensorMap xmap, const uint32_t* __
           break;
         }
         mbar_expect_tx(&sh.b_full[s], (uint32_t)b_bytes);
-        tma_load_2d(base + s * stage_bytes + a_bytes, &xmap, (c_begin + j) * kPfChunk, 0, &sh.b_full[s]);
+        tma_load(base + s * stage_bytes + a_bytes, &xmap, c_begin + j, 0, &sh.b_full[s]);
         issued = j + 1;
         if (++s == ns) s = 0, ++use;
       }
@@ -386,12 +387,13 @@ EncodeTiledFn encode_tiled() {
 
 }  // namespace
 
-bool encode_activation_map(CUtensorMap* map, const void* X, int T, int K, int box_rows) {
+bool encode_activation_map(CUtensorMap* map, const void* X, int T, int K, int box_rows, int chunks) {
   const EncodeTiledFn encode = encode_tiled();
   if (!encode) return false;
-  const cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)T}, strides[1] = {(cuuint64_t)K * 2};
-  const cuuint32_t box[2] = {(cuuint32_t)kPfChunk, (cuuint32_t)box_rows}, estr[2] = {1, 1};
-  return encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(X), dims, strides, box, estr,
+  const cuuint64_t dims[3] = {(cuuint64_t)kPfChunk, (cuuint64_t)T, (cuuint64_t)(K / kPfChunk)};
+  const cuuint64_t strides[2] = {(cuuint64_t)K * 2, (cuuint64_t)kPfChunk * 2};
+  const cuuint32_t box[3] = {(cuuint32_t)kPfChunk, (cuuint32_t)box_rows, (cuuint32_t)chunks}, estr[3] = {1, 1, 1};
+  return encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<void*>(X), dims, strides, box, estr,
                 CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                 CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
@@ -447,7 +449,7 @@ cudaError_t prefill_gemm_dispatch(const void* Wp, const void* SZ, const void* X,
   int cols = 32;
   while (cols < Tpad) cols *= 2;
   CUtensorMap xmap;
-  if (!encode_activation_map(&xmap, X, T, K, Tpad)) return cudaErrorInvalidValue;
+  if (!encode_activation_map(&xmap, X, T, K, Tpad, 1)) return cudaErrorInvalidValue;
   const size_t stage = (size_t)kPfRows * 128 + (size_t)Tpad * 128;
   int ns = (int)((kPfSmemLimit - 1024) / stage);
   ns = ns > kPfMaxStages ? kPfMaxStages : ns;   // >= kPfMinStages: four stages of the largest tile fit

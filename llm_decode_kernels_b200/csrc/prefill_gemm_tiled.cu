@@ -53,9 +53,6 @@ DEVI uint32_t in_cta(uint32_t local, uint32_t rank) {   // the same shared-memor
 DEVI void bar_arrive_cluster(uint32_t addr) {
   asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(addr) : "memory");
 }
-DEVI void bar_expect(uint64_t* b, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(sa(b)), "r"(bytes) : "memory");
-}
 DEVI bool bar_try(uint64_t* b, uint32_t parity) {
   uint32_t ok;
   asm volatile(
@@ -76,14 +73,16 @@ DEVI unsigned long long now_ns() {
 template <int SLEEP_NS>
 DEVI bool bar_wait(uint64_t* b, uint32_t parity, volatile int* fail, int code) {
   if (bar_try(b, parity)) return true;
-  const unsigned long long t0 = now_ns();
+  unsigned long long t0 = 0;   // the timer is slow to read: only a wait that is late anyway looks at it
 #pragma unroll 1
   for (int i = 0; i < kSpin; ++i) {
     if (SLEEP_NS > 0) __nanosleep(SLEEP_NS);
     if (bar_try(b, parity)) return true;
-    if ((i & 31) == 31) {
+    if ((i & 63) == 63) {
       if (*fail) return false;
-      if (now_ns() - t0 > kWaitNs) break;
+      const unsigned long long t = now_ns();
+      if (!t0) t0 = t;
+      if (t - t0 > kWaitNs) break;
     }
   }
   *fail = 1;
@@ -101,6 +100,17 @@ DEVI float4 ld_cluster4(uint32_t addr) {
 // K-major tile, 128-byte swizzle: see umma_desc_sw128 in prefill_gemm.cu
 DEVI uint64_t desc_sw128(uint32_t addr) {
   return (uint64_t)((addr & 0x3FFFFu) >> 4) | (1ull << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61);
+}
+
+// one arrival on `bar` in both CTAs of the pair when the MMAs issued so far by the elected lane have completed (whole warp)
+DEVI void commit_pair(uint64_t* bar, uint32_t ctas) {
+  asm volatile(
+      "{\n\t.reg .pred e;\n\t.reg .b16 m;\n\t"
+      "cvt.u16.u32 m, %1;\n\t"
+      "elect.sync _|e, 0xffffffff;\n\t"
+      "@e tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], m;\n\t}" ::"r"(sa(bar)),
+      "r"(ctas)
+      : "memory");
 }
 
 DEVI void tmem_ld16(uint32_t addr, uint32_t (&v)[16]) {
@@ -198,7 +208,7 @@ prefill_gemm_tiled_kernel(const __grid_constant__ CUtensorMap xmap, const uint8_
   extern __shared__ uint8_t raw[];
   __shared__ Shared sh;
   uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(raw) + 1023) & ~(uintptr_t)1023);
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;   // warp: known to be uniform
   uint32_t rank;
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
   const int csize = 2 * S, first = blockIdx.x / csize, stride = gridDim.x / csize;
@@ -234,29 +244,42 @@ prefill_gemm_tiled_kernel(const __grid_constant__ CUtensorMap xmap, const uint8_
     // ---- A: thread = row; group `grp` takes every third unit of the sequence, with the next two in registers
     const int grp = warp >> 2, r = (warp & 3) * 32 + lane;
     const uint32_t lanes = (uint32_t)((warp & 3) * 32) << 16;
-    Walk at = {first, u0};
-    at.step(grp, u0, u1, stride);
-    Walk ahead = at;
+    const int nu = u1 - u0, total = first < tiles ? ((tiles - 1 - first) / stride + 1) * nu : 0;   // units of this CTA's sequence
+    // the unit loaded next: its place in the sequence and in its tile, and where this row's weights of it are (null past the matrix)
+    int li = grp, lu = grp, ltile = first;
+    const uint8_t* lp;
+    auto seek = [&] {
+      const int rt = 16 * (ltile % feat_tiles) + 8 * side + (r >> 4);
+      lp = ltile < tiles && rt < row_tiles ? Wt + ((size_t)rt * nunit + u0 + lu) * kTileUnitBytes : nullptr;
+    };
+    auto wrap = [&] {
+      while (lu >= nu) lu -= nu, ltile += stride;
+      seek();
+    };
+    wrap();
     auto load = [&](RowUnit& d) {
-      const int rt = 16 * (ahead.tile % feat_tiles) + 8 * side + (r >> 4);
-#pragma unroll
-      for (int i = 0; i < 4; ++i) d.w[i] = make_uint4(0u, 0u, 0u, 0u);
-      d.sz = __float2half2_rn(0.f);
-      if (ahead.tile < tiles && rt < row_tiles) {   // rows past the matrix: zero words, zero scale
-        const uint8_t* p = Wt + ((size_t)rt * nunit + ahead.u) * kTileUnitBytes;
-        const uint8_t* q = p + 64 * (r & 15);
+      if (lp && li < total) {
+        const uint8_t* q = lp + 64 * (r & 15);
         ld32(q, d.w[0], d.w[1]);
         ld32(q + 32, d.w[2], d.w[3]);
-        d.sz = __ldg(reinterpret_cast<const half2*>(p + 1024) + (r & 15));
+        d.sz = __ldg(reinterpret_cast<const half2*>(lp + 1024) + (r & 15));
+      } else {   // rows past the matrix: zero words, zero scale
+#pragma unroll
+        for (int i = 0; i < 4; ++i) d.w[i] = make_uint4(0u, 0u, 0u, 0u);
+        d.sz = __float2half2_rn(0.f);
       }
-      ahead.step(kDqGroups, u0, u1, stride);
+      li += kDqGroups;
+      lu += kDqGroups;
+      if (lu >= nu) wrap();
+      else if (lp) lp += kDqGroups * kTileUnitBytes;
     };
     RowUnit cur, next, after;
     load(cur);
     load(next);
     Ring ring = {grp, 0};
+    const uint32_t a_full0 = in_cta(sa(&sh.a_full[0]), lead);
 #pragma unroll 1
-    for (; at.tile < tiles; at.step(kDqGroups, u0, u1, stride)) {
+    for (int i = grp; i < total; i += kDqGroups) {
       load(after);
       if (ring.use > 0 && !__all_sync(0xffffffffu, bar_wait<64>(&sh.empty[ring.s], (ring.use - 1) & 1, fail, WAIT_DQ))) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -266,68 +289,78 @@ prefill_gemm_tiled_kernel(const __grid_constant__ CUtensorMap xmap, const uint8_
       asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
-      if (lane == 0) bar_arrive_cluster(in_cta(sa(&sh.a_full[ring.s]), lead));
+      if (lane == 0) bar_arrive_cluster(a_full0 + 8 * ring.s);
       ring.step(kDqGroups, ns);
       cur = next;
       next = after;
     }
   } else if (warp == kMmaWarp) {
-    if (side == 0 && lane == 0) {
+    if (side == 0) {
+      // The whole warp runs the loop and one elected lane issues. In code that only one lane enters the compiler cannot keep the
+      // descriptors in uniform registers, and the eight MMAs of a unit took 580 cycles to issue, more than they take to run.
       // D fp32, A and B fp16, both K-major, N / 8 in bits 17-22, M / 16 in bits 24-28 (M = 256 over the pair)
       const uint32_t idesc = (1u << 4) | ((uint32_t)(nt >> 3) << 17) | ((256u >> 4) << 24);
-      const uint16_t both = (uint16_t)(3u << lead);
-      auto commit = [&](uint64_t* bar) {
-        asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(sa(bar)),
-                     "h"(both)
-                     : "memory");
-      };
+      const uint32_t both = 3u << lead;
       bool ok = true;
       int done = 0;
       Ring ring = {0, 0};
+#pragma unroll 1
       for (int tile = first; tile < tiles && ok; tile += stride, ++done) {
-        if (done > 0) ok = bar_wait<0>(&sh.acc_empty, (done - 1) & 1, fail, WAIT_MMA_ACC);
+        if (done > 0) ok = __all_sync(0xffffffffu, bar_wait<0>(&sh.acc_empty, (done - 1) & 1, fail, WAIT_MMA_ACC));
+#pragma unroll 1
         for (int u = u0; u < u1 && ok; ++u) {
-          ok = bar_wait<0>(&sh.b_full[ring.s], ring.use & 1, fail, WAIT_MMA_B) &&
-               bar_wait<0>(&sh.a_full[ring.s], ring.use & 1, fail, WAIT_MMA_A);
+          ok = __all_sync(0xffffffffu, bar_wait<0>(&sh.b_full[ring.s], ring.use & 1, fail, WAIT_MMA_B) &&
+                                           bar_wait<0>(&sh.a_full[ring.s], ring.use & 1, fail, WAIT_MMA_A));
           if (!ok) break;
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           const uint32_t a = tmem_a + (uint32_t)(kACols * ring.s), bs = sa(base + ring.s * stage_bytes);
-          const uint64_t b0 = desc_sw128(bs), b1 = desc_sw128(bs + half_bytes);
-#pragma unroll
-          for (int k = 0; k < 8; ++k)
-            asm volatile(
-                "{\n\t.reg .pred p;\n\t"
-                "setp.ne.b32 p, %4, 0;\n\t"
-                "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(tmem),
-                "r"(a + 8 * k), "l"((k < 4 ? b0 + 2 * k : b1 + 2 * (k - 4))), "r"(idesc), "r"((u > u0 || k > 0) ? 1u : 0u)
-                : "memory");
-          commit(&sh.empty[ring.s]);
+          asm volatile(
+              "{\n\t.reg .pred e, p;\n\t.reg .b32 a1;\n\t.reg .b64 d;\n\t"
+              "tcgen05.fence::after_thread_sync;\n\t"
+              "elect.sync _|e, 0xffffffff;\n\t"
+              "setp.ne.b32 p, %5, 0;\n\t"
+              "@e tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %4, p;\n\t"
+              "setp.eq.b32 p, 0, 0;\n\t"
+              "add.u32 a1, %1, 8;\n\tadd.u64 d, %2, 2;\n\t@e tcgen05.mma.cta_group::2.kind::f16 [%0], [a1], d, %4, p;\n\t"
+              "add.u32 a1, %1, 16;\n\tadd.u64 d, %2, 4;\n\t@e tcgen05.mma.cta_group::2.kind::f16 [%0], [a1], d, %4, p;\n\t"
+              "add.u32 a1, %1, 24;\n\tadd.u64 d, %2, 6;\n\t@e tcgen05.mma.cta_group::2.kind::f16 [%0], [a1], d, %4, p;\n\t"
+              "add.u32 a1, %1, 32;\n\t@e tcgen05.mma.cta_group::2.kind::f16 [%0], [a1], %3, %4, p;\n\t"
+              "add.u32 a1, %1, 40;\n\tadd.u64 d, %3, 2;\n\t@e tcgen05.mma.cta_group::2.kind::f16 [%0], [a1], d, %4, p;\n\t"
+              "add.u32 a1, %1, 48;\n\tadd.u64 d, %3, 4;\n\t@e tcgen05.mma.cta_group::2.kind::f16 [%0], [a1], d, %4, p;\n\t"
+              "add.u32 a1, %1, 56;\n\tadd.u64 d, %3, 6;\n\t@e tcgen05.mma.cta_group::2.kind::f16 [%0], [a1], d, %4, p;\n\t"
+              "}" ::"r"(tmem),
+              "r"(a), "l"(desc_sw128(bs)), "l"(desc_sw128(bs + half_bytes)), "r"(idesc), "r"(u > u0 ? 1u : 0u)
+              : "memory");
+          commit_pair(&sh.empty[ring.s], both);
           ring.step(1, ns);
         }
-        if (ok) commit(&sh.acc_full);
+        if (ok) commit_pair(&sh.acc_full, both);
       }
     }
   } else if (warp == kTmaWarp) {
-    if (lane == 0) {
-      pdl_wait();   // X is the predecessor's output
+    pdl_wait();   // X is the predecessor's output
+    {
+      // like the MMA warp, all lanes run the loop; one copy brings both 64-column halves of a unit (a third dimension of the tensor
+      // map). Two copies a unit from a single-lane branch took 440 cycles of the pair's 970 per unit at few tokens.
       Ring ring = {0, 0};
+#pragma unroll 1
       for (Walk at = {first, u0}; at.tile < tiles; at.step(1, u0, u1, stride), ring.step(1, ns)) {
         uint64_t* full = &sh.b_full[ring.s];
-        if (ring.use > 0 && !bar_wait<0>(&sh.empty[ring.s], (ring.use - 1) & 1, fail, WAIT_TMA)) break;
+        if (ring.use > 0 && !__all_sync(0xffffffffu, bar_wait<0>(&sh.empty[ring.s], (ring.use - 1) & 1, fail, WAIT_TMA))) break;
         // both CTAs' halves count on the even CTA's barrier
-        if (side == 0) bar_expect(full, 2 * stage_bytes);
         const uint32_t bar = in_cta(sa(full), lead), dst = sa(base + ring.s * stage_bytes);
         const int y = (at.tile / feat_tiles) * nt + side * (nt >> 1);
-#pragma unroll
-        for (int h = 0; h < 2; ++h)
-          asm volatile(
-              "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
-                  dst + h * half_bytes),
-              "l"(&xmap), "r"(at.u * 128 + 64 * h), "r"(y), "r"(bar)
-              : "memory");
+        asm volatile(
+            "{\n\t.reg .pred e, l;\n\t"
+            "elect.sync _|e, 0xffffffff;\n\t"
+            "setp.eq.and.b32 l, %6, 0, e;\n\t"
+            "@l mbarrier.arrive.expect_tx.shared::cta.b64 _, [%7], %8;\n\t"
+            "@e cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], "
+            "[%5];\n\t}" ::"r"(dst),
+            "l"(&xmap), "r"(0), "r"(y), "r"(2 * at.u), "r"(bar), "r"(side), "r"(sa(full)), "r"((uint32_t)(2 * stage_bytes))
+            : "memory");
       }
       // giving up: let the copies in flight land before the shared memory goes away (the even CTA holds the barriers)
-      if (*fail && side == 0)
+      if (*fail && side == 0 && lane == 0)
         for (int s = 0; s < ns; ++s) {
           const int uses = ring.use + (s < ring.s ? 1 : 0);   // how often stage s has been filled
           for (int i = 0; uses > 0 && i < (1 << 16) && !bar_try(&sh.b_full[s], (uses - 1) & 1); ++i) __nanosleep(64);
@@ -480,24 +513,25 @@ cudaError_t prefill_gemm_tiled_dispatch(const void* Wt, const void* X, void* Y, 
   cudaError_t e = allow_dynamic_smem(prefill_gemm_tiled_kernel<false>, smem_max, allowed[0]);
   if (e == cudaSuccess) e = allow_dynamic_smem(prefill_gemm_tiled_kernel<true>, smem_max, allowed[1]);
   if (e != cudaSuccess) return e;
-  // Split K where that shortens the longest CTA. Measured, in microseconds: a unit 0.53 at any token count (MMA issue and
-  // dequantization below 256 tokens, the MMA itself at 256); a launch 3.4 and 0.019 per token behind it when a pair works alone,
-  // 4.4 / 5.6 and 0.022 when 2 / 4 pairs exchange partial tiles.
+  // Split K where that shortens the longest CTA. Measured, in microseconds: a unit takes 0.38 (dequantization and issue) or its MMA
+  // time, 0.53 at 256 tokens; a launch 2.5 and 0.0145 per token beside that when a pair works alone, 3.9 / 4.4 and 0.02 when 2 / 4
+  // pairs exchange partial tiles.
   int S = 1;
   double best = 0;
   for (int c = 1; c <= kMaxSplit; c *= 2) {
     const int room = resident_clusters(c, smem_max);
     if (room == 0 || (c > 1 && nunit / c < 2)) continue;
     const int waves = (tiles + room - 1) / room, units = (nunit + c - 1) / c;
-    const double cost = c == 1 ? 3.4 + 0.019 * (nt - 32) + waves * (units * 0.53 + 0.3)
-                               : waves * (3.2 + 0.6 * c + 0.022 * (nt - 32) + units * 0.53);
+    const double unit = nt * 0.00207 > 0.38 ? nt * 0.00207 : 0.38;
+    const double cost = c == 1 ? 2.5 + 0.0145 * nt + waves * (units * unit + 0.3)
+                               : waves * (3.4 + 0.25 * c + 0.02 * nt + units * unit);
     if (best == 0 || cost < best) best = cost, S = c;
   }
   if (force_split) S = force_split;
   const int room = resident_clusters(S, smem_max);
   if (room == 0) return cudaErrorNotSupported;
   CUtensorMap xmap;
-  if (!encode_activation_map(&xmap, X, T, K, nt / 2)) return cudaErrorInvalidValue;
+  if (!encode_activation_map(&xmap, X, T, K, nt / 2, 2)) return cudaErrorInvalidValue;
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
