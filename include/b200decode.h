@@ -251,8 +251,6 @@ typedef struct {
   const int* pos;         /* [T]: start, start + 1, ... */
   int T, start;
   void *x, *normed, *qkv, *attn, *o, *act;   /* fp16 work buffers: [T,H] [T,H] [T,(n_q+2n_kv)D] [T,n_q D] [T,H] [T,I] */
-  float* scratch;         /* partials of split attention, or NULL: short prompts behind a long context then run unsplit */
-  size_t scratch_floats;
 } b200_prefill_desc;
 int b200_prefill_chunk(const b200_prefill_desc* d, void* stream);
 

@@ -271,10 +271,11 @@ int b200_gemm_w4a16_max_tokens(void) { return b200::prefill_gemm_max_tokens(); }
 
 int b200_gemm_w4a16_status(int* code) {
   REQUIRE(code, B200_ERR_ARG);
-  int tiled = 0;
+  int tiled = 0, attention = 0;
   cudaError_t e = b200::prefill_gemm_status(code);
   if (e == cudaSuccess) e = b200::prefill_gemm_tiled_status(&tiled);
-  *code |= tiled;
+  if (e == cudaSuccess) e = b200::prefill_attention_status(&attention);
+  *code |= tiled | attention;
   return finish(e);
 }
 
@@ -288,7 +289,7 @@ int b200_prefill_chunk(const b200_prefill_desc* d, void* stream) {
   REQUIRE(d->H % 128 == 0 && (d->n_q * d->D) % 128 == 0 && d->I % 128 == 0, B200_ERR_SHAPE);
   REQUIRE(d->H <= 32768 && d->T <= (1 << 20), B200_ERR_LIMIT);
   for (const void* q : {d->emb, d->norm_f, (const void*)d->cos_t, (const void*)d->sin_t, (const void*)d->x, (const void*)d->normed,
-                        (const void*)d->qkv, (const void*)d->attn, (const void*)d->o, (const void*)d->act, (const void*)d->scratch})
+                        (const void*)d->qkv, (const void*)d->attn, (const void*)d->o, (const void*)d->act})
     REQUIRE(aligned16(q), B200_ERR_ALIGN);
   b200::PrefillParams p = {};
   p.layers = reinterpret_cast<const b200::StepLayer*>(d->layers);
@@ -296,7 +297,6 @@ int b200_prefill_chunk(const b200_prefill_desc* d, void* stream) {
   p.eps = d->eps; p.emb = d->emb; p.norm_f = d->norm_f; p.cos_t = d->cos_t; p.sin_t = d->sin_t; p.bt = d->bt;
   p.ids = d->ids; p.pos = d->pos; p.T = d->T; p.start = d->start;
   p.x = d->x; p.normed = d->normed; p.qkv = d->qkv; p.attn = d->attn; p.o = d->o; p.act = d->act;
-  p.scratch = d->scratch; p.scratch_floats = d->scratch ? d->scratch_floats : 0;
   return finish(b200::prefill_chunk_dispatch(p, S(stream)));
 }
 

@@ -34,8 +34,7 @@ cudaError_t prefill_chunk_dispatch(const PrefillParams& p, cudaStream_t st) {
     TRY(add_rmsnorm_dispatch(p.x, delta, ly.ln1, p.normed, p.T, p.H, p.eps, st));
     TRY(prefill_gemm_tiled_dispatch(ly.w[0], p.normed, p.qkv, p.T, n_qkv, p.H, 0, 0, st));
     TRY(rope_append_dispatch(p.qkv, p.cos_t, p.sin_t, p.pos, p.bt, 0, ly.kc, ly.vc, p.T, p.n_q, p.n_kv, p.D, p.log2P, st));
-    TRY(prefill_attention_dispatch(p.qkv, n_qkv, ly.kc, ly.vc, p.bt, p.pos, p.start, p.T, p.n_q, p.n_kv, p.D, p.log2P, p.scratch,
-                                   p.scratch_floats, p.attn, st));
+    TRY(prefill_attention_dispatch(p.qkv, n_qkv, ly.kc, ly.vc, p.bt, p.start, p.T, p.n_q, p.n_kv, p.D, p.log2P, p.attn, st));
     TRY(prefill_gemm_tiled_dispatch(ly.w[1], p.attn, p.o, p.T, p.H, n_att, 0, 0, st));
     TRY(add_rmsnorm_dispatch(p.x, p.o, ly.ln2, p.normed, p.T, p.H, p.eps, st));
     TRY(prefill_gemm_tiled_dispatch(ly.w[2], p.normed, p.act, p.T, p.I, p.H, 1, 0, st));

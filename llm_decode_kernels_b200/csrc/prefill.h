@@ -22,15 +22,13 @@ struct PrefillParams {
   const int* pos;            // [T] start, start + 1, ...
   int T, start;
   void *x, *normed, *qkv, *attn, *o, *act;   // fp16 [T, H], [T, H], [T, (n_q + 2 n_kv) D], [T, n_q D], [T, H], [T, I]
-  float* scratch;            // attention partials, or null
-  size_t scratch_floats;
 };
 
 cudaError_t prefill_chunk_dispatch(const PrefillParams& p, cudaStream_t st);
 bool prefill_attention_takes(int D, int n_q, int n_kv);
-cudaError_t prefill_attention_dispatch(const void* q, int q_stride, const void* kc, const void* vc, const int* bt, const int* pos,
-                                       int start, int T, int n_q, int n_kv, int D, int log2P, float* scratch, size_t scratch_len,
-                                       void* out, cudaStream_t st);
+cudaError_t prefill_attention_dispatch(const void* q, int q_stride, const void* kc, const void* vc, const int* bt, int start, int T,
+                                       int n_q, int n_kv, int D, int log2P, void* out, cudaStream_t st);
+cudaError_t prefill_attention_status(int* code);
 cudaError_t prefill_gemm_tiled_dispatch(const void* Wt, const void* X, void* Y, int T, int N, int K, int swiglu, int force_split,
                                         cudaStream_t st);
 cudaError_t add_rmsnorm_dispatch(void* x, const void* delta, const void* w, void* out, int rows, int H, float eps,
@@ -38,7 +36,5 @@ cudaError_t add_rmsnorm_dispatch(void* x, const void* delta, const void* w, void
 cudaError_t rope_append_dispatch(void* qkv, const float* cos_t, const float* sin_t, const int* pos, const int* bt,
                                  int bt_stride, void* kc, void* vc, int B, int n_q, int n_kv, int D, int log2P,
                                  cudaStream_t st);
-cudaError_t attention_combine_dispatch(const float* o_part, const float* m_part, const float* l_part, const int* pos, int PS,
-                                       int max_splits, int n_q, int B, int D, void* out, cudaStream_t st);
 
 }  // namespace b200

@@ -21,10 +21,13 @@
 // joins the cluster barriers, frees its tensor memory, and b200_gemm_w4a16_status is non-zero.
 #include "common.cuh"
 #include "prefill.h"
+#include "umma.cuh"
 
 namespace b200 {
 
 namespace {
+
+using namespace umma;
 
 __device__ int g_tiled_status = 0;   // 0, or the code of the first wait inside prefill_gemm_tiled_kernel that ran out
 
@@ -34,73 +37,7 @@ constexpr int kMaxStages = 6;          // 128-column units in flight: A in tenso
 constexpr int kACols = 64;             // tensor-memory columns of an A stage
 constexpr int kMaxTokens = 256;        // tokens per tile = N of the MMA (a multiple of 32)
 constexpr int kMaxSplit = 4;           // pairs per tile: clusters of at most 8 CTAs
-constexpr int kSpin = 1 << 20;         // polls before a wait gives up ...
-constexpr unsigned long long kWaitNs = 100000000ull;   // ... or this long
-
 enum : int { WAIT_DQ = 1, WAIT_MMA_ACC = 2, WAIT_MMA_B = 3, WAIT_MMA_A = 4, WAIT_TMA = 5, WAIT_EP = 6 };
-
-DEVI uint32_t sa(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-DEVI void bar_init(uint64_t* b, int count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(sa(b)), "r"(count));
-}
-DEVI uint32_t in_cta(uint32_t local, uint32_t rank) {   // the same shared-memory offset in CTA `rank` of the cluster
-  uint32_t r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(local), "r"(rank));
-  return r;
-}
-// Arrivals and waits carry no cluster-scope fence: what they order is tensor memory (the tcgen05 fences beside them) and bulk
-// copies (their own transaction counts); an acquire at cluster scope would empty the L1 on every poll.
-DEVI void bar_arrive_cluster(uint32_t addr) {
-  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(addr) : "memory");
-}
-DEVI bool bar_try(uint64_t* b, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(sa(b)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-DEVI unsigned long long now_ns() {
-  unsigned long long t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
-}
-// false if the phase did not complete within the bound or another role of the CTA has given up
-template <int SLEEP_NS>
-DEVI bool bar_wait(uint64_t* b, uint32_t parity, volatile int* fail, int code) {
-  if (bar_try(b, parity)) return true;
-  unsigned long long t0 = 0;   // the timer is slow to read: only a wait that is late anyway looks at it
-#pragma unroll 1
-  for (int i = 0; i < kSpin; ++i) {
-    if (SLEEP_NS > 0) __nanosleep(SLEEP_NS);
-    if (bar_try(b, parity)) return true;
-    if ((i & 63) == 63) {
-      if (*fail) return false;
-      const unsigned long long t = now_ns();
-      if (!t0) t0 = t;
-      if (t - t0 > kWaitNs) break;
-    }
-  }
-  *fail = 1;
-  atomicCAS(&g_tiled_status, 0, code);
-  return false;
-}
-DEVI void cluster_barrier() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-DEVI float4 ld_cluster4(uint32_t addr) {
-  float4 v;
-  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
-  return v;
-}
-// K-major tile, 128-byte swizzle: see umma_desc_sw128 in prefill_gemm.cu
-DEVI uint64_t desc_sw128(uint32_t addr) {
-  return (uint64_t)((addr & 0x3FFFFu) >> 4) | (1ull << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61);
-}
 
 // one arrival on `bar` in both CTAs of the pair when the MMAs issued so far by the elected lane have completed (whole warp)
 DEVI void commit_pair(uint64_t* bar, uint32_t ctas) {
@@ -113,21 +50,9 @@ DEVI void commit_pair(uint64_t* bar, uint32_t ctas) {
       : "memory");
 }
 
-DEVI void tmem_ld16(uint32_t addr, uint32_t (&v)[16]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n\t"
-      "tcgen05.wait::ld.sync.aligned;"
-      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
-        "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-      : "r"(addr)
-      : "memory");
-}
-DEVI void tmem_st16(uint32_t addr, const uint32_t (&v)[16]) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(addr),
-      "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]), "r"(v[10]),
-      "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
-      : "memory");
+template <int SLEEP_NS>
+DEVI bool bar_wait(uint64_t* b, uint32_t parity, volatile int* fail, int code) {
+  return umma::bar_wait<SLEEP_NS>(b, parity, fail, &g_tiled_status, code);
 }
 
 struct Shared {
@@ -217,8 +142,6 @@ prefill_gemm_tiled_kernel(const __grid_constant__ CUtensorMap xmap, const uint8_
   const int u0 = nunit * split / S, u1 = nunit * (split + 1) / S;
   const int half_bytes = nt * 64, stage_bytes = 2 * half_bytes;   // 64 columns of K x nt / 2 tokens; a unit
   volatile int* fail = &sh.fail;
-  pdl_launch_dependents();
-
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(sa(&sh.tmem)) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
@@ -237,6 +160,9 @@ prefill_gemm_tiled_kernel(const __grid_constant__ CUtensorMap xmap, const uint8_
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   cluster_barrier();   // the peers' barriers exist before anything arrives on them
+  // only now, with its tensor memory allocated: a dependent CTA that got there first and then waited for this grid would not give
+  // it back
+  pdl_launch_dependents();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = sh.tmem, tmem_a = tmem + (uint32_t)(512 - kACols * ns);
 

@@ -111,8 +111,7 @@ class PrefillDesc(ctypes.Structure):
                 ("D", c_int), ("V", c_int), ("log2P", c_int), ("eps", c_float), ("emb", c_void_p), ("norm_f", c_void_p),
                 ("cos_t", c_void_p), ("sin_t", c_void_p), ("bt", c_void_p), ("ids", c_void_p), ("pos", c_void_p),
                 ("T", c_int), ("start", c_int), ("x", c_void_p), ("normed", c_void_p), ("qkv", c_void_p),
-                ("attn", c_void_p), ("o", c_void_p), ("act", c_void_p), ("scratch", c_void_p),
-                ("scratch_floats", c_size_t)]
+                ("attn", c_void_p), ("o", c_void_p), ("act", c_void_p)]
 
 
 def load_library(build_if_missing=True, path=None):

@@ -674,16 +674,15 @@ class Model:
         widths = (self.H, self.H, self.H, (self.n_q + 2 * self.n_kv) * self.D, self.n_q * self.D, self.I)
         per_token = 2 * sum(widths)
         chunk = max(256, min(4096, (256 << 20) // per_token // 256 * 256))
-        scratch = 2 * 128 * 2 * 148 * (self.D + 2)     # floats: two waves of attention blocks, 128 query rows each
-        need = min(n, chunk) * per_token + 4 * scratch
+        need = min(n, chunk) * per_token
         if self._prefill_work is None or self._prefill_work.numel() < need:
             self._prefill_work = torch.empty(need, dtype=torch.uint8, device=dev)
         base = self._prefill_work.data_ptr()
-        d.scratch, d.scratch_floats, d.bt = base, scratch, self.bt.data_ptr()
+        d.bt = self.bt.data_ptr()
         all_logits = torch.empty(n, self.V_full, dtype=torch.half, device=dev) if collect_logits else None
         for c0 in range(0, n, chunk):
             T = min(chunk, n - c0)
-            at = base + 4 * scratch
+            at = base
             for name, w in zip(("x", "normed", "o", "qkv", "attn", "act"), widths):
                 setattr(d, name, at)
                 at += 2 * T * w
