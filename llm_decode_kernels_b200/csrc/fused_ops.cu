@@ -10,11 +10,15 @@ namespace b200 {
 // ---- residual add + RMSNorm -----------------------------------------------------------------------------
 // Replaces add_rmsnorm_launch (reference kernels/fused_norm.cu:56-58). Rounding as in HF LlamaRMSNorm
 // (reference reference/ref_ops.py:15-20): x <- x +_fp16 delta (written back); h = half(float(x) * rsqrt(
-// mean(float(x)^2) + eps)); out = w *_fp16 h. One block; each thread keeps its 8-element chunks in
-// registers across the reduction, so x is read once. With a batch (the prompt's tokens) block b takes row b.
+// mean(float(x)^2) + eps)); out = w *_fp16 h. A block takes a row, a thread up to CH 8-element chunks of it, held in
+// registers across the reduction, so x is read once. Latency-bound for one row, bound by L2 for many: a block has just the
+// threads that its row needs and issues all its loads at once. 4096 rows of 2048: 8.0 us (20.3 with 512 threads for every row
+// and the loads of a row one behind the other); one row of 2048: 1.6 us. Fewer threads with more chunks each (2, 4, 8): the
+// same or slower at every size but 4096 rows of 2048 (7.4 us).
 constexpr int kNormThreads = 512;
 constexpr int kNormMaxChunks = 8;  // H <= 512 * 8 * 8 = 32768
 
+template <int CH>
 __global__ void __launch_bounds__(kNormThreads)
 add_rmsnorm_kernel(half* __restrict__ x, const half* __restrict__ delta, const half* __restrict__ w,
                    half* __restrict__ out, int H, float eps) {
@@ -24,42 +28,50 @@ add_rmsnorm_kernel(half* __restrict__ x, const half* __restrict__ delta, const h
   out += (size_t)blockIdx.x * H;
   if (delta) delta += (size_t)blockIdx.x * H;
   __shared__ float part[kNormThreads / 32];
-  const int tid = threadIdx.x, nchunk = H >> 3;
-  uint4 xv[kNormMaxChunks];
+  const int tid = threadIdx.x, nt = blockDim.x, nchunk = H >> 3;
+  uint4 xv[CH], dv[CH], wv[CH];
+#pragma unroll
+  for (int c = 0; c < CH; ++c) {   // all loads first: one round trip
+    const int i = tid + c * nt;
+    if (i < nchunk) {
+      xv[c] = reinterpret_cast<const uint4*>(x)[i];
+      if (delta) dv[c] = reinterpret_cast<const uint4*>(delta)[i];
+      if (CH == 1) wv[c] = __ldg(reinterpret_cast<const uint4*>(w) + i);
+    }
+  }
   float ss = 0.f;
 #pragma unroll
-  for (int c = 0; c < kNormMaxChunks; ++c) {
-    const int i = tid + c * kNormThreads;
+  for (int c = 0; c < CH; ++c) {
+    const int i = tid + c * nt;
     if (i < nchunk) {
-      uint4 v = reinterpret_cast<const uint4*>(x)[i];
       if (delta) {
-        const uint4 d = reinterpret_cast<const uint4*>(delta)[i];
-        v.x = as_u32(__hadd2(as_h2(v.x), as_h2(d.x)));
-        v.y = as_u32(__hadd2(as_h2(v.y), as_h2(d.y)));
-        v.z = as_u32(__hadd2(as_h2(v.z), as_h2(d.z)));
-        v.w = as_u32(__hadd2(as_h2(v.w), as_h2(d.w)));
-        reinterpret_cast<uint4*>(x)[i] = v;
+        xv[c].x = as_u32(__hadd2(as_h2(xv[c].x), as_h2(dv[c].x)));
+        xv[c].y = as_u32(__hadd2(as_h2(xv[c].y), as_h2(dv[c].y)));
+        xv[c].z = as_u32(__hadd2(as_h2(xv[c].z), as_h2(dv[c].z)));
+        xv[c].w = as_u32(__hadd2(as_h2(xv[c].w), as_h2(dv[c].w)));
+        reinterpret_cast<uint4*>(x)[i] = xv[c];
       }
       float f[8];
-      unpack8(v, f);
+      unpack8(xv[c], f);
 #pragma unroll
       for (int k = 0; k < 8; ++k) ss = fmaf(f[k], f[k], ss);
-      xv[c] = v;
     }
   }
   ss = warp_sum(ss);
-  if ((tid & 31) == 0) part[tid >> 5] = ss;
-  __syncthreads();
-  float tot = 0.f;
-#pragma unroll
-  for (int k = 0; k < kNormThreads / 32; ++k) tot += part[k];
+  float tot = ss;
+  if (nt > 32) {
+    if ((tid & 31) == 0) part[tid >> 5] = ss;
+    __syncthreads();
+    tot = 0.f;
+    for (int k = 0; k < nt / 32; ++k) tot += part[k];
+  }
   const float r = rsqrtf(tot / (float)H + eps);
 #pragma unroll
-  for (int c = 0; c < kNormMaxChunks; ++c) {
-    const int i = tid + c * kNormThreads;
+  for (int c = 0; c < CH; ++c) {
+    const int i = tid + c * nt;
     if (i < nchunk) {
-      const uint4 wv = __ldg(reinterpret_cast<const uint4*>(w) + i);
-      const uint32_t xu[4] = {xv[c].x, xv[c].y, xv[c].z, xv[c].w}, wu[4] = {wv.x, wv.y, wv.z, wv.w};
+      if (CH > 1) wv[c] = __ldg(reinterpret_cast<const uint4*>(w) + i);
+      const uint32_t xu[4] = {xv[c].x, xv[c].y, xv[c].z, xv[c].w}, wu[4] = {wv[c].x, wv[c].y, wv[c].z, wv[c].w};
       uint32_t o[4];
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
@@ -73,8 +85,11 @@ add_rmsnorm_kernel(half* __restrict__ x, const half* __restrict__ delta, const h
 
 cudaError_t add_rmsnorm_dispatch(void* x, const void* delta, const void* w, void* out, int rows, int H, float eps,
                                  cudaStream_t st) {
-  B200_LAUNCH(add_rmsnorm_kernel, dim3(rows), dim3(kNormThreads), 0, st, (half*)x, (const half*)delta, (const half*)w,
-              (half*)out, H, eps);
+  const int nchunk = H >> 3, ch = (nchunk + kNormThreads - 1) / kNormThreads;
+  const int threads = ((nchunk + ch - 1) / ch + 31) & ~31;
+  auto kern = ch == 1 ? add_rmsnorm_kernel<1> : ch == 2 ? add_rmsnorm_kernel<2> : ch <= 4 ? add_rmsnorm_kernel<4>
+                                                                                      : add_rmsnorm_kernel<kNormMaxChunks>;
+  B200_LAUNCH(kern, dim3(rows), dim3(threads), 0, st, (half*)x, (const half*)delta, (const half*)w, (half*)out, H, eps);
   return cudaPeekAtLastError();
 }
 
