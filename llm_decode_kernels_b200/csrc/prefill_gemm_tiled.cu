@@ -428,34 +428,39 @@ cudaError_t prefill_gemm_tiled_status(int* code) {
 // Y[T, N]; N = rows of W (swiglu: of outputs, W has 2 N rows in paired layout). force_split: 0, or the S to use.
 cudaError_t prefill_gemm_tiled_dispatch(const void* Wt, const void* X, void* Y, int T, int N, int K, int swiglu, int force_split,
                                         cudaStream_t st) {
-  const int nunit = K / 128, row_tiles = swiglu ? (N + 7) / 8 : (N + 15) / 16;
-  const int feat_tiles = (row_tiles + 15) / 16, ntt = (T + kMaxTokens - 1) / kMaxTokens;
-  const int nt = ((T + ntt - 1) / ntt + 31) / 32 * 32;   // equal token tiles, so that the last one is not nearly empty
-  const int tiles = feat_tiles * ((T + nt - 1) / nt);
-  const int ns = nt <= 128 ? 6 : 4;   // what tensor memory has left beside the accumulator
+  const int nunit = K / 128, row_tiles = swiglu ? (N + 7) / 8 : (N + 15) / 16, feat_tiles = (row_tiles + 15) / 16;
   auto bytes = [](int tokens, int stages) { return 1024 + (size_t)tokens * (128 * stages + 256); };   // stages + fp16 tile
-  const size_t smem = bytes(nt, ns), smem_max = bytes(kMaxTokens, 4);
+  const size_t smem_max = bytes(kMaxTokens, 4);
   static size_t allowed[2][kMaxDevices] = {};
   cudaError_t e = allow_dynamic_smem(prefill_gemm_tiled_kernel<false>, smem_max, allowed[0]);
   if (e == cudaSuccess) e = allow_dynamic_smem(prefill_gemm_tiled_kernel<true>, smem_max, allowed[1]);
   if (e != cudaSuccess) return e;
-  // Split K where that shortens the longest CTA. Measured, in microseconds: a unit takes 0.38 (dequantization and issue) or its MMA
-  // time, 0.53 at 256 tokens; a launch 2.5 and 0.0145 per token beside that when a pair works alone, 3.9 / 4.4 and 0.02 when 2 / 4
-  // pairs exchange partial tiles.
-  int S = 1;
+  // Tokens per tile (equal tiles, so that the last is not nearly empty; up to eight more of them than there have to be) and split of
+  // K, by estimated time. In microseconds, fitted to 1,100 measured launches (TinyLlama, 8B and 70B matrices, 16 .. 4096 tokens;
+  // the pick is 0.5 % off the best of them on average, 8 % at worst; always the widest tiles: 8 % and 44 %): a unit takes 0.385
+  // (dequantization and issue) or its MMA time, 0.68 at 256 tokens with the chip full; beside that a launch takes 1.0 + 0.0162 a
+  // token where a pair works alone and 2.1 / 2.7 + 0.0206 a token where 2 / 4 pairs exchange partial tiles; and up to 2.8 are lost
+  // with the SMs that the launch leaves none of to the start of the next one.
+  int S = 0, nt = 0, tiles = 0;
   double best = 0;
+  const int least = (T + kMaxTokens - 1) / kMaxTokens;
   for (int c = 1; c <= kMaxSplit; c *= 2) {
     const int room = resident_clusters(c, smem_max);
-    if (room == 0 || (c > 1 && nunit / c < 2)) continue;
-    const int waves = (tiles + room - 1) / room, units = (nunit + c - 1) / c;
-    const double unit = nt * 0.00207 > 0.38 ? nt * 0.00207 : 0.38;
-    const double cost = c == 1 ? 2.5 + 0.0145 * nt + waves * (units * unit + 0.3)
-                               : waves * (3.4 + 0.25 * c + 0.02 * nt + units * unit);
-    if (best == 0 || cost < best) best = cost, S = c;
+    if (room == 0 || (force_split ? c != force_split : c > 1 && nunit / c < 2)) continue;
+    const int units = (nunit + c - 1) / c;
+    for (int ntt = least; ntt < least + 8; ++ntt) {
+      const int n = ((T + ntt - 1) / ntt + 31) / 32 * 32, count = feat_tiles * ((T + n - 1) / n), waves = (count + room - 1) / room;
+      const double unit = units * (n * 0.00264 > 0.385 ? n * 0.00264 : 0.385), fill = (double)count / room;
+      const double cost = (c == 1 ? 1.0 + 0.0162 * n + waves * (unit + 0.2) : waves * (1.45 + 0.32 * c + 0.0206 * n + unit)) +
+                          2.8 * (fill < 0.36 ? 0 : fill > 0.86 ? 1 : 2 * (fill - 0.36));
+      if (S == 0 || cost < best) best = cost, S = c, nt = n, tiles = count;
+      if (n == 32) break;
+    }
   }
-  if (force_split) S = force_split;
+  if (S == 0) return cudaErrorNotSupported;
+  const int ns = nt <= 128 ? 6 : 4;   // what tensor memory has left beside the accumulator
+  const size_t smem = bytes(nt, ns);
   const int room = resident_clusters(S, smem_max);
-  if (room == 0) return cudaErrorNotSupported;
   CUtensorMap xmap;
   if (!encode_activation_map(&xmap, X, T, K, nt / 2, 2)) return cudaErrorInvalidValue;
   cudaLaunchConfig_t cfg = {};
