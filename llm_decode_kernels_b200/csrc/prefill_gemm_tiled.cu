@@ -37,7 +37,7 @@ constexpr int kMaxStages = 6;          // 128-column units in flight: A in tenso
 constexpr int kACols = 64;             // tensor-memory columns of an A stage
 constexpr int kMaxTokens = 256;        // tokens per tile = N of the MMA (a multiple of 32)
 constexpr int kMaxSplit = 4;           // pairs per tile: clusters of at most 8 CTAs
-enum : int { WAIT_DQ = 1, WAIT_MMA_ACC = 2, WAIT_MMA_B = 3, WAIT_MMA_A = 4, WAIT_TMA = 5, WAIT_EP = 6 };
+enum : int { WAIT_DQ = 1, WAIT_MMA_ACC = 2, WAIT_MMA_FULL = 3, WAIT_TMA = 5, WAIT_EP = 6 };
 
 // one arrival on `bar` in both CTAs of the pair when the MMAs issued so far by the elected lane have completed (whole warp)
 DEVI void commit_pair(uint64_t* bar, uint32_t ctas) {
@@ -56,18 +56,9 @@ DEVI bool bar_wait(uint64_t* b, uint32_t parity, volatile int* fail, int code) {
 }
 
 struct Shared {
-  uint64_t a_full[kMaxStages], b_full[kMaxStages], empty[kMaxStages], acc_full, acc_empty;
+  uint64_t full[kMaxStages], empty[kMaxStages], acc_full, acc_empty;
   uint32_t tmem;
   int fail;
-};
-
-// Position in the sequence of 128-column units a CTA works through: the units [u0, u1) of its first tile, of its second, ...
-struct Walk {
-  int tile, u;
-  DEVI void step(int n, int u0, int u1, int stride) {
-    u += n;
-    while (u >= u1) u -= u1 - u0, tile += stride;
-  }
 };
 
 // Stage and how often it has been used before, of a sequence that takes the stages in turn.
@@ -88,19 +79,14 @@ DEVI void ld32(const uint8_t* p, uint4& a, uint4& b) {   // one whole 32-byte se
                : "l"(p));
 }
 
-// (q - z) * s per pair of weights, as dequant_w4a16_kernel. HI: nibbles at bits 4-7 / 20-23 are taken where they stand, as
-// 1024 + 16 q, and multiplied by s / 16 - the same product whenever s / 16 is exact in fp16 and 1024 + 16 z is sixteen times
-// what 1024 + z rounds z to (sixteenths_exact: not for a subnormal scale); it saves two shifts per word.
-DEVI bool sixteenths_exact(half2 sz) {
-  const half k1024 = __float2half_rn(1024.f), k16 = __float2half_rn(16.f), s = __low2half(sz), z = __high2half(sz);
-  return __heq(__hmul(__hmul(s, __float2half_rn(0.0625f)), k16), s) &&
-         __heq(__hsub(__hfma(z, k16, k1024), k1024), __hmul(__hsub(__hadd(z, k1024), k1024), k16));
-}
-template <bool HI>
+// (q - z) * s per pair of weights, as dequant_w4a16_kernel. Nibbles at bits 0-3 / 16-19 become 1024 + q, those at bits 4-7 / 20-23
+// where they stand 64 + q (ulp 1 and 1/16: both exact), and 64 + z is made of what 1024 + z rounds z to: the same difference, bit for
+// bit, without a shift. (As 1024 + 16 q and s / 16, which a subnormal s does not survive, it took a second form of the loop and a vote
+// between the two: 0.35 instead of 0.30 us a unit.)
+DEVI half2 nib_hi64(uint32_t w) { return as_h2((w & 0x00F000F0u) | 0x54005400u); }
 DEVI void dequant_store(const RowUnit& d, uint32_t dst) {
-  const half2 k1024 = __float2half2_rn(1024.f), z2 = __half2half2(__high2half(d.sz)), s2 = __half2half2(__low2half(d.sz));
-  const half2 zl = __hadd2(z2, k1024), zh = __hfma2(z2, __float2half2_rn(16.f), k1024);
-  const half2 s16 = __hmul2(s2, __float2half2_rn(0.0625f));
+  const half2 z2 = __half2half2(__high2half(d.sz)), s2 = __half2half2(__low2half(d.sz));
+  const half2 k1024 = __float2half2_rn(1024.f), zl = __hadd2(z2, k1024), zh = __hadd2(__hsub2(zl, k1024), __float2half2_rn(64.f));
 #pragma unroll
   for (int h = 0; h < 4; ++h) {   // 32 columns of K = 16 columns of tensor memory
     const uint32_t w4[4] = {d.w[h].x, d.w[h].y, d.w[h].z, d.w[h].w};
@@ -109,9 +95,9 @@ DEVI void dequant_store(const RowUnit& d, uint32_t dst) {
     for (int j = 0; j < 4; ++j) {
       const uint32_t w = w4[j], wh = w >> 8;
       o[4 * j] = as_u32(__hmul2(__hsub2(nib_lo(w), zl), s2));
-      o[4 * j + 1] = HI ? as_u32(__hmul2(__hsub2(nib_hi(w), zh), s16)) : as_u32(__hmul2(__hsub2(nib_lo(w >> 4), zl), s2));
+      o[4 * j + 1] = as_u32(__hmul2(__hsub2(nib_hi64(w), zh), s2));
       o[4 * j + 2] = as_u32(__hmul2(__hsub2(nib_lo(wh), zl), s2));
-      o[4 * j + 3] = HI ? as_u32(__hmul2(__hsub2(nib_hi(wh), zh), s16)) : as_u32(__hmul2(__hsub2(nib_lo(w >> 12), zl), s2));
+      o[4 * j + 3] = as_u32(__hmul2(__hsub2(nib_hi64(wh), zh), s2));
     }
     tmem_st16(dst + 16 * h, o);
   }
@@ -148,8 +134,7 @@ prefill_gemm_tiled_kernel(const __grid_constant__ CUtensorMap xmap, const uint8_
   }
   if (tid == 0) {
     for (int s = 0; s < ns; ++s) {
-      bar_init(&sh.a_full[s], 2 * 4);   // one group of dequantizing warps in each CTA of the pair
-      bar_init(&sh.b_full[s], 1);
+      bar_init(&sh.full[s], 2 * 4 + 1);   // one group of dequantizing warps in each CTA of the pair, and the copies
       bar_init(&sh.empty[s], 1);
     }
     bar_init(&sh.acc_full, 1);
@@ -203,19 +188,18 @@ prefill_gemm_tiled_kernel(const __grid_constant__ CUtensorMap xmap, const uint8_
     load(cur);
     load(next);
     Ring ring = {grp, 0};
-    const uint32_t a_full0 = in_cta(sa(&sh.a_full[0]), lead);
+    const uint32_t full0 = in_cta(sa(&sh.full[0]), lead);
 #pragma unroll 1
     for (int i = grp; i < total; i += kDqGroups) {
       load(after);
       if (ring.use > 0 && !__all_sync(0xffffffffu, bar_wait<64>(&sh.empty[ring.s], (ring.use - 1) & 1, fail, WAIT_DQ))) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t dst = tmem_a + lanes + (uint32_t)(kACols * ring.s);
-      if (__all_sync(0xffffffffu, sixteenths_exact(cur.sz))) dequant_store<true>(cur, dst);
-      else dequant_store<false>(cur, dst);
+      dequant_store(cur, dst);
       asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
-      if (lane == 0) bar_arrive_cluster(a_full0 + 8 * ring.s);
+      if (lane == 0) bar_arrive_cluster(full0 + 8 * ring.s);
       ring.step(kDqGroups, ns);
       cur = next;
       next = after;
@@ -235,8 +219,7 @@ prefill_gemm_tiled_kernel(const __grid_constant__ CUtensorMap xmap, const uint8_
         if (done > 0) ok = __all_sync(0xffffffffu, bar_wait<0>(&sh.acc_empty, (done - 1) & 1, fail, WAIT_MMA_ACC));
 #pragma unroll 1
         for (int u = u0; u < u1 && ok; ++u) {
-          ok = __all_sync(0xffffffffu, bar_wait<0>(&sh.b_full[ring.s], ring.use & 1, fail, WAIT_MMA_B) &&
-                                           bar_wait<0>(&sh.a_full[ring.s], ring.use & 1, fail, WAIT_MMA_A));
+          ok = __all_sync(0xffffffffu, bar_wait<0>(&sh.full[ring.s], ring.use & 1, fail, WAIT_MMA_FULL));
           if (!ok) break;
           const uint32_t a = tmem_a + (uint32_t)(kACols * ring.s), bs = sa(base + ring.s * stage_bytes);
           asm volatile(
@@ -265,31 +248,38 @@ prefill_gemm_tiled_kernel(const __grid_constant__ CUtensorMap xmap, const uint8_
   } else if (warp == kTmaWarp) {
     pdl_wait();   // X is the predecessor's output
     {
-      // like the MMA warp, all lanes run the loop; one copy brings both 64-column halves of a unit (a third dimension of the tensor
+      // What a unit costs this warp is what few tokens pay a unit, as for the MMA warp: one barrier for both operands, the token offset
+      // (a division) once a tile. Like the MMA warp, all lanes run the loop; one copy brings both 64-column halves of a unit (a third dimension of the tensor
       // map). Two copies a unit from a single-lane branch took 440 cycles of the pair's 970 per unit at few tokens.
       Ring ring = {0, 0};
+      bool ok = true;
+      const uint32_t full0 = in_cta(sa(&sh.full[0]), lead), own0 = sa(&sh.full[0]), dst0 = sa(base);   // both CTAs' halves count on the even CTA's barrier
 #pragma unroll 1
-      for (Walk at = {first, u0}; at.tile < tiles; at.step(1, u0, u1, stride), ring.step(1, ns)) {
-        uint64_t* full = &sh.b_full[ring.s];
-        if (ring.use > 0 && !__all_sync(0xffffffffu, bar_wait<0>(&sh.empty[ring.s], (ring.use - 1) & 1, fail, WAIT_TMA))) break;
-        // both CTAs' halves count on the even CTA's barrier
-        const uint32_t bar = in_cta(sa(full), lead), dst = sa(base + ring.s * stage_bytes);
-        const int y = (at.tile / feat_tiles) * nt + side * (nt >> 1);
-        asm volatile(
-            "{\n\t.reg .pred e, l;\n\t"
-            "elect.sync _|e, 0xffffffff;\n\t"
-            "setp.eq.and.b32 l, %6, 0, e;\n\t"
-            "@l mbarrier.arrive.expect_tx.shared::cta.b64 _, [%7], %8;\n\t"
-            "@e cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], "
-            "[%5];\n\t}" ::"r"(dst),
-            "l"(&xmap), "r"(0), "r"(y), "r"(2 * at.u), "r"(bar), "r"(side), "r"(sa(full)), "r"((uint32_t)(2 * stage_bytes))
-            : "memory");
+      for (int tile = first; tile < tiles && ok; tile += stride) {
+        const int y = (tile / feat_tiles) * nt + side * (nt >> 1);
+#pragma unroll 1
+        for (int u = u0; u < u1; ++u) {
+          if (ring.use > 0 && !__all_sync(0xffffffffu, bar_wait<0>(&sh.empty[ring.s], (ring.use - 1) & 1, fail, WAIT_TMA))) {
+            ok = false;
+            break;
+          }
+          asm volatile(
+              "{\n\t.reg .pred e, l;\n\t"
+              "elect.sync _|e, 0xffffffff;\n\t"
+              "setp.eq.and.b32 l, %6, 0, e;\n\t"
+              "@l mbarrier.arrive.expect_tx.shared::cta.b64 _, [%7], %8;\n\t"
+              "@e cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], "
+              "[%5];\n\t}" ::"r"(dst0 + ring.s * stage_bytes),
+              "l"(&xmap), "r"(0), "r"(y), "r"(2 * u), "r"(full0 + 8 * ring.s), "r"(side), "r"(own0 + 8 * ring.s), "r"((uint32_t)(2 * stage_bytes))
+              : "memory");
+          ring.step(1, ns);
+        }
       }
       // giving up: let the copies in flight land before the shared memory goes away (the even CTA holds the barriers)
       if (*fail && side == 0 && lane == 0)
         for (int s = 0; s < ns; ++s) {
           const int uses = ring.use + (s < ring.s ? 1 : 0);   // how often stage s has been filled
-          for (int i = 0; uses > 0 && i < (1 << 16) && !bar_try(&sh.b_full[s], (uses - 1) & 1); ++i) __nanosleep(64);
+          for (int i = 0; uses > 0 && i < (1 << 16) && !bar_try(&sh.full[s], (uses - 1) & 1); ++i) __nanosleep(64);
         }
     }
   } else {
@@ -436,8 +426,8 @@ cudaError_t prefill_gemm_tiled_dispatch(const void* Wt, const void* X, void* Y, 
   if (e == cudaSuccess) e = allow_dynamic_smem(prefill_gemm_tiled_kernel<true>, smem_max, allowed[1]);
   if (e != cudaSuccess) return e;
   // Tokens per tile (equal tiles, so that the last is not nearly empty; up to eight more of them than there have to be) and split of
-  // K, by estimated time. In microseconds, fitted to 1,100 measured launches (TinyLlama, 8B and 70B matrices, 16 .. 4096 tokens;
-  // the pick is 0.5 % off the best of them on average, 8 % at worst; always the widest tiles: 8 % and 44 %): a unit takes 0.385
+  // K, by estimated time. In microseconds, fitted to 1,250 measured launches (TinyLlama, 8B and 70B matrices, 16 .. 4096 tokens;
+  // the pick is 0.7 % off the best of them on average, 11 % at worst; always the widest tiles: 10 % and 51 %): a unit takes 0.30 - 0.35
   // (dequantization and issue) or its MMA time, 0.68 at 256 tokens with the chip full; beside that a launch takes 1.0 + 0.0162 a
   // token where a pair works alone and 2.1 / 2.7 + 0.0206 a token where 2 / 4 pairs exchange partial tiles; and up to 2.8 are lost
   // with the SMs that the launch leaves none of to the start of the next one.
@@ -450,8 +440,8 @@ cudaError_t prefill_gemm_tiled_dispatch(const void* Wt, const void* X, void* Y, 
     const int units = (nunit + c - 1) / c;
     for (int ntt = least; ntt < least + 8; ++ntt) {
       const int n = ((T + ntt - 1) / ntt + 31) / 32 * 32, count = feat_tiles * ((T + n - 1) / n), waves = (count + room - 1) / room;
-      const double unit = units * (n * 0.00264 > 0.385 ? n * 0.00264 : 0.385), fill = (double)count / room;
-      const double cost = (c == 1 ? 1.0 + 0.0162 * n + waves * (unit + 0.2) : waves * (1.45 + 0.32 * c + 0.0206 * n + unit)) +
+      const double unit = units * (n * 0.00264 > 0.35 ? n * 0.00264 : 0.35), fill = (double)count / room;
+      const double cost = (c == 1 ? 1.0 + 0.0162 * n + waves * (unit + 0.4) : waves * (1.45 + 0.32 * c + 0.0206 * n + unit)) +
                           2.8 * (fill < 0.36 ? 0 : fill > 0.86 ? 1 : 2 * (fill - 0.36));
       if (S == 0 || cost < best) best = cost, S = c, nt = n, tiles = count;
       if (n == 32) break;
