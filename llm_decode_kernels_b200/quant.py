@@ -114,8 +114,10 @@ def quantize_gptq(w: torch.Tensor, H: torch.Tensor, group: int, clip: bool = Fal
 
 def _gptq_columns(W, U, group, clip, block):
     """Fixes the columns of W fp32 [N, K] left to right (W is used up): levels, scales and zero points."""
-    if not (W.is_cuda and block <= 128 and group >= 4 and group & (group - 1) == 0):
+    if not (W.is_cuda and U.device == W.device and W.numel() > 0 and block <= 128 and group >= 4
+            and group & (group - 1) == 0):
         return _gptq_columns_torch(W, U, group, clip, block)
+    W = W.contiguous()      # the kernel walks rows of K; a transposed weight keeps its strides up to here
     N, K = W.shape
     Q = torch.empty(N, K, dtype=torch.uint8, device=W.device)
     S, Z = (torch.empty(N, K // group, device=W.device) for _ in range(2))

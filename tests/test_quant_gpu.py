@@ -48,3 +48,28 @@ def test_gptq_kernel_equals_torch_loop(monkeypatch, N, K, G, block, clip):
     ref = PQ.quantize_gptq(w, H, G, clip=clip, block=block)
     assert (got[0] != ref[0]).float().mean() < 2e-3
     assert all((a != b).float().mean() < 2e-3 for a, b in zip(got[1:], ref[1:]))
+
+
+@pytest.mark.parametrize("form", ["transposed", "columns of a wider matrix", "every second row"])
+def test_gptq_kernel_takes_any_strides(form):
+    g = torch.Generator(device="cuda").manual_seed(5)
+    N, K = 64, 256
+    if form == "transposed":
+        w = (torch.randn(K, N, generator=g, device="cuda") * 0.02).half().t()
+    elif form == "columns of a wider matrix":
+        w = (torch.randn(N, K + 64, generator=g, device="cuda") * 0.02).half()[:, 32:K + 32]
+    else:
+        w = (torch.randn(2 * N, K, generator=g, device="cuda") * 0.02).half()[::2]
+    assert w.shape == (N, K) and not w.is_contiguous()
+    x = torch.randn(4 * K, K, generator=g, device="cuda")
+    H = 2 * x.t() @ x / x.shape[0]
+    for a, b in zip(PQ.quantize_gptq(w, H, 64), PQ.quantize_gptq(w.contiguous(), H, 64)):
+        assert torch.equal(a, b)
+
+
+def test_gptq_without_rows_and_with_a_hessian_elsewhere():
+    H = torch.eye(128)
+    q, s, z = PQ.quantize_gptq(torch.empty(0, 128, device="cuda"), H.cuda(), 64)
+    assert q.shape == (0, 128) and s.shape == z.shape == (0, 2)
+    with pytest.raises(RuntimeError, match="device"):       # torch's own refusal; no host pointer reaches the kernel
+        PQ.quantize_gptq(torch.ones(4, 128, device="cuda"), H, 64)
