@@ -8,11 +8,13 @@
 // 16 a clock and SM: that, 61 us for 4096 tokens x 32 heads, is the floor here, so everything else runs beside it: the scores have two
 // buffers, so that those of the next tile are there when a tile is done; one warp issues the MMAs; half the loading warps copy cached
 // rows of K, half of V (cp.async, into the 128-byte-swizzled layout); two CTAs share an SM. The running maximum follows with a delay:
-// O is rescaled only when the maximum has grown by more than 2^8 (Zadouri et al., FlashAttention-4), which fp16 probabilities and fp32
-// sums take without loss.
-//   4096 tokens, 32 heads on 4 kv heads x 64: 106 us (277 with warp-level MMAs; the decode kernel, one pass over the cache per query
-//   token, took 1.8 ms). 512 tokens: 11 us. 1000 tokens, 64 heads on 8 x 128: 29 us.
-// What it waited for on the way, at 4096 tokens: 127 us with K and V in one ring whose loaders handed a tile over late; 119 with two
+// O is rescaled only when the maximum has grown by more than 2^8 (Zadouri et al., FlashAttention-4). Against such a maximum no
+// probability of a row is exactly 1, so fp16 alone would lose what the exact maximum keeps: the probabilities enter the second product
+// twice, as fp16 value and as fp16 remainder. Error against 64 bits, 200 tokens behind 1800: 2.08e-4, which is the rounding of the
+// output (2.88e-4 with the values alone; 2.52e-4 in fp16 against the exact maximum). It costs 23 of the 129 us at 4096 tokens.
+//   4096 tokens, 32 heads on 4 kv heads x 64: 129 us (277 with warp-level MMAs; the decode kernel, one pass over the cache per query
+//   token, took 1.8 ms). 512 tokens: 11 us.
+// What it waited for on the way, at 4096 tokens and without the remainders: 127 us with K and V in one ring whose loaders handed a tile over late; 119 with two
 // groups of softmax warps that take turns (scores of the next tile then come only behind the product of this one); queries through
 // registers, one round trip after the other, cost 3 us a CTA.
 // Where a short prompt continues a long context the CTAs are few: up to 8 CTAs (a cluster) then share the context of a row block and
@@ -223,16 +225,20 @@ prefill_attn_kernel(const half* __restrict__ q, int q_stride, const half* __rest
       const uint64_t sub2 = pair(sub, sub), scale2 = pair(sl2, sl2);
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
-        uint32_t p[kTile / 4];
+        uint32_t p[kTile / 4], r[kTile / 4];   // fp16 values and remainders
 #pragma unroll
         for (int c = 0; c < kTile / 2; c += 2) {
           float u, v;
           unpair(fma2(pair(s[kTile / 2 * h + c], s[kTile / 2 * h + c + 1]), scale2, sub2), u, v);
           u = ex2(u), v = ex2(v);
           sum[(c >> 1) & 1] = add2(sum[(c >> 1) & 1], pair(u, v));
-          p[c / 2] = as_u32(__floats2half2_rn(u, v));
+          const half2 hi = __floats2half2_rn(u, v);
+          const float2 f = __half22float2(hi);
+          p[c / 2] = as_u32(hi);
+          r[c / 2] = as_u32(__floats2half2_rn(u - f.x, v - f.y));
         }
-        tmem_st16(ts + (uint32_t)(kTile / 4 * h), p);   // over the scores
+        tmem_st16(ts + (uint32_t)(kTile / 4 * h), p);   // over the scores: values, then remainders
+        tmem_st16(ts + (uint32_t)(kTile / 2 + kTile / 4 * h), r);
       }
       asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -272,8 +278,8 @@ prefill_attn_kernel(const half* __restrict__ q, int q_stride, const half* __rest
       if (!ok) break;
       const uint32_t v_s = ring_s + (NS + i % NS) * TILE;
 #pragma unroll
-      for (int k = 0; k < kTile / 16; ++k)
-        mma_ts(tmem + kO, tmem + (uint32_t)(kTile * (i & 1) + 8 * k), desc_sw128(v_s, kTile * 128) + 128 * k, idesc_o,
+      for (int k = 0; k < kTile / 8; ++k)   // values, then remainders, both against all of V
+        mma_ts(tmem + kO, tmem + (uint32_t)(kTile * (i & 1) + 8 * k), desc_sw128(v_s, kTile * 128) + 128 * (k % (kTile / 16)), idesc_o,
                i > 0 || k > 0);
       commit(&sh.pv_done[i & 1]);
       if (n < ntiles) scores(n);   // over the scores and probabilities of tile i, behind the product that reads them
