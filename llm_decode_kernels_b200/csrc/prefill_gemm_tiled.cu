@@ -37,6 +37,10 @@ constexpr int kMaxStages = 6;          // 128-column units in flight: A in tenso
 constexpr int kACols = 64;             // tensor-memory columns of an A stage
 constexpr int kMaxTokens = 256;        // tokens per tile = N of the MMA (a multiple of 32)
 constexpr int kMaxSplit = 4;           // pairs per tile: clusters of at most 8 CTAs
+// Units of K that one accumulator sums: the tensor core drops bits at every step of a chain. Error against 64 bits at K = 28672 (224
+// units): 2.097e-4 in one chain, 2.077e-4 in two, of which 2.070e-4 is the rounding of the output; up to K = 8192 one chain loses
+// nothing (2.0758e-4 and 2.0736e-4). Longer rows are split whatever the cost rule says.
+constexpr int kMaxChain = 112;
 enum : int { WAIT_DQ = 1, WAIT_MMA_ACC = 2, WAIT_MMA_FULL = 3, WAIT_TMA = 5, WAIT_EP = 6 };
 
 // one arrival on `bar` in both CTAs of the pair when the MMAs issued so far by the elected lane have completed (whole warp)
@@ -434,7 +438,9 @@ cudaError_t prefill_gemm_tiled_dispatch(const void* Wt, const void* X, void* Y, 
   int S = 0, nt = 0, tiles = 0;
   double best = 0;
   const int least = (T + kMaxTokens - 1) / kMaxTokens;
-  for (int c = 1; c <= kMaxSplit; c *= 2) {
+  int least_split = 1;   // kMaxChain
+  while (least_split < kMaxSplit && nunit > kMaxChain * least_split && resident_clusters(2 * least_split, smem_max) > 0) least_split *= 2;
+  for (int c = force_split ? 1 : least_split; c <= kMaxSplit; c *= 2) {
     const int room = resident_clusters(c, smem_max);
     if (room == 0 || (force_split ? c != force_split : c > 1 && nunit / c < 2)) continue;
     const int units = (nunit + c - 1) / c;

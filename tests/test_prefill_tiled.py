@@ -124,3 +124,18 @@ def test_prompt_attention_loses_no_precision(D, n_q, n_kv, start, T, peak):
         ref[:, h] = torch.softmax(s, -1) @ v[:, h * n_kv // n_q]
     rounding = (ref.half().double() - ref).norm()
     assert (buffer(d.attn, n_q * D).reshape(T, n_q, D).double() - ref).norm() <= 1.1 * rounding
+
+
+def test_long_rows_are_split_for_precision(K):
+    """The library's own choice at K = 28672 and many tokens, where one accumulation chain per tile is fastest: the error against 64
+    bits is no larger than with K split in two (a chain loses the low bits of its addends at every step)."""
+    N, Kd, T = 8192, 28672, 256
+    ql, tiled = matrix(K, N, Kd)
+    x = torch.randn(T, Kd, generator=torch.Generator(device=dev).manual_seed(1), device=dev).half()
+    ref = torch.cat([x.double() @ w.double().t() for w in ql.w_ref.split(1024)], 1)
+    err = {}
+    for split in (0, 1, 2):
+        y = torch.empty(T, N, dtype=torch.half, device=dev)
+        K.gemm_w4a16_tiled(tiled, x, y, N, Kd, split=split)
+        err[split] = ((y.double() - ref).norm() / ref.norm()).item()
+    assert err[0] <= err[2] * (1 + 1e-4) < err[1]
