@@ -945,14 +945,15 @@ paged_attn_cluster_kernel(const half* __restrict__ q, const half* __restrict__ k
   uint4 qf[CH];
   const half* qkv = q + (size_t)b * (ROPE ? n_q + 2 * n_kv : n_q) * D;
   const half* qh = qkv + (size_t)(kvh * HPG + (g < HPG ? g : 0)) * D;
-  const float *cs = ROPE ? ra.cos_t + (size_t)pos * (D / 2) : nullptr, *sn = ROPE ? ra.sin_t + (size_t)pos * (D / 2) : nullptr;
+  const size_t rope_at = (size_t)max(pos, 0) * (D / 2);
+  const float *cs = ROPE ? ra.cos_t + rope_at : nullptr, *sn = ROPE ? ra.sin_t + rope_at : nullptr;
 #pragma unroll
   for (int c = 0; c < CH; ++c) {
     qf[c] = ROPE ? rotated8<D>(qh, cs, sn, t, c) : reinterpret_cast<const uint4*>(qh + t * (D / 4))[c];
     if (g >= HPG) qf[c] = make_uint4(0u, 0u, 0u, 0u);
   }
   int i_new = -1;   // which of this warp's blocks holds the new token
-  if (ROPE && pos < ctx && ((pos >> 4) - rank) % C == 0) {   // in this CTA
+  if (ROPE && pos >= 0 && pos < ctx && ((pos >> 4) - rank) % C == 0) {   // in this CTA
     const int nb = (pos >> 4) - rank;
     if (nb >= C * warp && (nb / C - warp) % kClWarps == 0) i_new = (nb / C - warp) / kClWarps;
     if (tid < 4 * CH) {
@@ -1033,6 +1034,7 @@ paged_attn_cluster_kernel(const half* __restrict__ q, const half* __restrict__ k
     }
   }
 
+  if (nblk <= 0) return;   // an idle slot of the batch (position -1), for all CTAs of the cluster alike: out and caches stay as they are
   // the warps of the CTA: acc[n][e] = O[head g][dim 64 (n / 8) + 8 (2 t + e) + n % 8]
   l += __shfl_xor_sync(0xffffffffu, l, 1);
   l += __shfl_xor_sync(0xffffffffu, l, 2);

@@ -413,6 +413,41 @@ def test_attention_in_clusters(K, B, n_q, n_kv, D, page, ctxs):
         assert rel_err(out[b], want) <= ATTN_TOL
 
 
+def _cluster_case(n_q, n_kv, D, ctxs, page=16):
+    pages = max(1, -(-max(ctxs) // page))
+    kc, vc = (torch.randn(len(ctxs) * pages, n_kv, page, D, device=dev).half() for _ in range(2))
+    bt = torch.arange(len(ctxs) * pages, dtype=torch.int32, device=dev).view(len(ctxs), pages)
+    pos = torch.tensor([c - 1 for c in ctxs], dtype=torch.int32, device=dev)
+    S = -(-max(ctxs) // 64) + 1
+    return kc, vc, bt, pos, [torch.empty(len(ctxs), n_q, S, *w, device=dev) for w in ((D,), (), ())]
+
+
+@pytest.mark.parametrize("D", [64, 128])
+def test_attention_in_clusters_idle_slots(K, D):
+    """Position -1: nothing is attended to, out and (with RoPE) the caches stay as they are."""
+    torch.manual_seed(D)
+    n_q, n_kv, ctxs = 8, 2, [0, 40, 0, 300]
+    kc, vc, bt, pos, scratch = _cluster_case(n_q, n_kv, D, ctxs)
+    q = torch.randn(4, n_q, D, device=dev).half()
+    out = torch.full((4, n_q, D), 7.0, dtype=torch.half, device=dev)
+    K.paged_attention_batched(q, kc, vc, bt, pos, 64, *scratch, out)
+    assert bool((out[0] == 7).all()) and bool((out[2] == 7).all())
+    for b in (1, 3):
+        assert rel_err(out[b], R.paged_attention_ref(q[b].cpu(), kc.cpu(), vc.cpu(), bt[b].cpu(), ctxs[b], 16)) <= ATTN_TOL
+
+
+@pytest.mark.parametrize("D", [64, 128])
+def test_rope_attention_at_position_minus_one(K, D):
+    torch.manual_seed(D)
+    n_q, n_kv = 8, 2
+    kc, vc, bt, pos, scratch = _cluster_case(n_q, n_kv, D, [0])
+    cos, sin = (t.to(dev) for t in R.rope_tables(64, D))
+    k0, v0, out = kc.clone(), vc.clone(), torch.full((n_q, D), 7.0, dtype=torch.half, device=dev)
+    qkv = torch.randn((n_q + 2 * n_kv) * D, device=dev).half()
+    K.rope_paged_attention(qkv, cos, sin, pos, bt[0], kc, vc, n_q, n_kv, 64, *[t[0] for t in scratch], out)
+    assert torch.equal(kc, k0) and torch.equal(vc, v0) and bool((out == 7).all())
+
+
 @pytest.mark.parametrize("H", [2048, 8192, 128, 4104])
 def test_add_rmsnorm(K, H):
     torch.manual_seed(H)
