@@ -1057,7 +1057,7 @@ paged_attn_cluster_kernel(const half* __restrict__ q, const half* __restrict__ k
     float M = -CUDART_INF_F, o = 0.f, L = 0.f;
 #pragma unroll
     for (int w = 0; w < kClWarps; ++w) M = fmaxf(M, wm[w][h]);
-    if (M > -CUDART_INF_F) {   // a CTA without a block: nothing
+    if (rank < nblk) {   // a CTA without a block: nothing. (M does not tell: it is -inf as well where every score is NaN)
 #pragma unroll
       for (int w = 0; w < kClWarps; ++w) {
         const float a = exp2f(wm[w][h] - M);

@@ -448,6 +448,17 @@ def test_rope_attention_at_position_minus_one(K, D):
     assert torch.equal(kc, k0) and torch.equal(vc, v0) and bool((out == 7).all())
 
 
+@pytest.mark.parametrize("ctx", [129, 20, 1000])
+def test_attention_in_clusters_keeps_nan(K, ctx):
+    """A block of 16 tokens whose keys are all NaN (all that a CTA of the cluster has, at 129 tokens): the output is NaN."""
+    torch.manual_seed(ctx)
+    kc, vc, bt, pos, scratch = _cluster_case(8, 1, 64, [ctx])
+    kc[bt[0, 1]] = float("nan")
+    out = torch.zeros(1, 8, 64, dtype=torch.half, device=dev)
+    K.paged_attention_batched(torch.randn(1, 8, 64, device=dev).half(), kc, vc, bt, pos, 64, *scratch, out)
+    assert torch.isnan(out.float()).all()
+
+
 @pytest.mark.parametrize("H", [2048, 8192, 128, 4104])
 def test_add_rmsnorm(K, H):
     torch.manual_seed(H)
