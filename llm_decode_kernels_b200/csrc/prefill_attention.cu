@@ -115,6 +115,60 @@ DEVI void mma_ts(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t ac
       : "memory");
 }
 
+// A token must not depend on later ones, but the products above multiply whole tiles: a probability of zero against an infinity or a
+// NaN in the value row of a later token of the block is NaN. Where that may be why some of the dims [d0, d1) of a row came out NaN, they
+// are computed once more from the tokens the row sees, by one thread (a row that sees a NaN itself stays as it is). Kept out of
+// line, behind one test per row: the code of it in the epilogue costs a short prompt 1 us a launch.
+struct RowArgs {
+  const half *q, *kc, *vc;   // the row's query; the caches
+  const int* bt;
+  int kvh, n_kv, log2P, pos, last;   // last: the last position the row was multiplied with
+  float sl2;
+  half* out;                 // the row
+};
+template <int D>
+__device__ __noinline__ void redo_row(const RowArgs a, int d0, int d1) {
+  auto row = [&](int j) { return (((((size_t)a.bt[j >> a.log2P] * a.n_kv + a.kvh) << a.log2P) + (j & ((1 << a.log2P) - 1))) * D); };
+#pragma unroll 1
+  for (int d = d0; d < d1; d += 4) {
+    const uint2 was = *reinterpret_cast<const uint2*>(a.out + d);
+    const half2 z = __hadd2(as_h2(was.x), as_h2(was.y));
+    if (!__hisnan(__low2half(z)) && !__hisnan(__high2half(z))) continue;
+    bool hidden = false;
+#pragma unroll 1
+    for (int j = a.pos + 1; j <= a.last; ++j) {
+      const uint2 v = *reinterpret_cast<const uint2*>(a.vc + row(j) + d);
+      hidden |= (v.x & 0x7C00u) == 0x7C00u || (v.x & 0x7C000000u) == 0x7C000000u || (v.y & 0x7C00u) == 0x7C00u || (v.y & 0x7C000000u) == 0x7C000000u;
+    }
+    if (!hidden) continue;
+    float m = -CUDART_INF_F, l = 0.f, o[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 1
+    for (int j = 0; j <= a.pos; ++j) {
+      const size_t at = row(j);
+      float s = 0.f;
+#pragma unroll 1
+      for (int c = 0; c < D; c += 8) {
+        float x[8], y[8];
+        unpack8(*reinterpret_cast<const uint4*>(a.q + c), x);
+        unpack8(*reinterpret_cast<const uint4*>(a.kc + at + c), y);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) s = fmaf(x[e], y[e], s);
+      }
+      s *= a.sl2;
+      if (s != s) return;
+      const float mn = fmaxf(m, s), f = m == mn ? 1.f : exp2f(m - mn), p = s == -CUDART_INF_F ? 0.f : exp2f(s - mn);
+      m = mn, l = fmaf(l, f, p);
+      const uint2 v = *reinterpret_cast<const uint2*>(a.vc + at + d);
+      const float2 v0 = __half22float2(as_h2(v.x)), v1 = __half22float2(as_h2(v.y));
+      const float w[4] = {v0.x, v0.y, v1.x, v1.y};
+#pragma unroll
+      for (int e = 0; e < 4; ++e) o[e] = fmaf(p, w[e], o[e] * f);
+    }
+    const float f = 1.f / l;
+    *reinterpret_cast<uint2*>(a.out + d) = make_uint2(as_u32(__floats2half2_rn(o[0] * f, o[1] * f)), as_u32(__floats2half2_rn(o[2] * f, o[3] * f)));
+  }
+}
+
 }  // namespace
 
 // Grid (row blocks x n_kv, 1, splits), clusters (1, 1, splits). q rows: token t at q + t * q_stride, heads one after the other.
@@ -350,6 +404,7 @@ prefill_attn_kernel(const half* __restrict__ q, int q_stride, const half* __rest
   if (warp < kSoftWarps && !*fail) {
     const int r = row0 + tid, t = r >> log2hpg, h = (kvh << log2hpg) + (r & (hpg - 1));
     const float f = C == 1 ? 1.f / l : 1.f;
+    half2 any = __float2half2_rn(0.f);   // NaN if one of the row is (or if infinities of both signs are: redo_row looks closer)
     half* o = out + ((size_t)t * n_q + h) * D;
 #pragma unroll 1
     for (int c = 0; c < D; c += 16) {
@@ -368,6 +423,8 @@ prefill_attn_kernel(const half* __restrict__ q, int q_stride, const half* __rest
           reinterpret_cast<uint4*>(o + c)[0] = make_uint4(u[0], u[1], u[2], u[3]);
           reinterpret_cast<uint4*>(o + c)[1] = make_uint4(u[4], u[5], u[6], u[7]);
         }
+#pragma unroll
+        for (int e = 0; e < 8; ++e) any = __hadd2(any, as_h2(u[e]));
       } else {
 #pragma unroll
         for (int e = 0; e < 16; e += 4)
@@ -375,6 +432,8 @@ prefill_attn_kernel(const half* __restrict__ q, int q_stride, const half* __rest
       }
     }
     ml[tid] = make_float2(m, l);
+    if (t < T && (__hisnan(__low2half(any)) || __hisnan(__high2half(any))))
+      redo_row<D>(RowArgs{q + (size_t)t * q_stride + (size_t)h * D, kc, vc, bt, kvh, n_kv, log2P, start + t, last, sl2, o}, 0, D);
   }
   if (C > 1) {
     cluster_barrier();
@@ -402,9 +461,14 @@ prefill_attn_kernel(const half* __restrict__ q, int q_stride, const half* __rest
             o.x = fmaf(a, v[c].x, o.x), o.y = fmaf(a, v[c].y, o.y), o.z = fmaf(a, v[c].z, o.z), o.w = fmaf(a, v[c].w, o.w);
           }
         const float f = 1.f / L;
-        if (t < T)
-          *reinterpret_cast<uint2*>(out + ((size_t)t * n_q + (kvh << log2hpg) + (r & (hpg - 1))) * D + d) =
-              make_uint2(as_u32(__floats2half2_rn(o.x * f, o.y * f)), as_u32(__floats2half2_rn(o.z * f, o.w * f)));
+        if (t < T) {
+          const int h = (kvh << log2hpg) + (r & (hpg - 1));
+          half* to = out + ((size_t)t * n_q + h) * D + d;
+          *reinterpret_cast<uint2*>(to) = make_uint2(as_u32(__floats2half2_rn(o.x * f, o.y * f)), as_u32(__floats2half2_rn(o.z * f, o.w * f)));
+          const float any = (o.x + o.y + o.z + o.w) * f;
+          if (any != any)
+            redo_row<D>(RowArgs{q + (size_t)t * q_stride + (size_t)h * D, kc, vc, bt, kvh, n_kv, log2P, start + t, last, sl2, to - d}, d, d + 4);
+        }
       }
     }
     cluster_barrier();   // nobody's shared memory goes away while a peer still reads it

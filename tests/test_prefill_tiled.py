@@ -139,3 +139,25 @@ def test_long_rows_are_split_for_precision(K):
         K.gemm_w4a16_tiled(tiled, x, y, N, Kd, split=split)
         err[split] = ((y.double() - ref).norm() / ref.norm()).item()
     assert err[0] <= err[2] * (1 + 1e-4) < err[1]
+
+
+# A token whose keys and values are NaN (as after an overflow): the tokens before it are what they are without it - in the same tile
+# of 64, in the row block before, and where the context is split between CTAs.
+@pytest.mark.parametrize("D,n_q,n_kv,start,T,bad", [(64, 8, 1, 0, 40, 37), (64, 8, 8, 0, 150, 100), (64, 16, 2, 0, 70, 0), (128, 8, 2, 30, 90, 64),
+                                                    (64, 8, 1, 1500, 12, 9), (128, 8, 1, 1100, 20, 3)])
+def test_tokens_do_not_see_a_later_nan(D, n_q, n_kv, start, T, bad):
+    from llm_decode_kernels_b200.model import DecodeConfig, Model
+    from test_model import KERNEL_TOL, hf_cfg, random_state
+    c = hf_cfg(512, 2, n_q, n_kv, 1024, 1000, D=D)
+    m = Model(random_state(c, 3, D), c, DecodeConfig(group=128, max_ctx=start + T + 16, page=16, seed=1))
+    m.prepare(start + T + 8, use_graph=False)
+    m.kv.normal_(generator=torch.Generator(device=dev).manual_seed(2))
+    m.emb[999] = float("inf")
+    ids = torch.randint(0, 999, (T,), generator=torch.Generator().manual_seed(4))
+    m.reset(start)
+    want = m.prefill(ids, collect_logits=True).float()
+    ids[bad] = 999
+    m.reset(start)
+    got = m.prefill(ids, collect_logits=True).float()
+    assert torch.isnan(got[bad:]).all()
+    assert bad == 0 or (got[:bad] - want[:bad]).abs().max() <= KERNEL_TOL * want.abs().max()
