@@ -53,14 +53,27 @@ DEVI f2 fma2(f2 a, f2 b, f2 c) {
   return r;
 }
 
+// minimum and maximum that keep a NaN (fminf and fmaxf drop it): a damaged weight makes its group's parameters NaN, as torch's
+// amin, amax and clamp do, instead of ordinary ones that hide it
+DEVI float min_nan(float a, float b) {
+  float r;
+  asm("min.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+  return r;
+}
+DEVI float max_nan(float a, float b) {
+  float r;
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+  return r;
+}
+
 struct GroupScale { float s, z, rs; };   // scale, zero point, fl(1 / scale)
 
 // scale and zero point of a group with range [lo, hi]
 DEVI GroupScale scale_zero(float lo, float hi) {
   GroupScale g;
   const float c15 = 1.0f / 15.0f;
-  g.s = __half2float(__float2half_rn(fmaxf(__fmul_rn(__fsub_rn(hi, lo), c15), 1e-6f)));
-  g.z = fminf(fmaxf(rintf(__fdiv_rn(-lo, g.s)), 0.f), 15.f);
+  g.s = __half2float(__float2half_rn(max_nan(__fmul_rn(__fsub_rn(hi, lo), c15), 1e-6f)));
+  g.z = min_nan(max_nan(rintf(__fdiv_rn(-lo, g.s)), 0.f), 15.f);
   g.rs = __frcp_rn(g.s);
   return g;
 }
@@ -118,10 +131,10 @@ template <int V>
 DEVI GroupScale group_params(const float (&w)[V], int lanes, bool clip, float* wmax) {
   float lo = w[0], hi = w[0];
 #pragma unroll
-  for (int i = 1; i < V; ++i) lo = fminf(lo, w[i]), hi = fmaxf(hi, w[i]);
+  for (int i = 1; i < V; ++i) lo = min_nan(lo, w[i]), hi = max_nan(hi, w[i]);
   for (int o = 1; o < lanes; o <<= 1) {
-    lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
-    hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+    lo = min_nan(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+    hi = max_nan(hi, __shfl_xor_sync(0xffffffffu, hi, o));
   }
   *wmax = fmaxf(-lo, hi);
   if (!clip) return scale_zero(lo, hi);

@@ -73,3 +73,48 @@ def test_gptq_without_rows_and_with_a_hessian_elsewhere():
     assert q.shape == (0, 128) and s.shape == z.shape == (0, 2)
     with pytest.raises(RuntimeError, match="device"):       # torch's own refusal; no host pointer reaches the kernel
         PQ.quantize_gptq(torch.ones(4, 128, device="cuda"), H, 64)
+
+
+def damaged(N, K, G, dtype):
+    """Groups of every kind a damaged matrix holds, one per row: NaN alone or everywhere, infinities of one or both signs."""
+    g = torch.Generator(device="cuda").manual_seed(9)
+    w = torch.randn(N, K, generator=g, device="cuda") * 0.02
+    nan, inf = float("nan"), float("inf")
+    w[0, G + 3] = nan
+    w[1, :G] = nan
+    w[2, 2 * G - 1], w[2, G] = inf, -inf
+    w[3, G + 1] = inf
+    w[4, G + 2] = -inf
+    w[5, :G] = inf
+    w[6, :3] = torch.tensor([nan, inf, -inf])
+    return w.to(dtype)
+
+
+@pytest.mark.parametrize("G", [8, 32, 128])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("clip", [False, True])
+def test_quantize_kernel_shows_damaged_weights(G, dtype, clip):
+    w = damaged(9, 4 * G, G, dtype)
+    q0, s0, z0 = PQ._quantize_torch(w, G, clip)
+    q, s, z = PQ.quantize(w, G, clip)
+    assert torch.isnan(s0[:2]).any() and torch.isinf(s0[2, 1])
+    assert torch.equal(torch.isfinite(s), torch.isfinite(s0)) and torch.equal(torch.isfinite(z), torch.isfinite(z0))
+    bad = ~(torch.isfinite(s0) & torch.isfinite(z0))
+    assert torch.allclose(s[bad], s0[bad], rtol=0, equal_nan=True) and torch.allclose(z[bad], z0[bad], rtol=0, equal_nan=True)
+    rows = bad.repeat_interleave(G, 1)
+    assert torch.equal(q[rows], q0[rows])
+    ref = PQ.QuantLinear(w, G, clip=clip).w_ref
+    assert torch.allclose(ref[rows], PQ.dequantize(q0, s0, z0, G)[rows], rtol=0, equal_nan=True)
+
+
+@pytest.mark.parametrize("clip", [False, True])
+def test_gptq_kernel_shows_damaged_weights(monkeypatch, clip):
+    G = 64
+    w = damaged(9, 4 * G, G, torch.float32)
+    x = torch.randn(2048, 4 * G, generator=torch.Generator(device="cuda").manual_seed(1), device="cuda")
+    H = 2 * x.t() @ x / x.shape[0]
+    got = PQ.quantize_gptq(w, H, G, clip=clip)
+    monkeypatch.setattr(PQ, "_gptq_columns", PQ._gptq_columns_torch)
+    ref = PQ.quantize_gptq(w, H, G, clip=clip)
+    for a, b in zip(got[1:], ref[1:]):
+        assert torch.equal(torch.isnan(a), torch.isnan(b)) and torch.isnan(b[:2]).any()
