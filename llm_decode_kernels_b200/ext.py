@@ -526,6 +526,8 @@ class Ops:
         """w [N, K] fp16 / bf16 / fp32 -> whichever outputs are given: packed int32 [N, K/8], sz fp16 [N, K/G, 2], levels q
         uint8 [N, K], scale and zero fp16 [N, K/G], dequantized deq fp16 [N, K]."""
         w = _cuda(w.contiguous(), "w")
+        if w.data_ptr() % 16:      # a view that starts in the middle of a buffer; the kernel reads 16 bytes at a time
+            w = w.clone()
         N, K = w.shape
         ptr = [None if t is None else t.data_ptr() for t in (packed, sz, q, scale, zero, deq)]
         with torch.cuda.device(w.device):

@@ -118,3 +118,13 @@ def test_gptq_kernel_shows_damaged_weights(monkeypatch, clip):
     ref = PQ.quantize_gptq(w, H, G, clip=clip)
     for a, b in zip(got[1:], ref[1:]):
         assert torch.equal(torch.isnan(a), torch.isnan(b)) and torch.isnan(b[:2]).any()
+
+
+@pytest.mark.parametrize("dtype,offset", [(torch.float16, 1), (torch.float16, 4), (torch.bfloat16, 3), (torch.float32, 2)])
+def test_quantize_takes_views_off_a_16_byte_boundary(dtype, offset):
+    flat = torch.randn(offset + 32 * 256, generator=torch.Generator(device="cuda").manual_seed(2), device="cuda").to(dtype)
+    w = flat[offset:].view(32, 256)
+    assert w.is_contiguous() and w.data_ptr() % 16
+    for a, b in zip(PQ.quantize(w, 64), PQ.quantize(w.clone(), 64)):
+        assert torch.equal(a, b)
+    assert torch.equal(PQ.QuantLinear(w, 64).packed, PQ.QuantLinear(w.clone(), 64).packed)
