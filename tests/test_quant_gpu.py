@@ -128,3 +128,17 @@ def test_quantize_takes_views_off_a_16_byte_boundary(dtype, offset):
     for a, b in zip(PQ.quantize(w, 64), PQ.quantize(w.clone(), 64)):
         assert torch.equal(a, b)
     assert torch.equal(PQ.QuantLinear(w, 64).packed, PQ.QuantLinear(w.clone(), 64).packed)
+
+
+def test_quantize_under_autograd_and_vmap_is_the_torch_form():
+    w = torch.randn(4, 32, 256, generator=torch.Generator(device="cuda").manual_seed(3), device="cuda")
+    p = torch.nn.Parameter(w[0].clone())
+    _, s, _ = PQ.quantize(p, 64)
+    s.float().sum().backward()
+    want = w[0].clone().requires_grad_()
+    PQ._quantize_torch(want, 64)[1].float().sum().backward()
+    assert torch.equal(p.grad, want.grad)
+    with torch.no_grad():      # an ordinary parameter, as a loader passes it
+        assert not PQ.quantize(p, 64)[1].requires_grad
+    for a, b in zip(torch.vmap(lambda m: PQ.quantize(m, 64))(w), map(torch.stack, zip(*(PQ.quantize(m, 64) for m in w)))):
+        assert torch.equal(a, b)
