@@ -368,7 +368,7 @@ size_t b200_decode_step_xchg_bytes(int L, int H, int I, int n_q, int n_kv, int D
 size_t b200_decode_step_att_bytes(int L, int n_q, int n_kv, int D, int grid) {
   if (L <= 0 || grid <= 0 || n_q <= 0 || n_kv <= 0 || n_q % n_kv) return 0;
   const int wide = b200::step_att_max(grid, n_q, n_kv);
-  if (wide <= b200::step_att_slices(grid, n_q)) return 0;
+  if (wide <= b200::step_att_slices(grid, n_q)) return 0;   // a layer's block of the exchange holds as many
   return b200::step_att_words_per_layer(n_q, D, wide) * L * sizeof(uint32_t);
 }
 
@@ -405,7 +405,7 @@ int b200_decode_step(const b200_step_desc* d, void* stream) {
   p.trace = d->trace;
   p.att_slices = b200::step_att_slices(d->grid, d->n_q);
   p.att_groups = b200::step_att_groups(d->n_q, d->n_kv);
-  p.att_max = d->att_xchg ? b200::step_att_max(d->grid, d->n_q, d->n_kv) : 0;
+  p.att_max = d->att_xchg && b200_decode_step_att_bytes(d->L, d->n_q, d->n_kv, d->D, d->grid) ? b200::step_att_max(d->grid, d->n_q, d->n_kv) : 0;
   p.att_xchg = (uint32_t*)d->att_xchg;
   p.layer_words = (int)b200::step_words_per_layer(d->H, d->I, d->n_q, d->n_kv, d->D, p.att_slices);
   p.att_layer_words = (int)b200::step_att_words_per_layer(d->n_q, d->D, p.att_max);
@@ -440,7 +440,7 @@ int b200_decode_step(const b200_step_desc* d, void* stream) {
   int ns = (int)((budget - fixed) / p.stage_bytes);
   if (ns > b200::decode_step_max_stages()) ns = b200::decode_step_max_stages();
   p.ns = ns;
-  return finish(b200::decode_step_launch(p, d->grid, fixed + (size_t)ns * p.stage_bytes, S(stream)));
+  return finish(b200::decode_step_launch(p, d->ctx_cap, d->grid, fixed + (size_t)ns * p.stage_bytes, S(stream)));
 }
 
 int b200_argmax(const void* logits, int V, long long* tok, int* pos, long long* history, void* stream) {

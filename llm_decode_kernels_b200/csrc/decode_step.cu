@@ -160,10 +160,10 @@ DEVI void st_tagged2(uint32_t* p, uint32_t a, uint32_t b) {
 // from kHeaderBytes on: residual stream, then the areas whose offsets the host put into StepParams (off_*).
 // Pointers into it are formed where they are used (one add of a kernel parameter) instead of being carried in
 // registers through the whole step.
-// How a step's attention is cut: A slices of `per` cached tokens per kv head. two: their partials are merged by one CTA per
-// head, which publishes the attention output (otherwise the CTAs that stage it merge).
+// How a step's attention is cut: A slices of `per` cached tokens. two: per kv head, the partials merged by one CTA per head, which
+// publishes the attention output; staged: per query head, merged by the CTAs that stage it; neither: one CTA per query head.
 // units: attention units of a layer, dealt to the CTAs in turn.
-struct AttPlan { int A, per, two, refresh, pos, units; };
+struct AttPlan { int A, per, two, staged, refresh, pos, units; };
 
 // The shared memory is named where it is used and not carried as a pointer: a pointer that passes through a function or an asm
 // statement loses its address space, and every access through it becomes a generic one.
@@ -670,26 +670,35 @@ DEVI unsigned long long emit_logits(const Cta& c, const Slice& s, int tid) {
 }
 
 // ---- attention -------------------------------------------------------------------------------------------------------
-// The cut of a context of `pos` cached tokens: short ones by attention_head, longer ones in slices by attention_group, merged by a CTA
-// per head in one more exchange (~1.3 us), with every CTA taking part. Build-time knobs for measurements: tokens per slice and
-// where the sliced form begins.
+// The cut of a context of `pos` cached tokens: short ones by attention_head, longer ones in slices. With the wide exchange by
+// attention_group: every CTA takes part and a CTA per head merges the slices in one more exchange (~1.3 us). Without it (STAGED) a
+// layer's block has room for att_slices partials per query head: attention_head takes a slice of whole ring stages, and the CTAs
+// that stage the attention output merge. (4 layers behind 8192 tokens, us a token: 32 kv heads x 128 559 with one CTA per head, 298 with
+// four slices in the wide exchange, 268 this way. 32 / 4 heads x 64 without the wide exchange 152 with the groups of
+// attention_group, kv heads x 4 CTAs, and 130 this way.) Build-time knobs for measurements: tokens per slice and where the sliced
+// forms begin (the wide one by the bytes a CTA copies for one head).
 #ifndef B200_STEP_SLICE_TOKENS
 #define B200_STEP_SLICE_TOKENS 128
 #endif
 #ifndef B200_STEP_TWO_MIN
 #define B200_STEP_TWO_MIN 512
 #endif
+#ifndef B200_STEP_STAGED_MIN
+#define B200_STEP_STAGED_MIN 1152
+#endif
+template <bool STAGED>
 DEVI AttPlan att_plan(const StepParams& p, int pos, uint32_t epoch) {
   AttPlan r;
-  r.two = p.att_max > 1 && pos * p.D >= 64 * B200_STEP_TWO_MIN;   // by the bytes a CTA would copy for one head
+  r.two = !STAGED && p.att_max > 1 && pos * p.D >= 64 * B200_STEP_TWO_MIN;
+  r.staged = STAGED && pos >= B200_STEP_STAGED_MIN;
   const int want = (pos + B200_STEP_SLICE_TOKENS - 1) / B200_STEP_SLICE_TOKENS;
-  const int A = r.two ? min(p.att_max, want) : 1;   // one slice: attention_head
-  const int align = max(16, 1 << p.log2P);
+  const int A = r.two ? min(p.att_max, want) : (r.staged ? p.att_slices : 1);
+  const int align = r.staged ? kv_tokens_per_stage(p) : max(16, 1 << p.log2P);
   r.per = max(align, ((pos + A - 1) / A + align - 1) / align * align);
   r.A = max(1, (pos + r.per - 1) / r.per);   // no slice is empty
   r.refresh = (epoch & 1023u) == 0;
   r.pos = pos;
-  r.units = r.two ? p.att_groups * r.A : p.n_q;
+  r.units = r.two ? p.att_groups * r.A : p.n_q * r.A;
   return r;
 }
 
@@ -705,7 +714,7 @@ DEVI AttUnit att_unit(const StepParams& p, int u) {
   return r;
 }
 
-// Where slice j's partials go: the layer's block of the exchange (few slices) or of the wide exchange (two-level form).
+// Where slice j's partials go: the layer's block of the exchange (merged while staging) or of the wide exchange (two).
 struct AttOut { uint32_t* o; uint32_t* lse; int lsew; };
 DEVI AttOut att_out(const StepParams& p, int layer, bool two) {
   const int n_att = p.n_q * p.D;
@@ -731,14 +740,62 @@ __device__ __noinline__ void refresh_partials(const Cta c, int layer) {
   const int tid = threadIdx.x, n_att = p.n_q * p.D;
   for (int h = blockIdx.x; h < p.n_q; h += gridDim.x) {
     for (int two = 0; two < 2; ++two) {
-      const int slots = two ? p.att_max : p.att_slices;
-      if (two && slots <= p.att_slices) break;
       const AttOut out = att_out(p, layer, two);
-      const int used = two == pl.two ? pl.A : (two ? 0 : 1), used_l = two == pl.two ? pl.A + (pl.A & 1) : 0;
+      const bool partials = two ? pl.two : pl.staged;   // this step writes A of them here; otherwise the layer's block has one output
+      const int slots = two ? p.att_max : p.att_slices, used = partials ? pl.A : (two ? 0 : 1), used_l = partials ? pl.A + (pl.A & 1) : 0;
       for (int i = used * p.D + tid; i < slots * p.D; i += kNT) st_tagged(out.o + (size_t)(i / p.D) * n_att + h * p.D + i % p.D, c.tagw);
-      for (int i = 2 * used_l + tid; i < out.lsew; i += kNT) st_tagged(out.lse + (size_t)h * out.lsew + i, c.tagw);
+      for (int i = 2 * used_l + tid; slots > 0 && i < out.lsew; i += kNT) st_tagged(out.lse + (size_t)h * out.lsew + i, c.tagw);
     }
   }
+}
+
+// x <- the attention output, merged from the A slices of every head while it is staged: x = sum_j 2^(l_j - max l) o_j /
+// sum_j 2^(l_j - max l). Lane l of the warp that owns unit u holds 4 values of one head. Not inlined: the one loop body that
+// serves every phase of the step would have to find registers for it.
+__device__ __noinline__ void stage_attn(const Cta c, int layer, int warp, int lane) {
+  constexpr int NL = (kStepMaxAttSlices + 1) / 2;   // granules of log-sum-exp words per head
+  const StepParams& p = *c.p;
+  const AttOut in = att_out(p, layer, false);
+  const int nunit = p.n_att >> 7, A = c.plan().A;
+  const uint32_t lbase = (uint32_t)(in.lse - in.o);
+#pragma unroll 1
+  for (int u = warp; u < nunit; u += kNCW) {
+    const int i = 128 * u + 4 * lane, h = i / p.D;
+    // While the slices are still at work the warp polls the log-sum-exp words only: one or two addresses per head, the same for all
+    // lanes of a head, instead of A granules per lane - every CTA polls. When those are there the outputs are too, or nearly (the
+    // second poll checks their tags all the same).
+    uint32_t loff[NL], ooff[kStepMaxAttSlices];
+#pragma unroll
+    for (int g = 0; g < NL; ++g) loff[g] = lbase + (uint32_t)(h * in.lsew + 4 * g);
+#pragma unroll
+    for (int k = 0; k < kStepMaxAttSlices; ++k) ooff[k] = (uint32_t)(k * p.n_att + i);
+    uint2 lv[NL], v[kStepMaxAttSlices];
+    poll_list(c, in.o, loff, (1u << ((A + 1) >> 1)) - 1u, lv);
+    poll_list(c, in.o, ooff, (1u << A) - 1u, v);
+    float lse[kStepMaxAttSlices], M = -CUDART_INF_F;
+#pragma unroll
+    for (int k = 0; k < kStepMaxAttSlices; ++k) {
+      lse[k] = -CUDART_INF_F;
+      if (k < A) {
+        const float2 f = __half22float2(as_h2((k & 1) ? lv[k >> 1].y : lv[k >> 1].x));   // (value, remainder)
+        lse[k] = f.x + f.y;
+        M = fmaxf(M, lse[k]);
+      }
+    }
+    float W = 0.f, o[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int k = 0; k < kStepMaxAttSlices; ++k) {
+      if (k < A) {
+        const float w = exp2f(lse[k] - M);   // M is finite: no slice is empty
+        const float2 x01 = __half22float2(as_h2(v[k].x)), x23 = __half22float2(as_h2(v[k].y));
+        W += w;
+        o[0] = fmaf(w, x01.x, o[0]), o[1] = fmaf(w, x01.y, o[1]), o[2] = fmaf(w, x23.x, o[2]), o[3] = fmaf(w, x23.y, o[3]);
+      }
+    }
+    const float r = 1.f / W;
+    put_unit(c, u, make_float4(o[0] * r, o[1] * r, o[2] * r, o[3] * r), lane);
+  }
+  __syncwarp();
 }
 
 DEVI uint4 lds16(uint32_t addr) {
@@ -748,19 +805,21 @@ DEVI uint4 lds16(uint32_t addr) {
 }
 
 // ---- short contexts: one CTA per query head -------------------------------------------------------------------------
-// All consumer threads of the CTA. q, k, v of this step come from the tagged qkv exchange, the cached tokens from ring stages
-// filled by produce_kv. Lane (t = lane >> 3, c = lane & 7) of warp w owns token slot 4 w + t of a stage and dims
-// [c D/8, (c+1) D/8) of it, on the fp32 pipes; each warp keeps a private online-softmax state, merged once at the end. Against
+// All consumer threads of the CTA, for unit u = head u % n_q (and, STAGED, context slice u / n_q; the last one takes the token of this
+// step). q, k, v of this step come from the tagged qkv exchange, the cached tokens from ring stages filled by produce_kv. Lane
+// (t = lane >> 3, c = lane & 7) of warp w owns token slot 4 w + t of a stage and dims [c D/8, (c+1) D/8) of it, on the fp32 pipes; each warp keeps a private online-softmax state, merged once at the end. Against
 // attention_group: eight times the copies, but a head per CTA is less work on the way from q to the output, and up to a few
 // hundred tokens that way is what counts (TinyLlama shape, context 128: 359 us a token, 376 with the groups).
-template <int D>
-DEVI void attention_head(const Cta& c, const StepParams& p, const StepLayer& ly, uint32_t* E, int h, RingPos& rp, int tid,
+template <int D, bool STAGED>
+DEVI void attention_head(const Cta& c, const StepParams& p, const StepLayer& ly, uint32_t* E, int u, RingPos& rp, int tid,
                          int trace_at) {
   constexpr int D2 = D / 2, G4 = D / 4, DPL = D / 8;
   const int warp = tid >> 5, lane = tid & 31, ts = lane >> 3, ch = lane & 7, pos = c.plan().pos;
-  const int hpg = p.n_q / p.n_kv, kvh = h / hpg;
+  const int h = STAGED ? u % p.n_q : u, hpg = p.n_q / p.n_kv, kvh = h / hpg;
   const int tps = kv_tokens_per_stage(p);
-  const int nst = (pos + tps - 1) / tps;
+  const int t0 = STAGED ? u / p.n_q * c.plan().per : 0, len = STAGED ? min(c.plan().per, pos - t0) : pos;   // the slice's cached tokens
+  const bool takes_new = !STAGED || t0 + len == pos;
+  const int nst = (len + tps - 1) / tps;
   float* qf = reinterpret_cast<float*>(c.att());              // [D] rotated q * 1/sqrt(D)
   half* knew = reinterpret_cast<half*>(qf + D);           // [D] rotated k of this step
   half* vnew = knew + D;                                     // [D]
@@ -794,13 +853,13 @@ DEVI void attention_head(const Cta& c, const StepParams& p, const StepLayer& ly,
       } else {
         knew[i] = ra;
         knew[i + D2] = rb;
-        if (h % hpg == 0) { ly.kc[row_new + i] = ra; ly.kc[row_new + i + D2] = rb; }
+        if (takes_new && h % hpg == 0) { ly.kc[row_new + i] = ra; ly.kc[row_new + i + D2] = rb; }
       }
     } else {
       const int i = tid - D;
       const half v = raw[2 * D + i];
       vnew[i] = v;
-      if (h % hpg == 0) ly.vc[row_new + i] = v;
+      if (takes_new && h % hpg == 0) ly.vc[row_new + i] = v;
     }
   }
   consumer_sync();
@@ -861,7 +920,7 @@ DEVI void attention_head(const Cta& c, const StepParams& p, const StepLayer& ly,
   };
 
   // The cached tokens come stage by stage from the ring. The token of this step (rotated k, v in the attention scratch)
-  // rides along as token number nt of the last stage: a stage holds at most kMaxKvTokens tokens and the warps' slots cover
+  // rides along as token number nt of the (last slice's) last stage: a stage holds at most kMaxKvTokens tokens and the warps' slots cover
   // 4 kNCW kKvRounds > kMaxKvTokens, so there is always a slot for it and it costs no chain of its own.
   static_assert(4 * kNCW * kKvRounds > kMaxKvTokens, "a stage needs a spare slot for the token of this step");
   const uint32_t knew_off = (uint32_t)(reinterpret_cast<const uint8_t*>(knew) - step_smem) + ch * DPL * 2;
@@ -882,14 +941,14 @@ DEVI void attention_head(const Cta& c, const StepParams& p, const StepLayer& ly,
 #endif
     const uint32_t kbase = c.p->off_ring + (uint32_t)slot * c.p->stage_bytes + ch * DPL * 2;
     const uint32_t vbase = kbase + (uint32_t)tps * D * 2;
-    const int nt = have ? min(tps, pos - st * tps) : 0;
+    const int nt = have ? min(tps, len - st * tps) : 0;
     if (ok) {
       uint32_t koff[kKvRounds], voff[kKvRounds];
       bool valid[kKvRounds];
 #pragma unroll
       for (int r = 0; r < kKvRounds; ++r) {
         const int jt = 4 * warp + ts + 4 * kNCW * r;   // token slot of the stage
-        valid[r] = jt < nt || (last && jt == nt);
+        valid[r] = jt < nt || (takes_new && last && jt == nt);
         koff[r] = jt < nt ? kbase + (uint32_t)jt * (D * 2) : knew_off;
         voff[r] = jt < nt ? vbase + (uint32_t)jt * (D * 2) : vnew_off;
       }
@@ -932,7 +991,13 @@ DEVI void attention_head(const Cta& c, const StepParams& p, const StepLayer& ly,
       o = fmaf(a, wo[w * D + tid], o);
       L = fmaf(a, wl[w], L);
     }
-    st_tagged(E + p.n_qkv + (size_t)h * D + tid, c.tagw | (uint32_t)__half_as_ushort(__float2half(o / L)));
+    st_tagged(E + p.n_qkv + (size_t)u * D + tid, c.tagw | (uint32_t)__half_as_ushort(__float2half(o / L)));   // slot u / n_q, head h
+    if (STAGED && c.plan().staged && tid == 0) {
+      const int lsew = step_lse_words(p.att_slices), j = u / p.n_q;
+      uint32_t* lp = E + p.n_qkv + (size_t)p.att_slices * p.n_att + (size_t)h * lsew + 2 * j;
+      st_lse(c, lp, (M + __logf(L)) * 1.44269504088896340736f);
+      if ((c.plan().A & 1) && takes_new) st_tagged2(lp + 2, c.tagw | 0xFC00u, c.tagw);   // the other half of the last granule: -inf
+    }
   }
   stamp(c, trace_at + 2);
 }
@@ -1213,7 +1278,9 @@ __device__ __noinline__ AttDone attention_sliced(const Cta c, int layer, RingPos
 }  // namespace
 
 // ---- the kernel ------------------------------------------------------------------------------------------------------
-template <int D, bool WIDE>
+// STAGED: without the wide attention exchange (att_plan). A kernel of its own: the code that merges slices while staging, anywhere in
+// the kernel, makes the loop that serves every phase spill 40 to 100 bytes.
+template <int D, bool WIDE, bool STAGED>
 __global__ void __launch_bounds__(kThreads, 1) decode_step_kernel(const __grid_constant__ StepParams p) {
   uint8_t* smem = step_smem;
   Cta c;
@@ -1244,7 +1311,7 @@ __global__ void __launch_bounds__(kThreads, 1) decode_step_kernel(const __grid_c
   const uint32_t epoch = ((volatile StepCtrl*)p.ctrl)->epoch + 1u;
   c.tagw = ((epoch % 65535u) + 1u) << 16;
   const int pos = p.pos[0];
-  if (tid == 64) *reinterpret_cast<AttPlan*>(smem + 640) = att_plan(p, pos, epoch);
+  if (tid == 64) *reinterpret_cast<AttPlan*>(smem + 640) = att_plan<STAGED>(p, pos, epoch);
   __syncthreads();
   if (warp == kNCW) {
     // ================= producer =================
@@ -1262,8 +1329,8 @@ __global__ void __launch_bounds__(kThreads, 1) decode_step_kernel(const __grid_c
         for (int u = cta; u < c.plan().units && !*c.abort(); u += ncta) {
           const bool two = c.plan().two;
           const AttUnit un = att_unit(p, u);
-          const int t0 = two ? un.j * c.plan().per : 0;
-          produce_kv(c, p, ly, two ? un.kvh : u / (p.n_q / p.n_kv), t0, min(c.plan().pos, t0 + c.plan().per), rp, lane);
+          const int t0 = (two ? un.j : u / p.n_q) * c.plan().per;
+          produce_kv(c, p, ly, two ? un.kvh : u % p.n_q / (p.n_q / p.n_kv), t0, min(c.plan().pos, t0 + c.plan().per), rp, lane);
         }
     }
     // Leave only when every copy issued has landed. On the normal path the consumers have waited on every full
@@ -1356,7 +1423,8 @@ __global__ void __launch_bounds__(kThreads, 1) decode_step_kernel(const __grid_c
       stage_norm<WIDE ? kWideBatchNorm : kBatchNorm>(c, Ein, emb_row, nw, n_in, warp, lane);
     }
     else if (s.nt > 0) {
-      stage_plain<WIDE ? kWideBatch : kBatch>(c, Ein, n_in, warp, lane);
+      if (STAGED && ph == 1 && c.plan().staged) stage_attn(c, l, warp, lane);
+      else stage_plain<WIDE ? kWideBatch : kBatch>(c, Ein, n_in, warp, lane);
     }
     const int tr_at = kTraceHead + kTracePerLayer * l + kTracePerPhase * ph;
     stamp(c, tr_at);
@@ -1370,13 +1438,13 @@ __global__ void __launch_bounds__(kThreads, 1) decode_step_kernel(const __grid_c
     if (ph == 0) {
       if (c.plan().refresh) refresh_partials(c, l);
       const int tr_att = kTraceHead + kTracePerLayer * l + 4 * kTracePerPhase;
-      if (c.plan().two) {
+      if (!STAGED && c.plan().two) {
         const AttDone d = attention_sliced<D>(c, l, rp, tr_att);
         if (!d.ok) return;
         rp = d.rp;
       } else {
-        for (int u = cta; u < p.n_q; u += ncta) {
-          attention_head<D>(c, p, ly, E, u, rp, tid, tr_att);
+        for (int u = cta; u < (STAGED ? c.plan().units : p.n_q); u += ncta) {
+          attention_head<D, STAGED>(c, p, ly, E, u, rp, tid, tr_att);
           if (consumer_sync_or(*c.abort())) return;
         }
       }
@@ -1458,13 +1526,19 @@ int decode_step_max_stages() { return kMaxStages; }
 int decode_step_consumer_warps() { return kNCW; }
 int decode_step_max_kv_tokens() { return kMaxKvTokens; }
 
-cudaError_t decode_step_launch(const StepParams& p, int grid, size_t smem, cudaStream_t st) {
+// Whether a context of up to ctx_cap tokens can call for slices that are merged while staging.
+static bool decode_step_staged(const StepParams& p, int ctx_cap) {
+  return p.att_max <= 1 && p.att_slices > 1 && ctx_cap >= B200_STEP_STAGED_MIN;
+}
+
+cudaError_t decode_step_launch(const StepParams& p, int ctx_cap, int grid, size_t smem, cudaStream_t st) {
   const int kmax = p.H > p.I ? (p.H > p.n_att ? p.H : p.n_att) : (p.I > p.n_att ? p.I : p.n_att);
-  const bool wide = kmax > 128 * kNCW * kWideUnits;
-  auto kern = p.D == 64 ? (wide ? decode_step_kernel<64, true> : decode_step_kernel<64, false>)
-                        : (wide ? decode_step_kernel<128, true> : decode_step_kernel<128, false>);
-  static size_t allowed[4][kMaxDevices] = {};
-  const cudaError_t e = allow_dynamic_smem(kern, smem, allowed[2 * (p.D == 128) + wide]);
+  const bool staged = decode_step_staged(p, ctx_cap);
+  const bool wide = !staged && kmax > 128 * kNCW * kWideUnits;
+  auto kern = p.D == 64 ? (staged ? decode_step_kernel<64, false, true> : wide ? decode_step_kernel<64, true, false> : decode_step_kernel<64, false, false>)
+                        : (staged ? decode_step_kernel<128, false, true> : wide ? decode_step_kernel<128, true, false> : decode_step_kernel<128, false, false>);
+  static size_t allowed[6][kMaxDevices] = {};
+  const cudaError_t e = allow_dynamic_smem(kern, smem, allowed[3 * (p.D == 128) + 2 * staged + wide]);
   if (e != cudaSuccess) return e;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);

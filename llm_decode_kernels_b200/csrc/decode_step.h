@@ -53,15 +53,16 @@ struct StepParams {
   int part_stride_head;  // the same for the LM head (one buffer over the same area)
   int att_slices;        // J: partial attention outputs per query head a layer's exchange block has room for (step_att_slices)
   int att_groups;        // attention units per slice: kv heads x groups of up to 8 query heads
-  int att_max;           // slices the wide attention exchange has room for (0: there is none)
+  int att_max;           // slices the wide attention exchange has room for (0: there is none; the kernel's STAGED form serves then)
   int layer_words, att_layer_words;   // exchange words of a layer: step_words_per_layer, step_att_words_per_layer
   uint32_t* att_xchg;    // wide attention exchange, step_att_words_per_layer words per layer
 };
 
-// Attention of the step: a unit of work is one kv head (at most 8 of its query heads) and one slice of the context. Each slice
-// publishes, per query head, a normalised partial output and its log-sum-exp (two fp16 words: value and remainder). A layer's
-// exchange block has room for J = at most kStepMaxAttSlices of them, which the CTAs that stage the attention output merge; the
-// wide attention exchange has room for as many as the grid has CTAs per group, merged by one CTA per head.
+// Attention of the step. With the wide attention exchange a unit of work is one kv head (at most 8 of its query heads) and one slice of
+// the context, as many slices as the grid has CTAs per group; a slice publishes, per query head, a normalised partial output and its
+// log-sum-exp (two fp16 words: value and remainder), and one CTA per head merges them. Without it a unit is one query head and one of
+// at most J = kStepMaxAttSlices slices; a layer's exchange block has room for their partials, which the CTAs that stage the attention
+// output merge. Short contexts are not cut: one CTA per query head leaves the output in the block's first slot.
 #ifndef B200_STEP_MAX_SLICES
 #define B200_STEP_MAX_SLICES 4   // build-time knob for measurements: 1 = one CTA per query head
 #endif
@@ -91,6 +92,6 @@ int decode_step_threads();
 int decode_step_max_stages();
 int decode_step_consumer_warps();
 int decode_step_max_kv_tokens();
-cudaError_t decode_step_launch(const StepParams& p, int grid, size_t smem, cudaStream_t st);
+cudaError_t decode_step_launch(const StepParams& p, int ctx_cap, int grid, size_t smem, cudaStream_t st);
 
 }  // namespace b200

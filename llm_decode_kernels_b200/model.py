@@ -83,11 +83,16 @@ class DecodeConfig:
                                  # separate device ops); any entry implies one launch per operator
     step_kernel: str = "auto"    # "persistent": the whole step is one kernel (b200_decode_step); "multi": one launch
                                  # per operator, as the reference does; "auto": persistent when fused and the
-                                 # prepared context cap is within PERSISTENT_MAX_CTX
+                                 # prepared context cap is within PERSISTENT_MAX_CTX (.._FEW_CTAS)
 
 
-PERSISTENT_MAX_CTX = 1 << 20  # what the kernel takes; the one-launch-per-operator step is slower at every context (measured us
-                             # per token at 2048 / 16384 / 65000: persistent 403 / 467 / 665, multi-kernel 650 / 995 / 2278)
+# Prepared context cap up to which "auto" takes the persistent step. Measured us per token, persistent / one launch per operator:
+# 32 heads on 4 kv heads x 64 (22 layers) 403 / 650 at 2048 tokens, 467 / 995 at 16384, 665 / 2278 at 65000. Where the chip has few CTAs
+# for a kv head, the per-operator attention, which uses all of it, overtakes (4 layers, at 8192 and 16384 tokens): 32 kv heads x 128
+# 268 / 279 and 371 / 358, 64 x 64 266 / 273 and 375 / 345, 24 x 128 226 / 215 and 318 / 274; not with more CTAs or shorter rows: 32 x 64
+# 138 / 178 and 195 / 239, 16 x 128 158 / 202 and 218 / 270.
+PERSISTENT_MAX_CTX = 1 << 20          # what the kernel takes
+PERSISTENT_MAX_CTX_FEW_CTAS = 10240   # with fewer than four CTAs per 64 dims of a kv head
 
 
 class Linear:
@@ -365,13 +370,15 @@ class Model:
             raise ValueError("step_kernel='persistent' needs tile_weights, hidden, heads*head_dim and intermediate sizes "
                              "that are multiples of 128, a group size that is a multiple of 128 and pages of at most 64 "
                              "tokens; use step_kernel='multi' for this model")
-        self.persistent = mode == "persistent" or (mode == "auto" and not self.off and fits and self.tp == 1
-                                                   and self.ctx_cap <= PERSISTENT_MAX_CTX)
+        dev = self.cfg.device
+        sms = torch.cuda.get_device_properties(dev).multi_processor_count
+        few = sms // (self.n_kv * -(-self.n_q // self.n_kv // 8)) * 64 < 4 * self.D
+        self.persistent = mode == "persistent" or (mode == "auto" and not self.off and fits and self.tp == 1 and self.ctx_cap <=
+                                                   (PERSISTENT_MAX_CTX_FEW_CTAS if few else PERSISTENT_MAX_CTX))
         if not self.persistent:
             return
-        dev = self.cfg.device
         if getattr(self, "_step_static", None) is None:
-            grid = torch.cuda.get_device_properties(dev).multi_processor_count
+            grid = sms
             arr = self._layer_table()
             host = torch.frombuffer(bytearray(bytes(arr)), dtype=torch.uint8)
             nbytes = self.K.decode_step_xchg_bytes(self.L, self.H, self.I, self.n_q, self.n_kv, self.D, grid)

@@ -427,8 +427,11 @@ def test_rope_tables_match_oracle():
 # The step's attention: one CTA per head below 512 cached tokens (256 at head_dim 128), slices of 16-token blocks merged by a CTA per
 # head above. Groups of 1 .. 16 query heads per kv head, a first step on an empty cache, both sides of the change, ends of
 # blocks, ring stages and slices, more slices than the ring has stages, pages of 64.
-@pytest.mark.parametrize("D,n_q,n_kv,page", [(64, 16, 1, 16), (64, 8, 8, 16), (64, 8, 2, 64), (128, 8, 1, 16), (128, 4, 4, 32)])
-def test_persistent_attention_forms_match_the_multi_kernel_step(D, n_q, n_kv, page):
+# Without the wide exchange - by size with 30 kv heads and more, or because the caller has none - slices per query head from 1152 tokens on:
+# four, three (an odd number of log-sum-exps) and two.
+@pytest.mark.parametrize("D,n_q,n_kv,page", [(64, 16, 1, 16), (64, 8, 8, 16), (64, 8, 2, 64), (128, 8, 1, 16), (128, 4, 4, 32), (128, 32, 32, 16),
+                                             (64, 40, 40, 16), (64, 64, 64, 64)])
+def test_persistent_attention_forms_match_the_multi_kernel_step(D, n_q, n_kv, page, wide=True):
     c = hf_cfg(512, 2, n_q, n_kv, 1024, 1000, D=D)
     sd = random_state(c, 31, D)
     cap = 4700
@@ -438,7 +441,10 @@ def test_persistent_attention_forms_match_the_multi_kernel_step(D, n_q, n_kv, pa
     for m in pair:
         m.prepare(cap - 16, use_graph=False)
         m.kv.copy_(kv)
-    for ctx in (0, 15, 127, 128, 255, 256, 511, 512, 513, 640, 1023, 2049, 4600):
+        assert not m.persistent or (m._step_desc.att_xchg is None) == (n_kv >= 30)
+        if m.persistent and not wide:
+            m._step_desc.att_xchg = None
+    for ctx in (0, 15, 127, 128, 255, 256, 511, 512, 513, 640, 1023, 1151, 1152, 1537, 2049, 4600):
         outs = []
         for m in pair:
             m.reset(ctx)
@@ -452,3 +458,47 @@ def test_persistent_attention_forms_match_the_multi_kernel_step(D, n_q, n_kv, pa
             m.reset(ctx)
             want = m.prefill([17, 23], collect_logits=True).float()
             assert (outs[0] - want).abs().max() <= KERNEL_TOL * want.abs().max(), ctx
+
+
+@pytest.mark.parametrize("D,n_q,n_kv,page", [(64, 16, 1, 16), (64, 8, 2, 64), (128, 8, 1, 32), (64, 64, 8, 16)])
+def test_persistent_attention_without_the_wide_exchange(D, n_q, n_kv, page):
+    test_persistent_attention_forms_match_the_multi_kernel_step(D, n_q, n_kv, page, wide=False)
+
+
+def test_partials_that_no_step_wrote_stay_fresh():
+    """The tag of an exchange word repeats after 65535 steps. A word that a form of attention left alone for that long would pass for this
+    step's, so every 1024th step renews what it does not write: slices used at one step, short contexts across the renewal and
+    up to the epoch at which the old tags come round, slices again."""
+    c = hf_cfg(512, 1, 8, 2, 1024, 500)
+    sd = random_state(c, 5)
+    for wide in (True, False):
+        m = Model(sd, c, DecodeConfig(max_ctx=4200, seed=4, step_kernel="persistent"))
+        m.prepare(4100, use_graph=False)
+        if not wide:
+            m._step_desc.att_xchg = None
+        m.kv.normal_(generator=torch.Generator(device="cuda").manual_seed(1))
+        ctrl, kv = m._step_static["ctrl"], m.kv.clone()
+
+        def step(at, epoch=None):
+            if epoch is not None:
+                ctrl[0] = epoch
+            m.kv.copy_(kv)          # without the rows that earlier steps appended
+            m.reset(at)
+            m.teacher_force([7], use_graph=False)
+            assert m.step_error() == 0
+            return m.logits.clone()
+        first = step(4000, 500)
+        step(20, 1022), step(20), step(20)                     # renewal at epoch 1024
+        xchg = m._step_static["att_xchg" if wide else "xchg"].view(torch.int32)
+        stale = 501 % 65535 + 1
+        assert not ((xchg >> 16) & 0xFFFF == stale).any()      # nothing of the first step is left to be mistaken
+        assert torch.equal(step(4000, 500 + 65535), first)
+
+
+def test_automatic_step_kernel_by_context_and_ctas_per_kv_head():
+    for n_q, n_kv, D, limit in ((32, 32, 128, 10240), (8, 2, 64, None)):
+        c = hf_cfg(n_q * D, 1, n_q, n_kv, 256, 300, D=D)
+        m = Model(random_state(c, 2, D), c, DecodeConfig(max_ctx=20000, seed=1))
+        for cap in (4096, 10240, 10241, 20000):
+            m.set_attention_partition(cap, part_size=1)
+            assert m.persistent == (limit is None or cap <= limit), (n_kv, cap)
