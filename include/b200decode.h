@@ -276,14 +276,12 @@ typedef struct b200_step_desc {
   int grid;            /* CTAs = SMs of the device */
   long long* trace;    /* NULL. (A library built with -DB200_STEP_TRACE, which the normal build never is, fills an
                         * int64 [grid, 8 + 25 (L + 1)] array here with per-CTA globaltimer values inside every phase.) */
-  void* att_xchg;      /* NULL, or b200_decode_step_att_bytes() bytes, zeroed once by the caller: lets attention use every CTA on
-                        * long contexts (without it: at most four slices per query head) */
 } b200_step_desc;
 
 /* Bytes of exchange memory a step of these dimensions needs. */
 size_t b200_decode_step_xchg_bytes(int L, int H, int I, int n_q, int n_kv, int D, int grid);
 
-/* Bytes of the optional wide attention exchange (0: the dimensions leave no CTAs to spare). */
+/* Bytes of the wide attention exchange of b200_decode_step_wide (0: the dimensions leave no CTAs to spare). */
 size_t b200_decode_step_att_bytes(int L, int n_q, int n_kv, int D, int grid);
 
 /* Launch one step. B200_ERR_SHAPE if the dimensions do not fit the kernel (H, n_q D and I multiples of 128, group size
@@ -294,6 +292,11 @@ size_t b200_decode_step_att_bytes(int L, int n_q, int n_kv, int D, int grid);
  * outside [0, V) - row 0 of the embedding was used instead and the step completed. A logit vector with no comparable
  * entry (all NaN) yields token 0, as an in-range answer like torch.argmax's. */
 int b200_decode_step(const b200_step_desc* d, void* stream);
+
+/* The same with the wide attention exchange: b200_decode_step_att_bytes() bytes, 16B, zeroed once by the caller, then owned by the
+ * step. Attention of long contexts then uses every CTA; without it (NULL, or b200_decode_step) at most four slices per query head.
+ * Steps over one xchg may use either entry point in turn. */
+int b200_decode_step_wide(const b200_step_desc* d, void* att_xchg, void* stream);
 
 /* ---- tensor-parallel exchange over NVLink peer memory (one process per GPU, all GPUs in one node) ----
  * No counterpart in the reference, which is single-GPU; the 70B-shape configuration splits o_proj / down_proj by

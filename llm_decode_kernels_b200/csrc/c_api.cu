@@ -372,7 +372,9 @@ size_t b200_decode_step_att_bytes(int L, int n_q, int n_kv, int D, int grid) {
   return b200::step_att_words_per_layer(n_q, D, wide) * L * sizeof(uint32_t);
 }
 
-int b200_decode_step(const b200_step_desc* d, void* stream) {
+int b200_decode_step(const b200_step_desc* d, void* stream) { return b200_decode_step_wide(d, nullptr, stream); }
+
+int b200_decode_step_wide(const b200_step_desc* d, void* att_xchg, void* stream) {
   static_assert(sizeof(b200_step_layer) == sizeof(b200::StepLayer), "layer structs must match");
   REQUIRE(d && d->layers && d->emb && d->norm_f && d->w_head && d->cos_t && d->sin_t && d->bt &&
               d->tok && d->pos && d->logits && d->xchg && d->ctrl,
@@ -390,7 +392,7 @@ int b200_decode_step(const b200_step_desc* d, void* stream) {
     kmax = K > kmax ? K : kmax;
   }
   REQUIRE(aligned16(d->emb) && aligned16(d->norm_f) && aligned16(d->w_head) && aligned16(d->xchg) &&
-              aligned16(d->ctrl) && aligned16(d->layers) && aligned16(d->att_xchg),
+              aligned16(d->ctrl) && aligned16(d->layers) && aligned16(att_xchg),
           B200_ERR_ALIGN);
   REQUIRE(d->ctx_cap <= (1 << 20), B200_ERR_LIMIT);
 
@@ -405,8 +407,8 @@ int b200_decode_step(const b200_step_desc* d, void* stream) {
   p.trace = d->trace;
   p.att_slices = b200::step_att_slices(d->grid, d->n_q);
   p.att_groups = b200::step_att_groups(d->n_q, d->n_kv);
-  p.att_max = d->att_xchg && b200_decode_step_att_bytes(d->L, d->n_q, d->n_kv, d->D, d->grid) ? b200::step_att_max(d->grid, d->n_q, d->n_kv) : 0;
-  p.att_xchg = (uint32_t*)d->att_xchg;
+  p.att_max = att_xchg && b200_decode_step_att_bytes(d->L, d->n_q, d->n_kv, d->D, d->grid) ? b200::step_att_max(d->grid, d->n_q, d->n_kv) : 0;
+  p.att_xchg = (uint32_t*)att_xchg;
   p.layer_words = (int)b200::step_words_per_layer(d->H, d->I, d->n_q, d->n_kv, d->D, p.att_slices);
   p.att_layer_words = (int)b200::step_att_words_per_layer(d->n_q, d->D, p.att_max);
   // shared-memory plan

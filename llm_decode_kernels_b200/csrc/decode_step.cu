@@ -807,9 +807,10 @@ DEVI uint4 lds16(uint32_t addr) {
 // ---- short contexts: one CTA per query head -------------------------------------------------------------------------
 // All consumer threads of the CTA, for unit u = head u % n_q (and, STAGED, context slice u / n_q; the last one takes the token of this
 // step). q, k, v of this step come from the tagged qkv exchange, the cached tokens from ring stages filled by produce_kv. Lane
-// (t = lane >> 3, c = lane & 7) of warp w owns token slot 4 w + t of a stage and dims [c D/8, (c+1) D/8) of it, on the fp32 pipes; each warp keeps a private online-softmax state, merged once at the end. Against
-// attention_group: eight times the copies, but a head per CTA is less work on the way from q to the output, and up to a few
-// hundred tokens that way is what counts (TinyLlama shape, context 128: 359 us a token, 376 with the groups).
+// (t = lane >> 3, c = lane & 7) of warp w owns token slot 4 w + t of a stage and dims [c D/8, (c+1) D/8) of it, on the fp32 pipes;
+// each warp keeps a private online-softmax state, merged once at the end. Against attention_group: eight times the copies, but
+// a head per CTA is less work on the way from q to the output, and up to a few hundred tokens that way is what counts (TinyLlama
+// shape, context 128: 359 us a token, 376 with the groups).
 template <int D, bool STAGED>
 DEVI void attention_head(const Cta& c, const StepParams& p, const StepLayer& ly, uint32_t* E, int u, RingPos& rp, int tid,
                          int trace_at) {

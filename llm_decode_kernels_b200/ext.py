@@ -82,6 +82,7 @@ SIGNATURES = {
     "b200_gemm_w4a16_tiled": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p],
     "b200_prefill_chunk": [c_void_p, c_void_p],
     "b200_decode_step_att_bytes": [c_int] * 5,
+    "b200_decode_step_wide": [c_void_p, c_void_p, c_void_p],
     "b200_gemm_w4a16_max_tokens": [],
     "b200_gemm_w4a16_status": [c_void_p],
     "b200_embed_row": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p],
@@ -101,8 +102,7 @@ class StepDesc(ctypes.Structure):
                 ("D", c_int), ("V", c_int), ("log2G", c_int), ("log2P", c_int), ("eps", c_float), ("emb", c_void_p),
                 ("norm_f", c_void_p), ("w_head", c_void_p), ("sz_head", c_void_p), ("cos_t", c_void_p),
                 ("sin_t", c_void_p), ("bt", c_void_p), ("tok", c_void_p), ("pos", c_void_p), ("history", c_void_p),
-                ("logits", c_void_p), ("xchg", c_void_p), ("ctrl", c_void_p), ("ctx_cap", c_int), ("grid", c_int), ("trace", c_void_p),
-                ("att_xchg", c_void_p)]
+                ("logits", c_void_p), ("xchg", c_void_p), ("ctrl", c_void_p), ("ctx_cap", c_int), ("grid", c_int), ("trace", c_void_p)]
 
 
 class PrefillDesc(ctypes.Structure):
@@ -623,9 +623,10 @@ class Ops:
     def decode_step_att_bytes(self, L, n_q, n_kv, D, grid):
         return int(self.lib.b200_decode_step_att_bytes(L, n_q, n_kv, D, grid))
 
-    def decode_step(self, desc: "StepDesc"):
-        """One whole decode step as one persistent kernel (b200_decode_step) on the current stream."""
-        self._check(self.lib.b200_decode_step(ctypes.byref(desc), _stream()), "decode_step")
+    def decode_step(self, desc: "StepDesc", att_xchg=None):
+        """One whole decode step as one persistent kernel (b200_decode_step) on the current stream. att_xchg: None, or the
+        address of decode_step_att_bytes() zeroed bytes (b200_decode_step_wide)."""
+        self._check(self.lib.b200_decode_step_wide(ctypes.byref(desc), att_xchg, _stream()), "decode_step")
 
 
 def load(verbose=False):

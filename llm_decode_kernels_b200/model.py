@@ -396,9 +396,8 @@ class Model:
         d.cos_t, d.sin_t, d.bt = self.cos.data_ptr(), self.sin.data_ptr(), self.bt.data_ptr()
         d.tok, d.pos, d.history = self.tok.data_ptr(), self.pos.data_ptr(), self.history.data_ptr()
         d.logits, d.xchg, d.ctrl = self.logits.data_ptr(), st["xchg"].data_ptr(), st["ctrl"].data_ptr()
-        d.att_xchg = st["att_xchg"].data_ptr() or None
         d.ctx_cap, d.grid = min(self.ctx_cap, self.cfg.max_ctx + 1), st["grid"]
-        self._step_desc = d
+        self._step_desc, self._step_att = d, st["att_xchg"].data_ptr() or None
 
     def step_error(self):
         """Non-zero if a bounded wait inside a kernel of the step gave up (the step's outputs are then invalid): the
@@ -512,7 +511,7 @@ class Model:
     def step(self):
         """One token: reads self.tok / self.pos, writes self.logits, self.tok <- argmax, self.pos += 1."""
         if self.persistent:
-            self.K.decode_step(self._step_desc)
+            self.K.decode_step(self._step_desc, self._step_att)
             return
         self.K.embed_row(self.emb, self.tok, self.x)
         if self.norm_in_gemv:

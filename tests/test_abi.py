@@ -112,3 +112,13 @@ def test_native_call_path_mirrors_the_methods():
         ops.swiglu(1, 2, 3)
     with pytest.raises(TypeError):
         ops.swiglu(gu=1, nonsense=2)
+
+
+def test_descriptors_have_the_fields_of_the_header():
+    """Same fields in the same order; and b200_step_desc ends where callers built against the first headers have it end."""
+    text = re.sub(r"/\*.*?\*/", "", HEADER.read_text(), flags=re.S)
+    for cls, name in ((ext.StepLayer, "b200_step_layer"), (ext.StepDesc, "b200_step_desc"), (ext.PrefillDesc, "b200_prefill_desc")):
+        body = next(b for b, n in re.findall(r"typedef struct\s*\w*\s*\{([^{}]*)\}\s*(\w+);", text) if n == name)
+        fields = [re.sub(r"\[.*?\]", "", f).split()[-1].lstrip("*") for line in body.split(";") for f in line.split(",") if f.strip()]
+        assert fields == [f[0] for f in cls._fields_], name
+    assert ext.StepDesc._fields_[-1][0] == "trace" and ctypes.sizeof(ext.StepDesc) == 168

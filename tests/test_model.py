@@ -441,9 +441,9 @@ def test_persistent_attention_forms_match_the_multi_kernel_step(D, n_q, n_kv, pa
     for m in pair:
         m.prepare(cap - 16, use_graph=False)
         m.kv.copy_(kv)
-        assert not m.persistent or (m._step_desc.att_xchg is None) == (n_kv >= 30)
+        assert not m.persistent or (m._step_att is None) == (n_kv >= 30)
         if m.persistent and not wide:
-            m._step_desc.att_xchg = None
+            m._step_att = None
     for ctx in (0, 15, 127, 128, 255, 256, 511, 512, 513, 640, 1023, 1151, 1152, 1537, 2049, 4600):
         outs = []
         for m in pair:
@@ -475,7 +475,7 @@ def test_partials_that_no_step_wrote_stay_fresh():
         m = Model(sd, c, DecodeConfig(max_ctx=4200, seed=4, step_kernel="persistent"))
         m.prepare(4100, use_graph=False)
         if not wide:
-            m._step_desc.att_xchg = None
+            m._step_att = None
         m.kv.normal_(generator=torch.Generator(device="cuda").manual_seed(1))
         ctrl, kv = m._step_static["ctrl"], m.kv.clone()
 
