@@ -65,26 +65,20 @@ bool group_ok(int64_t n_q, int64_t n_kv) {
   return g == 1 || g == 2 || g == 4 || g == 8;
 }
 
-// C ABI entry points, bound by address (the library may be any build of it)
-void* g_fn[16] = {};
-enum : int { GEMV, TILED, TILED_NORM, ATTN, ATTN_B, ROPE_ATTN, NORM, SWIGLU, ROPE, ROPE_B, EMBED, ARGMAX, NUM_FN };
-const char* const kFnNames[NUM_FN] = {"b200_gemv_w4a16", "b200_gemv_w4a16_tiled", "b200_gemv_w4a16_tiled_norm", "b200_paged_attention",
-                                      "b200_paged_attention_batched_v", "b200_rope_paged_attention", "b200_add_rmsnorm", "b200_swiglu",
-                                      "b200_rope_append", "b200_rope_append_batched", "b200_embed_row", "b200_argmax"};
-
+// An operator's C ABI entry point; it is bound by address, per operator object (the library may be any build of it).
 // The call itself runs without the interpreter lock: a launch blocks while the device's queue is full.
 template <typename... A>
-bool call(int fn, A... a) {
+bool call(void* fn, A... a) {
   int rc;
   Py_BEGIN_ALLOW_THREADS
-  rc = reinterpret_cast<int (*)(A...)>(g_fn[fn])(a...);
+  rc = reinterpret_cast<int (*)(A...)>(fn)(a...);
   Py_END_ALLOW_THREADS
   return rc == 0;
 }
 #define CHECK(cond) \
   if (!(cond)) return false
 
-bool op_gemv(Args a) {   // stage, R, warps, pf, packed, sz, x, y, group
+bool op_gemv(void* fn, Args a) {   // stage, R, warps, pf, packed, sz, x, y, group
   int stage, R, warps, pf, group;
   CHECK(integer(a[0], &stage) && integer(a[1], &R) && integer(a[2], &warps) && integer(a[3], &pf) && integer(a[8], &group));
   const Tensor w = i32(a[4]), sz = f16(a[5]), x = f16(a[6]), y = f16(a[7]);
@@ -94,17 +88,17 @@ bool op_gemv(Args a) {   // stage, R, warps, pf, packed, sz, x, y, group
   CHECK(x.numel() == K && y.numel() == N && sz.size(0) == N && sz.size(1) == K / group && w.aligned16() && x.aligned16());
   const int lg = log2_exact(group);
   CHECK(lg >= 0);
-  return call(GEMV, stage, R, warps, pf, w.data(), sz.data(), x.data(), y.data(), (int)N, (int)K, lg, stream());
+  return call(fn, stage, R, warps, pf, w.data(), sz.data(), x.data(), y.data(), (int)N, (int)K, lg, stream());
 }
 
-bool op_tiled(Args a) {   // tiled, x, y, N, K, swiglu
+bool op_tiled(void* fn, Args a) {   // tiled, x, y, N, K, swiglu
   int N, K, sw;
   const Tensor w = get(a[0], at::kByte), x = f16(a[1]), y = f16(a[2]);
   CHECK(w && x && y && integer(a[3], &N) && integer(a[4], &K) && flag(a[5], &sw) && x.numel() == K && y.numel() == N);
-  return call(TILED, w.data(), x.data(), y.data(), N, K, sw, stream());
+  return call(fn, w.data(), x.data(), y.data(), N, K, sw, stream());
 }
 
-bool op_tiled_norm(Args a) {   // tiled, x_in, delta, norm_w, eps, x_out, y, N, K, swiglu
+bool op_tiled_norm(void* fn, Args a) {   // tiled, x_in, delta, norm_w, eps, x_out, y, N, K, swiglu
   int N, K, sw;
   float eps;
   const Tensor w = get(a[0], at::kByte), x = f16(a[1]), nw = f16(a[3]), xo = f16(a[5]), y = f16(a[6]);
@@ -116,10 +110,10 @@ bool op_tiled_norm(Args a) {   // tiled, x_in, delta, norm_w, eps, x_out, y, N, 
     CHECK(t);
     d = t.data();
   }
-  return call(TILED_NORM, w.data(), x.data(), d, nw.data(), eps, xo.data(), y.data(), N, K, sw, stream());
+  return call(fn, w.data(), x.data(), d, nw.data(), eps, xo.data(), y.data(), N, K, sw, stream());
 }
 
-bool op_attn(Args a) {   // q, kc, vc, bt, pos, part_size, o_part, m_part, l_part, out, version
+bool op_attn(void* fn, Args a) {   // q, kc, vc, bt, pos, part_size, o_part, m_part, l_part, out, version
   int part, version = 2;
   const Tensor q = f16(a[0]), kc = f16(a[1]), vc = f16(a[2]), bt = i32(a[3]), pos = i32(a[4]);
   const Tensor o = f32(a[6]), m = f32(a[7]), l = f32(a[8]), out = f16(a[9]);
@@ -131,11 +125,11 @@ bool op_attn(Args a) {   // q, kc, vc, bt, pos, part_size, o_part, m_part, l_par
   CHECK(o.dim() > 1 && m.dim() > 1 && l.dim() > 1);
   const int64_t S = o.size(1);
   CHECK(o.size(0) == n_q && m.size(1) == S && l.size(1) == S);
-  return call(ATTN, version, q.data(), kc.data(), vc.data(), bt.data(), pos.data(), (int)n_q, (int)n_kv, lp, part, (int)S, o.data(),
+  return call(fn, version, q.data(), kc.data(), vc.data(), bt.data(), pos.data(), (int)n_q, (int)n_kv, lp, part, (int)S, o.data(),
               m.data(), l.data(), out.data(), stream());
 }
 
-bool op_attn_b(Args a) {   // q, kc, vc, bt, pos, part_size, o_part, m_part, l_part, out, version
+bool op_attn_b(void* fn, Args a) {   // q, kc, vc, bt, pos, part_size, o_part, m_part, l_part, out, version
   int part, version = 0;
   const Tensor q = f16(a[0]), kc = f16(a[1]), vc = f16(a[2]), bt = i32(a[3]), pos = i32(a[4]);
   const Tensor o = f32(a[6]), m = f32(a[7]), l = f32(a[8]), out = f16(a[9]);
@@ -147,11 +141,11 @@ bool op_attn_b(Args a) {   // q, kc, vc, bt, pos, part_size, o_part, m_part, l_p
   CHECK(o.dim() == 4 && m.dim() == 3 && m.t->sizes() == l.t->sizes());
   const int64_t S = o.size(2);
   CHECK(o.size(0) == B && o.size(1) == n_q && o.size(3) == D && m.size(0) == B && m.size(1) == n_q && m.size(2) == S);
-  return call(ATTN_B, version, q.data(), kc.data(), vc.data(), bt.data(), (int)bt.size(1), pos.data(), (int)B, (int)n_q,
+  return call(fn, version, q.data(), kc.data(), vc.data(), bt.data(), (int)bt.size(1), pos.data(), (int)B, (int)n_q,
               (int)kc.size(1), (int)D, lp, part, (int)S, o.data(), m.data(), l.data(), out.data(), stream());
 }
 
-bool op_rope_attn(Args a) {   // qkv, cos_t, sin_t, pos, bt, kc, vc, n_q, n_kv, part_size, o_part, m_part, l_part, out, arrive
+bool op_rope_attn(void* fn, Args a) {   // qkv, cos_t, sin_t, pos, bt, kc, vc, n_q, n_kv, part_size, o_part, m_part, l_part, out, arrive
   int n_q, n_kv, part;
   const Tensor qkv = f16(a[0]), cs = f32(a[1]), sn = f32(a[2]), pos = i32(a[3]), bt = i32(a[4]), kc = f16(a[5]), vc = f16(a[6]);
   const Tensor o = f32(a[10]), m = f32(a[11]), l = f32(a[12]), out = f16(a[13]);
@@ -168,11 +162,11 @@ bool op_rope_attn(Args a) {   // qkv, cos_t, sin_t, pos, bt, kc, vc, n_q, n_kv, 
     CHECK(t && t.numel() >= n_kv);
     arrive = t.data();
   }
-  return call(ROPE_ATTN, qkv.data(), cs.data(), sn.data(), kc.data(), vc.data(), bt.data(), pos.data(), n_q, n_kv, (int)D, lp, part,
+  return call(fn, qkv.data(), cs.data(), sn.data(), kc.data(), vc.data(), bt.data(), pos.data(), n_q, n_kv, (int)D, lp, part,
               (int)S, o.data(), m.data(), l.data(), out.data(), arrive, stream());
 }
 
-bool op_norm(Args a) {   // x, delta, w, out, eps
+bool op_norm(void* fn, Args a) {   // x, delta, w, out, eps
   float eps;
   const Tensor x = f16(a[0]), w = f16(a[2]), out = f16(a[3]);
   CHECK(x && w && out && real(a[4], &eps) && x.numel() % 8 == 0 && x.aligned16() && w.aligned16() && out.aligned16());
@@ -182,25 +176,25 @@ bool op_norm(Args a) {   // x, delta, w, out, eps
     CHECK(t && t.aligned16());
     d = t.data();
   }
-  return call(NORM, x.data(), d, w.data(), out.data(), (int)x.numel(), eps, stream());
+  return call(fn, x.data(), d, w.data(), out.data(), (int)x.numel(), eps, stream());
 }
 
-bool op_swiglu(Args a) {   // gu, out
+bool op_swiglu(void* fn, Args a) {   // gu, out
   const Tensor gu = f16(a[0]), out = f16(a[1]);
   CHECK(gu && out && out.numel() % 8 == 0 && gu.numel() == 2 * out.numel() && gu.aligned16() && out.aligned16());
-  return call(SWIGLU, gu.data(), out.data(), (int)out.numel(), stream());
+  return call(fn, gu.data(), out.data(), (int)out.numel(), stream());
 }
 
-bool op_rope(Args a) {   // qkv, cos_t, sin_t, pos, bt, kc, vc, n_q, n_kv
+bool op_rope(void* fn, Args a) {   // qkv, cos_t, sin_t, pos, bt, kc, vc, n_q, n_kv
   int n_q, n_kv;
   const Tensor qkv = f16(a[0]), cs = f32(a[1]), sn = f32(a[2]), pos = i32(a[3]), bt = i32(a[4]), kc = f16(a[5]), vc = f16(a[6]);
   CHECK(qkv && cs && sn && pos && bt && kc && vc && integer(a[7], &n_q) && integer(a[8], &n_kv) && kc.dim() > 2 && cs.dim() > 1);
   const int lp = log2_exact(kc.size(2));
   CHECK(qkv.numel() == (n_q + 2 * (int64_t)n_kv) * 64 && cs.size(1) == 32 && lp >= 0);
-  return call(ROPE, qkv.data(), cs.data(), sn.data(), pos.data(), bt.data(), kc.data(), vc.data(), n_q, n_kv, lp, stream());
+  return call(fn, qkv.data(), cs.data(), sn.data(), pos.data(), bt.data(), kc.data(), vc.data(), n_q, n_kv, lp, stream());
 }
 
-bool op_rope_b(Args a) {   // the same for rows qkv [B, (n_q + 2 n_kv) D], bt [B, max_pages]
+bool op_rope_b(void* fn, Args a) {   // the same for rows qkv [B, (n_q + 2 n_kv) D], bt [B, max_pages]
   int n_q, n_kv;
   const Tensor qkv = f16(a[0]), cs = f32(a[1]), sn = f32(a[2]), pos = i32(a[3]), bt = i32(a[4]), kc = f16(a[5]), vc = f16(a[6]);
   CHECK(qkv && cs && sn && pos && bt && kc && vc && integer(a[7], &n_q) && integer(a[8], &n_kv));
@@ -208,17 +202,17 @@ bool op_rope_b(Args a) {   // the same for rows qkv [B, (n_q + 2 n_kv) D], bt [B
   const int64_t B = qkv.size(0), D = 2 * cs.size(1);
   const int lp = log2_exact(kc.size(2));
   CHECK(qkv.size(1) == (n_q + 2 * (int64_t)n_kv) * D && kc.size(3) == D && bt.size(0) == B && lp >= 0);
-  return call(ROPE_B, qkv.data(), cs.data(), sn.data(), pos.data(), bt.data(), (int)bt.size(1), kc.data(), vc.data(), (int)B, n_q, n_kv,
+  return call(fn, qkv.data(), cs.data(), sn.data(), pos.data(), bt.data(), (int)bt.size(1), kc.data(), vc.data(), (int)B, n_q, n_kv,
               (int)D, lp, stream());
 }
 
-bool op_embed(Args a) {   // emb, tok, x
+bool op_embed(void* fn, Args a) {   // emb, tok, x
   const Tensor emb = f16(a[0]), tok = i64(a[1]), x = f16(a[2]);
   CHECK(emb && tok && x && emb.dim() == 2 && emb.size(1) == x.numel());
-  return call(EMBED, emb.data(), tok.data(), x.data(), (int)x.numel(), (int)emb.size(0), stream());
+  return call(fn, emb.data(), tok.data(), x.data(), (int)x.numel(), (int)emb.size(0), stream());
 }
 
-bool op_argmax(Args a) {   // logits, tok, pos, history
+bool op_argmax(void* fn, Args a) {   // logits, tok, pos, history
   const Tensor lg = f16(a[0]), tok = i64(a[1]);
   CHECK(lg && tok);
   void *p = nullptr, *h = nullptr;
@@ -232,37 +226,39 @@ bool op_argmax(Args a) {   // logits, tok, pos, history
     CHECK(t);
     h = t.data();
   }
-  return call(ARGMAX, lg.data(), (int)lg.numel(), tok.data(), p, h, stream());
+  return call(fn, lg.data(), (int)lg.numel(), tok.data(), p, h, stream());
 }
 
 struct OpDef {
   const char* name;
-  bool (*fn)(Args);
+  bool (*fn)(void*, Args);
+  const char* entry;   // the C function
   int required, total;
   const char* args[kMaxArgs];
 };
 const OpDef kOps[] = {
-    {"gemv_w4a16", op_gemv, 9, 9, {"stage", "R", "warps", "pf", "packed", "sz", "x", "y", "group"}},
-    {"gemv_w4a16_tiled", op_tiled, 5, 6, {"tiled", "x", "y", "N", "K", "swiglu"}},
-    {"gemv_w4a16_tiled_norm", op_tiled_norm, 9, 10, {"tiled", "x_in", "delta", "norm_w", "eps", "x_out", "y", "N", "K", "swiglu"}},
-    {"paged_attention", op_attn, 10, 11,
+    {"gemv_w4a16", op_gemv, "b200_gemv_w4a16", 9, 9, {"stage", "R", "warps", "pf", "packed", "sz", "x", "y", "group"}},
+    {"gemv_w4a16_tiled", op_tiled, "b200_gemv_w4a16_tiled", 5, 6, {"tiled", "x", "y", "N", "K", "swiglu"}},
+    {"gemv_w4a16_tiled_norm", op_tiled_norm, "b200_gemv_w4a16_tiled_norm", 9, 10, {"tiled", "x_in", "delta", "norm_w", "eps", "x_out", "y", "N", "K", "swiglu"}},
+    {"paged_attention", op_attn, "b200_paged_attention", 10, 11,
      {"q", "kc", "vc", "bt", "pos", "part_size", "o_part", "m_part", "l_part", "out", "version"}},
-    {"paged_attention_batched", op_attn_b, 10, 11,
+    {"paged_attention_batched", op_attn_b, "b200_paged_attention_batched_v", 10, 11,
      {"q", "kc", "vc", "bt", "pos", "part_size", "o_part", "m_part", "l_part", "out", "version"}},
-    {"rope_paged_attention", op_rope_attn, 14, 15,
+    {"rope_paged_attention", op_rope_attn, "b200_rope_paged_attention", 14, 15,
      {"qkv", "cos_t", "sin_t", "pos", "bt", "kc", "vc", "n_q", "n_kv", "part_size", "o_part", "m_part", "l_part", "out", "arrive"}},
-    {"add_rmsnorm", op_norm, 5, 5, {"x", "delta", "w", "out", "eps"}},
-    {"swiglu", op_swiglu, 2, 2, {"gu", "out"}},
-    {"rope_append", op_rope, 9, 9, {"qkv", "cos_t", "sin_t", "pos", "bt", "kc", "vc", "n_q", "n_kv"}},
-    {"rope_append_batched", op_rope_b, 9, 9, {"qkv", "cos_t", "sin_t", "pos", "bt", "kc", "vc", "n_q", "n_kv"}},
-    {"embed_row", op_embed, 3, 3, {"emb", "tok", "x"}},
-    {"argmax", op_argmax, 2, 4, {"logits", "tok", "pos", "history"}},
+    {"add_rmsnorm", op_norm, "b200_add_rmsnorm", 5, 5, {"x", "delta", "w", "out", "eps"}},
+    {"swiglu", op_swiglu, "b200_swiglu", 2, 2, {"gu", "out"}},
+    {"rope_append", op_rope, "b200_rope_append", 9, 9, {"qkv", "cos_t", "sin_t", "pos", "bt", "kc", "vc", "n_q", "n_kv"}},
+    {"rope_append_batched", op_rope_b, "b200_rope_append_batched", 9, 9, {"qkv", "cos_t", "sin_t", "pos", "bt", "kc", "vc", "n_q", "n_kv"}},
+    {"embed_row", op_embed, "b200_embed_row", 3, 3, {"emb", "tok", "x"}},
+    {"argmax", op_argmax, "b200_argmax", 2, 4, {"logits", "tok", "pos", "history"}},
 };
 
 struct OpObject {
   PyObject_HEAD
   vectorcallfunc vectorcall;
   const OpDef* op;
+  void* entry;
   PyObject* fallback;
 };
 
@@ -282,7 +278,7 @@ PyObject* op_call(PyObject* self, PyObject* const* args, size_t nargsf, PyObject
   }
   for (int i = 0; ok && i < op.required; ++i) ok = a[i] != nullptr;
   try {
-    if (ok && op.fn(a)) Py_RETURN_NONE;
+    if (ok && op.fn(o->entry, a)) Py_RETURN_NONE;
   } catch (const std::exception&) {   // a tensor without storage and the like: the method says what is wrong
   }
   return PyObject_Vectorcall(o->fallback, args, nargsf & ~PY_VECTORCALL_ARGUMENTS_OFFSET, kwnames);
@@ -307,43 +303,42 @@ PyGetSetDef op_getset[] = {{"__doc__", op_doc, nullptr, nullptr, nullptr}, {"__w
 
 PyTypeObject OpType = {PyVarObject_HEAD_INIT(nullptr, 0)};
 
-// operator(name, fallback): the callable, or None if there is no native form of that name
+// operator(name, address of its C function, fallback): the callable
 PyObject* make_operator(PyObject*, PyObject* args) {
   const char* name;
-  PyObject* fallback;
-  if (!PyArg_ParseTuple(args, "sO", &name, &fallback)) return nullptr;
+  PyObject *address, *fallback;
+  if (!PyArg_ParseTuple(args, "sOO", &name, &address, &fallback)) return nullptr;
+  void* entry = PyLong_AsVoidPtr(address);
+  if (!entry) return PyErr_Occurred() ? nullptr : PyErr_Format(PyExc_ValueError, "%s: null address", name);
   for (const OpDef& d : kOps)
     if (strcmp(d.name, name) == 0) {
       OpObject* o = PyObject_GC_New(OpObject, &OpType);
       if (!o) return nullptr;
       o->vectorcall = op_call;
       o->op = &d;
+      o->entry = entry;
       o->fallback = Py_NewRef(fallback);
       PyObject_GC_Track(o);
       return reinterpret_cast<PyObject*>(o);
     }
-  Py_RETURN_NONE;
+  return PyErr_Format(PyExc_KeyError, "%s", name);
 }
 
-// bind(name -> address of the C function)
-PyObject* bind(PyObject*, PyObject* table) {
-  for (int i = 0; i < NUM_FN; ++i) {
-    PyObject* v = PyMapping_GetItemString(table, kFnNames[i]);
-    if (!v) return nullptr;
-    g_fn[i] = PyLong_AsVoidPtr(v);
+PyObject* entries(PyObject*, PyObject*) {   // {operator: its C function}
+  PyObject* o = PyDict_New();
+  for (const OpDef& d : kOps) {
+    PyObject* v = PyUnicode_FromString(d.entry);
+    PyDict_SetItemString(o, d.name, v);
     Py_DECREF(v);
-    if (!g_fn[i]) return PyErr_Occurred() ? nullptr : PyErr_Format(PyExc_ValueError, "%s is null", kFnNames[i]);
   }
-  Py_RETURN_NONE;
+  return o;
 }
-PyObject* names(PyObject*, PyObject*) {   // (C functions to bind, {operator: (argument names, how many are required)})
+PyObject* names(PyObject*, PyObject*) {   // (C functions, {operator: (argument names, how many are required)})
   PyObject *f = PyList_New(0), *o = PyDict_New();
-  for (const char* n : kFnNames) {
-    PyObject* s = PyUnicode_FromString(n);
+  for (const OpDef& d : kOps) {
+    PyObject* s = PyUnicode_FromString(d.entry);
     PyList_Append(f, s);
     Py_DECREF(s);
-  }
-  for (const OpDef& d : kOps) {
     PyObject* args = PyTuple_New(d.total);
     for (int i = 0; i < d.total; ++i) PyTuple_SET_ITEM(args, i, PyUnicode_FromString(d.args[i]));
     PyObject* v = Py_BuildValue("(Ni)", args, d.required);
@@ -353,7 +348,7 @@ PyObject* names(PyObject*, PyObject*) {   // (C functions to bind, {operator: (a
   return Py_BuildValue("(NN)", f, o);
 }
 
-PyMethodDef methods[] = {{"operator", make_operator, METH_VARARGS, nullptr}, {"bind", bind, METH_O, nullptr},
+PyMethodDef methods[] = {{"operator", make_operator, METH_VARARGS, nullptr}, {"entries", entries, METH_NOARGS, nullptr},
                          {"names", names, METH_NOARGS, nullptr}, {}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_host", nullptr, -1, methods};
 

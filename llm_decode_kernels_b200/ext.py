@@ -172,25 +172,38 @@ def _stream():
     return torch.cuda.current_stream().cuda_stream
 
 
-def _load_host(lib):
-    """The native call path (csrc/host_ops.cpp), built first if it is absent, bound to `lib`."""
+def _load_host():
+    """The native call path (csrc/host_ops.cpp), built first if it is absent."""
     if not HOST_PATH.exists():
         from . import build as _build
         _build.build_host()
     from . import _host
-    _host.bind({n: ctypes.cast(getattr(lib, n), c_void_p).value for n in _host.names()[0]})
     return _host
 
 
 class Ops:
     """The operator set. Every method launches on torch's current CUDA stream and returns None. The operators a decode step is
-    made of are called through native code that makes the same checks; what it does not accept comes to the methods here."""
+    made of are called through native code that makes the same checks; what it does not accept comes to the methods here. So
+    do all calls of a subclass's own methods, and of a `lib` that is not a loaded library but something in its place."""
 
     def __init__(self, lib):
         self.lib = lib
-        host = _load_host(lib)
-        for name in host.names()[1]:
-            setattr(self, name, host.operator(name, getattr(self, name)))
+
+    @property
+    def lib(self):
+        return self._lib
+
+    @lib.setter
+    def lib(self, lib):
+        self._lib = lib
+        for name in self.__dict__.pop("_native", ()):
+            del self.__dict__[name]
+        if isinstance(lib, ctypes.CDLL):
+            host = _load_host()
+            self._native = [n for n in host.entries() if getattr(type(self), n) is getattr(Ops, n)]
+            for name in self._native:
+                entry = ctypes.cast(getattr(lib, host.entries()[name]), c_void_p).value
+                setattr(self, name, host.operator(name, entry, getattr(type(self), name).__get__(self)))
 
     def _check(self, code, what):
         if code != 0:

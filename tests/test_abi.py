@@ -122,3 +122,33 @@ def test_descriptors_have_the_fields_of_the_header():
         fields = [re.sub(r"\[.*?\]", "", f).split()[-1].lstrip("*") for line in body.split(";") for f in line.split(",") if f.strip()]
         assert fields == [f[0] for f in cls._fields_], name
     assert ext.StepDesc._fields_[-1][0] == "trace" and ctypes.sizeof(ext.StepDesc) == 168
+
+
+def test_native_call_path_leaves_overrides_and_stand_ins_alone():
+    """A subclass's method, and whatever stands in for the library, are what a call reaches."""
+    import torch
+    real = ext.load_library()
+    calls = []
+
+    class Counting(ext.Ops):
+        def swiglu(self, gu, out):
+            calls.append("swiglu")
+    Counting(real).swiglu(1, 2)
+    assert calls == ["swiglu"]
+
+    class StandIn:
+        def __getattr__(self, name):
+            return lambda *a: calls.append(name) or 0
+    ops = ext.Ops(real)
+    native = type(ops.swiglu)
+    assert native.__name__ == "operator" and isinstance(ops.add_rmsnorm, native)
+    ops.lib = StandIn()
+    assert not isinstance(ops.swiglu, native) and ops.lib.b200_swiglu() == 0 and calls[-1] == "b200_swiglu"
+    with pytest.raises(RuntimeError, match="CUDA tensor"):
+        ops.swiglu(torch.zeros(16), torch.zeros(8))
+    ops.lib = real
+    assert isinstance(ops.swiglu, native)
+    assert not isinstance(ext.Ops(StandIn()).swiglu, native)
+    other = ext.Ops(real)                 # one object's binding is not another's
+    ops.lib = StandIn()
+    assert isinstance(other.swiglu, native)
