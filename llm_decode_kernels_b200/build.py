@@ -18,7 +18,7 @@ PKG = Path(__file__).resolve().parent
 CSRC = PKG / "csrc"
 INCLUDE = PKG.parent / "include"
 LIB = PKG / "libb200decode.so"
-HOST = PKG / "_host.so"          # the operators' call path (csrc/host_ops.cpp), a CPython extension module
+HOST_SRC = CSRC / "host_ops.cpp"   # the operators' call path, a CPython extension module
 
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-lineinfo", "-std=c++17",
               "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr"]
@@ -78,25 +78,44 @@ def build(force=False, verbose=False, defines=(), lib=LIB):
     return lib
 
 
+def host_path():
+    """Where _host lies. The name holds what the module was made for - source, C declarations, torch, Python - so that one made for
+    anything else is never loaded."""
+    import hashlib
+    import sysconfig
+    import torch
+    h = hashlib.sha256()
+    for part in (HOST_SRC.read_bytes(), (INCLUDE / "b200decode.h").read_bytes(), torch.__version__.encode(),
+                 sysconfig.get_config_var("SOABI").encode()):
+        h.update(part + b"\0")
+    return PKG / f"_host_{h.hexdigest()[:16]}.so"
+
+
 def build_host(force=False, verbose=False):
-    """Compile _host.so if it is stale. Returns its path."""
-    src = CSRC / "host_ops.cpp"
-    if not force and HOST.exists() and HOST.stat().st_mtime >= src.stat().st_mtime:
-        return HOST
+    """Compile the module of host_path() if it is not there. Returns its path."""
+    out = host_path()
+    if not force and out.exists():
+        return out
     import sysconfig
     import torch
     root = Path(torch.__file__).resolve().parent
     cuda = Path(nvcc()).resolve().parents[1]
+    tmp = out.with_name(f".{out.stem}.{os.getpid()}")   # several processes may build at once: each moves a whole file into place
     cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}", "-I", sysconfig.get_paths()["include"],
            "-I", str(root / "include"), "-I", str(root / "include/torch/csrc/api/include"), "-I", str(cuda / "include"),
-           str(src), "-o", str(HOST), "-L", str(root / "lib"), "-ltorch_python", "-ltorch_cpu", "-lc10", "-lc10_cuda"]
+           str(HOST_SRC), "-o", str(tmp), "-L", str(root / "lib"), "-ltorch_python", "-ltorch_cpu", "-lc10", "-lc10_cuda"]
     r = subprocess.run(cmd, capture_output=True, text=True)
     if verbose or r.returncode:
-        sys.stderr.write(f"--- {src.name}\n{r.stdout}{r.stderr}")
+        sys.stderr.write(f"--- {HOST_SRC.name}\n{r.stdout}{r.stderr}")
     if r.returncode:
-        raise RuntimeError(f"{cmd[0]} failed on {src.name}")
-    return HOST
+        tmp.unlink(missing_ok=True)
+        raise RuntimeError(f"{cmd[0]} failed on {HOST_SRC.name}")
+    os.replace(tmp, out)
+    for old in PKG.glob("_host*.so"):
+        if old != out:
+            old.unlink(missing_ok=True)
+    return out
 
 
 if __name__ == "__main__":

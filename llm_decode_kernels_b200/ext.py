@@ -13,7 +13,11 @@ rope_append_batched, embed_row, argmax, and the prompt's batched forms gemm_w4a1
 swiglu_batched.
 """
 import ctypes
+import importlib.machinery
+import importlib.util
 import math
+import sys
+import warnings
 from ctypes import c_float, c_int, c_longlong, c_size_t, c_void_p
 from pathlib import Path
 
@@ -21,8 +25,8 @@ import torch
 
 _LIB = None
 _OPS = None
+_HOST = None         # the native call path; False: cannot be had
 LIB_PATH = Path(__file__).resolve().parent / "libb200decode.so"
-HOST_PATH = LIB_PATH.with_name("_host.so")
 
 # name -> argtypes, exactly the declarations of include/b200decode.h (checked by tests/test_abi.py)
 SIGNATURES = {
@@ -173,12 +177,23 @@ def _stream():
 
 
 def _load_host():
-    """The native call path (csrc/host_ops.cpp), built first if it is absent."""
-    if not HOST_PATH.exists():
-        from . import build as _build
-        _build.build_host()
-    from . import _host
-    return _host
+    """The native call path (csrc/host_ops.cpp), built first if it is absent; None, with a warning, where it cannot be had: every
+    operator has its ctypes form."""
+    global _HOST
+    if _HOST is None:
+        try:
+            from . import build as _build
+            path = _build.build_host()
+            name = f"{__package__}._host"
+            spec = importlib.util.spec_from_file_location(name, path, loader=importlib.machinery.ExtensionFileLoader(name, str(path)))
+            _HOST = importlib.util.module_from_spec(spec)
+            spec.loader.exec_module(_HOST)
+            sys.modules[name] = _HOST
+            setattr(sys.modules[__package__], "_host", _HOST)
+        except Exception as e:      # no compiler, no headers, no write permission, a module that does not load
+            _HOST = False
+            warnings.warn(f"operators are called through ctypes, several microseconds slower each: {e}", RuntimeWarning, stacklevel=4)
+    return _HOST or None
 
 
 class Ops:
@@ -200,6 +215,8 @@ class Ops:
             del self.__dict__[name]
         if isinstance(lib, ctypes.CDLL):
             host = _load_host()
+            if host is None:
+                return
             self._native = [n for n in host.entries() if getattr(type(self), n) is getattr(Ops, n)]
             for name in self._native:
                 entry = ctypes.cast(getattr(lib, host.entries()[name]), c_void_p).value

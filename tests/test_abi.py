@@ -152,3 +152,40 @@ def test_native_call_path_leaves_overrides_and_stand_ins_alone():
     other = ext.Ops(real)                 # one object's binding is not another's
     ops.lib = StandIn()
     assert isinstance(other.swiglu, native)
+
+
+def test_operators_do_without_the_native_call_path(monkeypatch):
+    """No compiler, no headers: one warning, and every operator in its ctypes form."""
+    import warnings
+    from llm_decode_kernels_b200 import build as B
+    real = ext.load_library()
+
+    def no_compiler(*a, **k):
+        raise RuntimeError("no compiler")
+    monkeypatch.setattr(ext, "_HOST", None)
+    monkeypatch.setattr(B, "build_host", no_compiler)
+    with pytest.warns(RuntimeWarning, match="no compiler"):
+        ops = ext.Ops(real)
+    assert ops.swiglu.__func__ is ext.Ops.swiglu
+    with warnings.catch_warnings():
+        warnings.simplefilter("error")
+        ext.Ops(real)
+
+
+def test_native_call_path_is_made_for_what_loads_it(monkeypatch, tmp_path):
+    """Another torch, source or header has another file; the build puts a whole file in place and leaves nothing else behind."""
+    import torch
+    from llm_decode_kernels_b200 import build as B
+    here = B.host_path()
+    monkeypatch.setattr(torch, "__version__", "0.0.1")
+    assert B.host_path() != here
+    monkeypatch.undo()
+    src = tmp_path / "host_ops.cpp"
+    src.write_bytes(B.HOST_SRC.read_bytes() + b"\n")
+    monkeypatch.setattr(B, "HOST_SRC", src)
+    assert B.host_path() != here
+    monkeypatch.undo()
+    monkeypatch.setattr(B, "PKG", tmp_path)
+    (tmp_path / "_host_0123456789abcdef.so").write_bytes(b"made for something else")
+    out = B.build_host()
+    assert out.parent == tmp_path and [p.name for p in tmp_path.glob("*host*.so")] == [out.name] and not list(tmp_path.glob(".*"))
