@@ -185,7 +185,8 @@ int b200_gemm_w4a16(const void* Wp, const void* SZ, const void* X, void* Y, int 
  * of CTA pairs (1, 2, 4) that share an output tile by splitting K. Timed-out waits: b200_gemm_w4a16_status. */
 int b200_gemm_w4a16_tiled(const void* Wt, const void* X, void* Y, int T, int N, int K, int swiglu, int split, void* stream);
 int b200_gemm_w4a16_max_tokens(void);
-/* Synchronous read of the status word: 0, or 1 once a bounded wait ran out. */
+/* Synchronous read of the status of all prompt kernels (b200_gemm_w4a16, b200_gemm_w4a16_tiled, b200_prefill_chunk): 0, or 1 once a
+ * bounded wait ran out in one of them (sticky). */
 int b200_gemm_w4a16_status(int* code);
 
 /* out fp16 [N, K] (16B) = per-element dequantized weight, bit-identical to the quantizer's dequantize

@@ -271,11 +271,11 @@ int b200_gemm_w4a16_max_tokens(void) { return b200::prefill_gemm_max_tokens(); }
 
 int b200_gemm_w4a16_status(int* code) {
   REQUIRE(code, B200_ERR_ARG);
-  int tiled = 0, attention = 0;
-  cudaError_t e = b200::prefill_gemm_status(code);
+  int rows = 0, tiled = 0, attention = 0;   // the kernels' own words say which wait it was; here 0 or 1
+  cudaError_t e = b200::prefill_gemm_status(&rows);
   if (e == cudaSuccess) e = b200::prefill_gemm_tiled_status(&tiled);
   if (e == cudaSuccess) e = b200::prefill_attention_status(&attention);
-  *code |= tiled | attention;
+  if (e == cudaSuccess) *code = rows || tiled || attention;
   return finish(e);
 }
 

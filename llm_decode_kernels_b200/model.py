@@ -400,9 +400,9 @@ class Model:
         self._step_desc, self._step_att = d, st["att_xchg"].data_ptr() or None
 
     def step_error(self):
-        """Non-zero if a bounded wait inside a kernel of the step gave up (the step's outputs are then invalid): the
-        persistent kernel's code (4 = a token id outside the vocabulary was replaced by 0), the peer exchange's, or
-        the attention ring's. Synchronises."""
+        """Non-zero if a bounded wait inside a kernel of the step or of prefill() gave up (the outputs since are then
+        invalid): the persistent kernel's code (4 = a token id outside the vocabulary was replaced by 0), the peer
+        exchange's, the attention ring's, or 5 for the prompt kernels. Synchronises."""
         code = 0
         if getattr(self, "comm", None) is not None:
             code = self.comm.error()
@@ -410,6 +410,8 @@ class Model:
             code = code or int(self._step_static["ctrl"][1])
         else:
             code = code or self.K.paged_attention_status()
+        if getattr(self, "_prefilled", False):
+            code = code or 5 * self.K.gemm_status()
         return code
 
     def prepare(self, ctx_cap, use_graph=True, part_size=None):
@@ -777,6 +779,7 @@ class Model:
         if self.host_pos + n > limit:
             raise RuntimeError(f"context {self.host_pos + n} exceeds the prepared attention cap {limit}; call prepare()")
         dev, K, G = self.tok.device, self.K, self.cfg.group
+        self._prefilled = True
         ids = _ids_to(ids, dev)
         if self._tiled_prefill() is not None:
             all_logits, last = self._prefill_tiled(ids, collect_logits)
