@@ -686,6 +686,7 @@ class Model:
         need = min(n, chunk) * per_token
         if self._prefill_work is None or self._prefill_work.numel() < need:
             self._prefill_work = torch.empty(need, dtype=torch.uint8, device=dev)
+        self._prefill_work.record_stream(torch.cuda.current_stream(dev))   # a longer prompt, perhaps on another stream, replaces it
         base = self._prefill_work.data_ptr()
         d.bt = self.bt.data_ptr()
         all_logits = torch.empty(n, self.V_full, dtype=torch.half, device=dev) if collect_logits else None

@@ -161,3 +161,28 @@ def test_tokens_do_not_see_a_later_nan(D, n_q, n_kv, start, T, bad):
     got = m.prefill(ids, collect_logits=True).float()
     assert torch.isnan(got[bad:]).all()
     assert bad == 0 or (got[:bad] - want[:bad]).abs().max() <= KERNEL_TOL * want.abs().max()
+
+
+def test_prompts_on_two_streams_keep_their_work_buffer():
+    """A prompt on a side stream, then a longer one, which replaces the work buffer: its memory is not handed to the stream it was
+    allocated on while the side stream still uses it."""
+    from llm_decode_kernels_b200.model import DecodeConfig, Model
+    from test_model import hf_cfg, random_state
+    c = hf_cfg(512, 2, 8, 2, 1024, 1000)
+    m = Model(random_state(c, 3), c, DecodeConfig(group=128, max_ctx=2100, page=16, seed=1))
+    m.prepare(2048, use_graph=False)
+    ids = torch.randint(0, 1000, (1500,), generator=torch.Generator().manual_seed(4))   # on the host: checking them waits for nothing
+    m.reset(0)
+    m.prefill(ids[:700])                    # allocates the buffer, on the current stream
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        torch.cuda._sleep(200_000_000)      # the side stream is busy for a while
+        m.reset(0)
+        m.prefill(ids[:700])
+        used = m._prefill_work.data_ptr(), m._prefill_work.numel()
+        m.prefill(ids[700:])                # more than the buffer holds: it is replaced
+    assert m._prefill_work.data_ptr() != used[0]
+    again = torch.empty(used[1], dtype=torch.uint8, device=dev)     # on the current stream
+    assert again.data_ptr() != used[0]
+    torch.cuda.synchronize()
