@@ -459,6 +459,55 @@ def test_attention_in_clusters_keeps_nan(K, ctx):
     assert torch.isnan(out.float()).all()
 
 
+# The split kernels behind the cluster form: few (sequence, kv head) pairs and a cap of more than 16384 tokens, whatever the live context.
+# They leave partials in the scratch, the cluster kernel none, which is how the test knows what ran.
+SPLIT_CASES = [(64, 32, 4, 16), (64, 8, 8, 8), (64, 8, 4, 64), (64, 16, 8, 32), (128, 8, 1, 16), (128, 8, 8, 16), (128, 4, 2, 32), (128, 16, 4, 8)]
+
+
+def _split_scratch(n_q, D, PS, S):
+    return [torch.full((n_q, S, *w), float("nan"), device=dev) for w in ((D,), (), ())]
+
+
+@pytest.mark.parametrize("D,n_q,n_kv,page", SPLIT_CASES)
+def test_attention_on_both_sides_of_the_cluster_rule(K, D, n_q, n_kv, page):
+    torch.manual_seed(D + n_kv + page)
+    for ctx, PS in ((1, 512), (63, 64), (512, 512), (700, 512), (1537, 512), (16384, 512)):
+        kc, vc, bt, pos, _ = _cluster_case(n_q, n_kv, D, [ctx], page)
+        bt[0] = bt[0][torch.randperm(bt.shape[1], device=dev)]
+        q = torch.randn(n_q, D, device=dev).half()
+        want = R.paged_attention_ref(q.cpu(), kc.cpu(), vc.cpu(), bt[0].cpu(), ctx, page)
+        for S, ring in ((16384 // PS, False), (16384 // PS + 1, True)):
+            scratch, out = _split_scratch(n_q, D, PS, S), torch.full((n_q, D), float("nan"), dtype=torch.half, device=dev)
+            K.paged_attention_batched(q[None], kc, vc, bt, pos, PS, *[t[None] for t in scratch], out[None], version=3)
+            assert rel_err(out, want) <= ATTN_TOL, (ctx, PS, ring)
+            assert bool(torch.isfinite(scratch[0][:, 0]).all()) == (ring and ctx > PS), (ctx, PS, ring)
+    assert K.paged_attention_status() == 0
+
+
+@pytest.mark.parametrize("D,n_q,n_kv,page", SPLIT_CASES)
+def test_rope_attention_in_splits(K, D, n_q, n_kv, page):
+    """RoPE + append + attention with a cap beyond the cluster form, with the combine kernel and with the splits merged by the last
+    block to arrive (its count goes up, and back to zero), against the two kernels one after the other."""
+    torch.manual_seed(D + page)
+    arrive = torch.zeros(n_kv, dtype=torch.int32, device=dev)
+    cos, sin = (t.to(dev) for t in R.rope_tables(3000, D))
+    for ctx, PS in ((1, 64), (65, 64), (300, 128), (2049, 512)):
+        kc, vc, bt, pos, _ = _cluster_case(n_q, n_kv, D, [ctx], page)
+        qkv = torch.randn((n_q + 2 * n_kv) * D, device=dev).half()
+        S = 16384 // PS + 1
+        q2, kc2, vc2 = qkv.clone(), kc.clone(), vc.clone()
+        K.rope_append_batched(q2[None], cos, sin, pos, bt, kc2, vc2, n_q, n_kv)
+        want = R.paged_attention_ref(q2[:n_q * D].view(n_q, D).cpu(), kc2.cpu(), vc2.cpu(), bt[0].cpu(), ctx, page)
+        for counts in (None, arrive):
+            q1, kc1, vc1 = qkv.clone(), kc.clone(), vc.clone()
+            scratch, out = _split_scratch(n_q, D, PS, S), torch.full((n_q, D), float("nan"), dtype=torch.half, device=dev)
+            K.rope_paged_attention(q1, cos, sin, pos, bt[0], kc1, vc1, n_q, n_kv, PS, *scratch, out, counts)
+            assert rel_err(out, want) <= ATTN_TOL, (ctx, PS, counts is None)
+            assert torch.equal(kc1, kc2) and torch.equal(vc1, vc2) and torch.equal(q1, qkv)
+            assert bool(torch.isfinite(scratch[0][:, 0]).all()) == (ctx > PS) and int(arrive.abs().sum()) == 0
+    assert K.paged_attention_status() == 0
+
+
 @pytest.mark.parametrize("H", [2048, 8192, 128, 4104])
 def test_add_rmsnorm(K, H):
     torch.manual_seed(H)

@@ -175,3 +175,29 @@ def test_prefill_in_chunks_and_refusals():
     m2 = Model(sd, c, DecodeConfig(group=128, max_ctx=64, page=16, keep_packed=False))
     with pytest.raises(ValueError, match="keep_packed"):
         m2.prefill([1, 2, 3])
+
+
+@pytest.mark.parametrize("n_q,n_kv,D", [(8, 2, 64), (8, 1, 128)])
+def test_prefill_from_the_row_major_tensors(n_q, n_kv, D):
+    """Groups of 64, which the tile layout does not hold: chunks of gemm_max_tokens() through b200_gemm_w4a16, the third of them a
+    replayed graph, the last a partial one - against stepping; then a second prompt through the recorded graph."""
+    c = hf_cfg(512, 2, n_q, n_kv, 1024, 1000, D=D)
+    m = Model(random_state(c, 7, D), c, DecodeConfig(group=64, max_ctx=2600, page=16, seed=5))
+    m.prepare(2560, use_graph=False)
+    n = 3 * m.K.gemm_max_tokens() + 50
+    ids = torch.randint(0, 1000, (n,), generator=torch.Generator().manual_seed(2))
+    m.reset(0)
+    want = m.teacher_force(ids, use_graph=False, collect_logits=True).float()
+    kv, tok = m.kv.clone().float(), int(m.tok)
+    assert m._tiled_prefill() is None
+    for rerun in range(2):
+        m.kv.zero_()
+        m.reset(0)
+        got = m.prefill(ids, collect_logits=True).float()
+        assert (got - want).abs().max() <= KERNEL_TOL * want.abs().max()
+        assert torch.equal((m.kv != 0).any(-1), (kv != 0).any(-1))
+        assert (m.kv.float() - kv).abs().max() <= KERNEL_TOL * kv.abs().max()
+        assert m.host_pos == n and int(m.pos) == n and m.step_error() == 0
+        top = want[-1].sort(descending=True)[0]
+        assert int(m.tok) == tok or top[0] - top[1] <= 2 * KERNEL_TOL * want.abs().max()
+    assert any(st["graph"] is not None for st in m._prefill_cache.values())

@@ -65,9 +65,11 @@ def test_gemm_tiled_swiglu(K, I, Kd, T, split):
 
 
 # heads per group 1 .. 8, both head sizes, pages of 8 .. 64 tokens; prompts of one row block and several, with and without
-# a context before them, and a few tokens behind a long one (the context is then split between blocks)
+# a context before them, and a few tokens behind a long one (the context is then split between blocks); more than one chunk
+# of 4096 tokens
 @pytest.mark.parametrize("D,n_q,n_kv,page,start,T", [(64, 8, 8, 16, 0, 130), (64, 8, 4, 8, 37, 65), (64, 8, 2, 64, 0, 33),
                                                      (64, 8, 1, 16, 1500, 5), (64, 16, 2, 16, 700, 200), (128, 8, 1, 16, 0, 70),
+                                                     (64, 8, 2, 16, 0, 4500), (128, 8, 1, 16, 300, 4100),
                                                      (128, 4, 4, 16, 1100, 3), (64, 8, 1, 16, 0, 1), (64, 16, 2, 16, 4090, 7),
                                                      (128, 8, 1, 32, 191, 130), (64, 8, 2, 16, 500, 300)])
 def test_prefill_equals_stepping(D, n_q, n_kv, page, start, T):
