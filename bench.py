@@ -206,10 +206,10 @@ def peak_hbm_gbs():
 
 
 # Measured with ncu on the same kernel, TinyLlama shape cut to 6 layers (profiles/decode_step_kernel_tinyllama_6layers.md):
-# dram__bytes_read.sum + dram__bytes_write.sum of one launch (175,887,616 + 4,746,752) over the algorithmic bytes of
+# dram__bytes_read.sum + dram__bytes_write.sum of one launch (175,830,528 + 4,072,704) over the algorithmic bytes of
 # that launch (6 layers + LM head + embedding row + KV at context 40: 175,499,264). Traffic grows with the layers in
 # proportion to the bytes, so the 22-layer figure is this ratio times the step's bytes.
-STEP_TRAFFIC_OVER_ALGORITHMIC = 180634368 / 175499264
+STEP_TRAFFIC_OVER_ALGORITHMIC = 179903232 / 175499264
 
 
 def prompt_record(m, n):

@@ -58,9 +58,11 @@ int b200_bw_read(const void* p, size_t bytes, void* sink, int blocks, int thread
  * [n_q, max_splits]; out [n_q, 64]. n_q / n_kv in {1,2,4,8}. Tokens beyond max_splits * PS are ignored.
  * `version` (1..3, as in the reference, whose three versions are three generations of its kernel) selects the kernel:
  * 1 = K/V by register loads (any page and split size); 2 = K/V pages pulled into a shared-memory ring by bulk async
- * copies, arithmetic on the fp32 pipes; 3 = the same ring with both contractions as warp-level tensor-core MMAs
- * (the fastest; with 8 query heads per KV head the fp32 pipes cannot keep up with HBM). 2 and 3 need pages of 8..64
- * tokens and PS a multiple of the page size and otherwise run as 1. All three meet the same tolerance. */
+ * copies, arithmetic on the fp32 pipes; 3 = both contractions as warp-level tensor-core MMAs (the fastest; with 8 query
+ * heads per KV head the fp32 pipes cannot keep up with HBM): in one launch by clusters of CTAs, which leave o_part, m_part and
+ * l_part alone, where these fill half of the chip or the cap max_splits * PS is within 2048 tokens per CTA of a cluster
+ * (pages of 8 tokens and more), else from the ring of 2. The ring needs pages of 8..64 tokens and PS a multiple of the page
+ * size; without it 2 and 3 run as 1. All three meet the same tolerance. A position of -1 leaves out alone. */
 int b200_paged_attention(int version, const void* q, const void* kc, const void* vc, const int* bt, const int* pos,
                          int n_q, int n_kv, int log2P, int PS, int max_splits, float* o_part, float* m_part,
                          float* l_part, void* out, void* stream);

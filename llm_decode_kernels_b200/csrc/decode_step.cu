@@ -49,13 +49,14 @@
 // The per-element weight this stands for is the format's dequantized weight (dequant_w4a16 in gemv_w4a16.cu proves
 // the format bit-exactly).
 //
-// Phases per layer (the reference's operator order, with the same rounding points as its fused kernels):
+// Phases per layer (the reference's operator order and the rounding points of its fused kernels, but for the
+// normalised row, which is not rounded to fp16 before the product):
 //   A  resid += down[l-1] (layer 0: resid = embedding row);  x = RMSNorm(resid) * ln1;  qkv = Wqkv x
 //   B  attention: RoPE on q and k, append k, v to the paged cache, online softmax over the cached tokens (from the ring).
-//      Short contexts: one CTA per query head. Longer ones: a CTA takes one kv head and one slice of the context for ALL
-//      query heads of the group (up to 8), so every cached row is copied and read once, both contractions as warp-level
-//      MMAs; the slices' normalised outputs and log-sum-exps go to an exchange of their own, and one CTA per head merges
-//      them. (TinyLlama shape at 8192 cached tokens: 695 us a token with up to four CTAs per query head, 440 this way.)
+//      Short contexts: one CTA per query head. Longer ones, with an exchange of its own (the wide one): a CTA takes one kv head and
+//      one slice of the context for ALL query heads of the group (up to 8), so every cached row is copied and read once,
+//      both contractions as warp-level MMAs; one CTA per head merges the slices' outputs. (TinyLlama shape at 8192
+//      cached tokens: 695 us a token with up to four CTAs per query head, 440 this way.) Without: see att_plan.
 //   C  o = Wo attn
 //   D  resid += o;  x = RMSNorm(resid) * ln2;  act = SwiGLU(Wgate x, Wup x)
 //   E  down = Wdown act

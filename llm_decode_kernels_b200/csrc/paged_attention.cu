@@ -1260,8 +1260,8 @@ static cudaError_t launch_partial(int hpg, int kind, const AttnArgs& a, cudaStre
 // 0, or 1 once a block of the staged kernel gave up waiting for its own copies (its outputs are then invalid).
 cudaError_t paged_attention_status(int* code) { return cudaMemcpyFromSymbol(code, g_attn_status, sizeof(int)); }
 
-// version: 1 register-load kernel, 2 ring-staged kernel on the fp32 pipes, 3 ring-staged kernel with the contractions
-// on the tensor cores, 0 the library's choice (3). 2 and 3 fall back to 1 for shapes the ring does not cover.
+// version: 1 register-load kernel, 2 ring-staged kernel on the fp32 pipes, 0 and 3 on the tensor cores: the cluster kernel where
+// cluster_ctas() says so, else the ring-staged one. 2 and 3 fall back to 1 for shapes the ring does not cover.
 cudaError_t paged_attention_dispatch(int version, const void* q, const void* kc, const void* vc, const int* bt,
                                      int bt_stride, const int* pos, int B, int n_q, int n_kv, int D, int log2P, int PS,
                                      int max_splits, float* o_part, float* m_part, float* l_part, void* out,

@@ -556,13 +556,15 @@ class Ops:
         """w [N, K] fp16 / bf16 / fp32 -> whichever outputs are given: packed int32 [N, K/8], sz fp16 [N, K/G, 2], levels q
         uint8 [N, K], scale and zero fp16 [N, K/G], dequantized deq fp16 [N, K]."""
         w = _cuda(w.contiguous(), "w")
-        if w.data_ptr() % 16:      # a view that starts in the middle of a buffer; the kernel reads 16 bytes at a time
+        at = w.data_ptr()
+        if at % 16:      # a view that starts in the middle of a buffer; the kernel reads 16 bytes at a time
             w = w.clone()
+            at = w.data_ptr()
         N, K = w.shape
         ptr = [None if t is None else t.data_ptr() for t in (packed, sz, q, scale, zero, deq)]
         with torch.cuda.device(w.device):
             self._check(self.lib.b200_quantize_w4(
-                w.data_ptr(), (torch.float16, torch.bfloat16, torch.float32).index(w.dtype), N, K, int(group), int(clip),
+                at, (torch.float16, torch.bfloat16, torch.float32).index(w.dtype), N, K, int(group), int(clip),
                 *ptr, _stream()), "quantize_w4")
 
     def gptq_block(self, W, b0, b1, U, group, clip, Q, S, Z, Eb):

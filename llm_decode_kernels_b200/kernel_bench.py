@@ -179,7 +179,7 @@ def attention_fp32(q, kc, vc, bt, ctxs, page):
     return out
 
 
-ATTN_VERSIONS = ((1, "v1 register loads"), (2, "v2 ring, fp32 pipes"), (3, "v3 ring, tensor cores"))
+ATTN_VERSIONS = ((1, "v1 register loads"), (2, "v2 ring, fp32 pipes"), (3, "v3 tensor cores"))
 ATTN_CONTEXTS = (128, 512, 2048, 8192)
 
 
@@ -238,7 +238,7 @@ def write_attn_policy(rows, path=POLICY_PATH):
     policy.append({"max_ctx": 1 << 30, "part_size": int(rows[ctxs[-1]])})
     path.parent.mkdir(exist_ok=True)
     path.write_text(json.dumps({"gpu": torch.cuda.get_device_name(0), "heads": "32q/4kv x64", "page": 16,
-                                "kernel": "v3 ring, tensor cores", "policy": policy}, indent=1) + "\n")
+                                "kernel": "v3 tensor cores", "policy": policy}, indent=1) + "\n")
 
 
 def bench_attention(K, write_policy=True):
@@ -248,7 +248,7 @@ def bench_attention(K, write_policy=True):
     for c in ATTN_CONTEXTS:
         row = attention_case(K, 1, [c])
         out[f"batch 1 ctx {c}"] = row
-        best_ps[c] = row["v3 ring, tensor cores"]["part_size"]
+        best_ps[c] = row["v3 tensor cores"]["part_size"]
     ctxs = torch.randint(128, 8193, (8,), generator=g).tolist()
     out[f"batch 8 ctx U[128,8192] sum {sum(ctxs)}"] = attention_case(K, 8, ctxs)
     if write_policy:

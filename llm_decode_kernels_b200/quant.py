@@ -60,12 +60,15 @@ def group_params(wf, clip=False):
     return best_scale, best_zero
 
 
+_transform = torch._C._functorch.peek_interpreter_stack   # the innermost vmap, grad, jvp ... around the call, or None
+
+
 def _kernel_takes(w, group):
     """Whether the CUDA quantizer covers this input: groups of 8 to 256 weights, a power of two (a group is then at most
     one warp of 8-weight threads), and a floating type it reads; and nothing records or transforms the call (the torch form's
     scales have a gradient)."""
     return (w.is_cuda and type(w) in (torch.Tensor, torch.nn.Parameter) and not (w.requires_grad and torch.is_grad_enabled())
-            and torch._C._functorch.peek_interpreter_stack() is None and w.numel() > 0 and w.dtype in (torch.float16, torch.bfloat16, torch.float32)
+            and _transform() is None and w.numel() > 0 and w.dtype in (torch.float16, torch.bfloat16, torch.float32)
             and 8 <= group <= 256 and group & (group - 1) == 0)
 
 

@@ -84,7 +84,8 @@ def main():
             d[:, :, i + 1] -= w
         prev = lay[:, :, PER_PHASE - 1]             # attention follows the qkv emit
         for i in range(G, PER_LAYER - 1):
-            d[:, :, i] = np.where(lay[:, :, i] > 0, lay[:, :, i] - prev, 0.0)
+            # only a CTA with a unit of this step has stamped all of them (one more slice may start within the measured steps)
+            d[:, :, i] = np.where((lay[:, :, i] > 0) & (prev > 0), lay[:, :, i] - prev, 0.0)
             prev = lay[:, :, i]
         d[:, :, PER_LAYER - 1] = lay[:, :, PER_LAYER - 1]   # a duration
         acc.append(d)
