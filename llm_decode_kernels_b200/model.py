@@ -118,8 +118,8 @@ class Linear:
         if cfg.quant == "pre" and pre is None:
             pre = (cfg.qparams or {}).get(key)
             assert pre is not None, f"no precomputed weights for {key}"
-        with torch.no_grad():    # parameters as a state: nothing here has a gradient
-            ql = QuantLinear(w.to(cfg.device), cfg.group, keep_ref=keep_ref, clip=cfg.quant == "clip", qsz=pre)
+        # detached: a state of parameters records nothing here
+        ql = QuantLinear(w.detach().to(cfg.device), cfg.group, keep_ref=keep_ref, clip=cfg.quant == "clip", qsz=pre)
         self.packed, self.sz = ql.packed.to(cfg.device), ql.sz.to(cfg.device)
         self.w_ref = ql.w_ref
         self.nbytes = ql.nbytes()
