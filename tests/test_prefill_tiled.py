@@ -173,18 +173,21 @@ def test_prompts_on_two_streams_keep_their_work_buffer():
     c = hf_cfg(512, 2, 8, 2, 1024, 1000)
     m = Model(random_state(c, 3), c, DecodeConfig(group=128, max_ctx=2100, page=16, seed=1))
     m.prepare(2048, use_graph=False)
-    ids = torch.randint(0, 1000, (1500,), generator=torch.Generator().manual_seed(4))   # on the host: checking them waits for nothing
+    # on the host and pinned: neither checking nor copying them waits for the side stream
+    ids = torch.randint(0, 1000, (1500,), generator=torch.Generator().manual_seed(4)).pin_memory()
     m.reset(0)
     m.prefill(ids[:700])                    # allocates the buffer, on the current stream
     side = torch.cuda.Stream()
     side.wait_stream(torch.cuda.current_stream())
     with torch.cuda.stream(side):
-        torch.cuda._sleep(200_000_000)      # the side stream is busy for a while
+        torch.cuda._sleep(1_000_000_000)    # the side stream is busy for about half a second
         m.reset(0)
         m.prefill(ids[:700])
         used = m._prefill_work.data_ptr(), m._prefill_work.numel()
         m.prefill(ids[700:])                # more than the buffer holds: it is replaced
+        done = side.record_event()
     assert m._prefill_work.data_ptr() != used[0]
+    assert not done.query(), "the host was too slow for this test"
     again = torch.empty(used[1], dtype=torch.uint8, device=dev)     # on the current stream
     assert again.data_ptr() != used[0]
     torch.cuda.synchronize()
