@@ -5,8 +5,9 @@
 namespace b200 {
 namespace umma {
 
-constexpr int kSpin = 1 << 20;                         // polls before a wait gives up ...
-constexpr unsigned long long kWaitNs = 100000000ull;   // ... or this long
+// Polls before a wait gives up: about a second (a poll that is not met suspends the warp for 7,760 clocks). Counted and not timed: the
+// clock runs on while the GPU is given to another process, and a wait that is about to be met must not end for that.
+constexpr int kSpin = 1 << 18;
 
 DEVI uint32_t sa(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 DEVI void bar_init(uint64_t* b, int count) {
@@ -34,27 +35,16 @@ DEVI bool bar_try(uint64_t* b, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
-DEVI unsigned long long now_ns() {
-  unsigned long long t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
-}
 // false if the phase did not complete within the bound or another role of the CTA has given up; *status <- code of the first wait
 // that ran out
 template <int SLEEP_NS>
 DEVI bool bar_wait(uint64_t* b, uint32_t parity, volatile int* fail, int* status, int code) {
   if (bar_try(b, parity)) return true;
-  unsigned long long t0 = 0;   // the timer is slow to read: only a wait that is late anyway looks at it
 #pragma unroll 1
   for (int i = 0; i < kSpin; ++i) {
     if (SLEEP_NS > 0) __nanosleep(SLEEP_NS);
     if (bar_try(b, parity)) return true;
-    if ((i & 63) == 63) {
-      if (*fail) return false;
-      const unsigned long long t = now_ns();
-      if (!t0) t0 = t;
-      if (t - t0 > kWaitNs) break;
-    }
+    if ((i & 63) == 63 && *fail) return false;
   }
   *fail = 1;
   atomicCAS(status, 0, code);
