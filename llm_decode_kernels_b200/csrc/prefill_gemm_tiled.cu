@@ -114,12 +114,67 @@ DEVI uint32_t gated2(uint32_t gate, uint32_t up) {
   return as_u32(__hmul2(s, as_h2(up)));
 }
 
+// The accumulator of a CTA's 128 rows x nt tokens -> rows[token pair][128 rows], two tokens of a row in a word: columns c0 .. c0 + 31 of
+// every `step`, by a warp that reaches lanes 32 q .. . The next tile's MMAs wait for this: with a token's row as a half of its own
+// (single conversions, 2-byte stores) it took 1.8 us for 128 tokens, a quarter of a tile's time at 256.
+DEVI void park_tile(uint32_t tmem, int q, int lane, uint32_t* rows, int c0, int step, int nt) {
+  const uint32_t from = tmem + ((uint32_t)(32 * q) << 16);
+#pragma unroll 1
+  for (int c = c0; c < nt; c += step) {   // nt is a multiple of 32
+    float v[32];
+    tmem_ld16_async(from + c, v);
+    tmem_ld16_async(from + c + 16, v + 16);
+    tmem_wait_ld(v);
+    uint32_t* to = rows + (c >> 1) * 128 + 32 * q + lane;
+#pragma unroll
+    for (int j = 0; j < 16; ++j) to[128 * j] = as_u32(__floats2half2_rn(v[2 * j], v[2 * j + 1]));
+  }
+}
+
+// rows -> Y: tokens t0 .. of the tile, features from row0 (SWIGLU: half of it) on; thread `at` of `threads`. A thread takes eight outputs of
+// two tokens.
+template <bool SWIGLU>
+DEVI void store_tile(const uint32_t* rows, half* Y, int T, int N, int t0, int row0, int nt, int at, int threads) {
+  constexpr int kPieces = SWIGLU ? 8 : 16;   // pieces of 8 outputs per token
+  const bool vec = (N & 7) == 0 && (reinterpret_cast<uintptr_t>(Y) & 15) == 0;
+  const int pairs = (min(nt, T - t0) + 1) >> 1;
+#pragma unroll 1
+  for (int i = at; i < pairs * kPieces; i += threads) {
+    const int tp = i / kPieces, pc = i % kPieces, f = (SWIGLU ? row0 >> 1 : row0) + 8 * pc;
+    const uint4* src = reinterpret_cast<const uint4*>(rows + tp * 128 + (SWIGLU ? 16 : 8) * pc);
+    const uint4 a = src[0], b = src[1];
+    uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+    if (SWIGLU) {   // rows 16 k + 0..7 are gates, 16 k + 8..15 their up rows
+      const uint4 c = src[2], d = src[3];
+      const uint32_t u[8] = {c.x, c.y, c.z, c.w, d.x, d.y, d.z, d.w};
+#pragma unroll
+      for (int e = 0; e < 8; ++e) w[e] = gated2(w[e], u[e]);
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int t = t0 + 2 * tp + h;
+      if (t >= T) break;
+      uint32_t o[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) o[e] = __byte_perm(w[2 * e], w[2 * e + 1], h ? 0x7632 : 0x5410);
+      half* y = Y + (size_t)t * N + f;
+      if (vec && f + 7 < N) {
+        *reinterpret_cast<uint4*>(y) = make_uint4(o[0], o[1], o[2], o[3]);
+      } else {
+#pragma unroll
+        for (int e = 0; e < 8; ++e)
+          if (f + e < N) y[e] = __ushort_as_half((unsigned short)(o[e >> 1] >> (16 * (e & 1))));
+      }
+    }
+  }
+}
+
 }  // namespace
 
 template <bool SWIGLU>
 __global__ void __launch_bounds__(kThreads, 1)
 prefill_gemm_tiled_kernel(const __grid_constant__ CUtensorMap xmap, const uint8_t* __restrict__ Wt, half* __restrict__ Y, int T,
-                          int N, int row_tiles, int nunit, int nt, int S, int feat_tiles, int tiles, int ns) {
+                          int N, int row_tiles, int nunit, int nt, int S, int feat_tiles, int tiles, int ns, int p_apart) {
   extern __shared__ uint8_t raw[];
   __shared__ Shared sh;
   uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(raw) + 1023) & ~(uintptr_t)1023);
@@ -131,12 +186,14 @@ prefill_gemm_tiled_kernel(const __grid_constant__ CUtensorMap xmap, const uint8_
   const uint32_t lead = rank & ~1u;
   const int u0 = nunit * split / S, u1 = nunit * (split + 1) / S;
   const int half_bytes = nt * 64, stage_bytes = 2 * half_bytes;   // 64 columns of K x nt / 2 tokens; a unit
+  uint32_t* rows = reinterpret_cast<uint32_t*>(base + ns * stage_bytes);   // a finished tile, see park_tile
   volatile int* fail = &sh.fail;
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(sa(&sh.tmem)) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
   }
   if (tid == 0) {
+    asm volatile("prefetch.tensormap [%0];" ::"l"(&xmap) : "memory");   // before the wait for X, not behind it
     for (int s = 0; s < ns; ++s) {
       bar_init(&sh.full[s], 2 * 4 + 1);   // one group of dequantizing warps in each CTA of the pair, and the copies
       bar_init(&sh.empty[s], 1);
@@ -287,84 +344,88 @@ prefill_gemm_tiled_kernel(const __grid_constant__ CUtensorMap xmap, const uint8_
         }
     }
   } else {
-    // ---- epilogue: a warp reaches the 32 lanes (rows) of its quarter
-    const int q = warp & 3, et = tid - 32 * kDqWarps;
-    const uint32_t taddr = tmem + ((uint32_t)(32 * q) << 16);
-    half* rows = reinterpret_cast<half*>(base + ns * stage_bytes);   // [token][128 rows]
+    // ---- epilogue of all tiles but the CTA's last: a warp reaches the 32 lanes (rows) of its quarter
+    const int et = tid - 32 * kDqWarps;
     auto epilogue_sync = [] { asm volatile("bar.sync 1, %0;" ::"n"(32 * kEpWarps) : "memory"); };
-    const bool vec = (N & 7) == 0 && (reinterpret_cast<uintptr_t>(Y) & 15) == 0;
+    auto any_failed = [&] {   // the same barrier, and one answer for all: a warp that left alone would strand the others at the next one
+      uint32_t p;
+      asm volatile(
+          "{\n\t.reg .pred q, p;\n\t"
+          "setp.ne.s32 q, %1, 0;\n\t"
+          "bar.red.or.pred p, 1, %2, q;\n\t"
+          "selp.u32 %0, 1, 0, p;\n\t}"
+          : "=r"(p)
+          : "r"(*fail), "n"(32 * kEpWarps)
+          : "memory");
+      return p != 0;
+    };
     int done = 0;
 #pragma unroll 1
     for (int tile = first; tile < tiles; tile += stride, ++done) {
       const bool ok = __all_sync(0xffffffffu, bar_wait<128>(&sh.acc_full, done & 1, fail, WAIT_EP));
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      if (S > 1) {   // one tile per cluster: park the partial tile P[token][128 rows] as fp32 over the idle stages
-        float* P = reinterpret_cast<float*>(base);
-#pragma unroll 1
-        for (int c = 0; ok && c < nt; c += 16) {
-          uint32_t v[16];
-          tmem_ld16(taddr + c, v);
-#pragma unroll
-          for (int j = 0; j < 16; ++j) P[(c + j) * 128 + 32 * q + lane] = __uint_as_float(v[j]);
-        }
-        break;
-      }
-#pragma unroll 1
-      for (int c = 0; ok && c < nt; c += 16) {
-        uint32_t v[16];
-        tmem_ld16(taddr + c, v);
-#pragma unroll
-        for (int j = 0; j < 16; ++j) rows[(c + j) * 128 + 32 * q + lane] = __float2half_rn(__uint_as_float(v[j]));
-      }
+      if (tile + stride >= tiles) break;
+      if (ok) park_tile(tmem, warp & 3, lane, rows, 0, 32, nt);
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-      epilogue_sync();   // the tile is complete; a warp that gave up has raised the flag before
-      if (*fail) break;
+      if (any_failed()) break;   // otherwise the tile is complete: a warp that gave up has raised the flag before
       if (lane == 0) bar_arrive_cluster(in_cta(sa(&sh.acc_empty), lead));
       if (done == 0) pdl_wait();   // Y may still be read by the kernel before this one
-      const int t0 = (tile / feat_tiles) * nt, row0 = (tile % feat_tiles) * 256 + side * 128, tn = min(nt, T - t0);
-      constexpr int kPieces = SWIGLU ? 8 : 16;   // pieces of 8 outputs per token
-#pragma unroll 2
-      for (int i = et; i < tn * kPieces; i += 32 * kEpWarps) {
-        const int t = i / kPieces, pc = i % kPieces, f = (SWIGLU ? row0 >> 1 : row0) + 8 * pc;
-        const uint4* src = reinterpret_cast<const uint4*>(rows + t * 128 + (SWIGLU ? 16 : 8) * pc);
-        uint4 o = src[0];
-        if (SWIGLU) {   // rows 16 k + 0..7 are gates, 16 k + 8..15 their up rows
-          const uint4 u = src[1];
-          o = make_uint4(gated2(o.x, u.x), gated2(o.y, u.y), gated2(o.z, u.z), gated2(o.w, u.w));
-        }
-        half* y = Y + (size_t)(t0 + t) * N + f;
-        if (vec && f + 7 < N) {
-          *reinterpret_cast<uint4*>(y) = o;
-        } else {
-          const uint32_t w[4] = {o.x, o.y, o.z, o.w};
-#pragma unroll
-          for (int e = 0; e < 8; ++e)
-            if (f + e < N) y[e] = __ushort_as_half((unsigned short)(w[e >> 1] >> (16 * (e & 1))));
-        }
-      }
+      store_tile<SWIGLU>(rows, Y, T, N, (tile / feat_tiles) * nt, (tile % feat_tiles) * 256 + side * 128, nt, et, 32 * kEpWarps);
       epilogue_sync();   // `rows` is free for the next tile
     }
   }
+  // ---- the CTA's last tile, by all warps: those that are not the epilogue's are idle by now
   __syncwarp();
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-  cluster_barrier();   // partial tiles are parked; every MMA that reads a peer's shared memory has completed
-  if (S > 1 && first < tiles && !*fail) {
-    pdl_wait();
-    // CTA (split, side) finishes tokens split, split + S, ... of its side's rows: sum in split order, four rows a lane
-    const int t_base = (first / feat_tiles) * nt, row0 = (first % feat_tiles) * 256 + side * 128;
-    for (int t = warp * S + split; t < nt && t_base + t < T; t += (kThreads / 32) * S) {
-      const uint32_t local = sa(base) + (uint32_t)((t * 128 + 4 * lane) * sizeof(float));
-      float4 v[kMaxSplit];
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const bool live = first < tiles && !*fail;
+  const int last_tile = first < tiles ? first + (tiles - 1 - first) / stride * stride : 0;
+  const int t_base = (last_tile / feat_tiles) * nt, row0 = (last_tile % feat_tiles) * 256 + side * 128;
+  if (S == 1) {
+    if (live && warp < 16) park_tile(tmem, warp & 3, lane, rows, 32 * (warp >> 2), 128, nt);
+    __syncthreads();
+    if (live) {
+      pdl_wait();
+      store_tile<SWIGLU>(rows, Y, T, N, t_base, row0, nt, tid, kThreads);
+    }
+  } else {
+    // The split tile meets in the CTA that finishes a token: CTA (split, side) does tokens [split nt / S, (split + 1) nt / S) of its side's
+    // rows. Every CTA writes its fp32 partials there, P[split][token][128 rows], and reads only its own shared memory afterwards: one
+    // cluster barrier. (Partials parked locally and fetched by the finishing CTA: a round trip of distributed shared memory and a second
+    // barrier more, 1.5 us a launch at 96 tokens.) Where P does not fit beside the stages it lies over them: then all CTAs' MMAs have
+    // to be done first.
+    const int chunk = nt / S;
+    float* P = reinterpret_cast<float*>(base + (p_apart ? ns * stage_bytes : 0));
+    if (!p_apart) cluster_barrier();
+    if (live && warp < 16) {
+#pragma unroll 1
+      for (int c = 8 * (warp >> 2); c < nt; c += 32) {
+        uint32_t v[8];
+        tmem_ld8(tmem + ((uint32_t)(32 * (warp & 3)) << 16) + c, v);
+        const int owner = c / chunk;
+        const uint32_t to = in_cta(sa(P + (size_t)(split * chunk + c - owner * chunk) * 128 + 32 * (warp & 3) + lane), 2 * owner + side);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(to + 512 * j), "r"(v[j]) : "memory");
+      }
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    cluster_barrier();   // every CTA's partials are there, and nobody writes here any more
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    if (live) pdl_wait();
+    for (int k = warp; live && k < chunk; k += kThreads / 32) {
+      const int t = t_base + split * chunk + k;
+      if (t >= T) break;
+      float4 v[kMaxSplit];   // sum in split order, four rows a lane
 #pragma unroll
       for (int s = 0; s < kMaxSplit; ++s)
-        if (s < S) v[s] = ld_cluster4(in_cta(local, 2 * s + side));
+        if (s < S) v[s] = reinterpret_cast<const float4*>(P + (size_t)(s * chunk + k) * 128)[lane];
       float4 a = v[0];
 #pragma unroll
       for (int s = 1; s < kMaxSplit; ++s)
         if (s < S) a.x += v[s].x, a.y += v[s].y, a.z += v[s].z, a.w += v[s].w;
       half2 h01 = __floats2half2_rn(a.x, a.y), h23 = __floats2half2_rn(a.z, a.w);
-      half* y = Y + (size_t)(t_base + t) * N;
+      half* y = Y + (size_t)t * N;
       if (SWIGLU) {   // rows 16 k + 0..7 gates, 16 k + 8..15 their up rows: two lanes further on
         const uint32_t u01 = __shfl_xor_sync(0xffffffffu, as_u32(h01), 2), u23 = __shfl_xor_sync(0xffffffffu, as_u32(h23), 2);
         if ((lane & 2) == 0) {
@@ -388,7 +449,9 @@ prefill_gemm_tiled_kernel(const __grid_constant__ CUtensorMap xmap, const uint8_
       }
     }
   }
-  if (S > 1) cluster_barrier();   // nobody's shared memory goes away while a peer still reads it
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (S == 1) cluster_barrier();   // the pair is done with its tensor memory and with each other's barriers (S > 1: since the barrier above)
   if (warp == 0) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
@@ -423,8 +486,8 @@ cudaError_t prefill_gemm_tiled_status(int* code) {
 cudaError_t prefill_gemm_tiled_dispatch(const void* Wt, const void* X, void* Y, int T, int N, int K, int swiglu, int force_split,
                                         cudaStream_t st) {
   const int nunit = K / 128, row_tiles = swiglu ? (N + 7) / 8 : (N + 15) / 16, feat_tiles = (row_tiles + 15) / 16;
-  auto bytes = [](int tokens, int stages) { return 1024 + (size_t)tokens * (128 * stages + 256); };   // stages + fp16 tile
-  const size_t smem_max = bytes(kMaxTokens, 4);
+  auto bytes = [](int tokens, int stages, int per_token) { return 1024 + (size_t)tokens * (128 * stages + per_token); };
+  const size_t smem_max = 226 * 1024;   // the largest of what follows, beside the static part
   static size_t allowed[2][kMaxDevices] = {};
   cudaError_t e = allow_dynamic_smem(prefill_gemm_tiled_kernel<false>, smem_max, allowed[0]);
   if (e == cudaSuccess) e = allow_dynamic_smem(prefill_gemm_tiled_kernel<true>, smem_max, allowed[1]);
@@ -455,7 +518,9 @@ cudaError_t prefill_gemm_tiled_dispatch(const void* Wt, const void* X, void* Y, 
   }
   if (S == 0) return cudaErrorNotSupported;
   const int ns = nt <= 128 ? 6 : 4;   // what tensor memory has left beside the accumulator
-  const size_t smem = bytes(nt, ns);
+  // beside the stages: the fp16 tile, or the fp32 partials of a split one where they fit
+  const int p_apart = S > 1 && bytes(nt, ns, 512) <= smem_max;
+  const size_t smem = bytes(nt, ns, S == 1 ? 256 : p_apart ? 512 : 0);
   const int room = resident_clusters(S, smem_max);
   CUtensorMap xmap;
   if (!encode_activation_map(&xmap, X, T, K, nt / 2, 2)) return cudaErrorInvalidValue;
@@ -472,7 +537,7 @@ cudaError_t prefill_gemm_tiled_dispatch(const void* Wt, const void* X, void* Y, 
   cfg.attrs = attr;
   cfg.numAttrs = 2;
   return cudaLaunchKernelEx(&cfg, swiglu ? prefill_gemm_tiled_kernel<true> : prefill_gemm_tiled_kernel<false>, xmap,
-                            (const uint8_t*)Wt, (half*)Y, T, N, row_tiles, nunit, nt, S, feat_tiles, tiles, ns);
+                            (const uint8_t*)Wt, (half*)Y, T, N, row_tiles, nunit, nt, S, feat_tiles, tiles, ns, p_apart);
 }
 
 }  // namespace b200
