@@ -39,8 +39,6 @@ cudaError_t gptq_block_dispatch(const float* W, int ldw, int N, int nb, const fl
                                 int group, int clip, uint8_t* Q, int ldq, float* S, float* Z, int lds, float* E, int lde,
                                 cudaStream_t st);
 cudaError_t prefill_gemm_status(int* code);
-cudaError_t prefill_gemm_tiled_dispatch(const void* Wt, const void* X, void* Y, int T, int N, int K, int swiglu, int force_split,
-                                        cudaStream_t st);
 cudaError_t prefill_gemm_tiled_status(int* code);
 cudaError_t rope_append_dispatch(void* qkv, const float* cos_t, const float* sin_t, const int* pos, const int* bt,
                                  int bt_stride, void* kc, void* vc, int B, int n_q, int n_kv, int D, int log2P,
@@ -304,7 +302,7 @@ int b200_gemm_w4a16_tiled(const void* Wt, const void* X, void* Y, int T, int N, 
   REQUIRE(Wt && X && Y && T > 0 && N > 0 && K > 0 && (split == 0 || split == 1 || split == 2 || split == 4), B200_ERR_ARG);
   REQUIRE(K % 128 == 0 && split <= K / 128, B200_ERR_SHAPE);
   REQUIRE(aligned16(Wt) && aligned16(X) && (reinterpret_cast<uintptr_t>(Y) & 7u) == 0, B200_ERR_ALIGN);
-  return finish(b200::prefill_gemm_tiled_dispatch(Wt, X, Y, T, N, K, swiglu, split, S(stream)));
+  return finish(b200::prefill_gemm_tiled_dispatch(Wt, X, Y, T, N, K, swiglu, split, nullptr, S(stream)));
 }
 
 int b200_rope_append_batched(void* qkv, const float* cos_t, const float* sin_t, const int* pos, const int* bt,

@@ -10,6 +10,20 @@ namespace b200 {
 // boxes of 64 columns x box_rows tokens x chunks. False if the driver refuses (alignment).
 bool encode_activation_map(CUtensorMap* map, const void* X, int T, int K, int box_rows, int chunks);
 
+// RMSNorm inside the GEMMs of a prompt. The norm's factor is one number per token, so a GEMM may read rows that lack it and apply it to its
+// outputs. What it reads is xw = fp16(x * w * scale), written by the GEMM that finished the residual row x (RESIDUAL of
+// prefill_gemm_tiled_kernel: x += its output) together with the sums of x^2 over each 128 columns; the power of two `scale` keeps xw near
+// 1, whatever the size of the row, and follows from the row as it was before this addition, whose sum all its writers know.
+struct PrefillNorm {
+  const float* ss_in;    // [T][parts] sums of squares: of the rows behind X (to be normalised), or of x before this GEMM's addition
+  const float* inv_in;   // [T] 1 / scale of the rows X; null with RESIDUAL
+  half *x, *xw;          // RESIDUAL: [T, N]; otherwise null
+  const half* w;         // [N] the next norm's weight
+  float *ss_out, *inv_out;
+  int parts;             // H / 128
+  float inv_h, eps;
+};
+
 // One chunk of a prompt: T tokens at positions start .. start + T - 1 of the sequence whose block table is bt.
 struct PrefillParams {
   const StepLayer* layers;   // host array; matrices in tile layout, gate|up paired
@@ -29,8 +43,9 @@ bool prefill_attention_takes(int D, int n_q, int n_kv);
 cudaError_t prefill_attention_dispatch(const void* q, int q_stride, const void* kc, const void* vc, const int* bt, int start, int T,
                                        int n_q, int n_kv, int D, int log2P, void* out, cudaStream_t st);
 cudaError_t prefill_attention_status(int* code);
+// norm: null, or the norm of X's rows to apply, or (norm->x) the residual row to finish instead of storing Y
 cudaError_t prefill_gemm_tiled_dispatch(const void* Wt, const void* X, void* Y, int T, int N, int K, int swiglu, int force_split,
-                                        cudaStream_t st);
+                                        const PrefillNorm* norm, cudaStream_t st);
 cudaError_t add_rmsnorm_dispatch(void* x, const void* delta, const void* w, void* out, int rows, int H, float eps,
                                  cudaStream_t st);
 cudaError_t rope_append_dispatch(void* qkv, const float* cos_t, const float* sin_t, const int* pos, const int* bt,

@@ -114,10 +114,39 @@ DEVI uint32_t gated2(uint32_t gate, uint32_t up) {
   return as_u32(__hmul2(s, as_h2(up)));
 }
 
+// norm: what the epilogue multiplies a token by. Plain: rsqrt(mean square + eps) / scale, or 1; RESIDUAL: the scale of its row of xw.
+DEVI float token_factor(const PrefillNorm& nm, int t, bool residual) {
+  float a = 0.f, b = 0.f;   // two chains, always the same order
+  const float* p = nm.ss_in + (size_t)t * nm.parts;
+#pragma unroll 8
+  for (int i = 0; i + 1 < nm.parts; i += 2) a += p[i], b += p[i + 1];
+  if (nm.parts & 1) a += p[nm.parts - 1];
+  const float ms = (a + b) * nm.inv_h;
+  return residual ? 1.f / row_inv_scale(ms) : rsqrtf(ms + nm.eps) * nm.inv_in[t];
+}
+
+// Eight columns of a finished residual row: x += y, xw = x * w * scale; returns the sum of x^2.
+DEVI float residual8(const uint4& y, const uint4& w, half* x, half* xw, float scale) {
+  uint4 r = *reinterpret_cast<const uint4*>(x);
+  const uint32_t yu[4] = {y.x, y.y, y.z, y.w}, wu[4] = {w.x, w.y, w.z, w.w};
+  uint32_t ru[4] = {r.x, r.y, r.z, r.w}, o[4];
+  float ss = 0.f;
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    ru[e] = as_u32(__hadd2(as_h2(ru[e]), as_h2(yu[e])));
+    const float2 f = __half22float2(as_h2(ru[e])), g = __half22float2(as_h2(wu[e]));
+    ss = fmaf(f.x, f.x, fmaf(f.y, f.y, ss));
+    o[e] = as_u32(__floats2half2_rn(f.x * g.x * scale, f.y * g.y * scale));
+  }
+  *reinterpret_cast<uint4*>(x) = make_uint4(ru[0], ru[1], ru[2], ru[3]);
+  *reinterpret_cast<uint4*>(xw) = make_uint4(o[0], o[1], o[2], o[3]);
+  return ss;
+}
+
 // The accumulator of a CTA's 128 rows x nt tokens -> rows[token pair][128 rows], two tokens of a row in a word: columns c0 .. c0 + 31 of
 // every `step`, by a warp that reaches lanes 32 q .. . The next tile's MMAs wait for this: with a token's row as a half of its own
 // (single conversions, 2-byte stores) it took 1.8 us for 128 tokens, a quarter of a tile's time at 256.
-DEVI void park_tile(uint32_t tmem, int q, int lane, uint32_t* rows, int c0, int step, int nt) {
+DEVI void park_tile(uint32_t tmem, int q, int lane, uint32_t* rows, int c0, int step, int nt, const float* fac) {
   const uint32_t from = tmem + ((uint32_t)(32 * q) << 16);
 #pragma unroll 1
   for (int c = c0; c < nt; c += step) {   // nt is a multiple of 32
@@ -125,6 +154,13 @@ DEVI void park_tile(uint32_t tmem, int q, int lane, uint32_t* rows, int c0, int 
     tmem_ld16_async(from + c, v);
     tmem_ld16_async(from + c + 16, v + 16);
     tmem_wait_ld(v);
+    if (fac) {
+#pragma unroll
+      for (int j = 0; j < 32; j += 4) {
+        const float4 f = *reinterpret_cast<const float4*>(fac + c + j);
+        v[j] *= f.x, v[j + 1] *= f.y, v[j + 2] *= f.z, v[j + 3] *= f.w;
+      }
+    }
     uint32_t* to = rows + (c >> 1) * 128 + 32 * q + lane;
 #pragma unroll
     for (int j = 0; j < 16; ++j) to[128 * j] = as_u32(__floats2half2_rn(v[2 * j], v[2 * j + 1]));
@@ -169,14 +205,53 @@ DEVI void store_tile(const uint32_t* rows, half* Y, int T, int N, int t0, int ro
   }
 }
 
+// rows -> the residual stream (PrefillNorm): 16 lanes take a token pair's 128 columns, so each of the two sums is one of theirs.
+DEVI void store_residual(const uint32_t* rows, const PrefillNorm& nm, const float* fac, int T, int N, int t0, int row0, int nt, int at,
+                         int threads) {
+  const int lane = at & 31, pairs = (min(nt, T - t0) + 1) >> 1, pc = at & 15, f = row0 + 8 * pc;
+  if (row0 >= N) return;   // N is a multiple of 128
+  const uint4 w8 = __ldg(reinterpret_cast<const uint4*>(nm.w + f));
+#pragma unroll 1
+  for (int i = at; i - lane < pairs * 16; i += threads) {
+    const int tp = i >> 4;
+    float ss[2] = {0.f, 0.f};
+    if (tp < pairs) {
+      const uint4* src = reinterpret_cast<const uint4*>(rows + tp * 128 + 8 * pc);
+      const uint4 a = src[0], b = src[1];
+      const uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int t = t0 + 2 * tp + h;
+        if (t < T) {
+          uint32_t o[4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e) o[e] = __byte_perm(w[2 * e], w[2 * e + 1], h ? 0x7632 : 0x5410);
+          ss[h] = residual8(make_uint4(o[0], o[1], o[2], o[3]), w8, nm.x + (size_t)t * N + f, nm.xw + (size_t)t * N + f, fac[2 * tp + h]);
+        }
+      }
+    }
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) {
+      ss[0] += __shfl_xor_sync(0xffffffffu, ss[0], o);
+      ss[1] += __shfl_xor_sync(0xffffffffu, ss[1], o);
+    }
+    const int t = t0 + 2 * tp + pc;   // lanes 0 and 1 of the sixteen
+    if (tp < pairs && pc < 2 && t < T) {
+      nm.ss_out[(size_t)t * nm.parts + (row0 >> 7)] = pc ? ss[1] : ss[0];
+      if (row0 == 0) nm.inv_out[t] = 1.f / fac[2 * tp + pc];
+    }
+  }
+}
+
 }  // namespace
 
-template <bool SWIGLU>
+template <bool SWIGLU, bool RESIDUAL>
 __global__ void __launch_bounds__(kThreads, 1)
 prefill_gemm_tiled_kernel(const __grid_constant__ CUtensorMap xmap, const uint8_t* __restrict__ Wt, half* __restrict__ Y, int T,
-                          int N, int row_tiles, int nunit, int nt, int S, int feat_tiles, int tiles, int ns, int p_apart) {
+                          int N, int row_tiles, int nunit, int nt, int S, int feat_tiles, int tiles, int ns, int p_apart, const PrefillNorm nm) {
   extern __shared__ uint8_t raw[];
   __shared__ Shared sh;
+  __shared__ __align__(16) float token_fac[kMaxTokens];
   uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(raw) + 1023) & ~(uintptr_t)1023);
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;   // warp: known to be uniform
   uint32_t rank;
@@ -187,6 +262,7 @@ prefill_gemm_tiled_kernel(const __grid_constant__ CUtensorMap xmap, const uint8_
   const int u0 = nunit * split / S, u1 = nunit * (split + 1) / S;
   const int half_bytes = nt * 64, stage_bytes = 2 * half_bytes;   // 64 columns of K x nt / 2 tokens; a unit
   uint32_t* rows = reinterpret_cast<uint32_t*>(base + ns * stage_bytes);   // a finished tile, see park_tile
+  const float* fac = !RESIDUAL && nm.ss_in ? token_fac : nullptr;   // multiplies the outputs
   volatile int* fail = &sh.fail;
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(sa(&sh.tmem)) : "memory");
@@ -360,17 +436,24 @@ prefill_gemm_tiled_kernel(const __grid_constant__ CUtensorMap xmap, const uint8_
       return p != 0;
     };
     int done = 0;
+    if (first < tiles) pdl_wait();   // Y may still be read by the kernel before this one; the norm's sums come from it or from earlier ones
 #pragma unroll 1
     for (int tile = first; tile < tiles; tile += stride, ++done) {
+      if (nm.ss_in) {
+        const int t0 = (tile / feat_tiles) * nt;
+        for (int i = et; i < nt; i += 32 * kEpWarps) token_fac[i] = t0 + i < T ? token_factor(nm, t0 + i, RESIDUAL) : 0.f;
+        epilogue_sync();
+      }
       const bool ok = __all_sync(0xffffffffu, bar_wait<128>(&sh.acc_full, done & 1, fail, WAIT_EP));
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       if (tile + stride >= tiles) break;
-      if (ok) park_tile(tmem, warp & 3, lane, rows, 0, 32, nt);
+      if (ok) park_tile(tmem, warp & 3, lane, rows, 0, 32, nt, fac);
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       if (any_failed()) break;   // otherwise the tile is complete: a warp that gave up has raised the flag before
       if (lane == 0) bar_arrive_cluster(in_cta(sa(&sh.acc_empty), lead));
-      if (done == 0) pdl_wait();   // Y may still be read by the kernel before this one
-      store_tile<SWIGLU>(rows, Y, T, N, (tile / feat_tiles) * nt, (tile % feat_tiles) * 256 + side * 128, nt, et, 32 * kEpWarps);
+      const int t0 = (tile / feat_tiles) * nt, row0 = (tile % feat_tiles) * 256 + side * 128;
+      if (RESIDUAL) store_residual(rows, nm, token_fac, T, N, t0, row0, nt, et, 32 * kEpWarps);
+      else store_tile<SWIGLU>(rows, Y, T, N, t0, row0, nt, et, 32 * kEpWarps);
       epilogue_sync();   // `rows` is free for the next tile
     }
   }
@@ -383,11 +466,12 @@ prefill_gemm_tiled_kernel(const __grid_constant__ CUtensorMap xmap, const uint8_
   const int last_tile = first < tiles ? first + (tiles - 1 - first) / stride * stride : 0;
   const int t_base = (last_tile / feat_tiles) * nt, row0 = (last_tile % feat_tiles) * 256 + side * 128;
   if (S == 1) {
-    if (live && warp < 16) park_tile(tmem, warp & 3, lane, rows, 32 * (warp >> 2), 128, nt);
+    if (live && warp < 16) park_tile(tmem, warp & 3, lane, rows, 32 * (warp >> 2), 128, nt, fac);
     __syncthreads();
     if (live) {
       pdl_wait();
-      store_tile<SWIGLU>(rows, Y, T, N, t_base, row0, nt, tid, kThreads);
+      if (RESIDUAL) store_residual(rows, nm, token_fac, T, N, t_base, row0, nt, tid, kThreads);
+      else store_tile<SWIGLU>(rows, Y, T, N, t_base, row0, nt, tid, kThreads);
     }
   } else {
     // The split tile meets in the CTA that finishes a token: CTA (split, side) does tokens [split nt / S, (split + 1) nt / S) of its side's
@@ -424,7 +508,25 @@ prefill_gemm_tiled_kernel(const __grid_constant__ CUtensorMap xmap, const uint8_
 #pragma unroll
       for (int s = 1; s < kMaxSplit; ++s)
         if (s < S) a.x += v[s].x, a.y += v[s].y, a.z += v[s].z, a.w += v[s].w;
-      half2 h01 = __floats2half2_rn(a.x, a.y), h23 = __floats2half2_rn(a.z, a.w);
+      const float f = fac ? token_fac[split * chunk + k] : 1.f;
+      half2 h01 = __floats2half2_rn(a.x * f, a.y * f), h23 = __floats2half2_rn(a.z * f, a.w * f);
+      if (RESIDUAL) {   // as residual8
+        if (row0 >= N) break;
+        const float scale = token_fac[split * chunk + k];
+        const size_t at = (size_t)t * N + row0 + 4 * lane;
+        const uint2 r = *reinterpret_cast<const uint2*>(nm.x + at), w4 = __ldg(reinterpret_cast<const uint2*>(nm.w + row0 + 4 * lane));
+        h01 = __hadd2(as_h2(r.x), h01), h23 = __hadd2(as_h2(r.y), h23);
+        const float2 x01 = __half22float2(h01), x23 = __half22float2(h23), w01 = __half22float2(as_h2(w4.x)), w23 = __half22float2(as_h2(w4.y));
+        *reinterpret_cast<uint2*>(nm.x + at) = make_uint2(as_u32(h01), as_u32(h23));
+        *reinterpret_cast<uint2*>(nm.xw + at) = make_uint2(as_u32(__floats2half2_rn(x01.x * w01.x * scale, x01.y * w01.y * scale)),
+                                                           as_u32(__floats2half2_rn(x23.x * w23.x * scale, x23.y * w23.y * scale)));
+        const float ss = warp_sum(fmaf(x01.x, x01.x, fmaf(x01.y, x01.y, fmaf(x23.x, x23.x, x23.y * x23.y))));
+        if (lane == 0) {
+          nm.ss_out[(size_t)t * nm.parts + (row0 >> 7)] = ss;
+          if (row0 == 0) nm.inv_out[t] = 1.f / scale;
+        }
+        continue;
+      }
       half* y = Y + (size_t)t * N;
       if (SWIGLU) {   // rows 16 k + 0..7 gates, 16 k + 8..15 their up rows: two lanes further on
         const uint32_t u01 = __shfl_xor_sync(0xffffffffu, as_u32(h01), 2), u23 = __shfl_xor_sync(0xffffffffu, as_u32(h23), 2);
@@ -469,7 +571,7 @@ static int resident_clusters(int S, size_t smem) {   // clusters of 2 S CTAs the
     attr[0].val.clusterDim.x = 2 * S, attr[0].val.clusterDim.y = 1, attr[0].val.clusterDim.z = 1;
     cfg.gridDim = dim3(2 * S), cfg.blockDim = dim3(kThreads), cfg.dynamicSmemBytes = smem, cfg.attrs = attr, cfg.numAttrs = 1;
     int num = 0;
-    if (cudaOccupancyMaxActiveClusters(&num, prefill_gemm_tiled_kernel<false>, &cfg) != cudaSuccess) {
+    if (cudaOccupancyMaxActiveClusters(&num, prefill_gemm_tiled_kernel<false, false>, &cfg) != cudaSuccess) {
       (void)cudaGetLastError();
       num = 0;
     }
@@ -484,13 +586,16 @@ cudaError_t prefill_gemm_tiled_status(int* code) {
 
 // Y[T, N]; N = rows of W (swiglu: of outputs, W has 2 N rows in paired layout). force_split: 0, or the S to use.
 cudaError_t prefill_gemm_tiled_dispatch(const void* Wt, const void* X, void* Y, int T, int N, int K, int swiglu, int force_split,
-                                        cudaStream_t st) {
+                                        const PrefillNorm* norm, cudaStream_t st) {
   const int nunit = K / 128, row_tiles = swiglu ? (N + 7) / 8 : (N + 15) / 16, feat_tiles = (row_tiles + 15) / 16;
   auto bytes = [](int tokens, int stages, int per_token) { return 1024 + (size_t)tokens * (128 * stages + per_token); };
-  const size_t smem_max = 226 * 1024;   // the largest of what follows, beside the static part
-  static size_t allowed[2][kMaxDevices] = {};
-  cudaError_t e = allow_dynamic_smem(prefill_gemm_tiled_kernel<false>, smem_max, allowed[0]);
-  if (e == cudaSuccess) e = allow_dynamic_smem(prefill_gemm_tiled_kernel<true>, smem_max, allowed[1]);
+  const size_t smem_max = 225 * 1024 + 512;   // no less than what follows, and room for the static part
+  static size_t allowed[3][kMaxDevices] = {};
+  const bool residual = norm && norm->x;
+  if (residual && (swiglu || N % 128)) return cudaErrorInvalidValue;
+  auto kern = residual ? prefill_gemm_tiled_kernel<false, true> : swiglu ? prefill_gemm_tiled_kernel<true, false> : prefill_gemm_tiled_kernel<false, false>;
+  cudaError_t e = allow_dynamic_smem(prefill_gemm_tiled_kernel<false, false>, smem_max, allowed[0]);   // resident_clusters asks for this one
+  if (e == cudaSuccess && kern != prefill_gemm_tiled_kernel<false, false>) e = allow_dynamic_smem(kern, smem_max, allowed[residual ? 2 : 1]);
   if (e != cudaSuccess) return e;
   // Tokens per tile (equal tiles, so that the last is not nearly empty; up to eight more of them than there have to be) and split of
   // K, by estimated time. In microseconds, fitted to 1,250 measured launches (TinyLlama, 8B and 70B matrices, 16 .. 4096 tokens;
@@ -536,8 +641,8 @@ cudaError_t prefill_gemm_tiled_dispatch(const void* Wt, const void* X, void* Y, 
   cfg.stream = st;
   cfg.attrs = attr;
   cfg.numAttrs = 2;
-  return cudaLaunchKernelEx(&cfg, swiglu ? prefill_gemm_tiled_kernel<true> : prefill_gemm_tiled_kernel<false>, xmap,
-                            (const uint8_t*)Wt, (half*)Y, T, N, row_tiles, nunit, nt, S, feat_tiles, tiles, ns, p_apart);
+  return cudaLaunchKernelEx(&cfg, kern, xmap, (const uint8_t*)Wt, (half*)Y, T, N, row_tiles, nunit, nt, S, feat_tiles, tiles, ns, p_apart,
+                            norm ? *norm : PrefillNorm{});
 }
 
 }  // namespace b200
