@@ -302,7 +302,7 @@ int b200_gemm_w4a16_tiled(const void* Wt, const void* X, void* Y, int T, int N, 
   REQUIRE(Wt && X && Y && T > 0 && N > 0 && K > 0 && (split == 0 || split == 1 || split == 2 || split == 4), B200_ERR_ARG);
   REQUIRE(K % 128 == 0 && split <= K / 128, B200_ERR_SHAPE);
   REQUIRE(aligned16(Wt) && aligned16(X) && (reinterpret_cast<uintptr_t>(Y) & 7u) == 0, B200_ERR_ALIGN);
-  return finish(b200::prefill_gemm_tiled_dispatch(Wt, X, Y, T, N, K, swiglu, split, nullptr, S(stream)));
+  return finish(b200::prefill_gemm_tiled_dispatch(Wt, X, Y, T, N, K, swiglu, split, nullptr, nullptr, S(stream)));
 }
 
 int b200_rope_append_batched(void* qkv, const float* cos_t, const float* sin_t, const int* pos, const int* bt,

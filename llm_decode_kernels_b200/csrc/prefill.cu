@@ -1,4 +1,4 @@
-// A whole chunk of a prompt in one host call: embedding rows, then per layer six launches, then the final norm. The launches are
+// A whole chunk of a prompt in one host call: embedding rows, then per layer five launches, then the final norm. The launches are
 // issued from here and not from Python because a short prompt is bound by them: 242 calls through ctypes took 2.7 ms for 77 tokens,
 // more than the GPU needs.
 #include "prefill.h"
@@ -14,8 +14,10 @@ __global__ void __launch_bounds__(256)
 embed_rows_kernel(const uint4* __restrict__ emb, const long long* __restrict__ ids, const uint4* __restrict__ w, uint4* __restrict__ x,
                   uint4* __restrict__ xw, float* __restrict__ ss_out, float* __restrict__ inv_out, int nchunk, int parts, float inv_h, int V) {
   __shared__ float part[8];
-  pdl_launch_dependents();
   pdl_wait();
+  // behind the wait: no kernel of the chunk starts before what precedes the chunk has completed, so each of them may read what the
+  // chunk's kernels do not write (weights, positions, block table) ahead of its own wait
+  pdl_launch_dependents();
   long long t = ids[blockIdx.x];
   if (t < 0 || t >= V) t = 0;
   emb += (size_t)t * nchunk, x += (size_t)blockIdx.x * nchunk, xw += (size_t)blockIdx.x * nchunk;
@@ -49,6 +51,11 @@ embed_rows_kernel(const uint4* __restrict__ emb, const long long* __restrict__ i
 
 }  // namespace
 
+// Up to this many tokens the qkv GEMM does RoPE and the append itself. Beyond, a launch of its own costs no more than the epilogue, and
+// attention's CTAs, which do not fit beside a GEMM's, start up beside it. Whole prompt, TinyLlama shape, us (launch of its own / in the GEMM): 8
+// tokens 897 / 865, 77 1,045 / 1,045, 512 1,681 / 1,650, 700 2,038 / 2,002, 1000 2,380 / 2,418, 1400 2,986 / 3,016, 2000 4,100 / 4,061.
+constexpr int kRopeInGemm = 768;
+
 cudaError_t prefill_chunk_dispatch(const PrefillParams& p, cudaStream_t st) {
 #define TRY(call)                        \
   do {                                   \
@@ -70,12 +77,13 @@ cudaError_t prefill_chunk_dispatch(const PrefillParams& p, cudaStream_t st) {
     const PrefillNorm to_mlp = {ss_a, nullptr, x, xw, ly.ln2, ss_m, inv_m, parts, inv_h, p.eps};
     const PrefillNorm at_mlp = {ss_m, inv_m, nullptr, nullptr, nullptr, nullptr, nullptr, parts, inv_h, p.eps};
     const PrefillNorm to_next = {ss_m, nullptr, x, xw, last ? nullptr : p.layers[l + 1].ln1, ss_a, inv_a, parts, inv_h, p.eps};
-    TRY(prefill_gemm_tiled_dispatch(ly.w[0], p.normed, p.qkv, p.T, n_qkv, p.H, 0, 0, &at_qkv, st));
-    TRY(rope_append_dispatch(p.qkv, p.cos_t, p.sin_t, p.pos, p.bt, 0, ly.kc, ly.vc, p.T, p.n_q, p.n_kv, p.D, p.log2P, st));
+    const PrefillRope rope = {p.cos_t, p.sin_t, p.pos, p.bt, ly.kc, ly.vc, p.n_q, p.n_kv, p.D, p.log2P};
+    TRY(prefill_gemm_tiled_dispatch(ly.w[0], p.normed, p.qkv, p.T, n_qkv, p.H, 0, 0, &at_qkv, p.T <= kRopeInGemm ? &rope : nullptr, st));
+    if (p.T > kRopeInGemm) TRY(prefill_rope_append_dispatch(p, ly, st));
     TRY(prefill_attention_dispatch(p.qkv, n_qkv, ly.kc, ly.vc, p.bt, p.start, p.T, p.n_q, p.n_kv, p.D, p.log2P, p.attn, st));
-    TRY(prefill_gemm_tiled_dispatch(ly.w[1], p.attn, nullptr, p.T, p.H, n_att, 0, 0, &to_mlp, st));
-    TRY(prefill_gemm_tiled_dispatch(ly.w[2], p.normed, p.act, p.T, p.I, p.H, 1, 0, &at_mlp, st));
-    TRY(prefill_gemm_tiled_dispatch(ly.w[3], p.act, p.o, p.T, p.H, p.I, 0, 0, last ? nullptr : &to_next, st));
+    TRY(prefill_gemm_tiled_dispatch(ly.w[1], p.attn, nullptr, p.T, p.H, n_att, 0, 0, &to_mlp, nullptr, st));
+    TRY(prefill_gemm_tiled_dispatch(ly.w[2], p.normed, p.act, p.T, p.I, p.H, 1, 0, &at_mlp, nullptr, st));
+    TRY(prefill_gemm_tiled_dispatch(ly.w[3], p.act, p.o, p.T, p.H, p.I, 0, 0, last ? nullptr : &to_next, nullptr, st));
   }
   return add_rmsnorm_dispatch(p.x, p.o, p.norm_f, p.normed, p.T, p.H, p.eps, st);
 #undef TRY

@@ -24,6 +24,15 @@ struct PrefillNorm {
   float inv_h, eps;
 };
 
+// RoPE and the append to the paged cache inside the qkv GEMM (rope_append_rows_kernel's arithmetic on the fp16 outputs): q goes to Y
+// rotated, k rotated and v as they are to the caches.
+struct PrefillRope {
+  const float *cos_t, *sin_t;   // [positions, D / 2]
+  const int *pos, *bt;          // [T]; block table
+  half *kc, *vc;                // null: no RoPE
+  int n_q, n_kv, D, log2P;
+};
+
 // One chunk of a prompt: T tokens at positions start .. start + T - 1 of the sequence whose block table is bt.
 struct PrefillParams {
   const StepLayer* layers;   // host array; matrices in tile layout, gate|up paired
@@ -43,13 +52,12 @@ bool prefill_attention_takes(int D, int n_q, int n_kv);
 cudaError_t prefill_attention_dispatch(const void* q, int q_stride, const void* kc, const void* vc, const int* bt, int start, int T,
                                        int n_q, int n_kv, int D, int log2P, void* out, cudaStream_t st);
 cudaError_t prefill_attention_status(int* code);
-// norm: null, or the norm of X's rows to apply, or (norm->x) the residual row to finish instead of storing Y
+// norm: null, or the norm of X's rows to apply, or (norm->x) the residual row to finish instead of storing Y. rope: null, or what the
+// qkv GEMM does with its outputs.
 cudaError_t prefill_gemm_tiled_dispatch(const void* Wt, const void* X, void* Y, int T, int N, int K, int swiglu, int force_split,
-                                        const PrefillNorm* norm, cudaStream_t st);
+                                        const PrefillNorm* norm, const PrefillRope* rope, cudaStream_t st);
+cudaError_t prefill_rope_append_dispatch(const PrefillParams& p, const StepLayer& ly, cudaStream_t st);   // 16-byte aligned caches
 cudaError_t add_rmsnorm_dispatch(void* x, const void* delta, const void* w, void* out, int rows, int H, float eps,
-                                 cudaStream_t st);
-cudaError_t rope_append_dispatch(void* qkv, const float* cos_t, const float* sin_t, const int* pos, const int* bt,
-                                 int bt_stride, void* kc, void* vc, int B, int n_q, int n_kv, int D, int log2P,
                                  cudaStream_t st);
 
 }  // namespace b200

@@ -211,6 +211,16 @@ prefill_attn_kernel(const half* __restrict__ q, int q_stride, const half* __rest
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   pdl_launch_dependents();   // with this CTA's tensor memory allocated (see prefill_gemm_tiled_kernel)
   const uint32_t tmem = sh.tmem;
+  // a loading warp's rows lane and lane + 32 of its first tile: the block table does not come from the kernels before this one, and its
+  // round trip would stand in front of every other (embed_rows_kernel lets nothing of a chunk start before what precedes the chunk is done)
+  constexpr int RW = kTile / (LW / 2);   // rows of a tile per loading warp
+  const int first = ((warp - kMmaWarp - 1) >> 1) * RW;
+  auto row = [&](int i, int r) {   // row r of this warp's part of tile i in the cache, in units of D; behind the context: the last (masked)
+    const int j = min(k0 + i * kTile + first + r, last);
+    return ((__ldg(bt + (j >> log2P)) * n_kv + kvh) << log2P) + (j & ((1 << log2P) - 1));
+  };
+  int lo = 0, hi = 0;
+  if (warp > kMmaWarp && ntiles > 0) lo = row(0, lane), hi = RW > 32 ? row(0, lane + 32) : 0;
   pdl_wait();
 
   float m = -CUDART_INF_F, l = 0.f;   // softmax thread: reference maximum (base-2 units) and sum of its row
@@ -346,9 +356,9 @@ prefill_attn_kernel(const half* __restrict__ q, int q_stride, const half* __rest
   } else {
     // Half the warps copy K, half V; a warp takes RW rows of a tile, 32 / PP at a time, and hands a tile over when it has issued
     // kLag more. (One TMA box per page instead: 80 ns a box of 2 KB, a third slower in all.)
-    constexpr int RW = kTile / (LW / 2), IT = 16;
+    constexpr int IT = 16;
     static_assert(RW * PP == 32 * IT, "16 copies a lane and tile");
-    const int w = warp - kMmaWarp - 1, p = lane % PP, first = (w >> 1) * RW;   // K: even warps
+    const int w = warp - kMmaWarp - 1, p = lane % PP;   // K: even warps
     const bool is_v = w & 1;
     uint64_t *full = is_v ? sh.v_full : sh.k_full, *empty = is_v ? sh.v_empty : sh.k_empty;
     const half* from = (is_v ? vc : kc) + 8 * p;
@@ -356,18 +366,12 @@ prefill_attn_kernel(const half* __restrict__ q, int q_stride, const half* __rest
     uint32_t to[8 / (32 / PP)];   // rows 8 apart have one position in the swizzle
 #pragma unroll
     for (int k = 0; k < 8 / (32 / PP); ++k) to[k] = at + swz_piece(lane / PP + k * (32 / PP), p, kTile);
-    auto row = [&](int i, int r) {   // row r of this warp's part of tile i in the cache, in units of D; behind the context: the last (masked)
-      const int j = min(k0 + i * kTile + first + r, last);
-      return ((__ldg(bt + (j >> log2P)) * n_kv + kvh) << log2P) + (j & ((1 << log2P) - 1));
-    };
     auto hand_over = [&](int i) {   // this warp's part of tile i has landed
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       __syncwarp();
       if (lane == 0) bar_arrive(&full[i % NS]);
     };
     bool ok = true;
-    int lo = 0, hi = 0;   // rows lane and lane + 32 of the next tile
-    if (ntiles > 0) lo = row(0, lane), hi = RW > 32 ? row(0, lane + 32) : 0;
 #pragma unroll 1
     for (int i = 0; i < ntiles; ++i) {
       const int a = lo, b = hi, n = min(i + 1, ntiles - 1);

@@ -126,8 +126,7 @@ DEVI float token_factor(const PrefillNorm& nm, int t, bool residual) {
 }
 
 // Eight columns of a finished residual row: x += y, xw = x * w * scale; returns the sum of x^2.
-DEVI float residual8(const uint4& y, const uint4& w, half* x, half* xw, float scale) {
-  uint4 r = *reinterpret_cast<const uint4*>(x);
+DEVI float residual8(const uint4& r, const uint4& y, const uint4& w, half* x, half* xw, float scale) {   // r: x as it was
   const uint32_t yu[4] = {y.x, y.y, y.z, y.w}, wu[4] = {w.x, w.y, w.z, w.w};
   uint32_t ru[4] = {r.x, r.y, r.z, r.w}, o[4];
   float ss = 0.f;
@@ -211,10 +210,21 @@ DEVI void store_residual(const uint32_t* rows, const PrefillNorm& nm, const floa
   const int lane = at & 31, pairs = (min(nt, T - t0) + 1) >> 1, pc = at & 15, f = row0 + 8 * pc;
   if (row0 >= N) return;   // N is a multiple of 128
   const uint4 w8 = __ldg(reinterpret_cast<const uint4*>(nm.w + f));
+  uint4 next[2];   // the pair's rows of x, one round ahead
+  auto fetch = [&](int i) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int t = t0 + 2 * (i >> 4) + h;
+      if ((i >> 4) < pairs && t < T) next[h] = *reinterpret_cast<const uint4*>(nm.x + (size_t)t * N + f);
+    }
+  };
+  fetch(at);
 #pragma unroll 1
   for (int i = at; i - lane < pairs * 16; i += threads) {
     const int tp = i >> 4;
     float ss[2] = {0.f, 0.f};
+    const uint4 was[2] = {next[0], next[1]};
+    fetch(i + threads);
     if (tp < pairs) {
       const uint4* src = reinterpret_cast<const uint4*>(rows + tp * 128 + 8 * pc);
       const uint4 a = src[0], b = src[1];
@@ -226,7 +236,7 @@ DEVI void store_residual(const uint32_t* rows, const PrefillNorm& nm, const floa
           uint32_t o[4];
 #pragma unroll
           for (int e = 0; e < 4; ++e) o[e] = __byte_perm(w[2 * e], w[2 * e + 1], h ? 0x7632 : 0x5410);
-          ss[h] = residual8(make_uint4(o[0], o[1], o[2], o[3]), w8, nm.x + (size_t)t * N + f, nm.xw + (size_t)t * N + f, fac[2 * tp + h]);
+          ss[h] = residual8(was[h], make_uint4(o[0], o[1], o[2], o[3]), w8, nm.x + (size_t)t * N + f, nm.xw + (size_t)t * N + f, fac[2 * tp + h]);
         }
       }
     }
@@ -243,15 +253,81 @@ DEVI void store_residual(const uint32_t* rows, const PrefillNorm& nm, const floa
   }
 }
 
+// Where head `head` of token t goes from its first dim on: rotated q to Y, k and v to their row of the cache.
+DEVI half* head_row(const PrefillRope& rp, half* Y, int N, int head, int t, int page, int slot) {
+  if (head < rp.n_q) return Y + (size_t)t * N + head * rp.D;
+  const bool k = head < rp.n_q + rp.n_kv;
+  const int kvh = head - rp.n_q - (k ? 0 : rp.n_kv);
+  return (k ? rp.kc : rp.vc) + ((((size_t)page * rp.n_kv + kvh) << rp.log2P) + slot) * rp.D;
+}
+
+// rows -> q, K and V: a thread takes eight rotation pairs of two tokens (128 rows are whole heads: two of 64 dims or one of 128).
+DEVI void store_rope(const uint32_t* rows, const PrefillRope& rp, const int* positions, half* Y, int T, int N, int t0, int row0, int nt, int at, int threads) {
+  const int pairs = (min(nt, T - t0) + 1) >> 1, d2 = rp.D >> 1, heads = rp.n_q + 2 * rp.n_kv;
+#pragma unroll 1
+  for (int i = at; i < pairs * 8; i += threads) {
+    const int tp = i >> 3, j = 8 * (i & 7), local = j & (d2 - 1), lo_row = (j & ~(d2 - 1)) * 2 + local;   // pair j of the 64 of these rows
+    const int head = (row0 + lo_row) / rp.D;
+    if (head >= heads) continue;
+    const bool rotate = head < rp.n_q + rp.n_kv;
+    const int pos[2] = {positions[2 * tp], positions[2 * tp + 1]};   // of a token behind the last: the last one's
+    float4 cs[2][2], sn[2][2];   // both tokens' factors are in flight together
+    int page[2] = {0, 0};
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      if (rotate) {
+#pragma unroll
+        for (int v = 0; v < 2; ++v) {
+          cs[h][v] = __ldg(reinterpret_cast<const float4*>(rp.cos_t + (size_t)pos[h] * d2 + local) + v);
+          sn[h][v] = __ldg(reinterpret_cast<const float4*>(rp.sin_t + (size_t)pos[h] * d2 + local) + v);
+        }
+      }
+      if (head >= rp.n_q) page[h] = __ldg(rp.bt + (pos[h] >> rp.log2P));
+    }
+    const uint4 *lp = reinterpret_cast<const uint4*>(rows + tp * 128 + lo_row), *hp = reinterpret_cast<const uint4*>(rows + tp * 128 + lo_row + d2);
+    const uint4 l0 = lp[0], l1 = lp[1], h0 = hp[0], h1 = hp[1];
+    const uint32_t lw[8] = {l0.x, l0.y, l0.z, l0.w, l1.x, l1.y, l1.z, l1.w}, hw[8] = {h0.x, h0.y, h0.z, h0.w, h1.x, h1.y, h1.z, h1.w};
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int t = t0 + 2 * tp + h;
+      uint32_t lo[4], hi[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const uint32_t sel = h ? 0x7632 : 0x5410;
+        lo[e] = __byte_perm(lw[2 * e], lw[2 * e + 1], sel), hi[e] = __byte_perm(hw[2 * e], hw[2 * e + 1], sel);
+      }
+      if (rotate) {
+#pragma unroll
+        for (int v = 0; v < 2; ++v) {
+          const float4 c = cs[h][v], s = sn[h][v];
+          const float2 a01 = __half22float2(as_h2(lo[2 * v])), a23 = __half22float2(as_h2(lo[2 * v + 1]));
+          const float2 b01 = __half22float2(as_h2(hi[2 * v])), b23 = __half22float2(as_h2(hi[2 * v + 1]));
+          lo[2 * v] = as_u32(__floats2half2_rn(a01.x * c.x - b01.x * s.x, a01.y * c.y - b01.y * s.y));
+          lo[2 * v + 1] = as_u32(__floats2half2_rn(a23.x * c.z - b23.x * s.z, a23.y * c.w - b23.y * s.w));
+          hi[2 * v] = as_u32(__floats2half2_rn(b01.x * c.x + a01.x * s.x, b01.y * c.y + a01.y * s.y));
+          hi[2 * v + 1] = as_u32(__floats2half2_rn(b23.x * c.z + a23.x * s.z, b23.y * c.w + a23.y * s.w));
+        }
+      }
+      if (t >= T) break;
+      half* to = head_row(rp, Y, N, head, t, page[h], pos[h] & ((1 << rp.log2P) - 1)) + local;
+      *reinterpret_cast<uint4*>(to) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+      *reinterpret_cast<uint4*>(to + d2) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+    }
+  }
+}
+
+enum : int { PLAIN, GATED, RESIDUAL, ROPE };   // what the epilogue does: Y as it is, SwiGLU, PrefillNorm's residual row, PrefillRope
+
 }  // namespace
 
-template <bool SWIGLU, bool RESIDUAL>
+template <int MODE>
 __global__ void __launch_bounds__(kThreads, 1)
 prefill_gemm_tiled_kernel(const __grid_constant__ CUtensorMap xmap, const uint8_t* __restrict__ Wt, half* __restrict__ Y, int T,
-                          int N, int row_tiles, int nunit, int nt, int S, int feat_tiles, int tiles, int ns, int p_apart, const PrefillNorm nm) {
+                          int N, int row_tiles, int nunit, int nt, int S, int feat_tiles, int tiles, int ns, int p_apart, const PrefillNorm nm, const PrefillRope rp) {
   extern __shared__ uint8_t raw[];
   __shared__ Shared sh;
   __shared__ __align__(16) float token_fac[kMaxTokens];
+  __shared__ int token_pos[MODE == ROPE ? kMaxTokens : 1];
   uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(raw) + 1023) & ~(uintptr_t)1023);
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;   // warp: known to be uniform
   uint32_t rank;
@@ -262,7 +338,7 @@ prefill_gemm_tiled_kernel(const __grid_constant__ CUtensorMap xmap, const uint8_
   const int u0 = nunit * split / S, u1 = nunit * (split + 1) / S;
   const int half_bytes = nt * 64, stage_bytes = 2 * half_bytes;   // 64 columns of K x nt / 2 tokens; a unit
   uint32_t* rows = reinterpret_cast<uint32_t*>(base + ns * stage_bytes);   // a finished tile, see park_tile
-  const float* fac = !RESIDUAL && nm.ss_in ? token_fac : nullptr;   // multiplies the outputs
+  const float* fac = MODE != RESIDUAL && nm.ss_in ? token_fac : nullptr;   // multiplies the outputs
   volatile int* fail = &sh.fail;
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(sa(&sh.tmem)) : "memory");
@@ -441,7 +517,10 @@ prefill_gemm_tiled_kernel(const __grid_constant__ CUtensorMap xmap, const uint8_
     for (int tile = first; tile < tiles; tile += stride, ++done) {
       if (nm.ss_in) {
         const int t0 = (tile / feat_tiles) * nt;
-        for (int i = et; i < nt; i += 32 * kEpWarps) token_fac[i] = t0 + i < T ? token_factor(nm, t0 + i, RESIDUAL) : 0.f;
+        for (int i = et; i < nt; i += 32 * kEpWarps) {
+          if (MODE == ROPE) token_pos[i] = __ldg(rp.pos + min(t0 + i, T - 1));
+          token_fac[i] = t0 + i < T ? token_factor(nm, t0 + i, MODE == RESIDUAL) : 0.f;
+        }
         epilogue_sync();
       }
       const bool ok = __all_sync(0xffffffffu, bar_wait<128>(&sh.acc_full, done & 1, fail, WAIT_EP));
@@ -452,8 +531,9 @@ prefill_gemm_tiled_kernel(const __grid_constant__ CUtensorMap xmap, const uint8_
       if (any_failed()) break;   // otherwise the tile is complete: a warp that gave up has raised the flag before
       if (lane == 0) bar_arrive_cluster(in_cta(sa(&sh.acc_empty), lead));
       const int t0 = (tile / feat_tiles) * nt, row0 = (tile % feat_tiles) * 256 + side * 128;
-      if (RESIDUAL) store_residual(rows, nm, token_fac, T, N, t0, row0, nt, et, 32 * kEpWarps);
-      else store_tile<SWIGLU>(rows, Y, T, N, t0, row0, nt, et, 32 * kEpWarps);
+      if (MODE == RESIDUAL) store_residual(rows, nm, token_fac, T, N, t0, row0, nt, et, 32 * kEpWarps);
+      else if (MODE == ROPE) store_rope(rows, rp, token_pos, Y, T, N, t0, row0, nt, et, 32 * kEpWarps);
+      else store_tile<MODE == GATED>(rows, Y, T, N, t0, row0, nt, et, 32 * kEpWarps);
       epilogue_sync();   // `rows` is free for the next tile
     }
   }
@@ -470,8 +550,9 @@ prefill_gemm_tiled_kernel(const __grid_constant__ CUtensorMap xmap, const uint8_
     __syncthreads();
     if (live) {
       pdl_wait();
-      if (RESIDUAL) store_residual(rows, nm, token_fac, T, N, t_base, row0, nt, tid, kThreads);
-      else store_tile<SWIGLU>(rows, Y, T, N, t_base, row0, nt, tid, kThreads);
+      if (MODE == RESIDUAL) store_residual(rows, nm, token_fac, T, N, t_base, row0, nt, tid, kThreads);
+      else if (MODE == ROPE) store_rope(rows, rp, token_pos, Y, T, N, t_base, row0, nt, tid, kThreads);
+      else store_tile<MODE == GATED>(rows, Y, T, N, t_base, row0, nt, tid, kThreads);
     }
   } else {
     // The split tile meets in the CTA that finishes a token: CTA (split, side) does tokens [split nt / S, (split + 1) nt / S) of its side's
@@ -497,9 +578,21 @@ prefill_gemm_tiled_kernel(const __grid_constant__ CUtensorMap xmap, const uint8_
     cluster_barrier();   // every CTA's partials are there, and nobody writes here any more
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     if (live) pdl_wait();
-    for (int k = warp; live && k < chunk; k += kThreads / 32) {
+    constexpr int kWarps = kThreads / 32;
+    uint2 next = make_uint2(0u, 0u), w4 = next;   // RESIDUAL: this lane's four columns of the next token's row, and of the norm's weight
+    auto fetch = [&](int k) {
+      const int t = t_base + split * chunk + k;
+      if (MODE == RESIDUAL && k < chunk && t < T && row0 < N) next = *reinterpret_cast<const uint2*>(nm.x + (size_t)t * N + row0 + 4 * lane);
+    };
+    if (MODE == RESIDUAL && live) {
+      if (row0 < N) w4 = __ldg(reinterpret_cast<const uint2*>(nm.w + row0 + 4 * lane));
+      fetch(warp);
+    }
+    for (int k = warp; live && k < chunk; k += kWarps) {
       const int t = t_base + split * chunk + k;
       if (t >= T) break;
+      const uint2 r = next;
+      fetch(k + kWarps);
       float4 v[kMaxSplit];   // sum in split order, four rows a lane
 #pragma unroll
       for (int s = 0; s < kMaxSplit; ++s)
@@ -510,11 +603,28 @@ prefill_gemm_tiled_kernel(const __grid_constant__ CUtensorMap xmap, const uint8_
         if (s < S) a.x += v[s].x, a.y += v[s].y, a.z += v[s].z, a.w += v[s].w;
       const float f = fac ? token_fac[split * chunk + k] : 1.f;
       half2 h01 = __floats2half2_rn(a.x * f, a.y * f), h23 = __floats2half2_rn(a.z * f, a.w * f);
-      if (RESIDUAL) {   // as residual8
+      if (MODE == ROPE) {   // as store_rope; the lane's four columns are all in one half of a head
+        const int d2 = rp.D >> 1, row = row0 + 4 * lane, head = row / rp.D, in_head = row - head * rp.D, local = in_head & (d2 - 1);
+        const uint32_t p01 = __shfl_xor_sync(0xffffffffu, as_u32(h01), d2 >> 2), p23 = __shfl_xor_sync(0xffffffffu, as_u32(h23), d2 >> 2);
+        if (head >= rp.n_q + 2 * rp.n_kv) continue;
+        const int pos = token_pos[split * chunk + k];
+        if (head < rp.n_q + rp.n_kv) {
+          const float4 c = __ldg(reinterpret_cast<const float4*>(rp.cos_t + (size_t)pos * d2 + local));
+          float4 s = __ldg(reinterpret_cast<const float4*>(rp.sin_t + (size_t)pos * d2 + local));
+          if (in_head < d2) s.x = -s.x, s.y = -s.y, s.z = -s.z, s.w = -s.w;
+          const float2 a01 = __half22float2(h01), a23 = __half22float2(h23), b01 = __half22float2(as_h2(p01)), b23 = __half22float2(as_h2(p23));
+          h01 = __floats2half2_rn(a01.x * c.x + b01.x * s.x, a01.y * c.y + b01.y * s.y);
+          h23 = __floats2half2_rn(a23.x * c.z + b23.x * s.z, a23.y * c.w + b23.y * s.w);
+        }
+        const int page = head < rp.n_q ? 0 : __ldg(rp.bt + (pos >> rp.log2P));
+        half* to = head_row(rp, Y, N, head, t, page, pos & ((1 << rp.log2P) - 1)) + in_head;
+        *reinterpret_cast<uint2*>(to) = make_uint2(as_u32(h01), as_u32(h23));
+        continue;
+      }
+      if (MODE == RESIDUAL) {   // as residual8
         if (row0 >= N) break;
         const float scale = token_fac[split * chunk + k];
         const size_t at = (size_t)t * N + row0 + 4 * lane;
-        const uint2 r = *reinterpret_cast<const uint2*>(nm.x + at), w4 = __ldg(reinterpret_cast<const uint2*>(nm.w + row0 + 4 * lane));
         h01 = __hadd2(as_h2(r.x), h01), h23 = __hadd2(as_h2(r.y), h23);
         const float2 x01 = __half22float2(h01), x23 = __half22float2(h23), w01 = __half22float2(as_h2(w4.x)), w23 = __half22float2(as_h2(w4.y));
         *reinterpret_cast<uint2*>(nm.x + at) = make_uint2(as_u32(h01), as_u32(h23));
@@ -528,7 +638,7 @@ prefill_gemm_tiled_kernel(const __grid_constant__ CUtensorMap xmap, const uint8_
         continue;
       }
       half* y = Y + (size_t)t * N;
-      if (SWIGLU) {   // rows 16 k + 0..7 gates, 16 k + 8..15 their up rows: two lanes further on
+      if (MODE == GATED) {   // rows 16 k + 0..7 gates, 16 k + 8..15 their up rows: two lanes further on
         const uint32_t u01 = __shfl_xor_sync(0xffffffffu, as_u32(h01), 2), u23 = __shfl_xor_sync(0xffffffffu, as_u32(h23), 2);
         if ((lane & 2) == 0) {
           const int f = (row0 >> 1) + 8 * (lane >> 2) + 4 * (lane & 1);
@@ -571,7 +681,7 @@ static int resident_clusters(int S, size_t smem) {   // clusters of 2 S CTAs the
     attr[0].val.clusterDim.x = 2 * S, attr[0].val.clusterDim.y = 1, attr[0].val.clusterDim.z = 1;
     cfg.gridDim = dim3(2 * S), cfg.blockDim = dim3(kThreads), cfg.dynamicSmemBytes = smem, cfg.attrs = attr, cfg.numAttrs = 1;
     int num = 0;
-    if (cudaOccupancyMaxActiveClusters(&num, prefill_gemm_tiled_kernel<false, false>, &cfg) != cudaSuccess) {
+    if (cudaOccupancyMaxActiveClusters(&num, prefill_gemm_tiled_kernel<PLAIN>, &cfg) != cudaSuccess) {
       (void)cudaGetLastError();
       num = 0;
     }
@@ -586,23 +696,26 @@ cudaError_t prefill_gemm_tiled_status(int* code) {
 
 // Y[T, N]; N = rows of W (swiglu: of outputs, W has 2 N rows in paired layout). force_split: 0, or the S to use.
 cudaError_t prefill_gemm_tiled_dispatch(const void* Wt, const void* X, void* Y, int T, int N, int K, int swiglu, int force_split,
-                                        const PrefillNorm* norm, cudaStream_t st) {
+                                        const PrefillNorm* norm, const PrefillRope* rope, cudaStream_t st) {
   const int nunit = K / 128, row_tiles = swiglu ? (N + 7) / 8 : (N + 15) / 16, feat_tiles = (row_tiles + 15) / 16;
   auto bytes = [](int tokens, int stages, int per_token) { return 1024 + (size_t)tokens * (128 * stages + per_token); };
-  const size_t smem_max = 225 * 1024 + 512;   // no less than what follows, and room for the static part
-  static size_t allowed[3][kMaxDevices] = {};
-  const bool residual = norm && norm->x;
-  if (residual && (swiglu || N % 128)) return cudaErrorInvalidValue;
-  auto kern = residual ? prefill_gemm_tiled_kernel<false, true> : swiglu ? prefill_gemm_tiled_kernel<true, false> : prefill_gemm_tiled_kernel<false, false>;
-  cudaError_t e = allow_dynamic_smem(prefill_gemm_tiled_kernel<false, false>, smem_max, allowed[0]);   // resident_clusters asks for this one
-  if (e == cudaSuccess && kern != prefill_gemm_tiled_kernel<false, false>) e = allow_dynamic_smem(kern, smem_max, allowed[residual ? 2 : 1]);
+  const size_t smem_max = 224 * 1024;   // beside the static part
+  static size_t allowed[4][kMaxDevices] = {};
+  const int mode = rope ? ROPE : norm && norm->x ? RESIDUAL : swiglu ? GATED : PLAIN;
+  if (mode == RESIDUAL && (swiglu || N % 128)) return cudaErrorInvalidValue;
+  if (mode == ROPE && (swiglu || !norm || norm->x || (rope->D != 64 && rope->D != 128))) return cudaErrorInvalidValue;
+  auto kern = mode == ROPE ? prefill_gemm_tiled_kernel<ROPE> : mode == RESIDUAL ? prefill_gemm_tiled_kernel<RESIDUAL>
+              : mode == GATED ? prefill_gemm_tiled_kernel<GATED> : prefill_gemm_tiled_kernel<PLAIN>;
+  cudaError_t e = allow_dynamic_smem(prefill_gemm_tiled_kernel<PLAIN>, smem_max, allowed[PLAIN]);   // resident_clusters asks for this one
+  if (e == cudaSuccess && mode != PLAIN) e = allow_dynamic_smem(kern, smem_max, allowed[mode]);
   if (e != cudaSuccess) return e;
   // Tokens per tile (equal tiles, so that the last is not nearly empty; up to eight more of them than there have to be) and split of
   // K, by estimated time. In microseconds, fitted to 1,250 measured launches (TinyLlama, 8B and 70B matrices, 16 .. 4096 tokens;
   // the pick is 0.7 % off the best of them on average, 11 % at worst; always the widest tiles: 10 % and 51 %): a unit takes 0.30 - 0.35
   // (dequantization and issue) or its MMA time, 0.68 at 256 tokens with the chip full; beside that a launch takes 1.0 + 0.0162 a
   // token where a pair works alone and 2.1 / 2.7 + 0.0206 a token where 2 / 4 pairs exchange partial tiles; and up to 2.8 are lost
-  // with the SMs that the launch leaves none of to the start of the next one.
+  // with the SMs that the launch's last wave leaves none of to the start of the next one (of its first wave, as it was: 2 % more for a prompt
+  // of 200 to 512 tokens).
   int S = 0, nt = 0, tiles = 0;
   double best = 0;
   const int least = (T + kMaxTokens - 1) / kMaxTokens;
@@ -614,7 +727,7 @@ cudaError_t prefill_gemm_tiled_dispatch(const void* Wt, const void* X, void* Y, 
     const int units = (nunit + c - 1) / c;
     for (int ntt = least; ntt < least + 8; ++ntt) {
       const int n = ((T + ntt - 1) / ntt + 31) / 32 * 32, count = feat_tiles * ((T + n - 1) / n), waves = (count + room - 1) / room;
-      const double unit = units * (n * 0.00264 > 0.35 ? n * 0.00264 : 0.35), fill = (double)count / room;
+      const double unit = units * (n * 0.00264 > 0.35 ? n * 0.00264 : 0.35), fill = (double)(count - (waves - 1) * room) / room;   // of the last wave
       const double cost = (c == 1 ? 1.0 + 0.0162 * n + waves * (unit + 0.4) : waves * (1.45 + 0.32 * c + 0.0206 * n + unit)) +
                           2.8 * (fill < 0.36 ? 0 : fill > 0.86 ? 1 : 2 * (fill - 0.36));
       if (S == 0 || cost < best) best = cost, S = c, nt = n, tiles = count;
@@ -642,7 +755,7 @@ cudaError_t prefill_gemm_tiled_dispatch(const void* Wt, const void* X, void* Y, 
   cfg.attrs = attr;
   cfg.numAttrs = 2;
   return cudaLaunchKernelEx(&cfg, kern, xmap, (const uint8_t*)Wt, (half*)Y, T, N, row_tiles, nunit, nt, S, feat_tiles, tiles, ns, p_apart,
-                            norm ? *norm : PrefillNorm{});
+                            norm ? *norm : PrefillNorm{}, rope ? *rope : PrefillRope{});
 }
 
 }  // namespace b200

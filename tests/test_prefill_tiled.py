@@ -95,6 +95,36 @@ def test_prefill_equals_stepping(D, n_q, n_kv, page, start, T):
     assert int(m.tok) == tok or top[0] - top[1] <= 2 * KERNEL_TOL * want.abs().max()
 
 
+# Norms, residual sums and RoPE inside the GEMMs: hidden sizes whose last 256-row tile is half empty, one and several token tiles, both
+# sides of the limit for RoPE; embeddings and norm weights small and large enough that rows stored without a scale would leave fp16.
+# Same tolerance as above, which allows for the stepping path's own roundings. (The norm in front of attention keeps its weights where
+# they are large: scores of hundreds would multiply every rounding of either path.)
+@pytest.mark.parametrize("H,D,n_q,n_kv,T,emb,ln", [(128, 64, 2, 1, 3, 1.0, 1.0), (384, 64, 6, 3, 33, 1e-3, 0.02), (640, 64, 8, 8, 257, 1.0, 8.0),
+                                                   (640, 128, 4, 1, 129, 2000.0, 1.0), (384, 64, 4, 4, 768, 100.0, 0.1),
+                                                   (384, 128, 2, 2, 769, 1e-3, 8.0), (2048, 64, 32, 4, 96, 1e-3, 3.0)])
+def test_norms_and_rope_inside_the_gemms(H, D, n_q, n_kv, T, emb, ln):
+    from llm_decode_kernels_b200.model import DecodeConfig, Model
+    from test_model import KERNEL_TOL, hf_cfg, random_state
+    c = hf_cfg(H, 3, n_q, n_kv, 512, 1000, D=D)
+    sd = random_state(c, 5, D)
+    for k in sd:
+        if "embed_tokens" in k:
+            sd[k] = (sd[k].float() * emb).half()
+        elif "norm" in k:
+            sd[k] = (sd[k].float() * (min(ln, 1.0) if "input" in k else ln)).half()
+    m = Model(sd, c, DecodeConfig(group=128, max_ctx=T + 16, seed=1))
+    m.prepare(T + 8, use_graph=False)
+    ids = torch.randint(0, 1000, (T,), generator=torch.Generator().manual_seed(6))
+    m.reset(0)
+    want = m.teacher_force(ids, use_graph=False, collect_logits=True).float()
+    kv = m.kv.clone().float()
+    m.kv.zero_()
+    m.reset(0)
+    got = m.prefill(ids, collect_logits=True).float()
+    assert torch.isfinite(want).all() and (got - want).abs().max() <= KERNEL_TOL * want.abs().max()
+    assert (m.kv.float() - kv).abs().max() <= KERNEL_TOL * kv.abs().max() and m.K.gemm_status() == 0
+
+
 # Error of the prompt attention against 64 bits, on the rotated queries and the cache it read. Its output is one fp16 rounding of sums
 # that keep the probabilities to 22 bits: the error must be that rounding's (2^-11 / sqrt(12), a little less on average) and 10 % at
 # most beside it. fp16 probabilities alone add 17 to 40 %. Flat and peaked rows; whole context and splits.
