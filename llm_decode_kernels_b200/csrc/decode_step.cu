@@ -441,7 +441,10 @@ struct Mat {
   int paired;          // 1: gate|up tiles (8 gate rows + their 8 up rows)
 };
 
-struct Slice { int t0, nt; };   // this CTA's tiles [t0, t0 + nt) of a matrix
+// This CTA's tiles [t0, t0 + nt) of a matrix, in ring stages of `ups` blocks. whole: a stage holds whole tiles and a warp has at most two units
+// of each (rows of up to 2048 weights whose units divide a stage). Rows of 44 units (5632 weights) come in two stages of 22, two units a
+// warp in each: stages of 32 and 12 are three passes of the loop instead of two. (The step at context 256: 361 -> 359 us.)
+struct Slice { int t0, nt, ups, whole; };
 
 // Position in the ring. Stages are used strictly in order by producer and consumers alike, so a slot index and a
 // parity bit that flips on wrap-around replace a stage counter (and the divisions by the ring size it would need).
@@ -479,11 +482,11 @@ DEVI void produce(const Cta& c, const uint8_t* base, int nunit, const Slice& s, 
   const int NU = s.nt * nunit;
   const uint8_t* src = base + (size_t)s.t0 * nunit * kTileUnitBytes;
 #pragma unroll 1
-  for (int i0 = 0; i0 < NU; i0 += c.p->ups, advance(rp, c.p->ns)) {
+  for (int i0 = 0; i0 < NU; i0 += s.ups, advance(rp, c.p->ns)) {
     const int slot = rp.slot;
     if (!wait_bar(c, c.empty(slot), rp.parity, ERR_EMPTY, 200)) return;
     if (lane == 0) {
-      const uint32_t bytes = (uint32_t)(min(c.p->ups, NU - i0) * kTileUnitBytes);
+      const uint32_t bytes = (uint32_t)(min(s.ups, NU - i0) * kTileUnitBytes);
       mbar_expect_tx(c.full(slot), bytes);
       bulk_g2s(c.stage(slot), src + (size_t)i0 * kTileUnitBytes, bytes, c.full(slot));
     }
@@ -519,21 +522,22 @@ DEVI void produce_kv(const Cta& c, const StepParams& p, const StepLayer& ly, int
   }
 }
 
-// One tile-unit block (at `tu` in the ring) against unit u of x: the dot products of row slots g (ya) and g + 8 (yb)
+// One tile-unit block (at byte `tu` of shared memory: 32-bit offsets from one base, not pointers, which would take 64-bit arithmetic for
+// every block) against unit u of x: the dot products of row slots g (ya) and g + 8 (yb)
 // over the unit's 128 columns, scaled and with the zero-point term; meaningful on lanes t == 0.
 // Lane (g, t) reads 16 bytes of row slot g and of row slot g + 8 (columns 32 t .. 32 t + 31 of the unit); lanes
 // (0, t) carry the hi digits of the matching 32 activations as the B operand, lanes (1, t) the lo digits, the other
 // lanes zeros. Four MMAs in two independent chains.
-DEVI void tile_unit(const Cta& c, const uint8_t* tu, int u, int lane, float& ya, float& yb) {
+DEVI void tile_unit(const Cta& c, uint32_t tu, int u, int lane, float& ya, float& yb) {
   const int g = lane >> 2, t = lane & 3;
   uint4 x0 = make_uint4(0u, 0u, 0u, 0u), x1 = x0;
   if (g < 2) {
-    const uint4* xp = reinterpret_cast<const uint4*>(c.xin()) + (size_t)u * 16 + (g * 4 + t) * 2;
+    const uint4* xp = reinterpret_cast<const uint4*>(step_smem + (uint32_t)(c.p->off_xin + 256 * u + 32 * (g * 4 + t)));
     x0 = xp[0];   // MMAs 0, 1: registers (m0 r0, m0 r1, m1 r0, m1 r1)
     x1 = xp[1];   // MMAs 2, 3
   }
-  const uint4 wa = *reinterpret_cast<const uint4*>(tu + 16 * lane);
-  const uint4 wb = *reinterpret_cast<const uint4*>(tu + 512 + 16 * lane);
+  const uint4 wa = *reinterpret_cast<const uint4*>(step_smem + (tu + 16 * lane));
+  const uint4 wb = *reinterpret_cast<const uint4*>(step_smem + (tu + 16 * lane) + 512);
   constexpr uint32_t kNib = 0x0F0F0F0Fu;
   int c0[4] = {0, 0, 0, 0}, c1[4] = {0, 0, 0, 0};
   mma16832_u8s8(c0, wa.x & kNib, wb.x & kNib, wa.y & kNib, wb.y & kNib, x0.x, x0.y);
@@ -541,13 +545,20 @@ DEVI void tile_unit(const Cta& c, const uint8_t* tu, int u, int lane, float& ya,
   mma16832_u8s8(c0, wa.z & kNib, wb.z & kNib, wa.w & kNib, wb.w & kNib, x1.x, x1.y);
   mma16832_u8s8(c1, (wa.z >> 4) & kNib, (wb.z >> 4) & kNib, (wa.w >> 4) & kNib, (wb.w >> 4) & kNib, x1.z, x1.w);
   // lanes t == 0: C columns 0 (hi digits) and 1 (lo digits) of rows g (c[0], c[1]) and g + 8 (c[2], c[3])
-  const float2 sa = __half22float2(*reinterpret_cast<const half2*>(tu + 1024 + 4 * g));
-  const float2 sc = __half22float2(*reinterpret_cast<const half2*>(tu + 1024 + 4 * (g + 8)));
-  const float xs = c.xsum()[2 * u], resc = c.xsum()[2 * u + 1];
+  const uint8_t* sz = step_smem + (tu + 4 * g) + 1024;
+  const float2 sa = __half22float2(*reinterpret_cast<const half2*>(sz)), sc = __half22float2(*reinterpret_cast<const half2*>(sz + 32));
+  const float2 xf = *reinterpret_cast<const float2*>(step_smem + (uint32_t)(c.p->off_xsum + 8 * u));
+  const float xs = xf.x, resc = xf.y;
   const float va = (float)(((c0[0] + c1[0]) << 8) + (c0[1] + c1[1]));
   const float vb = (float)(((c0[2] + c1[2]) << 8) + (c0[3] + c1[3]));
   ya = fmaf(sa.x, fmaf(va, resc, -sa.y * xs), ya);
   yb = fmaf(sc.x, fmaf(vb, resc, -sc.y * xs), yb);
+}
+
+// The same for two blocks, of two tiles, against one unit of x: two independent chains.
+DEVI void tile_unit2(const Cta& c, uint32_t tu, uint32_t tv, int u, int lane, float& ya, float& yb, float& za, float& zb) {
+  tile_unit(c, tu, u, lane, ya, yb);
+  tile_unit(c, tv, u, lane, za, zb);
 }
 
 // Consumer side of one matrix slice, one warp's share. The slice is the sequence of tile-unit blocks
@@ -560,18 +571,64 @@ DEVI void tile_unit(const Cta& c, const uint8_t* tu, int u, int lane, float& ya,
 // too and loses 3 %. When the warp has passed its last unit of a tile, lanes t == 0 leave the
 // two partial sums of rows g and g + 8 in part[warp][16 * tile + row slot]. A warp whose units do not exist
 // (K < 1024) only keeps the ring's barriers moving.
+//
+// TILES: slices of whole tiles have a loop of their own, which knows where a warp's one or two units of every tile are and takes two tiles
+// at a time: a tile of 16 units on 11 warps takes 690 cycles in the general loop, which keeps track of tile, unit and stage, and 555 in a plain
+// one over tiles (measured by themselves); with two tiles every warp has two chains in flight, also those with one unit of a tile. TinyLlama shape, us a token, with 32-bit offsets
+// instead of pointers into the ring, this loop, and the stages of 22 (Slice): context 128 354 -> 339, 256 368 -> 353, 2048 400 -> 385,
+// 8192 440 -> 423. Not in the STAGED form at head_dim 128, whose registers it exceeds (152 -> 157 us for 4 layers, 32 kv heads).
+// Four units of a row of 5632 at once, both stages: 1 % slower than two and two.
+template <bool TILES>
 DEVI void gemv(const Cta& c, const Mat& m, const Slice& s, float* part, int pstride, RingPos& rp, int warp, int lane,
                int trace_at) {
   const int g = lane >> 2, t = lane & 3;
   const int nunit = m.K >> 7, NU = s.nt * nunit;
   const bool active = warp < nunit;
+  if (TILES && s.whole) {
+    const bool two = warp + kNCW < nunit;
+    int row = 0;
+#pragma unroll 1
+    for (int i0 = 0; i0 < NU; i0 += c.p->ups, advance(rp, c.p->ns)) {
+      const int slot = rp.slot;
+      if (wait_bar(c, c.full(slot), rp.parity, ERR_FULL) && active) {
+        uint32_t tu = (uint32_t)(c.p->off_ring + slot * c.p->stage_bytes + warp * kTileUnitBytes);
+        const int n = min(c.p->ups, NU - i0);
+#pragma unroll 1
+        for (int b = 0; b < n;) {
+          if (b + nunit < n) {
+            const uint32_t tv = tu + nunit * kTileUnitBytes;
+            float ya = 0.f, yb = 0.f, za = 0.f, zb = 0.f;
+            tile_unit2(c, tu, tv, warp, lane, ya, yb, za, zb);
+            if (two) tile_unit2(c, tu + kNCW * kTileUnitBytes, tv + kNCW * kTileUnitBytes, warp + kNCW, lane, ya, yb, za, zb);
+            if (t == 0) {
+              float* to = part + warp * pstride + row + g;
+              to[0] = ya, to[8] = yb, to[16] = za, to[24] = zb;
+            }
+            b += 2 * nunit, tu += 2 * nunit * kTileUnitBytes, row += 32;
+            continue;
+          }
+          float ya = 0.f, yb = 0.f, ya2 = 0.f, yb2 = 0.f;
+          tile_unit(c, tu, warp, lane, ya, yb);
+          if (two) tile_unit(c, tu + kNCW * kTileUnitBytes, warp + kNCW, lane, ya2, yb2);
+          if (t == 0) {
+            part[warp * pstride + row + g] = ya + ya2;
+            part[warp * pstride + row + g + 8] = yb + yb2;
+          }
+          b += nunit, tu += nunit * kTileUnitBytes, row += 16;
+        }
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(c.empty(slot));
+    }
+    return;
+  }
   int tl = 0, u = warp, idx = warp;   // the warp's next block: local tile, unit, place in the sequence
   float ya = 0.f, yb = 0.f;
 #ifdef B200_STEP_TRACE
   long long waited = 0;
 #endif
 #pragma unroll 1
-  for (int i0 = 0; i0 < NU; i0 += c.p->ups, advance(rp, c.p->ns)) {
+  for (int i0 = 0; i0 < NU; i0 += s.ups, advance(rp, c.p->ns)) {
     const int slot = rp.slot;
 #ifdef B200_STEP_TRACE
     const long long w0 = now_ns();
@@ -580,15 +637,15 @@ DEVI void gemv(const Cta& c, const Mat& m, const Slice& s, float* part, int pstr
 #ifdef B200_STEP_TRACE
     waited += now_ns() - w0;   // time this warp spent waiting for ring stages of the matrix
 #endif
-    const int end = min(NU, i0 + c.p->ups);
-    const uint8_t* sb = c.stage(slot) - (size_t)i0 * kTileUnitBytes;   // block idx of the sequence is at sb + idx * 1088
+    const int end = min(NU, i0 + s.ups);
+    const uint32_t sb = (uint32_t)(c.p->off_ring + slot * c.p->stage_bytes - i0 * kTileUnitBytes);   // block idx of the sequence is at sb + idx * 1088
     if (ok && active) {
 #pragma unroll 1
       while (idx < end) {
         const bool two = u + kNCW < nunit && idx + kNCW < end;   // the next unit of the same tile is in this stage too
         float ya2 = 0.f, yb2 = 0.f;
-        tile_unit(c, sb + (size_t)idx * kTileUnitBytes, u, lane, ya, yb);
-        if (two) tile_unit(c, sb + (size_t)(idx + kNCW) * kTileUnitBytes, u + kNCW, lane, ya2, yb2);
+        tile_unit(c, sb + (uint32_t)(idx * kTileUnitBytes), u, lane, ya, yb);
+        if (two) tile_unit(c, sb + (uint32_t)((idx + kNCW) * kTileUnitBytes), u + kNCW, lane, ya2, yb2);
         ya += ya2;
         yb += yb2;
         const int step = two ? 2 * kNCW : kNCW;
@@ -1304,6 +1361,9 @@ __global__ void __launch_bounds__(kThreads, 1) decode_step_kernel(const __grid_c
   if (tid < 5) {
     const int rows = tid == 0 ? p.n_qkv : (tid == 2 ? p.I : (tid == 4 ? p.V : p.H));
     sl[tid] = slice_of(rows, tid == 2, cta, ncta);
+    const int nunit = (tid == 1 ? p.n_att : tid == 3 ? p.I : p.H) >> 7;
+    sl[tid].ups = nunit > p.ups && nunit <= 2 * p.ups && nunit % (2 * kNCW) == 0 && 2 * kNCW <= p.ups ? 2 * kNCW : p.ups;
+    sl[tid].whole = nunit <= 2 * kNCW && p.ups % nunit == 0;
   }
   {
     const uint4* src = reinterpret_cast<const uint4*>(p.layers);
@@ -1430,7 +1490,7 @@ __global__ void __launch_bounds__(kThreads, 1) decode_step_kernel(const __grid_c
     }
     const int tr_at = kTraceHead + kTracePerLayer * l + kTracePerPhase * ph;
     stamp(c, tr_at);
-    gemv(c, m, s, part, pstride, rp, warp, lane, tr_at + 1);
+    gemv<!(STAGED && D == 128)>(c, m, s, part, pstride, rp, warp, lane, tr_at + 1);
     stamp(c, tr_at + 2);
     if (consumer_sync_or(*c.abort())) return;
     stamp(c, tr_at + 3);

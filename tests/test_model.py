@@ -502,3 +502,22 @@ def test_automatic_step_kernel_by_context_and_ctas_per_kv_head():
         for cap in (4096, 10240, 10241, 20000):
             m.set_attention_partition(cap, part_size=1)
             assert m.persistent == (limit is None or cap <= limit), (n_kv, cap)
+
+
+# Slices of whole tiles (rows of 1 to 16 units), rows of 44 units in two stages, rows that fit neither; one, two, an odd number and many
+# tiles a CTA. Against the multi-kernel step, with the tolerance of a kernel's output.
+@pytest.mark.gpu
+@pytest.mark.parametrize("H,n_q,n_kv,I,V", [(128, 2, 1, 128, 333), (256, 4, 2, 5632, 5000), (512, 8, 2, 4864, 2400), (1024, 16, 2, 2816, 12000),
+                                            (2048, 32, 4, 5632, 7200), (640, 10, 5, 5632, 4000)])
+def test_slices_of_whole_tiles_match_the_multi_kernel_step(H, n_q, n_kv, I, V):
+    c = hf_cfg(H, 2, n_q, n_kv, I, V)
+    sd = random_state(c, 11)
+    ids = torch.randint(0, V, (12,), generator=torch.Generator().manual_seed(7))
+    out = {}
+    for step in ("persistent", "multi"):
+        m = Model(sd, c, DecodeConfig(group=128, max_ctx=64, seed=1, step_kernel=step))
+        m.prepare(32, use_graph=False)
+        m.reset(0)
+        out[step] = m.teacher_force(ids, use_graph=False, collect_logits=True).float()
+        assert m.step_error() == 0
+    assert (out["persistent"] - out["multi"]).abs().max() <= KERNEL_TOL * out["multi"].abs().max()
