@@ -10,9 +10,11 @@
 //     into tensor memory, and the MMA reads its A operand there;
 //   * a CTA pair is persistent: it walks over output tiles, the dequantizing and copying warps run four to six 128-column units
 //     ahead across tile borders, and the epilogue warps empty the accumulator into shared memory (rounded to fp16) before they
-//     store, so the next tile's MMAs wait only for that;
+//     store, so the next tile's MMAs wait only for that; the CTA's last tile is emptied and stored by all warps;
 //   * where there are fewer tiles than pairs, S = 2 or 4 pairs (one cluster) share a tile by splitting K; their fp32 partial tiles
-//     meet through distributed shared memory in a fixed order.
+//     are written into the shared memory of the CTA that finishes a token and added there in a fixed order.
+// What follows the product in a prompt rides in the epilogue (MODE): SwiGLU, the residual row with the next norm's input and sums, RoPE
+// and the append to the cache; and the norm's factor, which is applied to fp32 outputs.
 // Warps: 0-11 dequantize (three groups of four, every third unit: a unit is ~2000 cycles of latency for a warp and 1024 of MMA at
 // 256 tokens), 12-15 epilogue, 16 MMA issue (even CTA of a pair), 17 TMA.
 // Tensor memory: accumulator (128 lanes = rows, one column per token; 128 or 256 columns), then six or four A stages of 64 columns.
@@ -714,8 +716,8 @@ cudaError_t prefill_gemm_tiled_dispatch(const void* Wt, const void* X, void* Y, 
   // the pick is 0.7 % off the best of them on average, 11 % at worst; always the widest tiles: 10 % and 51 %): a unit takes 0.30 - 0.35
   // (dequantization and issue) or its MMA time, 0.68 at 256 tokens with the chip full; beside that a launch takes 1.0 + 0.0162 a
   // token where a pair works alone and 2.1 / 2.7 + 0.0206 a token where 2 / 4 pairs exchange partial tiles; and up to 2.8 are lost
-  // with the SMs that the launch's last wave leaves none of to the start of the next one (of its first wave, as it was: 2 % more for a prompt
-  // of 200 to 512 tokens).
+  // with the SMs that the launch's last wave leaves none of to the start of the next one (counted over all waves instead: 2 % more for a
+  // prompt of 200 to 512 tokens).
   int S = 0, nt = 0, tiles = 0;
   double best = 0;
   const int least = (T + kMaxTokens - 1) / kMaxTokens;
