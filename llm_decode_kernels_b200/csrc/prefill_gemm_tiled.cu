@@ -65,6 +65,7 @@ struct Shared {
   uint64_t full[kMaxStages], empty[kMaxStages], acc_full, acc_empty;
   uint32_t tmem;
   int fail;
+  float top[kEpWarps];   // norm_top
 };
 
 // Stage and how often it has been used before, of a sequence that takes the stages in turn.
@@ -116,16 +117,31 @@ DEVI uint32_t gated2(uint32_t gate, uint32_t up) {
   return as_u32(__hmul2(s, as_h2(up)));
 }
 
-// norm: what the epilogue multiplies a token by. Plain: rsqrt(mean square + eps) / scale, or 1; RESIDUAL: the scale of its row of xw.
-DEVI float token_factor(const PrefillNorm& nm, int t, bool residual) {
+// what the epilogue multiplies a token's outputs by: the norm's factor rsqrt(mean square + eps), and what its row of X lacks beside it
+DEVI float token_factor(const PrefillNorm& nm, int t) {
   float a = 0.f, b = 0.f;   // two chains, always the same order
   const float* p = nm.ss_in + (size_t)t * nm.parts;
 #pragma unroll 8
   for (int i = 0; i + 1 < nm.parts; i += 2) a += p[i], b += p[i + 1];
   if (nm.parts & 1) a += p[nm.parts - 1];
-  const float ms = (a + b) * nm.inv_h;
-  return residual ? 1.f / row_inv_scale(ms) : rsqrtf(ms + nm.eps) * nm.inv_in[t];
+  return rsqrtf((a + b) * nm.inv_h + nm.eps) * nm.inv_in[t];
 }
+
+// The largest |w| of the next norm, each warp's of the epilogue (thread et of their 128) in sh.top; norm_scale: the p made of it (PrefillNorm). w is
+// none of the chunk's outputs: read ahead of the wait, while the first units are on their way. (NaN is no maximum; its column is NaN anyway.)
+DEVI void norm_top(const PrefillNorm& nm, int N, Shared& sh, int et) {
+  float m = 0.f;
+#pragma unroll 4
+  for (int i = et; i < N >> 3; i += 32 * kEpWarps) {
+    float f[8];
+    unpack8(__ldg(reinterpret_cast<const uint4*>(nm.w) + i), f);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) m = fmaxf(m, fabsf(f[k]));
+  }
+  m = warp_max(m);
+  if ((et & 31) == 0) sh.top[et >> 5] = m;
+}
+DEVI float norm_scale(const Shared& sh) { return pow2_above(fmaxf(fmaxf(sh.top[0], sh.top[1]), fmaxf(sh.top[2], sh.top[3]))); }
 
 // Eight columns of a finished residual row: x += y, xw = x * w * scale; returns the sum of x^2.
 DEVI float residual8(const uint4& r, const uint4& y, const uint4& w, half* x, half* xw, float scale) {   // r: x as it was
@@ -207,11 +223,11 @@ DEVI void store_tile(const uint32_t* rows, half* Y, int T, int N, int t0, int ro
 }
 
 // rows -> the residual stream (PrefillNorm): 16 lanes take a token pair's 128 columns, so each of the two sums is one of theirs.
-DEVI void store_residual(const uint32_t* rows, const PrefillNorm& nm, const float* fac, int T, int N, int t0, int row0, int nt, int at,
-                         int threads) {
+DEVI void store_residual(const uint32_t* rows, const PrefillNorm& nm, float p, int T, int N, int t0, int row0, int nt, int at, int threads) {
   const int lane = at & 31, pairs = (min(nt, T - t0) + 1) >> 1, pc = at & 15, f = row0 + 8 * pc;
   if (row0 >= N) return;   // N is a multiple of 128
   const uint4 w8 = __ldg(reinterpret_cast<const uint4*>(nm.w + f));
+  const float scale = 1.f / p;
   uint4 next[2];   // the pair's rows of x, one round ahead
   auto fetch = [&](int i) {
 #pragma unroll
@@ -238,7 +254,7 @@ DEVI void store_residual(const uint32_t* rows, const PrefillNorm& nm, const floa
           uint32_t o[4];
 #pragma unroll
           for (int e = 0; e < 4; ++e) o[e] = __byte_perm(w[2 * e], w[2 * e + 1], h ? 0x7632 : 0x5410);
-          ss[h] = residual8(was[h], make_uint4(o[0], o[1], o[2], o[3]), w8, nm.x + (size_t)t * N + f, nm.xw + (size_t)t * N + f, fac[2 * tp + h]);
+          ss[h] = residual8(was[h], make_uint4(o[0], o[1], o[2], o[3]), w8, nm.x + (size_t)t * N + f, nm.xw + (size_t)t * N + f, scale);
         }
       }
     }
@@ -250,7 +266,7 @@ DEVI void store_residual(const uint32_t* rows, const PrefillNorm& nm, const floa
     const int t = t0 + 2 * tp + pc;   // lanes 0 and 1 of the sixteen
     if (tp < pairs && pc < 2 && t < T) {
       nm.ss_out[(size_t)t * nm.parts + (row0 >> 7)] = pc ? ss[1] : ss[0];
-      if (row0 == 0) nm.inv_out[t] = 1.f / fac[2 * tp + pc];
+      if (row0 == 0) nm.inv_out[t] = p;
     }
   }
 }
@@ -328,7 +344,7 @@ prefill_gemm_tiled_kernel(const __grid_constant__ CUtensorMap xmap, const uint8_
                           int N, int row_tiles, int nunit, int nt, int S, int feat_tiles, int tiles, int ns, int p_apart, const PrefillNorm nm, const PrefillRope rp) {
   extern __shared__ uint8_t raw[];
   __shared__ Shared sh;
-  __shared__ __align__(16) float token_fac[kMaxTokens];
+  __shared__ __align__(16) float token_fac[MODE == RESIDUAL ? 4 : kMaxTokens];
   __shared__ int token_pos[MODE == ROPE ? kMaxTokens : 1];
   uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(raw) + 1023) & ~(uintptr_t)1023);
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;   // warp: known to be uniform
@@ -514,14 +530,18 @@ prefill_gemm_tiled_kernel(const __grid_constant__ CUtensorMap xmap, const uint8_
       return p != 0;
     };
     int done = 0;
+    if (MODE == RESIDUAL) {
+      norm_top(nm, N, sh, et);
+      epilogue_sync();
+    }
     if (first < tiles) pdl_wait();   // Y may still be read by the kernel before this one; the norm's sums come from it or from earlier ones
 #pragma unroll 1
     for (int tile = first; tile < tiles; tile += stride, ++done) {
-      if (nm.ss_in) {
+      if (MODE != RESIDUAL && nm.ss_in) {
         const int t0 = (tile / feat_tiles) * nt;
         for (int i = et; i < nt; i += 32 * kEpWarps) {
           if (MODE == ROPE) token_pos[i] = __ldg(rp.pos + min(t0 + i, T - 1));
-          token_fac[i] = t0 + i < T ? token_factor(nm, t0 + i, MODE == RESIDUAL) : 0.f;
+          token_fac[i] = t0 + i < T ? token_factor(nm, t0 + i) : 0.f;
         }
         epilogue_sync();
       }
@@ -533,7 +553,7 @@ prefill_gemm_tiled_kernel(const __grid_constant__ CUtensorMap xmap, const uint8_
       if (any_failed()) break;   // otherwise the tile is complete: a warp that gave up has raised the flag before
       if (lane == 0) bar_arrive_cluster(in_cta(sa(&sh.acc_empty), lead));
       const int t0 = (tile / feat_tiles) * nt, row0 = (tile % feat_tiles) * 256 + side * 128;
-      if (MODE == RESIDUAL) store_residual(rows, nm, token_fac, T, N, t0, row0, nt, et, 32 * kEpWarps);
+      if (MODE == RESIDUAL) store_residual(rows, nm, norm_scale(sh), T, N, t0, row0, nt, et, 32 * kEpWarps);
       else if (MODE == ROPE) store_rope(rows, rp, token_pos, Y, T, N, t0, row0, nt, et, 32 * kEpWarps);
       else store_tile<MODE == GATED>(rows, Y, T, N, t0, row0, nt, et, 32 * kEpWarps);
       epilogue_sync();   // `rows` is free for the next tile
@@ -552,7 +572,7 @@ prefill_gemm_tiled_kernel(const __grid_constant__ CUtensorMap xmap, const uint8_
     __syncthreads();
     if (live) {
       pdl_wait();
-      if (MODE == RESIDUAL) store_residual(rows, nm, token_fac, T, N, t_base, row0, nt, tid, kThreads);
+      if (MODE == RESIDUAL) store_residual(rows, nm, norm_scale(sh), T, N, t_base, row0, nt, tid, kThreads);
       else if (MODE == ROPE) store_rope(rows, rp, token_pos, Y, T, N, t_base, row0, nt, tid, kThreads);
       else store_tile<MODE == GATED>(rows, Y, T, N, t_base, row0, nt, tid, kThreads);
     }
@@ -586,6 +606,7 @@ prefill_gemm_tiled_kernel(const __grid_constant__ CUtensorMap xmap, const uint8_
       const int t = t_base + split * chunk + k;
       if (MODE == RESIDUAL && k < chunk && t < T && row0 < N) next = *reinterpret_cast<const uint2*>(nm.x + (size_t)t * N + row0 + 4 * lane);
     };
+    const float p = MODE == RESIDUAL ? norm_scale(sh) : 1.f, scale = 1.f / p;
     if (MODE == RESIDUAL && live) {
       if (row0 < N) w4 = __ldg(reinterpret_cast<const uint2*>(nm.w + row0 + 4 * lane));
       fetch(warp);
@@ -625,7 +646,6 @@ prefill_gemm_tiled_kernel(const __grid_constant__ CUtensorMap xmap, const uint8_
       }
       if (MODE == RESIDUAL) {   // as residual8
         if (row0 >= N) break;
-        const float scale = token_fac[split * chunk + k];
         const size_t at = (size_t)t * N + row0 + 4 * lane;
         h01 = __hadd2(as_h2(r.x), h01), h23 = __hadd2(as_h2(r.y), h23);
         const float2 x01 = __half22float2(h01), x23 = __half22float2(h23), w01 = __half22float2(as_h2(w4.x)), w23 = __half22float2(as_h2(w4.y));
@@ -635,7 +655,7 @@ prefill_gemm_tiled_kernel(const __grid_constant__ CUtensorMap xmap, const uint8_
         const float ss = warp_sum(fmaf(x01.x, x01.x, fmaf(x01.y, x01.y, fmaf(x23.x, x23.x, x23.y * x23.y))));
         if (lane == 0) {
           nm.ss_out[(size_t)t * nm.parts + (row0 >> 7)] = ss;
-          if (row0 == 0) nm.inv_out[t] = 1.f / scale;
+          if (row0 == 0) nm.inv_out[t] = p;
         }
         continue;
       }

@@ -58,11 +58,10 @@ DEVI float4 ld_cluster4(uint32_t addr) {
   asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
   return v;
 }
-// 1 / scale of a row with mean square ms (PrefillNorm): 16 times the power of two below its root, at least 1 so that xw stays in range
-// where w and x are, at most 2^20.
-DEVI float row_inv_scale(float ms) {
-  const int e = (int)((__float_as_uint(ms) >> 23) & 255u) - 127;   // infinity and NaN: 128
-  return __int_as_float((min(max(e >> 1, -4), 16) + 4 + 127) << 23);
+// The power of two p with m < p <= 2 m, within 2^-59 .. 2^41 (0: the smallest, infinity: the largest).
+DEVI float pow2_above(float m) {
+  const int e = (int)((__float_as_uint(m) >> 23) & 255u) + 1;
+  return __int_as_float(min(max(e, 68), 168) << 23);
 }
 // Shared-memory matrix descriptor, 128-byte swizzle, rows of 128 bytes, eight rows per 1024-byte block. K-major operand: rows are M or
 // N, 64 fp16 of K each; `lead` unused (1). MN-major operand: rows are K, 64 fp16 of M or N each; `lead` = bytes from one 64-wide block

@@ -125,6 +125,78 @@ def test_norms_and_rope_inside_the_gemms(H, D, n_q, n_kv, T, emb, ln):
     assert (m.kv.float() - kv).abs().max() <= KERNEL_TOL * kv.abs().max() and m.K.gemm_status() == 0
 
 
+def prompt_in_64_bits(m, sd, ids):
+    """Logits [T, V], K and V rows [T, L, n_kv D] of a prompt at position 0, from the fp16 weights as dequantized."""
+    def weight(lin):
+        w = torch.empty(lin.packed.shape[0], lin.K, dtype=torch.half, device=dev)
+        m.K.dequant_w4a16(lin.packed, lin.sz, w, 128)
+        return w.double()
+    T, D, n_q, n_kv, d2 = ids.numel(), m.D, m.n_q, m.n_kv, m.D // 2
+    cos, sin = m.cos[:T, None].double(), m.sin[:T, None].double()
+    norm = lambda x, w: x * torch.rsqrt((x * x).mean(-1, keepdim=True) + m.eps) * w.double()
+    rope = lambda v: torch.cat([v[..., :d2] * cos - v[..., d2:] * sin, v[..., d2:] * cos + v[..., :d2] * sin], -1)
+    later = torch.ones(T, T, dtype=torch.bool, device=dev).triu(1)
+    x, ks, vs = sd["model.embed_tokens.weight"][ids].to(dev).double(), [], []
+    for lw in m.layers:
+        q, k, v = (norm(x, lw["ln1"]) @ weight(lw["qkv"]).t()).view(T, -1, D).split([n_q, n_kv, n_kv], 1)
+        q, k = rope(q), rope(k)
+        ks.append(k.reshape(T, -1)), vs.append(v.reshape(T, -1))
+        k, v = (t.repeat_interleave(n_q // n_kv, 1) for t in (k, v))
+        s = torch.einsum("thd,shd->hts", q, k) / D ** 0.5
+        a = torch.einsum("hts,shd->thd", s.masked_fill(later, float("-inf")).softmax(-1), v).reshape(T, -1)
+        x = x + a @ weight(lw["o"]).t()
+        gate, up = (norm(x, lw["ln2"]) @ weight(lw["gu"]).t()).split(m.I, 1)
+        x = x + (torch.nn.functional.silu(gate) * up) @ weight(lw["down"]).t()
+    return norm(x, m.norm_f) @ weight(m.lm_head).t(), torch.stack(ks, 1), torch.stack(vs, 1)
+
+
+# The rows between the GEMMs of a prompt lose neither range nor precision against RMSNorm as an operator of its own, which the
+# row-major path still has: small embeddings under small and large weights, large rows, rows of which one addition makes one channel a
+# million times as large as the rest, under weights above 1 (`jump`: by what its weights in o are multiplied; channel 7 and positive
+# weights for it give all tokens the same sign there), rows that one channel of weight zero dominates (`massive`: that channel's embedding). K and V
+# rows and logits against 64 bits: no further off than the operators, but for 5 % between two sets of roundings.
+@pytest.mark.parametrize("H,D,n_q,n_kv,I,T,emb,ln,jump,massive", [
+    (512, 64, 8, 2, 512, 40, 0.02, 0.005, 0, 0), (512, 64, 8, 2, 512, 40, 2e-3, 0.02, 0, 0), (512, 128, 4, 2, 512, 40, 2e-3, 0.005, 0, 0),
+    (512, 64, 8, 2, 512, 300, 1e-3, 0.02, 0, 0), (512, 64, 8, 2, 512, 40, 1e-4, 1.0, 0, 0), (512, 64, 8, 2, 512, 40, 0.04, 8.0, 800.0, 0),
+    (1024, 128, 8, 8, 512, 300, 0.04, 8.0, 400.0, 0), (2048, 64, 32, 4, 512, 40, 0.6, 0.1, 0, 15000.0), (512, 64, 8, 2, 512, 40, 600.0, 1.0, 0, 0)])
+def test_norms_inside_the_gemms_lose_nothing(H, D, n_q, n_kv, I, T, emb, ln, jump, massive):
+    from llm_decode_kernels_b200.model import DecodeConfig, Model
+    from test_model import hf_cfg, random_state
+    c = hf_cfg(H, 2, n_q, n_kv, I, 1000, D=D)
+    sd = random_state(c, 5, D)
+    for k in sd:
+        if "norm" in k:
+            sd[k] = (sd[k].float() * (min(ln, 1.0) if "input" in k else ln)).half()
+            if massive:
+                sd[k][5] = 0
+    E = sd["model.embed_tokens.weight"] = (sd["model.embed_tokens.weight"].float() * emb).half()
+    if jump:
+        E[:, 7] = 2
+        sd["model.layers.0.self_attn.v_proj.weight"][:, 7].abs_()
+        sd["model.layers.0.self_attn.o_proj.weight"][5].abs_().mul_(jump)
+    if massive:
+        E[:, 5] = massive
+    m = Model(sd, c, DecodeConfig(group=128, max_ctx=T + 16, seed=1, keep_packed=True))
+    m.prepare(T + 8, use_graph=False)
+    ids = torch.randint(0, 1000, (T,), generator=torch.Generator().manual_seed(6))
+    want, err = prompt_in_64_bits(m, sd, ids), {}
+    for path in ("tiled", "operators"):
+        if path == "operators":
+            m._prefill_desc = None          # what a model whose shape rules the tile layout out has there
+        m.kv.zero_()
+        m.reset(0)
+        logits = m.prefill(ids, collect_logits=True)
+        rows = m.kv[:, :, m.bt[:-(-T // 16)].long()].permute(1, 2, 4, 0, 3, 5).reshape(2, -1, 2, n_kv * D)[:, :T]
+        assert torch.isfinite(logits).all()
+        got = {"logits": (logits, want[0]), "k0": (rows[0, :, 0], want[1][:, 0]), "k1": (rows[0, :, 1], want[1][:, 1]),
+               "v0": (rows[1, :, 0], want[2][:, 0]), "v1": (rows[1, :, 1], want[2][:, 1])}
+        err[path] = {n: ((a.double() - b).norm() / b.norm()).item() for n, (a, b) in got.items()}
+    print(err)
+    assert m.K.gemm_status() == 0
+    for n, e in err["tiled"].items():
+        assert e <= 1.05 * err["operators"][n], (n, err)
+
+
 # Error of the prompt attention against 64 bits, on the rotated queries and the cache it read. Its output is one fp16 rounding of sums
 # that keep the probabilities to 22 bits: the error must be that rounding's (2^-11 / sqrt(12), a little less on average) and 10 % at
 # most beside it. fp16 probabilities alone add 17 to 40 %. Flat and peaked rows; whole context and splits.
