@@ -441,9 +441,14 @@ struct Mat {
   int paired;          // 1: gate|up tiles (8 gate rows + their 8 up rows)
 };
 
-// This CTA's tiles [t0, t0 + nt) of a matrix, in ring stages of `ups` blocks. whole: a stage holds whole tiles and a warp has at most two units
-// of each (rows of up to 2048 weights whose units divide a stage). Rows of 44 units (5632 weights) come in two stages of 22, two units a
-// warp in each: stages of 32 and 12 are three passes of the loop instead of two. (The step at context 256: 361 -> 359 us.)
+// This CTA's tiles [t0, t0 + nt) of a matrix, in ring stages of `ups` blocks: as many as a stage holds, but
+//  - rows of which a stage holds two and more (up to 16 units): whole tiles, and the loop over tiles in gemv (`whole`). us a token of 8 layers
+//    in the general loop / this one: 1280 columns (stages of 30) 138 / 133, 1536 (24) 144 / 139. One tile a stage leaves too much of the ring empty: 2560
+//    columns 168 / 170, 2816 174.0 / 174.6;
+//  - one tile of a row that fills more than a stage and no more than two passes of two units a warp (33 to 44 units): two stages of
+//    22 at most, which are those two passes; 32 and the rest are three. 8 layers of 2048 columns, down's rows 4352 / 4608 / 5120 / 5504 / 5632:
+//    122.0 / 120.5 / 122.1 / 123.0 / 124.0 -> 119.0 / 118.7 / 119.9 / 121.3 / 122.7. Not with more tiles, which want the ring full: 4096 columns, two
+//    tiles of 5632 104.9 -> 105.3; 5120 columns (three and four tiles a matrix) 144.7 -> 151.6.
 struct Slice { int t0, nt, ups, whole; };
 
 // Position in the ring. Stages are used strictly in order by producer and consumers alike, so a slot index and a
@@ -567,17 +572,16 @@ DEVI void tile_unit2(const Cta& c, uint32_t tu, uint32_t tv, int u, int lane, fl
 // streams for the scheduler to interleave). Rows of 2048 weights are 16 units for 11 warps: sharing the last five between two warps
 // each (half of a block's MMAs) evens the warps out on paper, and measured 20 us a token slower than leaving them. The activations are re-read from shared memory for every block: keeping
 // them in registers across tiles was measured and loses - it pushes the kernel over its registers, and a spilled
-// register costs an L2 round trip here. Doing two tiles of a stage together (four independent blocks) was measured
-// too and loses 3 %. When the warp has passed its last unit of a tile, lanes t == 0 leave the
+// register costs an L2 round trip here. When the warp has passed its last unit of a tile, lanes t == 0 leave the
 // two partial sums of rows g and g + 8 in part[warp][16 * tile + row slot]. A warp whose units do not exist
-// (K < 1024) only keeps the ring's barriers moving.
+// (K < 1408) only keeps the ring's barriers moving.
 //
-// TILES: slices of whole tiles have a loop of their own, which knows where a warp's one or two units of every tile are and takes two tiles
-// at a time: a tile of 16 units on 11 warps takes 690 cycles in the general loop, which keeps track of tile, unit and stage, and 555 in a plain
-// one over tiles (measured by themselves); with two tiles every warp has two chains in flight, also those with one unit of a tile. TinyLlama shape, us a token, with 32-bit offsets
-// instead of pointers into the ring, this loop, and the stages of 22 (Slice): context 128 354 -> 339, 256 368 -> 353, 2048 400 -> 385,
-// 8192 440 -> 423. Not in the STAGED form at head_dim 128, whose registers it exceeds (152 -> 157 us for 4 layers, 32 kv heads).
-// Four units of a row of 5632 at once, both stages: 1 % slower than two and two.
+// TILES: slices of whole tiles (Slice) have a loop of their own, which knows where a warp's one or two units of every tile are and takes
+// two tiles at a time: a tile of 16 units on 11 warps takes 690 cycles in the general loop, which keeps track of tile, unit and stage,
+// and 555 in a plain one over tiles (measured by themselves); with two tiles every warp has two chains in flight, also those with one
+// unit of a tile. TinyLlama shape, us a token, this loop, 32-bit offsets instead of pointers into the ring, and the stages of 22: context 128
+// 354 -> 339, 256 368 -> 353, 2048 400 -> 385, 8192 440 -> 423. Not in the STAGED form at head_dim 128, whose registers it exceeds (152 -> 157
+// us for 4 layers, 32 kv heads). Two tiles at once in the general loop lost 3 %; four units of a row of 5632 at once, both stages, 1 %.
 template <bool TILES>
 DEVI void gemv(const Cta& c, const Mat& m, const Slice& s, float* part, int pstride, RingPos& rp, int warp, int lane,
                int trace_at) {
@@ -588,11 +592,11 @@ DEVI void gemv(const Cta& c, const Mat& m, const Slice& s, float* part, int pstr
     const bool two = warp + kNCW < nunit;
     int row = 0;
 #pragma unroll 1
-    for (int i0 = 0; i0 < NU; i0 += c.p->ups, advance(rp, c.p->ns)) {
+    for (int i0 = 0; i0 < NU; i0 += s.ups, advance(rp, c.p->ns)) {
       const int slot = rp.slot;
       if (wait_bar(c, c.full(slot), rp.parity, ERR_FULL) && active) {
         uint32_t tu = (uint32_t)(c.p->off_ring + slot * c.p->stage_bytes + warp * kTileUnitBytes);
-        const int n = min(c.p->ups, NU - i0);
+        const int n = min(s.ups, NU - i0);
 #pragma unroll 1
         for (int b = 0; b < n;) {
           if (b + nunit < n) {
@@ -1362,8 +1366,9 @@ __global__ void __launch_bounds__(kThreads, 1) decode_step_kernel(const __grid_c
     const int rows = tid == 0 ? p.n_qkv : (tid == 2 ? p.I : (tid == 4 ? p.V : p.H));
     sl[tid] = slice_of(rows, tid == 2, cta, ncta);
     const int nunit = (tid == 1 ? p.n_att : tid == 3 ? p.I : p.H) >> 7;
-    sl[tid].ups = nunit > p.ups && nunit <= 2 * p.ups && nunit % (2 * kNCW) == 0 && 2 * kNCW <= p.ups ? 2 * kNCW : p.ups;
-    sl[tid].whole = nunit <= 2 * kNCW && p.ups % nunit == 0;
+    constexpr int kPass = 2 * kNCW;
+    sl[tid].whole = nunit <= kPass && 2 * nunit <= p.ups;
+    sl[tid].ups = sl[tid].whole ? p.ups / nunit * nunit : sl[tid].nt == 1 && nunit > p.ups && nunit <= 2 * kPass ? min(kPass, p.ups) : p.ups;
   }
   {
     const uint4* src = reinterpret_cast<const uint4*>(p.layers);

@@ -504,11 +504,13 @@ def test_automatic_step_kernel_by_context_and_ctas_per_kv_head():
             assert m.persistent == (limit is None or cap <= limit), (n_kv, cap)
 
 
-# Slices of whole tiles (rows of 1 to 16 units), rows of 44 units in two stages, rows that fit neither; one, two, an odd number and many
-# tiles a CTA. Against the multi-kernel step, with the tolerance of a kernel's output.
+# Slices of whole tiles (rows of 1 to 16 units, also where a stage of 32 is no multiple of them), rows of 34 to 44 units in two stages (one tile a
+# CTA) and not (two), rows that fit neither; one, two, an odd number and many tiles a CTA; both head sizes. Against the multi-kernel step, with the tolerance of a kernel's output.
 @pytest.mark.gpu
 @pytest.mark.parametrize("H,n_q,n_kv,I,V", [(128, 2, 1, 128, 333), (256, 4, 2, 5632, 5000), (512, 8, 2, 4864, 2400), (1024, 16, 2, 2816, 12000),
-                                            (2048, 32, 4, 5632, 7200), (640, 10, 5, 5632, 4000)])
+                                            (2048, 32, 4, 5632, 7200), (640, 10, 5, 5632, 4000),
+                                            (1280, 10, 5, 5504, 2400), (1536, 24, 6, 5120, 4000), (1920, 15, 15, 4352, 9000),
+                                            (2048, 16, 4, 4224, 3000), (2816, 22, 11, 5632, 3000), (4096, 32, 8, 5120, 2500)])
 def test_slices_of_whole_tiles_match_the_multi_kernel_step(H, n_q, n_kv, I, V):
     c = hf_cfg(H, 2, n_q, n_kv, I, V)
     sd = random_state(c, 11)
