@@ -219,6 +219,8 @@ DEVI long long now_ns() {
 DEVI void stamp_value(const Cta& c, int at, long long v) {
   if (c.tr && threadIdx.x == 0) c.tr[at] = v;
 }
+#else
+DEVI void stamp_value(const Cta&, int, long long) {}
 #endif
 constexpr int kTraceHead = 8, kTracePerPhase = 5, kTraceAttn = 5, kTracePerLayer = 4 * kTracePerPhase + kTraceAttn;
 
@@ -242,6 +244,18 @@ DEVI bool wait_bar(const Cta& c, uint64_t* bar, uint32_t parity, int code, unsig
   }
   raise(c, code);
   return false;
+}
+
+// Consumer side of a ring stage; a build under trace adds to `waited` what it took.
+DEVI bool wait_full(const Cta& c, int slot, uint32_t parity, long long& waited) {
+#ifdef B200_STEP_TRACE
+  const long long w0 = now_ns();
+  const bool ok = wait_bar(c, c.full(slot), parity, ERR_FULL);
+  waited += now_ns() - w0;
+  return ok;
+#else
+  return wait_bar(c, c.full(slot), parity, ERR_FULL);
+#endif
 }
 
 // ---- tagged exchange words -----------------------------------------------------------------------------------------
@@ -588,13 +602,14 @@ DEVI void gemv(const Cta& c, const Mat& m, const Slice& s, float* part, int pstr
   const int g = lane >> 2, t = lane & 3;
   const int nunit = m.K >> 7, NU = s.nt * nunit;
   const bool active = warp < nunit;
+  long long waited = 0;   // for the ring stages of the matrix
   if (TILES && s.whole) {
     const bool two = warp + kNCW < nunit;
     int row = 0;
 #pragma unroll 1
     for (int i0 = 0; i0 < NU; i0 += s.ups, advance(rp, c.p->ns)) {
       const int slot = rp.slot;
-      if (wait_bar(c, c.full(slot), rp.parity, ERR_FULL) && active) {
+      if (wait_full(c, slot, rp.parity, waited) && active) {
         uint32_t tu = (uint32_t)(c.p->off_ring + slot * c.p->stage_bytes + warp * kTileUnitBytes);
         const int n = min(s.ups, NU - i0);
 #pragma unroll 1
@@ -624,23 +639,15 @@ DEVI void gemv(const Cta& c, const Mat& m, const Slice& s, float* part, int pstr
       __syncwarp();
       if (lane == 0) mbar_arrive(c.empty(slot));
     }
+    stamp_value(c, trace_at, waited);
     return;
   }
   int tl = 0, u = warp, idx = warp;   // the warp's next block: local tile, unit, place in the sequence
   float ya = 0.f, yb = 0.f;
-#ifdef B200_STEP_TRACE
-  long long waited = 0;
-#endif
 #pragma unroll 1
   for (int i0 = 0; i0 < NU; i0 += s.ups, advance(rp, c.p->ns)) {
     const int slot = rp.slot;
-#ifdef B200_STEP_TRACE
-    const long long w0 = now_ns();
-#endif
-    const bool ok = wait_bar(c, c.full(slot), rp.parity, ERR_FULL);
-#ifdef B200_STEP_TRACE
-    waited += now_ns() - w0;   // time this warp spent waiting for ring stages of the matrix
-#endif
+    const bool ok = wait_full(c, slot, rp.parity, waited);
     const int end = min(NU, i0 + s.ups);
     const uint32_t sb = (uint32_t)(c.p->off_ring + slot * c.p->stage_bytes - i0 * kTileUnitBytes);   // block idx of the sequence is at sb + idx * 1088
     if (ok && active) {
@@ -671,9 +678,7 @@ DEVI void gemv(const Cta& c, const Mat& m, const Slice& s, float* part, int pstr
     __syncwarp();
     if (lane == 0) mbar_arrive(c.empty(slot));
   }
-#ifdef B200_STEP_TRACE
   stamp_value(c, trace_at, waited);
-#endif
 }
 
 // Sum of one row slot over the nwa warps that hold a share of it, always in the same order: pairs, then the pair sums. The
@@ -988,20 +993,12 @@ DEVI void attention_head(const Cta& c, const StepParams& p, const StepLayer& ly,
   static_assert(4 * kNCW * kKvRounds > kMaxKvTokens, "a stage needs a spare slot for the token of this step");
   const uint32_t knew_off = (uint32_t)(reinterpret_cast<const uint8_t*>(knew) - step_smem) + ch * DPL * 2;
   const uint32_t vnew_off = (uint32_t)(reinterpret_cast<const uint8_t*>(vnew) - step_smem) + ch * DPL * 2;
-#ifdef B200_STEP_TRACE
   long long waited = 0;
-#endif
 #pragma unroll 1
   for (int st = 0; st < nst || (nst == 0 && st == 0); ++st) {   // an empty cache: one pass without a ring stage
     const bool have = st < nst, last = st + 1 >= nst;
     const int slot = rp.slot;
-#ifdef B200_STEP_TRACE
-    const long long w0 = now_ns();
-#endif
-    const bool ok = have ? wait_bar(c, c.full(slot), rp.parity, ERR_FULL) : true;
-#ifdef B200_STEP_TRACE
-    waited += now_ns() - w0;
-#endif
+    const bool ok = have ? wait_full(c, slot, rp.parity, waited) : true;
     const uint32_t kbase = c.p->off_ring + (uint32_t)slot * c.p->stage_bytes + ch * DPL * 2;
     const uint32_t vbase = kbase + (uint32_t)tps * D * 2;
     const int nt = have ? min(tps, len - st * tps) : 0;
@@ -1024,9 +1021,7 @@ DEVI void attention_head(const Cta& c, const StepParams& p, const StepLayer& ly,
     }
   }
   stamp(c, trace_at + 1);
-#ifdef B200_STEP_TRACE
   stamp_value(c, trace_at + 4, waited);   // a duration: what warp 0 waited for the K/V stages
-#endif
 
   // merge: token slots inside the warp, then the warps
   float lw = l;
@@ -1129,20 +1124,12 @@ DEVI RingPos attention_group(const Cta& c, int layer, int u, RingPos rp, int tra
   const uint32_t qaddr = smem_u32(&sc.q[g][t * D4]), kaddr = smem_u32(sc.k), vaddr = smem_u32(sc.v);
   const int tps = kv_tokens_per_stage(p), bps = tps >> 4;   // tokens and blocks per stage
   int bid = 0, nblk = 0;                                     // first block of the stage mod kNCW; blocks of the slice
-#ifdef B200_STEP_TRACE
   long long waited = 0;
-#endif
 #pragma unroll 1
   for (int t0 = t_begin; t0 < t_end || nblk == 0; t0 += tps) {   // an empty cache: one pass without a ring stage
     const bool have = t0 < t_end, last = t0 + tps >= t_end;
     const int slot = rp.slot;
-#ifdef B200_STEP_TRACE
-    const long long w0 = now_ns();
-#endif
-    const bool ok = have ? wait_bar(c, c.full(slot), rp.parity, ERR_FULL) : true;
-#ifdef B200_STEP_TRACE
-    waited += now_ns() - w0;
-#endif
+    const bool ok = have ? wait_full(c, slot, rp.parity, waited) : true;
     const int nt = have ? min(tps, t_end - t0) : 0, ntot = nt + (takes_new && last ? 1 : 0);   // the new token rides behind the last one
     const uint32_t kst = smem_u32(c.stage(slot)), vst = kst + (uint32_t)(tps * D * 2);
     int b = team - bid;
@@ -1216,9 +1203,7 @@ DEVI RingPos attention_group(const Cta& c, int layer, int u, RingPos rp, int tra
     }
   }
   stamp(c, trace_at + 1);
-#ifdef B200_STEP_TRACE
   stamp_value(c, trace_at + 4, waited);   // a duration: what warp 0 waited for the K/V stages
-#endif
 
   // merge the teams: acc[n][e] = O[head g][dim0 + 8 (2 t + e) + n]
   const int nw = min(TEAMS, nblk);

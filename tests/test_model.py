@@ -6,7 +6,13 @@ numerical noise of fp16 logits; anything else is a failure. Streams are compared
 tokens are fed to the runtime), so one near-tie flip cannot make everything after it incomparable, and then
 free-running as well, where the streams must be identical up to the first near-tie.
 """
+import json
+import os
+import shutil
+import subprocess
+import sys
 import types
+from pathlib import Path
 
 import numpy as np
 import pytest
@@ -523,3 +529,15 @@ def test_slices_of_whole_tiles_match_the_multi_kernel_step(H, n_q, n_kv, I, V):
         out[step] = m.teacher_force(ids, use_graph=False, collect_logits=True).float()
         assert m.step_error() == 0
     assert (out["persistent"] - out["multi"]).abs().max() <= KERNEL_TOL * out["multi"].abs().max()
+
+
+@pytest.mark.gpu
+@pytest.mark.skipif(shutil.which("nvcc") is None and not os.path.exists("/usr/local/cuda/bin/nvcc"), reason="builds the step under trace")
+def test_step_trace_sees_the_waits_for_weights(tmp_path):
+    """Every matrix of a layer reports its waits for ring stages, those of the loop over whole tiles (rows of 16 units: qkv, o, gate|up) and
+    those of the general one (down)."""
+    out = tmp_path / "trace.json"
+    subprocess.run([sys.executable, "-m", "llm_decode_kernels_b200.step_trace", "--layers", "2", "--ctx", "16", "--reps", "2", "--out", str(out)],
+                   check=True, cwd=Path(__file__).resolve().parents[1], stdout=subprocess.DEVNULL, timeout=600)
+    phases = json.loads(out.read_text())["phases_us"]
+    assert all(phases[f"{m}.wait_weights"]["slowest_cta"] > 0 for m in ("qkv", "o", "gate_up", "down"))
