@@ -732,12 +732,14 @@ cudaError_t prefill_gemm_tiled_dispatch(const void* Wt, const void* X, void* Y, 
   if (e == cudaSuccess && mode != PLAIN) e = allow_dynamic_smem(kern, smem_max, allowed[mode]);
   if (e != cudaSuccess) return e;
   // Tokens per tile (equal tiles, so that the last is not nearly empty; up to eight more of them than there have to be) and split of
-  // K, by estimated time. In microseconds, fitted to 1,250 measured launches (TinyLlama, 8B and 70B matrices, 16 .. 4096 tokens;
-  // the pick is 0.7 % off the best of them on average, 11 % at worst; always the widest tiles: 10 % and 51 %): a unit takes 0.30 - 0.35
-  // (dequantization and issue) or its MMA time, 0.68 at 256 tokens with the chip full; beside that a launch takes 1.0 + 0.0162 a
-  // token where a pair works alone and 2.1 / 2.7 + 0.0206 a token where 2 / 4 pairs exchange partial tiles; and up to 2.8 are lost
-  // with the SMs that the launch's last wave leaves none of to the start of the next one (counted over all waves instead: 2 % more for a
-  // prompt of 200 to 512 tokens).
+  // K, by estimated time. In microseconds: a unit takes 0.35 (dequantization and issue) or, from 126 tokens on, 0.11 + 0.0019 a token (MMA and
+  // activations with the chip full); beside that a launch takes 1.0 + 0.0162 a token where a pair works alone and 2.1 / 2.7 + 0.0206 a token
+  // where 2 / 4 pairs exchange partial tiles; and up to 2.8 are lost with the SMs that the launch's last wave leaves none of to the start of the
+  // next one. Measured on launches in a row of the four matrices of TinyLlama, 8B and 70B shapes, 16 .. 4096 tokens, every choice (3,570; plain and
+  // SwiGLU epilogues): the pick is 0.2 % off the best on average, 6 % at worst (TinyLlama, down, 150 tokens). With a unit in proportion to its tokens
+  // (0.00264) the pick was 0.75 % off and 14 % at worst: 128-token tiles in many waves looked cheap. Whole prompts, that unit / this one, us:
+  // 70B shape (4 layers) 230 tokens 1,788 / 1,734, 256 1,853 / 1,771, 512 3,397 / 3,196, 1200 7,865 / 7,609; 8B shape (8 layers) 512 tokens
+  // 1,815 / 1,882, 700 2,485 / 2,418, 1000 3,388 / 3,252; TinyLlama within 0.7 %, but 1200 and 2000 tokens 1 % faster.
   int S = 0, nt = 0, tiles = 0;
   double best = 0;
   const int least = (T + kMaxTokens - 1) / kMaxTokens;
@@ -749,7 +751,7 @@ cudaError_t prefill_gemm_tiled_dispatch(const void* Wt, const void* X, void* Y, 
     const int units = (nunit + c - 1) / c;
     for (int ntt = least; ntt < least + 8; ++ntt) {
       const int n = ((T + ntt - 1) / ntt + 31) / 32 * 32, count = feat_tiles * ((T + n - 1) / n), waves = (count + room - 1) / room;
-      const double unit = units * (n * 0.00264 > 0.35 ? n * 0.00264 : 0.35), fill = (double)(count - (waves - 1) * room) / room;   // of the last wave
+      const double unit = units * (n * 0.0019 + 0.11 > 0.35 ? n * 0.0019 + 0.11 : 0.35), fill = (double)(count - (waves - 1) * room) / room;   // of the last wave
       const double cost = (c == 1 ? 1.0 + 0.0162 * n + waves * (unit + 0.4) : waves * (1.45 + 0.32 * c + 0.0206 * n + unit)) +
                           2.8 * (fill < 0.36 ? 0 : fill > 0.86 ? 1 : 2 * (fill - 0.36));
       if (S == 0 || cost < best) best = cost, S = c, nt = n, tiles = count;
