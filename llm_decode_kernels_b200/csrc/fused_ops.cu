@@ -3,7 +3,6 @@
 // and the number of dependent memory round trips matter, not bandwidth: every kernel makes one pass with the
 // data held in registers between its phases.
 #include "common.cuh"
-#include "prefill.h"
 #include <math_constants.h>
 
 namespace b200 {
@@ -158,25 +157,14 @@ __global__ void rope_append_kernel(half* __restrict__ qkv, const float* __restri
 
 // The same for the rows of a prompt: one block per token, 8 pairs per thread in 16-byte pieces. A block per (token, head) of 32
 // threads each, as above, is 164,000 blocks for 4096 tokens and 110 us; this form takes 12.
-// IN_CHUNK: inside b200_prefill_chunk positions, block table and factors do not come from the kernels before this one and are read ahead of
-// the wait (see embed_rows_kernel): 1 us a launch.
-template <bool IN_CHUNK>
 __global__ void __launch_bounds__(256)
 rope_append_rows_kernel(half* __restrict__ qkv, const float* __restrict__ cos_t, const float* __restrict__ sin_t,
                         const int* __restrict__ pos_ptr, const int* __restrict__ bt, int bt_stride, half* __restrict__ kc,
                         half* __restrict__ vc, int n_q, int n_kv, int D, int log2P) {
   pdl_launch_dependents();
-  if (!IN_CHUNK) pdl_wait();
+  pdl_wait();
   const int b = blockIdx.x, d2 = D >> 1, per_head = D >> 4, heads = n_q + 2 * n_kv;
   const int pos = pos_ptr[b], page = bt[(size_t)b * bt_stride + (pos >> log2P)], slot = pos & ((1 << log2P) - 1);
-  if (IN_CHUNK) {   // the factors on their way into the L1, too
-    if (threadIdx.x < per_head) {
-      asm volatile("prefetch.global.L1 [%0];" ::"l"(cos_t + (size_t)pos * d2 + 8 * threadIdx.x));
-      asm volatile("prefetch.global.L1 [%0];" ::"l"(sin_t + (size_t)pos * d2 + 8 * threadIdx.x));
-    }
-    asm volatile("" ::"r"(page));
-    pdl_wait();
-  }
   for (int c = threadIdx.x; c < heads * per_head; c += blockDim.x) {
     const int head = c / per_head, i = (c - head * per_head) * 8;
     half* v = qkv + ((size_t)b * heads + head) * D + i;
@@ -216,18 +204,12 @@ cudaError_t rope_append_dispatch(void* qkv, const float* cos_t, const float* sin
                                  cudaStream_t st) {
   auto aligned = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };
   if (B >= 4 && D % 16 == 0 && aligned(qkv) && aligned(cos_t) && aligned(sin_t) && aligned(kc) && aligned(vc)) {
-    B200_LAUNCH(rope_append_rows_kernel<false>, dim3(B), dim3(256), 0, st, (half*)qkv, cos_t, sin_t, pos, bt, bt_stride, (half*)kc,
+    B200_LAUNCH(rope_append_rows_kernel, dim3(B), dim3(256), 0, st, (half*)qkv, cos_t, sin_t, pos, bt, bt_stride, (half*)kc,
                 (half*)vc, n_q, n_kv, D, log2P);
     return cudaPeekAtLastError();
   }
   B200_LAUNCH(rope_append_kernel, dim3(n_q + 2 * n_kv, B), dim3(D / 2), 0, st, (half*)qkv, cos_t, sin_t, pos, bt,
               bt_stride, (half*)kc, (half*)vc, n_q, n_kv, D, log2P);
-  return cudaPeekAtLastError();
-}
-
-cudaError_t prefill_rope_append_dispatch(const PrefillParams& p, const StepLayer& ly, cudaStream_t st) {
-  B200_LAUNCH(rope_append_rows_kernel<true>, dim3(p.T), dim3(256), 0, st, (half*)p.qkv, p.cos_t, p.sin_t, p.pos, p.bt, 0, ly.kc, ly.vc, p.n_q,
-              p.n_kv, p.D, p.log2P);
   return cudaPeekAtLastError();
 }
 

@@ -53,11 +53,6 @@ embed_rows_kernel(const uint4* __restrict__ emb, const long long* __restrict__ i
 
 }  // namespace
 
-// Up to this many tokens the qkv GEMM does RoPE and the append itself. Beyond, a launch of its own costs no more than the epilogue, and
-// attention's CTAs, which do not fit beside a GEMM's, start up beside it. Whole prompt, TinyLlama shape, us (launch of its own / in the GEMM): 8
-// tokens 897 / 865, 77 1,045 / 1,045, 512 1,681 / 1,650, 700 2,038 / 2,002, 1000 2,380 / 2,418, 1400 2,986 / 3,016, 2000 4,100 / 4,061.
-constexpr int kRopeInGemm = 768;
-
 cudaError_t prefill_chunk_dispatch(const PrefillParams& p, cudaStream_t st) {
 #define TRY(call)                        \
   do {                                   \
@@ -80,8 +75,7 @@ cudaError_t prefill_chunk_dispatch(const PrefillParams& p, cudaStream_t st) {
     const PrefillNorm at_mlp = {ss_m, inv_m, nullptr, nullptr, nullptr, nullptr, nullptr, parts, inv_h, p.eps};
     const PrefillNorm to_next = {nullptr, nullptr, x, xw, last ? nullptr : p.layers[l + 1].ln1, ss_a, inv_a, parts, inv_h, p.eps};
     const PrefillRope rope = {p.cos_t, p.sin_t, p.pos, p.bt, ly.kc, ly.vc, p.n_q, p.n_kv, p.D, p.log2P};
-    TRY(prefill_gemm_tiled_dispatch(ly.w[0], p.normed, p.qkv, p.T, n_qkv, p.H, 0, 0, &at_qkv, p.T <= kRopeInGemm ? &rope : nullptr, st));
-    if (p.T > kRopeInGemm) TRY(prefill_rope_append_dispatch(p, ly, st));
+    TRY(prefill_gemm_tiled_dispatch(ly.w[0], p.normed, p.qkv, p.T, n_qkv, p.H, 0, 0, &at_qkv, &rope, st));
     TRY(prefill_attention_dispatch(p.qkv, n_qkv, ly.kc, ly.vc, p.bt, p.start, p.T, p.n_q, p.n_kv, p.D, p.log2P, p.attn, st));
     TRY(prefill_gemm_tiled_dispatch(ly.w[1], p.attn, nullptr, p.T, p.H, n_att, 0, 0, &to_mlp, nullptr, st));
     TRY(prefill_gemm_tiled_dispatch(ly.w[2], p.normed, p.act, p.T, p.I, p.H, 1, 0, &at_mlp, nullptr, st));

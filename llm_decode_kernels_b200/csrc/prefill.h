@@ -31,7 +31,11 @@ struct PrefillNorm {
 };
 
 // RoPE and the append to the paged cache inside the qkv GEMM (rope_append_rows_kernel's arithmetic on the fp16 outputs): q goes to Y
-// rotated, k rotated and v as they are to the caches.
+// rotated, k rotated and v as they are to the caches. A launch of its own for that was 1 us a layer at few tokens and 4 at 512. Whole prompt
+// us, own launch / here: TinyLlama shape 8 tokens 829 / 782, 77 976 / 966, 512 1,631 / 1,598, 768 2,021 / 1,980, 1000 2,411 / 2,442, 1400 3,274 /
+// 3,306, 2000 4,532 / 4,482, 4000 9,733 / 9,638; 8B shape (8 layers) 77 697 / 683, 1000 3,491 / 3,456, 4000 13,365 / 13,195; 70B shape (4 layers) 77
+// 908 / 900, 1000 6,019 / 5,980, 4000 25,162 / 25,046. Behind only for TinyLlama at 900 to 1400 tokens (1 %: attention's CTAs, one wave there, started
+// up beside the small launch), which is not worth a second form.
 struct PrefillRope {
   const float *cos_t, *sin_t;   // [positions, D / 2]
   const int *pos, *bt;          // [T]; block table
@@ -62,7 +66,6 @@ cudaError_t prefill_attention_status(int* code);
 // qkv GEMM does with its outputs.
 cudaError_t prefill_gemm_tiled_dispatch(const void* Wt, const void* X, void* Y, int T, int N, int K, int swiglu, int force_split,
                                         const PrefillNorm* norm, const PrefillRope* rope, cudaStream_t st);
-cudaError_t prefill_rope_append_dispatch(const PrefillParams& p, const StepLayer& ly, cudaStream_t st);   // 16-byte aligned caches
 cudaError_t add_rmsnorm_dispatch(void* x, const void* delta, const void* w, void* out, int rows, int H, float eps,
                                  cudaStream_t st);
 

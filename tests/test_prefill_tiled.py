@@ -136,7 +136,7 @@ def prompt_in_64_bits(m, sd, ids):
     norm = lambda x, w: x * torch.rsqrt((x * x).mean(-1, keepdim=True) + m.eps) * w.double()
     rope = lambda v: torch.cat([v[..., :d2] * cos - v[..., d2:] * sin, v[..., d2:] * cos + v[..., :d2] * sin], -1)
     later = torch.ones(T, T, dtype=torch.bool, device=dev).triu(1)
-    x, ks, vs = sd["model.embed_tokens.weight"][ids].to(dev).double(), [], []
+    x, ks, vs = sd["model.embed_tokens.weight"].to(dev)[ids.to(dev)].double(), [], []
     for lw in m.layers:
         q, k, v = (norm(x, lw["ln1"]) @ weight(lw["qkv"]).t()).view(T, -1, D).split([n_q, n_kv, n_kv], 1)
         q, k = rope(q), rope(k)
@@ -148,6 +148,24 @@ def prompt_in_64_bits(m, sd, ids):
         gate, up = (norm(x, lw["ln2"]) @ weight(lw["gu"]).t()).split(m.I, 1)
         x = x + (torch.nn.functional.silu(gate) * up) @ weight(lw["down"]).t()
     return norm(x, m.norm_f) @ weight(m.lm_head).t(), torch.stack(ks, 1), torch.stack(vs, 1)
+
+
+def errors(m, sd, ids):
+    """How far a prompt is from 64 bits (2-norms), on the tile layout and operator by operator: {path: {output: error}}."""
+    want, T, err = prompt_in_64_bits(m, sd, ids), ids.numel(), {}
+    for path in ("tiled", "operators"):
+        if path == "operators":
+            m._prefill_desc = None          # what a model whose shape rules the tile layout out has there
+        m.kv.zero_()
+        m.reset(0)
+        logits = m.prefill(ids, collect_logits=True)
+        rows = m.kv[:, :, m.bt[:-(-T // 16)].long()].permute(1, 2, 4, 0, 3, 5).reshape(2, -1, 2, m.n_kv * m.D)[:, :T]
+        assert torch.isfinite(logits).all() and m.K.gemm_status() == 0
+        got = {"logits": (logits, want[0]), "k0": (rows[0, :, 0], want[1][:, 0]), "k1": (rows[0, :, 1], want[1][:, 1]),
+               "v0": (rows[1, :, 0], want[2][:, 0]), "v1": (rows[1, :, 1], want[2][:, 1])}
+        err[path] = {n: ((a.double() - b).norm() / b.norm()).item() for n, (a, b) in got.items()}
+    print(err)
+    return err
 
 
 # The rows between the GEMMs of a prompt lose neither range nor precision against RMSNorm as an operator of its own, which the
@@ -179,20 +197,28 @@ def test_norms_inside_the_gemms_lose_nothing(H, D, n_q, n_kv, I, T, emb, ln, jum
     m = Model(sd, c, DecodeConfig(group=128, max_ctx=T + 16, seed=1, keep_packed=True))
     m.prepare(T + 8, use_graph=False)
     ids = torch.randint(0, 1000, (T,), generator=torch.Generator().manual_seed(6))
-    want, err = prompt_in_64_bits(m, sd, ids), {}
-    for path in ("tiled", "operators"):
-        if path == "operators":
-            m._prefill_desc = None          # what a model whose shape rules the tile layout out has there
-        m.kv.zero_()
-        m.reset(0)
-        logits = m.prefill(ids, collect_logits=True)
-        rows = m.kv[:, :, m.bt[:-(-T // 16)].long()].permute(1, 2, 4, 0, 3, 5).reshape(2, -1, 2, n_kv * D)[:, :T]
-        assert torch.isfinite(logits).all()
-        got = {"logits": (logits, want[0]), "k0": (rows[0, :, 0], want[1][:, 0]), "k1": (rows[0, :, 1], want[1][:, 1]),
-               "v0": (rows[1, :, 0], want[2][:, 0]), "v1": (rows[1, :, 1], want[2][:, 1])}
-        err[path] = {n: ((a.double() - b).norm() / b.norm()).item() for n, (a, b) in got.items()}
-    print(err)
-    assert m.K.gemm_status() == 0
+    err = errors(m, sd, ids)
+    for n, e in err["tiled"].items():
+        assert e <= 1.05 * err["operators"][n], (n, err)
+
+
+# The same where a CTA pair walks over several tiles of the qkv, o and down matrices (3400 tokens: 144 to 324 and 108 tiles for 74
+# pairs), where four pairs split K in front of RoPE and of a residual row, and where the partials of a split lie over the stages (rows
+# of more than 14336 weights and 256-token tiles). By the dispatch's own choice.
+@pytest.mark.parametrize("H,D,n_q,n_kv,I,T", [(1536, 128, 12, 12, 256, 3400), (1536, 64, 24, 3, 256, 3391), (8192, 64, 2, 1, 256, 40),
+                                              (256, 64, 4, 2, 8192, 37), (4352, 64, 2, 1, 14464, 256)])
+def test_epilogues_over_many_tiles_and_splits(H, D, n_q, n_kv, I, T):
+    from llm_decode_kernels_b200.model import DecodeConfig, Model
+    from llm_decode_kernels_b200.shapes import random_llama_state
+    from test_model import hf_cfg
+    c = hf_cfg(H, 2, n_q, n_kv, I, 1000, D=D)
+    sd, g = random_llama_state(c, dev, 7), torch.Generator(device=dev).manual_seed(8)
+    for k in sd:
+        if "norm" in k:
+            sd[k] = (0.5 + torch.rand(H, generator=g, device=dev)).half()
+    m = Model(sd, c, DecodeConfig(group=128, max_ctx=T + 16, seed=1, keep_packed=True))
+    m.prepare(T + 8, use_graph=False)
+    err = errors(m, sd, torch.randint(0, 1000, (T,), generator=torch.Generator().manual_seed(6)))
     for n, e in err["tiled"].items():
         assert e <= 1.05 * err["operators"][n], (n, err)
 
