@@ -456,7 +456,7 @@ struct Mat {
 };
 
 // This CTA's tiles [t0, t0 + nt) of a matrix, in ring stages of `ups` blocks: as many as a stage holds, but
-//  - rows of which a stage holds two and more (up to 16 units): whole tiles, and the loop over tiles in gemv (`whole`). us a token of 8 layers
+//  - rows of which a stage holds two and more (up to 16 units): whole tiles, `whole` of them, and the loop over tiles in gemv. us a token of 8 layers
 //    in the general loop / this one: 1280 columns (stages of 30) 138 / 133, 1536 (24) 144 / 139. One tile a stage leaves too much of the ring empty: 2560
 //    columns 168 / 170, 2816 174.0 / 174.6;
 //  - one tile of a row that fills more than a stage and no more than two passes of two units a warp (33 to 44 units): two stages of
@@ -605,35 +605,28 @@ DEVI void gemv(const Cta& c, const Mat& m, const Slice& s, float* part, int pstr
   long long waited = 0;   // for the ring stages of the matrix
   if (TILES && s.whole) {
     const bool two = warp + kNCW < nunit;
-    int row = 0;
+    float* to = part + warp * pstride + g;
 #pragma unroll 1
-    for (int i0 = 0; i0 < NU; i0 += s.ups, advance(rp, c.p->ns)) {
+    for (int left = s.nt; left > 0; left -= s.whole, advance(rp, c.p->ns)) {
       const int slot = rp.slot;
       if (wait_full(c, slot, rp.parity, waited) && active) {
         uint32_t tu = (uint32_t)(c.p->off_ring + slot * c.p->stage_bytes + warp * kTileUnitBytes);
-        const int n = min(s.ups, NU - i0);
 #pragma unroll 1
-        for (int b = 0; b < n;) {
-          if (b + nunit < n) {
+        for (int n = min(s.whole, left); n > 0;) {
+          if (n > 1) {
             const uint32_t tv = tu + nunit * kTileUnitBytes;
             float ya = 0.f, yb = 0.f, za = 0.f, zb = 0.f;
             tile_unit2(c, tu, tv, warp, lane, ya, yb, za, zb);
             if (two) tile_unit2(c, tu + kNCW * kTileUnitBytes, tv + kNCW * kTileUnitBytes, warp + kNCW, lane, ya, yb, za, zb);
-            if (t == 0) {
-              float* to = part + warp * pstride + row + g;
-              to[0] = ya, to[8] = yb, to[16] = za, to[24] = zb;
-            }
-            b += 2 * nunit, tu += 2 * nunit * kTileUnitBytes, row += 32;
+            if (t == 0) to[0] = ya, to[8] = yb, to[16] = za, to[24] = zb;
+            n -= 2, tu += 2 * nunit * kTileUnitBytes, to += 32;
             continue;
           }
           float ya = 0.f, yb = 0.f, ya2 = 0.f, yb2 = 0.f;
           tile_unit(c, tu, warp, lane, ya, yb);
           if (two) tile_unit(c, tu + kNCW * kTileUnitBytes, warp + kNCW, lane, ya2, yb2);
-          if (t == 0) {
-            part[warp * pstride + row + g] = ya + ya2;
-            part[warp * pstride + row + g + 8] = yb + yb2;
-          }
-          b += nunit, tu += nunit * kTileUnitBytes, row += 16;
+          if (t == 0) to[0] = ya + ya2, to[8] = yb + yb2;
+          --n, tu += nunit * kTileUnitBytes, to += 16;
         }
       }
       __syncwarp();
@@ -1352,8 +1345,8 @@ __global__ void __launch_bounds__(kThreads, 1) decode_step_kernel(const __grid_c
     sl[tid] = slice_of(rows, tid == 2, cta, ncta);
     const int nunit = (tid == 1 ? p.n_att : tid == 3 ? p.I : p.H) >> 7;
     constexpr int kPass = 2 * kNCW;
-    sl[tid].whole = nunit <= kPass && 2 * nunit <= p.ups;
-    sl[tid].ups = sl[tid].whole ? p.ups / nunit * nunit : sl[tid].nt == 1 && nunit > p.ups && nunit <= 2 * kPass ? min(kPass, p.ups) : p.ups;
+    sl[tid].whole = nunit <= kPass && 2 * nunit <= p.ups ? p.ups / nunit : 0;
+    sl[tid].ups = sl[tid].whole ? sl[tid].whole * nunit : sl[tid].nt == 1 && nunit > p.ups && nunit <= 2 * kPass ? min(kPass, p.ups) : p.ups;
   }
   {
     const uint4* src = reinterpret_cast<const uint4*>(p.layers);
