@@ -14,12 +14,12 @@ bool encode_activation_map(CUtensorMap* map, const void* X, int T, int K, int bo
 // outputs. What it reads is xw = fp16(x * w / p), written by the GEMM that finished the residual row x (RESIDUAL of
 // prefill_gemm_tiled_kernel: x += its output) together with the sums of x^2 over each 128 columns.
 // Range: p is the power of two that brings the largest |w| into [0.5, 1). |x * w / p| < 65504 then for every finite x, so nothing
-// overflows however much a row grows in one addition, and small weights do not push a row among the subnormals. (A scale taken from the
-// row as it was before the addition overflows where that addition makes it large.)
+// overflows however much a row grows in one addition, and small weights do not push a row among the subnormals. (A scale taken from
+// the row as it was before the addition overflows where that addition makes it large.)
 // Precision: one rounding, where w * fp16(x * factor) has two: a row is 2.07e-4 off instead of 2.9e-4. Products below 2^-14 are
 // subnormal and keep 2^-25, as additions leave it in x; that is less than the two roundings keep where the products' root mean square
-// is below 8e-5: rows of rms 1e-3 whose typical weight is below 0.08 of the largest, rows of rms 1e-2 below 0.008. Embeddings, which may be so small, are
-// scaled row by row (embed_rows_kernel).
+// is below 8e-5: rows of rms 1e-3 whose typical weight is below 0.08 p, rows of rms 1e-2 below 0.008 p. Embeddings, which may be
+// so small, are scaled row by row (embed_rows_kernel).
 struct PrefillNorm {
   const float* ss_in;    // [T][parts] sums of squares of the rows behind X, which are to be normalised
   const float* inv_in;   // [T] what X lacks beside the norm's factor (p)

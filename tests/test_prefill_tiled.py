@@ -95,8 +95,8 @@ def test_prefill_equals_stepping(D, n_q, n_kv, page, start, T):
     assert int(m.tok) == tok or top[0] - top[1] <= 2 * KERNEL_TOL * want.abs().max()
 
 
-# Norms, residual sums and RoPE inside the GEMMs: hidden sizes whose last 256-row tile is half empty, one and several token tiles, both
-# sides of the limit for RoPE; embeddings and norm weights small and large enough that rows stored without a scale would leave fp16.
+# Norms, residual sums and RoPE inside the GEMMs: hidden sizes whose last 256-row tile is half empty, one and several token tiles;
+# embeddings and norm weights small and large enough that rows stored as x * w would leave fp16.
 # Same tolerance as above, which allows for the stepping path's own roundings. (The norm in front of attention keeps its weights where
 # they are large: scores of hundreds would multiply every rounding of either path.)
 @pytest.mark.parametrize("H,D,n_q,n_kv,T,emb,ln", [(128, 64, 2, 1, 3, 1.0, 1.0), (384, 64, 6, 3, 33, 1e-3, 0.02), (640, 64, 8, 8, 257, 1.0, 8.0),
